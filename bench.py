@@ -277,10 +277,10 @@ def kernel_table(fb, path, c, poisson="int8x8", sweeps=2):
         ("gemm_bwd (cuBLAS DGEMM)", "gemm_bwd", 0, gemm, "tensor"),
     ]
     if poisson == "int8x8":
-        # 36 digit-pair products of 2*n2m*n3m^2 integer ops each; the digit cut
+        # 28 digit-pair products of 2*n2m*n3m^2 integer ops each; the digit cut
         # reads the FP64 operand and writes 8 int8 planes (16 B per cell)
         transform = [
-            ("i8x8 GEMM (tcgen05 kind::i8, 36 digit pairs)", "i8x8_gemm", 6, 36 * gemm, "tensor_i8"),
+            ("i8x8 GEMM (tcgen05 kind::i8, 28 digit pairs)", "i8x8_gemm", 6, 28 * gemm, "tensor_i8"),
             ("i8 digit cut (row maxima from the producers)", "i8_split", 6, 2.0 * B, "hbm"),
             ("poisson_tri", "poisson_tri", 3, 3 * B, "hbm"),
         ] + dgemm_rows
@@ -752,7 +752,7 @@ def device_arm(args, rank, world, local):
                     "peak_source": ("of measured: MEASURED_PEAKS.json bf16_tflops x 2 (dense INT8 rate; "
                                     "integer ops counted as flop)" if "bf16_tflops" in peaks
                                     else "of fallback 1.59 PFLOP/s bf16 x 2"),
-                    "work_per_launch": f"36 digit pairs x 2*n2m*n3m^2 = {dom['work']:.4g} integer ops",
+                    "work_per_launch": f"28 digit pairs x 2*n2m*n3m^2 = {dom['work']:.4g} integer ops",
                     "fp64_equivalent_tflops": dom["work"] / 36.0 / (dom["ms"] * 1e-3) / 1e12}
         elif dom["bound"] == "tensor":
             achieved = dom["work"] / (dom["ms"] * 1e-3) / 1e12

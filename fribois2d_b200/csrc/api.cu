@@ -101,7 +101,7 @@ struct fb_ctx {
     bool cond_graph = true;                    // coupled step as a graph WHILE node (else a host loop)
     int tune_tk = 64;         // windowed helsolve tile height (autotuned per grid size)
     int tune_bn = 128;        // 3xTF32 GEMM tile width (autotuned per grid size)
-    int tune_i8bn = fb::kI8BN;  // INT8 digit-product tile width, 32, 48 or 64 (autotuned per grid size)
+    int tune_i8bn = fb::kI8BN;  // INT8 digit-product tile width, 16, 32, 48 or 64 (by grid size)
     bool i8_fixed = false;      // the width set by FRIBOIS2D_I8_TILE: not tuned
     // precision form of the Poisson solve (3xTF32 tensor-core transforms + one
     // FP64 refinement sweep); planes of TF32 splits, tensor maps, FP64 scratch
@@ -430,9 +430,9 @@ int create_impl(const char *dir, int device, fb_ctx *c) {
     }
     c->device = device;
     if (const char *hv = std::getenv("FRIBOIS2D_HELSOLVE")) c->allow_win = std::strcmp(hv, "scan") != 0;
-    if (const char *tw = std::getenv("FRIBOIS2D_I8_TILE")) {   // fixed INT8 product tile width (32, 48 or 64)
+    if (const char *tw = std::getenv("FRIBOIS2D_I8_TILE")) {   // fixed INT8 product tile width (16, 32, 48 or 64)
         const int w = std::atoi(tw);
-        if (w == 32 || w == 48 || w == 64) {
+        if (w == 16 || w == 32 || w == 48 || w == 64) {
             c->tune_i8bn = w;
             c->i8_fixed = true;
         }
@@ -861,6 +861,8 @@ int setup_i8(fb_ctx *c) {
     const Dev &d = c->d;
     int st;
     if ((st = fb::i8_configure())) return st;
+    // the width is a rule on the grid's size: no tuning call needed
+    if (!c->i8_fixed) c->tune_i8bn = fb::i8_step_width(d.n2m, d.n3m);
     const long ldk = (d.n3m + fb::kI8BK - 1) / fb::kI8BK * fb::kI8BK;
     auto make = [&](fb::I8Plan &p, int rows, int box) -> int {
         p.ldk = ldk;
@@ -873,11 +875,17 @@ int setup_i8(fb_ctx *c) {
     if ((st = make(c->i8a, d.n2m, 128)) || (st = make(c->i8f, d.n3m, c->tune_i8bn)) ||
         (st = make(c->i8b, d.n3m, c->tune_i8bn)))
         return st;
-    if ((st = dnew(c, &c->i8max, 2 * static_cast<size_t>(d.ldh)))) return st;   // zeroed
+    // the row maxima (zeroed): at first the two eigenvector operands', then the
+    // data operand's of every step
+    const size_t nmx = 2 * static_cast<size_t>(std::max(d.ldh, d.n3m));
+    if ((st = dnew(c, &c->i8max, nmx))) return st;
     // forward B(m, k) = zmmt(m, k); backward B(k, m) = zmm(k, m): both column-major
-    fb::launch_i8_split(c->zmmt, d.n3m, d.n3m, d.n3m, c->i8f, c->stream);
-    fb::launch_i8_split(c->zmm, d.n3m, d.n3m, d.n3m, c->i8b, c->stream);
+    fb::launch_i8_rowmax(c->zmmt, d.n3m, d.n3m, d.n3m, c->i8max, c->stream);
+    fb::launch_i8_rowmax(c->zmm, d.n3m, d.n3m, d.n3m, c->i8max + d.n3m, c->stream);
+    fb::launch_i8_cut_rows(c->zmmt, d.n3m, d.n3m, d.n3m, c->i8f, c->i8max, nullptr, c->stream);
+    fb::launch_i8_cut_rows(c->zmm, d.n3m, d.n3m, d.n3m, c->i8b, c->i8max + d.n3m, nullptr, c->stream);
     CK(cudaGetLastError());
+    CK(cudaMemsetAsync(c->i8max, 0, nmx * sizeof(double), c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->i8_ready = true;
     return FB_OK;
@@ -2372,18 +2380,24 @@ int group_setup_i8(BatchGroup *bg) {
     const int n = static_cast<int>(bg->members.size());
     std::vector<fb::I8SplitTask> sp(static_cast<size_t>(2 * n));
     std::vector<fb::I8Task> gt(static_cast<size_t>(2 * n));
+    // the group's products fill the GPU together: the tile width by the waves
+    // of all of them, over maps of its own
+    const fb_ctx *c0 = bg->members[0];
+    bg->i8bn = c0->i8_fixed ? c0->tune_i8bn : fb::i8_step_width(c0->d.n2m, c0->d.n3m, 148, n);
     for (int i = 0; i < n; ++i) {
         const fb_ctx *c = bg->members[static_cast<size_t>(i)];
         const Dev &d = c->d;
+        fb::I8Plan f = c->i8f, b = c->i8b;
+        int r;
+        if ((r = fb::i8_plan(f, d.n3m, d.n3m, bg->i8bn)) || (r = fb::i8_plan(b, d.n3m, d.n3m, bg->i8bn))) return r;
         const size_t k = static_cast<size_t>(i), m = static_cast<size_t>(n);
         const fb::I8Plan &a = c->i8a;
         const int *gate = couple_gate(c);
         sp[k] = {d.dph + d.P, d.P, a.dig, a.ldk, a.scale, a.rows_pad, gate};
         sp[m + k] = {d.hmn, d.ldh, a.dig, a.ldk, a.scale, a.rows_pad, gate};
-        gt[k] = {a.map, c->i8f.map, fb::I8Out{d.hmn, d.ldh, a.scale, c->i8f.scale, d.n2m, d.n3m}, d.n3m, d.status,
-                 gate};
-        gt[m + k] = {a.map, c->i8b.map, fb::I8Out{d.dph + d.P, d.P, a.scale, c->i8b.scale, d.n2m, d.n3m}, d.n3m,
-                     d.status, gate};
+        gt[k] = {a.map, f.map, fb::I8Out{d.hmn, d.ldh, a.scale, f.scale, d.n2m, d.n3m}, d.n3m, d.status, gate};
+        gt[m + k] = {a.map, b.map, fb::I8Out{d.dph + d.P, d.P, a.scale, b.scale, d.n2m, d.n3m}, d.n3m, d.status,
+                     gate};
     }
     CK(cudaMalloc(&bg->i8s, sizeof(fb::I8SplitTask) * sp.size()));
     CK(cudaMalloc(&bg->i8t, sizeof(fb::I8Task) * gt.size()));
@@ -2391,7 +2405,6 @@ int group_setup_i8(BatchGroup *bg) {
     CK(cudaMemcpyAsync(bg->i8t, gt.data(), sizeof(fb::I8Task) * gt.size(), cudaMemcpyHostToDevice, bg->st));
     CK(cudaStreamSynchronize(bg->st));
     bg->i8rep = bg->members[0]->i8a;
-    bg->i8bn = bg->members[0]->i8b.box;
     bg->i8 = true;
     return FB_OK;
 }
@@ -2992,7 +3005,7 @@ int fb_autotune(fb_ctx *c, int32_t choice[2]) {
             // favours narrow two-wave tiles; inside the time step the next
             // kernel is another stage (galloping rectangle, the same process:
             // 480 us per step with 48 columns, 513 with 64).
-            ibn = fb::i8_tile_width(d.n2m, d.n3m);   // C = dph (n2m rows) x eigenvectors (n3m)
+            ibn = fb::i8_step_width(d.n2m, d.n3m);   // C = dph (n2m rows) x eigenvectors (n3m)
             r = i8_tile(ibn);
         }
         if (!r && want_bn && !bn) {
@@ -3258,8 +3271,8 @@ int fb_gemm_i8x8(int device, int M, int N, int K, const double *A, const double 
     double *dA = static_cast<double *>(alloc(sizeof(double) * M * K));
     double *dB = static_cast<double *>(alloc(sizeof(double) * N * K));
     double *dC = static_cast<double *>(alloc(sizeof(double) * M * N));
-    pa.dig = static_cast<int8_t *>(alloc(static_cast<size_t>(fb::kI8S) * pa.rows_pad * ldk));
-    pb.dig = static_cast<int8_t *>(alloc(static_cast<size_t>(fb::kI8S) * pb.rows_pad * ldk));
+    pa.dig = static_cast<int8_t *>(alloc(static_cast<size_t>(fb::kI8SPub) * pa.rows_pad * ldk));
+    pb.dig = static_cast<int8_t *>(alloc(static_cast<size_t>(fb::kI8SPub) * pb.rows_pad * ldk));
     pa.scale = static_cast<double *>(alloc(sizeof(double) * pa.rows_pad));
     pb.scale = static_cast<double *>(alloc(sizeof(double) * pb.rows_pad));
     int *status = static_cast<int *>(alloc(sizeof(int)));
@@ -3274,8 +3287,8 @@ int fb_gemm_i8x8(int device, int M, int N, int K, const double *A, const double 
                 cudaMemset(mxA, 0, sizeof(double) * M) != cudaSuccess ||
                 cudaMemset(mxB, 0, sizeof(double) * N) != cudaSuccess))
         st = FB_ERR_CUDA;
-    if (!st) st = fb::i8_plan(pa, M, K, 128);
-    if (!st) st = fb::i8_plan(pb, N, K, fb::kI8BN);
+    if (!st) st = fb::i8_plan(pa, M, K, 128, fb::kI8SPub);
+    if (!st) st = fb::i8_plan(pb, N, K, fb::kI8BN, fb::kI8SPub);
     if (!st) {
         // row maxima, then the cut of each operand (the step's kernels)
         fb::launch_i8_rowmax(dA, M, M, K, mxA, nullptr);

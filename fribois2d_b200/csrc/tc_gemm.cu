@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <type_traits>
 
 #include "../../include/fribois2d.h"
 #include "device.cuh"
@@ -631,85 +632,142 @@ __global__ void __launch_bounds__(256) kg_poisson_residual(const GroupCase *__re
 // ---- FP64 products on the INT8 tensor cores -------------------------------
 // C = A B^T to FP64 accuracy from exact integer products (the Ozaki scheme
 // with power-of-two row scaling, Ozaki, Ogita, Oishi and Rump): every row r
-// of A is scaled by 2^-e(r) (|A(r,k)| < 2^e(r)) and cut into kI8S signed
-// 8-bit digits, a = sum_i d_i 128^-(i+1), likewise the rows of B with f(c).
-// Then
-//   C(r,c) = 2^(e(r)+f(c)) sum_t 128^-(t+2) G_t(r,c),  G_t = sum_{i+j=t} D_i E_j^T,
-// keeping the digit pairs with i + j < kI8S.  Each G_t is an exact int32
-// sum of tcgen05.mma kind::i8 products accumulated in its own TMEM columns
-// (exact while K <= kI8MaxK); the epilogue adds the G_t in FP64 from the
-// smallest weight up and applies the power-of-two scales (exact).  The
-// error is absolute, relative to the row and column maxima: the digit
-// truncation and the dropped pairs leave at most about
-// K 2^-55 max|A(r,:)| max|B(c,:)| (each operand is cut to 56 bits of its
-// row maximum), plus the rounding of the FP64 additions.  For rows of
-// moderate dynamic range that is ~2e-16 of sum |a||b| at K = 1024, as FP64
-// DGEMM; a row whose entries span many decades is reproduced only to
-// 2^-55 of its largest entry.
+// of A is scaled by 2^-e(r) and cut into S signed digits D_i, likewise the
+// rows of B (E_j, f(c)).  Then
+//   C(r,c) = 2^(e(r)+f(c)) sum_t w_t G_t(r,c),  G_t = sum_{i+j=t} D_i E_j^T,
+// keeping the digit pairs with i + j < S.  Each G_t is an exact int32 sum of
+// tcgen05.mma kind::i8 products accumulated in its own TMEM columns (exact
+// while K <= kI8MaxK); the epilogue adds the G_t in FP64 from the smallest
+// weight up and applies the power-of-two scales (exact).
+//
+// The time step uses S = 7 balanced base-256 digits (each operand rounded to
+// 55 bits of its row maximum; w_t = 256^-t 2^-14, 28 pairs).  The public
+// product keeps S = 8 digits of 7 bits with the operand's sign (truncated to
+// 56 bits; w_t = 128^-(t+2), 36 pairs).  Fewer products and a smaller error:
+// digits of either sign leave dropped pairs that cancel on average, where the
+// sign-magnitude digits' all carry the sign of a b.  Against extended
+// precision, relative 2-norm error of 96 x 1024 random rows times the
+// galloping rectangle's eigenvectors: 5.9e-16 (S = 7), 1.26e-15 (S = 8),
+// 5.3e-16 (FP64 product); with rows decaying over 12 e-folds 1.0e-15,
+// 2.1e-15, 0.9e-15.  The error is absolute, relative to the row and column
+// maxima: a row whose entries span many decades is reproduced only to 2^-55
+// of its largest entry.
+// Per launch, S = 8 -> S = 7: 768 x 1024 22.8 -> 18.4 us (48 columns), 256 x
+// 384 8.7 -> 7.5 us (32 columns; 6.5 with 16).
 
-// Two forms of the digit cut.  k_i8_cut_rows (the time step, the public
-// product) takes each row's maximum from an array that the operand's producer
-// (or k_i8_rowmax) accumulated, so its blocks are independent.  k_i8_cut (the
-// eigenvector operands at set-up, the batched launches) finds the maxima
-// itself: a cluster of kCutCl CTAs per 32 rows, each CTA over its own range of
-// 8 V columns.  Thread (lane, warp w) holds V
-// consecutive columns of row lane in registers, all its loads in flight at
-// once (each load coalesced over the 32 rows); the CTA's row maxima go to the
-// cluster through distributed shared memory, so every CTA derives each row's
-// exponent from the whole row; then each thread turns its values into 56-bit
-// integers (one conversion each), takes the digits from them with shifts,
-// four columns to a 32-bit word, and stores each slice's V digit bytes of its
-// row with 16-byte stores.  The operand is read once.
-// Columns past K and rows past R get zero digits, up to ldk and rows_pad.
+// Two forms of the digit cut.  k_i8_cut_rows (the single-case step, the
+// eigenvector operands, the public product) takes each row's maximum from an
+// array that the operand's producer (or k_i8_rowmax) accumulated, so its
+// blocks are independent.  kg_i8_cut (the batched launches) finds the maxima
+// itself: a cluster of kCutCl CTAs per 32 rows, each CTA over its own range
+// of 8 V columns, whose row maxima go to the cluster through distributed
+// shared memory.  In both, thread (lane, warp w) holds V consecutive columns
+// of row lane in registers, all its loads in flight at once (each load
+// coalesced over the 32 rows), turns its values into integers (one
+// conversion each), takes the digits from them four columns to a 32-bit word,
+// and stores each slice's V digit bytes of its row with 16-byte stores.  The
+// operand is read once.  Columns past K and rows past R get zero digits, up
+// to ldk and rows_pad.  k_i8_cut_rows has V = 16 for every K: with V = 32 at
+// K = 1500 a thread's two rounds of loads and half as many blocks took 13.3 us.
 constexpr int kCutCl = 8;
 
-// the digits of a thread's V values a of row r (columns c0 ..) at the row's
-// scale s = 2^-e into the kI8S slices
+// The exponent of a row whose largest |a| is mm: its digits are those of
+// a 2^-e.  8 slices: |a| 2^-e < 1.  7 slices: at most 0.994, so that the
+// leading balanced digit, round(127.3 + 0.5) at most, stays below 128.
+template <int S>
+__device__ __forceinline__ int i8_row_exp(double mm) {
+    int e = 0;
+    if (mm > 0.0) {
+        const double m = frexp(mm, &e);   // mm = m 2^e, m < 1
+        if (S == kI8S && m > 0.994) ++e;
+    }
+    return e;
+}
+
+// stores one slice's V digit bytes of a row (16-byte stores)
 template <int V>
+__device__ __forceinline__ void i8_store_slice(int8_t *o, const uint32_t (&word)[V / 4]) {
+#pragma unroll
+    for (int v4 = 0; v4 < V / 16; ++v4)
+        reinterpret_cast<uint4 *>(o)[v4] =
+            make_uint4(word[4 * v4], word[4 * v4 + 1], word[4 * v4 + 2], word[4 * v4 + 3]);
+}
+
+// the digits of a thread's V values a of row r (columns c0 ..) at the row's
+// scale s = 2^-e into the S slices; each slice's V digits of row r are V
+// consecutive bytes: the thread stores them itself (a whole 32-byte sector
+// between neighbouring warps), no shared-memory transpose; rows up to
+// rows_pad get digits (zero past R)
+template <int V, int S>
 __device__ __forceinline__ void i8_cut_emit(const double (&a)[V / 4][4], double s, int r, int c0, int8_t *dig,
                                             long ldk, long plane) {
     constexpr int kP = V / 4;   // 32-bit words (four columns) per thread and slice
-    // |a s| < 1, so a s 2^(7 kI8S) (exact: powers of two) truncated toward
-    // zero is an integer below 2^(7 kI8S) whose base-128 digits, carrying the
-    // sign of a, are the kI8S digits: d_i = sign(a) floor(|a s| 128^(i+1)) mod 128
-    unsigned long long u[kP][4];
-    uint32_t neg[kP];
-#pragma unroll
-    for (int p = 0; p < kP; ++p) {
-        neg[p] = 0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const long long v = __double2ll_rz((a[p][q] * s) * 72057594037927936.0);   // 2^56
-            u[p][q] = static_cast<unsigned long long>(v < 0 ? -v : v);
-            neg[p] |= (v < 0 ? 0xFFu : 0u) << (8 * q);
-        }
-    }
-    static_assert(kI8S == 8, "2^56 = 128^kI8S");
-    // each slice's V digits of row r are V consecutive bytes: the thread
-    // stores them itself (a whole 32-byte sector between neighbouring warps),
-    // no shared-memory transpose; rows up to rows_pad get digits (zero past R)
     const bool live = c0 < ldk;   // ldk is a multiple of 128, so a run is inside or wholly past it
     int8_t *out = dig + static_cast<size_t>(r) * ldk + c0;
-    constexpr int kUnroll = (V <= 32) ? kI8S : 1;   // constant shifts where registers allow
-#pragma unroll kUnroll
-    for (int i = 0; i < kI8S; ++i) {
-        const int sh = 7 * (kI8S - 1 - i);
-        uint32_t word[kP];
+    if constexpr (S == kI8S) {
+        // a s 2^55 rounded to an integer v = sum_i d_i 256^(6 - i), |d_i| <= 128:
+        // with 128 added to each of the six lower digits (one 64-bit addition)
+        // every digit is a byte of the sum, biased by 128; the exclusive or
+        // takes the bias off again.  Byte i of four values becomes the word of
+        // slice 6 - i by byte permutations.
+        constexpr unsigned long long kBias = 0x0000808080808080ull;
+        uint32_t lo[kP][4], hi[kP][4];
+#pragma unroll
+        for (int p = 0; p < kP; ++p)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const long long v = __double2ll_rn((a[p][q] * s) * 36028797018963968.0);   // 2^55
+                const unsigned long long u = (static_cast<unsigned long long>(v) + kBias) ^ kBias;
+                lo[p][q] = static_cast<uint32_t>(u);
+                hi[p][q] = static_cast<uint32_t>(u >> 32);
+            }
+        if (!live) return;
+#pragma unroll
+        for (int i = 0; i < S; ++i) {
+            constexpr int kTop = S - 1;
+            const int byte = (kTop - i) & 3;   // of the low word for slices 3 .. 6, of the high one above
+            const uint32_t sel = static_cast<uint32_t>(byte) | (static_cast<uint32_t>(byte + 4) << 4);
+            uint32_t word[kP];
+#pragma unroll
+            for (int p = 0; p < kP; ++p) {
+                const uint32_t(&x)[4] = (kTop - i < 4) ? lo[p] : hi[p];
+                word[p] = __byte_perm(__byte_perm(x[0], x[1], sel), __byte_perm(x[2], x[3], sel), 0x5410);
+            }
+            i8_store_slice<V>(out + static_cast<size_t>(i) * plane, word);
+        }
+    } else {
+        // |a s| < 1, so a s 2^(7 S) (exact: powers of two) truncated toward
+        // zero is an integer below 2^(7 S) whose base-128 digits, carrying the
+        // sign of a, are the S digits: d_i = sign(a) floor(|a s| 128^(i+1)) mod 128
+        unsigned long long u[kP][4];
+        uint32_t neg[kP];
 #pragma unroll
         for (int p = 0; p < kP; ++p) {
-            uint32_t mag = 0;
+            neg[p] = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) mag |= static_cast<uint32_t>((u[p][q] >> sh) & 127u) << (8 * q);
-            // the negative values' bytes negated (bytewise, no carries between bytes)
-            const uint32_t mk = neg[p];
-            word[p] = (mag & ~mk) | (__vsub4(0u, mag) & mk);
+            for (int q = 0; q < 4; ++q) {
+                const long long v = __double2ll_rz((a[p][q] * s) * 72057594037927936.0);   // 2^56
+                u[p][q] = static_cast<unsigned long long>(v < 0 ? -v : v);
+                neg[p] |= (v < 0 ? 0xFFu : 0u) << (8 * q);
+            }
         }
-        if (live) {
-            int8_t *o = out + static_cast<size_t>(i) * plane;
+        static_assert(S == 8, "2^56 = 128^S");
+        if (!live) return;
+        constexpr int kUnroll = (V <= 32) ? S : 1;   // constant shifts where registers allow
+#pragma unroll kUnroll
+        for (int i = 0; i < S; ++i) {
+            const int sh = 7 * (S - 1 - i);
+            uint32_t word[kP];
 #pragma unroll
-            for (int v4 = 0; v4 < V / 16; ++v4)
-                reinterpret_cast<uint4 *>(o)[v4] =
-                    make_uint4(word[4 * v4], word[4 * v4 + 1], word[4 * v4 + 2], word[4 * v4 + 3]);
+            for (int p = 0; p < kP; ++p) {
+                uint32_t mag = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) mag |= static_cast<uint32_t>((u[p][q] >> sh) & 127u) << (8 * q);
+                // the negative values' bytes negated (bytewise, no carries between bytes)
+                const uint32_t mk = neg[p];
+                word[p] = (mag & ~mk) | (__vsub4(0u, mag) & mk);
+            }
+            i8_store_slice<V>(out + static_cast<size_t>(i) * plane, word);
         }
     }
 }
@@ -751,26 +809,24 @@ __device__ __forceinline__ void i8_cut_body(const double *__restrict__ src, long
     if (w == 0) {
         double mm = 0.0;
         for (int q = 0; q < kCutCl; ++q) mm = fmax(mm, *cl.map_shared_rank(&part[lane], q));
-        int e = 0;
-        if (mm > 0.0) frexp(mm, &e);   // mm < 2^e
+        const int e = i8_row_exp<kI8S>(mm);
         sc[lane] = ldexp(1.0, -e);
         if (rank == 0 && r < R) rowscale[r] = ldexp(1.0, e);
     }
     cl.sync();   // no CTA leaves while another still reads its maxima
-    i8_cut_emit<V>(a, sc[lane], r, c0, dig, ldk, plane);
+    i8_cut_emit<V, kI8S>(a, sc[lane], r, c0, dig, ldk, plane);
 }
 
 // The cut with the rows' maxima of |a| given (accumulated by the operand's
 // producer, or by k_i8_rowmax): no exchange between blocks.  Block (x, y):
-// rows 32 x .. 32 x + 31 (lane = row), columns 8 V y + V w .. (warp w), the
-// layout of the cluster form.  Column group 0 stores the row scales and, for
+// rows 32 x .. 32 x + 31 (lane = row), columns 128 y + 16 w .. (warp w).  Column group 0 stores the row scales and, for
 // the next producer, clears its maxima (clear, may be null).
-template <int V>
+template <int S>
 __global__ void __launch_bounds__(256)
     k_i8_cut_rows(const double *__restrict__ src, long lds, int R, int K, int8_t *dig, long ldk, long plane,
                   double *rowscale, const double *__restrict__ rmax, double *clear) {
     FB_GRID_WAIT();
-    constexpr int kP = V / 4;
+    constexpr int V = 16, kP = V / 4;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int r = blockIdx.x * 32 + lane;
     const int c0 = blockIdx.y * 8 * V + V * w;
@@ -783,13 +839,12 @@ __global__ void __launch_bounds__(256)
             a[p][q] = (r < R && k < K) ? src[static_cast<size_t>(k) * lds + r] : 0.0;
         }
     const double mm = (r < R) ? rmax[r] : 0.0;
-    int e = 0;
-    if (mm > 0.0) frexp(mm, &e);   // mm < 2^e
+    const int e = i8_row_exp<S>(mm);
     if (blockIdx.y == 0 && w == 0 && r < R) {
         rowscale[r] = ldexp(1.0, e);
         if (clear) clear[r] = 0.0;
     }
-    i8_cut_emit<V>(a, ldexp(1.0, -e), r, c0, dig, ldk, plane);
+    i8_cut_emit<V, S>(a, ldexp(1.0, -e), r, c0, dig, ldk, plane);
 }
 
 // rmax[r] = max(rmax[r], max_k |src[k lds + r]|) for rows r < R, columns k < K
@@ -811,14 +866,6 @@ __global__ void __launch_bounds__(256) k_i8_rowmax(const double *__restrict__ sr
     }
 }
 
-template <int V>
-__global__ void __cluster_dims__(kCutCl, 1, 1) __launch_bounds__(256)
-    k_i8_cut(const double *__restrict__ src, long lds, int R, int K, int8_t *dig, long ldk, long plane,
-             double *rowscale) {
-    FB_GRID_WAIT();
-    i8_cut_body<V>(src, lds, R, K, dig, ldk, plane, rowscale);
-}
-
 // grouped (blockIdx.z = case; a cluster never spans two cases)
 template <int V>
 __global__ void __cluster_dims__(kCutCl, 1, 1) __launch_bounds__(256)
@@ -836,37 +883,43 @@ inline int cut_values(long ldk) {
     return per <= 16 ? 16 : per <= 32 ? 32 : 64;
 }
 
-// BN: output tile width, 64, 48 or 32 (a 128 x 48 tile puts 132 CTAs on a
-// 768 x 1024 product where 128 x 64 tiles leave a third of the 148 SMs idle;
-// 32 spreads small products over more SMs, one MMA of N = 32 (8 - i) per A slice)
-template <int BN>
+// S: digit slices; BN: output tile width, 64, 48, 32 or 16 (a 128 x 48 tile
+// puts 132 CTAs on a 768 x 1024 product where 128 x 64 tiles leave a third of
+// the 148 SMs idle; 32 and 16 spread small products over more SMs)
+template <int S, int BN>
 struct I8Cfg {
     static constexpr uint32_t kATile = 128 * kI8BK;                 // one A digit slice: 128 rows x 128 B
     static constexpr uint32_t kBSlice = BN * kI8BK;                 // one B digit slice
-    static constexpr uint32_t kBStage = kI8S * BN * kI8BK;          // all B slices of a k-block
-    // as many A slots as the shared memory holds beside two B stages
-    static constexpr int kASlots = static_cast<int>((227u * 1024u - 1280u - 2u * kBStage) / kATile);
+    static constexpr uint32_t kBStage = S * BN * kI8BK;             // all B slices of a k-block
+    // as many A slots (in pairs) as the shared memory holds beside two B stages, at most 10
+    static constexpr int kAFit = static_cast<int>((227u * 1024u - 1280u - 2u * kBStage) / kATile);
+    static constexpr int kASlots = (kAFit < 10 ? kAFit : 10) / 2 * 2;
     static constexpr size_t kSmem = 2 * kBStage + kASlots * kATile + 1024 + 256;
-    static constexpr uint32_t kTmemCols = 512;                      // kI8S class accumulators of BN columns
+    static constexpr uint32_t kTmemCols = (S * BN > 256) ? 512 : (S * BN > 128) ? 256 : 128;   // S class accumulators of BN columns
     // D s32 (2), A and B signed 8-bit (1), both K-major, M = 128; N set per MMA
     static constexpr uint32_t kIdescBase = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(128 >> 4) << 24);
-    static_assert(kI8S * BN <= 512, "TMEM columns");
+    // weight class t: 2^-(kShift t + kW0)
+    static constexpr int kShift = (S == kI8S) ? 8 : 7, kW0 = 14;
+    static_assert(S * BN <= 512, "TMEM columns");
     static_assert(BN % 16 == 0 && BN <= 256, "MMA N: a multiple of 16, at most 256");
-    static_assert(kASlots >= 2 && kSmem <= 227 * 1024, "shared memory per CTA");
+    static_assert(kBSlice % 1024 == 0, "B slices start on swizzle atoms");
+    static_assert(kASlots >= 4 && kSmem <= 227 * 1024, "shared memory per CTA");
 };
 
 // One CTA per 128 x BN tile of C.  Per k-block of 128: the producer
-// thread loads all B slices (one barrier) and streams the A slices through
-// a ring, two slices per barrier; the MMA thread multiplies A slice i with B
-// slices j < kI8S - i into accumulators i + j (MMAs of K = 32 over up to
-// 256 / BN slices at once); eight warps drain the accumulators.  Every wait
-// gives up after one second with FB_ERR_TIMEOUT.
-template <int BN, bool kGlobalMaps>
+// thread loads all B slices (one copy, one barrier) and streams the A slices
+// through a ring, two consecutive slices of the stream per barrier (with an
+// odd S a pair may straddle two k-blocks, and the last pair may hold one
+// slice); the MMA thread multiplies A slice i with B slices j < S - i into
+// accumulators i + j (MMAs of K = 32 over up to 256 / BN slices at once);
+// eight warps drain the accumulators.  Every wait gives up after one second
+// with FB_ERR_TIMEOUT.
+template <int S, int BN, bool kGlobalMaps>
 __device__ __forceinline__ void i8x8_body(const CUtensorMap *ma, const CUtensorMap *mb, const I8Out &o, int K,
                                           int *status) {
-    using Cfg = I8Cfg<BN>;
-    constexpr int kS = kI8S, kAS = Cfg::kASlots, kAP = kAS / 2;   // A slots, in pairs of slices
-    static_assert(kAS % 2 == 0 && kS % 2 == 0, "A slices move in pairs");
+    using Cfg = I8Cfg<S, BN>;
+    constexpr int kS = S, kAS = Cfg::kASlots, kAP = kAS / 2;   // A slots, in pairs of slices
+    static_assert(kAS % 2 == 0, "A slices move in pairs");
     extern __shared__ uint8_t smraw[];
     const uint32_t raw = smem_u32(smraw);
     const uint32_t pad = (1024u - (raw & 1023u)) & 1023u;
@@ -931,14 +984,14 @@ __device__ __forceinline__ void i8x8_body(const CUtensorMap *ma, const CUtensorM
         if (!kGlobalMaps && o.b_const) {
             for (; pre < 2 && pre < nk; ++pre) {
                 mbar_expect_tx(bfull0 + 8 * pre, Cfg::kBStage);
-                for (int j = 0; j < kS; ++j)
-                    tma_load_3d(sB + pre * Cfg::kBStage + j * Cfg::kBSlice, mb, bfull0 + 8 * pre, pre * kI8BK, n0, j);
+                tma_load_3d(sB + pre * Cfg::kBStage, mb, bfull0 + 8 * pre, pre * kI8BK, n0, 0);
             }
         }
         if (!kGlobalMaps) FB_GRID_WAIT();
         load_scales();
         int ip = 0, nb = pre, ps = 0;   // A slice pairs issued, B stages issued, pair slot
         uint32_t aph = 0;
+        int half = 0;   // slices of the current pair already issued
         for (int kb = 0; kb < nk && ok; ++kb) {
             const int sb = kb & 1;
             if (kb >= pre) {
@@ -947,21 +1000,23 @@ __device__ __forceinline__ void i8x8_body(const CUtensorMap *ma, const CUtensorM
                     break;
                 }
                 mbar_expect_tx(bfull0 + 8 * sb, Cfg::kBStage);
-                for (int j = 0; j < kS; ++j)
-                    tma_load_3d(sB + sb * Cfg::kBStage + j * Cfg::kBSlice, mb, bfull0 + 8 * sb, kb * kI8BK, n0, j);
+                tma_load_3d(sB + sb * Cfg::kBStage, mb, bfull0 + 8 * sb, kb * kI8BK, n0, 0);
                 nb = kb + 1;
             }
 #pragma unroll
-            for (int i = 0; i < kS; i += 2) {   // slices i, i + 1 on one barrier
-                if (!mbar_wait(aempty0 + 8 * ps, aph ^ 1u)) {
-                    ok = false;
-                    break;
+            for (int i = 0; i < kS; ++i) {
+                if (half == 0) {
+                    if (!mbar_wait(aempty0 + 8 * ps, aph ^ 1u)) {
+                        ok = false;
+                        break;
+                    }
+                    const bool single = (kS % 2) && kb == nk - 1 && i == kS - 1;   // the stream's odd last slice
+                    mbar_expect_tx(afull0 + 8 * ps, (single ? 1 : 2) * Cfg::kATile);
+                    ++ip;
                 }
-                mbar_expect_tx(afull0 + 8 * ps, 2 * Cfg::kATile);
-                tma_load_3d(sA + (2 * ps) * Cfg::kATile, ma, afull0 + 8 * ps, kb * kI8BK, m0, i);
-                tma_load_3d(sA + (2 * ps + 1) * Cfg::kATile, ma, afull0 + 8 * ps, kb * kI8BK, m0, i + 1);
-                ++ip;
-                if (++ps == kAP) {
+                tma_load_3d(sA + (2 * ps + half) * Cfg::kATile, ma, afull0 + 8 * ps, kb * kI8BK, m0, i);
+                half ^= 1;
+                if (half == 0 && ++ps == kAP) {
                     ps = 0;
                     aph ^= 1u;
                 }
@@ -981,46 +1036,46 @@ __device__ __forceinline__ void i8x8_body(const CUtensorMap *ma, const CUtensorM
         const uint64_t adesc = sw128_desc(sA), bdesc = sw128_desc(sB);
         int ps = 0;
         uint32_t aph = 0;
-        for (int kb = 0; kb < nk && ok; ++kb) {
+        // one k-block; kPar: the parity of its first slice in the A stream
+        auto kblock = [&](auto par, int kb) -> bool {
+            constexpr int kPar = decltype(par)::value;
             const int sb = kb & 1;
-            if (!mbar_wait(bfull0 + 8 * sb, static_cast<uint32_t>(kb >> 1) & 1u)) {
-                ok = false;
-                break;
-            }
+            if (!mbar_wait(bfull0 + 8 * sb, static_cast<uint32_t>(kb >> 1) & 1u)) return false;
             tc_fence_after();
             const uint64_t bst = bdesc + static_cast<uint64_t>((sb * Cfg::kBStage) >> 4);
 #pragma unroll
-            for (int i2 = 0; i2 < kS; i2 += 2) {   // A slices i2, i2 + 1: one wait, one commit
-                if (!mbar_wait(afull0 + 8 * ps, aph)) {
-                    ok = false;
-                    break;
+            for (int i = 0; i < kS; ++i) {
+                const int e = (kPar + i) & 1;   // slot of the pair
+                // (the first k-block half of a straddling pair has waited for it)
+                if (e == 0 && !mbar_wait(afull0 + 8 * ps, aph)) return false;
+                const uint64_t ast = adesc + static_cast<uint64_t>(((2 * ps + e) * Cfg::kATile) >> 4);
+                // B slices j0 .. j0+nsl-1 are consecutive rows in shared memory and
+                // their classes i+j0 .. consecutive TMEM column blocks: one MMA of
+                // N = nsl * BN covers nsl digit pairs
+#pragma unroll
+                for (int j0 = 0; j0 < kS - i; j0 += kG) {
+                    const int nsl = (kS - i - j0 < kG) ? kS - i - j0 : kG;
+                    const uint32_t idesc = Cfg::kIdescBase | (static_cast<uint32_t>((nsl * BN) >> 3) << 17);
+                    const uint32_t acc_t = tmem + static_cast<uint32_t>((i + j0) * BN);
+                    const uint64_t bj = bst + static_cast<uint64_t>((j0 * Cfg::kBSlice) >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < kI8BK / 32; ++kk)   // K = 32 bytes per MMA: +2 in the address field
+                        mma_i8(acc_t, ast + 2 * kk, bj + 2 * kk, idesc, (kb > 0 || i > 0 || kk > 0) ? 1u : 0u);
                 }
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int i = i2 + e;
-                    const uint64_t ast = adesc + static_cast<uint64_t>(((2 * ps + e) * Cfg::kATile) >> 4);
-                    // B slices j0 .. j0+nsl-1 are consecutive rows in shared memory and
-                    // their classes i+j0 .. consecutive TMEM column blocks: one MMA of
-                    // N = nsl * BN covers nsl digit pairs
-#pragma unroll
-                    for (int j0 = 0; j0 < kS - i; j0 += kG) {
-                        const int nsl = (kS - i - j0 < kG) ? kS - i - j0 : kG;
-                        const uint32_t idesc = Cfg::kIdescBase | (static_cast<uint32_t>((nsl * BN) >> 3) << 17);
-                        const uint32_t acc_t = tmem + static_cast<uint32_t>((i + j0) * BN);
-                        const uint64_t bj = bst + static_cast<uint64_t>((j0 * Cfg::kBSlice) >> 4);
-#pragma unroll
-                        for (int kk = 0; kk < kI8BK / 32; ++kk)   // K = 32 bytes per MMA: +2 in the address field
-                            mma_i8(acc_t, ast + 2 * kk, bj + 2 * kk, idesc, (kb > 0 || i > 0 || kk > 0) ? 1u : 0u);
+                if (e == 1 || (i == kS - 1 && kb == nk - 1)) {   // the pair (or the odd last slice) is done
+                    mma_commit(aempty0 + 8 * ps);   // frees its A slots once these MMAs have read them
+                    if (++ps == kAP) {
+                        ps = 0;
+                        aph ^= 1u;
                     }
                 }
-                mma_commit(aempty0 + 8 * ps);   // frees the two A slots once these MMAs have read them
-                if (++ps == kAP) {
-                    ps = 0;
-                    aph ^= 1u;
-                }
             }
-            if (!ok) break;
             mma_commit(bempty0 + 8 * sb);
+            return true;
+        };
+        for (int kb = 0; kb < nk && ok; kb += 1 + kS % 2) {
+            ok = kblock(std::integral_constant<int, 0>{}, kb);
+            if (kS % 2 && ok && kb + 1 < nk) ok = kblock(std::integral_constant<int, 1>{}, kb + 1);
         }
         mma_commit(done);
     }
@@ -1048,7 +1103,7 @@ __device__ __forceinline__ void i8x8_body(const CUtensorMap *ma, const CUtensorM
         for (int q = 0; q < 8; ++q) acc[q] = 0.0;
 #pragma unroll
         for (int t = kS - 1; t >= 0; --t) {
-            const double wgt = ldexp(1.0, -7 * (t + 2));
+            const double wgt = ldexp(1.0, -(Cfg::kShift * t + Cfg::kW0));
 #pragma unroll
             for (int q = 0; q < 8; ++q) acc[q] = acc[q] + i32_as_f64(v[t][q]) * wgt;
         }
@@ -1068,11 +1123,11 @@ __device__ __forceinline__ void i8x8_body(const CUtensorMap *ma, const CUtensorM
     }
 }
 
-template <int BN>
+template <int S, int BN>
 __global__ void __launch_bounds__(kI8Threads, 1)
     k_i8x8_gemm(const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb, I8Out o, int K,
                 int *status) {
-    i8x8_body<BN, false>(&ma, &mb, o, K, status);   // waits for the previous kernel after its set-up
+    i8x8_body<S, BN, false>(&ma, &mb, o, K, status);   // waits for the previous kernel after its set-up
 }
 
 // grouped: blockIdx.z selects the product
@@ -1082,7 +1137,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) kg_i8x8_gemm(const I8Task *__re
     const I8Task &tk = t[blockIdx.z];
     if (tk.gate && !*tk.gate) return;
     const I8Out o = tk.o;
-    i8x8_body<BN, true>(&tk.a, &tk.b, o, tk.K, tk.status);
+    i8x8_body<kI8S, BN, true>(&tk.a, &tk.b, o, tk.K, tk.status);
 }
 
 void launch_poisson_residual(const Dev &d, const double *phi, const SplitPlane &dst, cudaStream_t st,
@@ -1218,9 +1273,10 @@ void launch_split_t(const double *src, long lds, int R, int C, const SplitPlane 
 
 
 // ---- INT8 FP64 products: buffers, maps, launches
-int i8_plan(I8Plan &p, int rows, int K, int box_rows) {
+int i8_plan(I8Plan &p, int rows, int K, int box_rows, int slices) {
     if (K > kI8MaxK) return FB_ERR_UNSUPPORTED;   // the int32 class sums would overflow
-    if (box_rows != 128 && box_rows != 64 && box_rows != 48 && box_rows != 32) return FB_ERR_STATE;
+    if (box_rows != 128 && box_rows != 64 && box_rows != 48 && box_rows != 32 && box_rows != 16) return FB_ERR_STATE;
+    if (slices != kI8S && (slices != kI8SPub || (box_rows != 128 && box_rows != kI8BN))) return FB_ERR_STATE;
     if (!p.dig || (p.ldk % 128) || p.rows_pad < rows) return FB_ERR_STATE;
     if (!g_encode) {
         void *fn = nullptr;
@@ -1232,10 +1288,11 @@ int i8_plan(I8Plan &p, int rows, int K, int box_rows) {
     }
     if (reinterpret_cast<uintptr_t>(p.dig) & 15u) return FB_ERR_STATE;
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(p.ldk), static_cast<cuuint64_t>(p.rows_pad),
-                                static_cast<cuuint64_t>(kI8S)};
+                                static_cast<cuuint64_t>(slices)};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(p.ldk),
                                    static_cast<cuuint64_t>(p.ldk) * static_cast<cuuint64_t>(p.rows_pad)};
-    const cuuint32_t box[3] = {static_cast<cuuint32_t>(kI8BK), static_cast<cuuint32_t>(box_rows), 1};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(kI8BK), static_cast<cuuint32_t>(box_rows),
+                               box_rows == 128 ? 1u : static_cast<cuuint32_t>(slices)};
     const cuuint32_t es[3] = {1, 1, 1};
     const CUresult r = g_encode(&p.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, p.dig, dims, strides, box, es,
                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1243,22 +1300,22 @@ int i8_plan(I8Plan &p, int rows, int K, int box_rows) {
     p.rows = rows;
     p.K = K;
     p.box = box_rows;
+    p.slices = slices;
     return r == CUDA_SUCCESS ? FB_OK : FB_ERR_CUDA;
 }
 
 int i8_configure() {
-    const bool ok = cudaFuncSetAttribute(k_i8x8_gemm<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(I8Cfg<64>::kSmem)) == cudaSuccess &&
-                    cudaFuncSetAttribute(kg_i8x8_gemm<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(I8Cfg<64>::kSmem)) == cudaSuccess &&
-                    cudaFuncSetAttribute(k_i8x8_gemm<48>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(I8Cfg<48>::kSmem)) == cudaSuccess &&
-                    cudaFuncSetAttribute(kg_i8x8_gemm<48>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(I8Cfg<48>::kSmem)) == cudaSuccess &&
-                    cudaFuncSetAttribute(k_i8x8_gemm<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(I8Cfg<32>::kSmem)) == cudaSuccess &&
-                    cudaFuncSetAttribute(kg_i8x8_gemm<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(I8Cfg<32>::kSmem)) == cudaSuccess;
+    bool ok = true;
+    auto allow = [&](auto kern, size_t smem) {
+        ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) ==
+                       cudaSuccess;
+    };
+    allow(k_i8x8_gemm<kI8SPub, kI8BN>, I8Cfg<kI8SPub, kI8BN>::kSmem);
+#define FB_I8_ALLOW(BN)                                 \
+    allow(k_i8x8_gemm<kI8S, BN>, I8Cfg<kI8S, BN>::kSmem); \
+    allow(kg_i8x8_gemm<BN>, I8Cfg<kI8S, BN>::kSmem);
+    FB_I8_ALLOW(64) FB_I8_ALLOW(48) FB_I8_ALLOW(32) FB_I8_ALLOW(16)
+#undef FB_I8_ALLOW
     return ok ? FB_OK : FB_ERR_CUDA;
 }
 
@@ -1275,38 +1332,18 @@ void launch_i8_split_group(const I8SplitTask *tasks, const I8Plan &rep, int R, i
 
 void launch_i8x8_group(const I8Task *tasks, int M, int N, int n, int bn, cudaStream_t st) {
     const dim3 grid((M + 127) / 128, (N + bn - 1) / bn, n);
-    if (bn == 48) pdl(kg_i8x8_gemm<48>, grid, dim3(kI8Threads), I8Cfg<48>::kSmem, st, tasks);
-    else if (bn == 32) pdl(kg_i8x8_gemm<32>, grid, dim3(kI8Threads), I8Cfg<32>::kSmem, st, tasks);
-    else pdl(kg_i8x8_gemm<64>, grid, dim3(kI8Threads), I8Cfg<64>::kSmem, st, tasks);
-}
-
-void launch_i8_split(const double *src, long lds, int R, int K, const I8Plan &p, cudaStream_t st) {
-    const dim3 grid(p.rows_pad / 32 * kCutCl);
-    const long plane = p.ldk * static_cast<long>(p.rows_pad);
-    switch (cut_values(p.ldk)) {
-#define FB_CUT_CASE(V) \
-    case V: pdl(k_i8_cut<V>, grid, dim3(256), 0, st, src, lds, R, K, p.dig, p.ldk, plane, p.scale); break;
-        FB_CUT_CASE(16) FB_CUT_CASE(32)
-#undef FB_CUT_CASE
-    default: pdl(k_i8_cut<64>, grid, dim3(256), 0, st, src, lds, R, K, p.dig, p.ldk, plane, p.scale); break;
-    }
+    if (bn == 48) pdl(kg_i8x8_gemm<48>, grid, dim3(kI8Threads), I8Cfg<kI8S, 48>::kSmem, st, tasks);
+    else if (bn == 32) pdl(kg_i8x8_gemm<32>, grid, dim3(kI8Threads), I8Cfg<kI8S, 32>::kSmem, st, tasks);
+    else if (bn == 16) pdl(kg_i8x8_gemm<16>, grid, dim3(kI8Threads), I8Cfg<kI8S, 16>::kSmem, st, tasks);
+    else pdl(kg_i8x8_gemm<64>, grid, dim3(kI8Threads), I8Cfg<kI8S, 64>::kSmem, st, tasks);
 }
 
 void launch_i8_cut_rows(const double *src, long lds, int R, int K, const I8Plan &p, const double *rmax,
                         double *clear, cudaStream_t st) {
-    const dim3 grid(p.rows_pad / 32, kCutCl);
+    const dim3 grid(p.rows_pad / 32, static_cast<unsigned>(p.ldk / 128));
     const long plane = p.ldk * static_cast<long>(p.rows_pad);
-    switch (cut_values(p.ldk)) {
-#define FB_CUT_CASE(V)                                                                                           \
-    case V:                                                                                                      \
-        pdl(k_i8_cut_rows<V>, grid, dim3(256), 0, st, src, lds, R, K, p.dig, p.ldk, plane, p.scale, rmax, clear); \
-        break;
-        FB_CUT_CASE(16) FB_CUT_CASE(32)
-#undef FB_CUT_CASE
-    default:
-        pdl(k_i8_cut_rows<64>, grid, dim3(256), 0, st, src, lds, R, K, p.dig, p.ldk, plane, p.scale, rmax, clear);
-        break;
-    }
+    pdl(p.slices == kI8SPub ? k_i8_cut_rows<kI8SPub> : k_i8_cut_rows<kI8S>, grid, dim3(256), 0, st, src, lds, R, K,
+        p.dig, p.ldk, plane, p.scale, rmax, clear);
 }
 
 void launch_i8_rowmax(const double *src, long lds, int R, int K, double *rmax, cudaStream_t st) {
@@ -1319,9 +1356,14 @@ void launch_i8x8(const I8Plan &a, const I8Plan &b, double *out, long ldo, int *s
                  bool b_const) {
     I8Out o{out, ldo, a.scale, b.scale, a.rows, b.rows, b_const ? 1 : 0};
     const dim3 grid((a.rows + 127) / 128, (b.rows + b.box - 1) / b.box);
-    if (b.box == 48) pdl(k_i8x8_gemm<48>, grid, dim3(kI8Threads), I8Cfg<48>::kSmem, st, a.map, b.map, o, a.K, status);
-    else if (b.box == 32) pdl(k_i8x8_gemm<32>, grid, dim3(kI8Threads), I8Cfg<32>::kSmem, st, a.map, b.map, o, a.K, status);
-    else pdl(k_i8x8_gemm<64>, grid, dim3(kI8Threads), I8Cfg<64>::kSmem, st, a.map, b.map, o, a.K, status);
+    auto go = [&](auto kern, size_t smem) {
+        pdl(kern, grid, dim3(kI8Threads), smem, st, a.map, b.map, o, a.K, status);
+    };
+    if (b.slices == kI8SPub) go(k_i8x8_gemm<kI8SPub, kI8BN>, I8Cfg<kI8SPub, kI8BN>::kSmem);
+    else if (b.box == 48) go(k_i8x8_gemm<kI8S, 48>, I8Cfg<kI8S, 48>::kSmem);
+    else if (b.box == 32) go(k_i8x8_gemm<kI8S, 32>, I8Cfg<kI8S, 32>::kSmem);
+    else if (b.box == 16) go(k_i8x8_gemm<kI8S, 16>, I8Cfg<kI8S, 16>::kSmem);
+    else go(k_i8x8_gemm<kI8S, 64>, I8Cfg<kI8S, 64>::kSmem);
 }
 
 }  // namespace fb

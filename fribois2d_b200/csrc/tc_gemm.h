@@ -56,23 +56,29 @@ struct ResidualTask {    // one Poisson residual: phi -> hi, lo (ldd), row facto
     const double *kscale;
 };
 
-// FP64 products C = A B^T on the INT8 tensor cores (kI8S digit slices per
-// operand; tc_gemm.cu).  An operand: digit planes [slice][row][k] of
-// rows_pad x ldk bytes (ldk a multiple of 128), 2^e per row, its tensor map.
-constexpr int kI8S = 8;       // digit slices per operand
+// FP64 products C = A B^T on the INT8 tensor cores (digit slices; tc_gemm.cu).
+// An operand: digit planes [slice][row][k] of rows_pad x ldk bytes (ldk a
+// multiple of 128), 2^e per row, its tensor map.  Two digit schemes, named by
+// their slices per operand: 7 balanced 8-bit digits (28 digit pairs; the time
+// step) and 8 sign-magnitude 7-bit digits (36 pairs; the public product
+// fb_gemm_i8x8, whose digits and summation order are its documented result).
+constexpr int kI8S = 7;       // digit slices per operand of the time step
+constexpr int kI8SPub = 8;    // ... of fb_gemm_i8x8
 constexpr int kI8BK = 128;    // K bytes per k-block (one 128-byte swizzle row)
-constexpr int kI8BN = 64;     // output tile width (the default; 48 is the other choice)
-// Largest K of one product: weight class t = kI8S - 1 sums kI8S digit pairs
-// of at most 127 * 127 per k into an int32 TMEM accumulator, so
-// K * kI8S * 127^2 must stay below 2^31 (K <= 16642); i8_plan rejects more.
+constexpr int kI8BN = 64;     // widest output tile
+// Largest K of one product: the last weight class sums S digit pairs (7 of at
+// most 128 * 128, or 8 of at most 127 * 127) per k into an int32 TMEM
+// accumulator, so K * 8 * 127^2 and K * 7 * 128^2 must stay below 2^31
+// (K <= 16642); i8_plan rejects more.
 constexpr int kI8MaxK = 16384;
 
 // The INT8 product's tile width for C[rows x cols] (one CTA per 128 x width
 // tile): the width of 64, 48 or 32 that minimises (CTA waves on sms SMs) x
 // width, ties to the wider tile.  A CTA's time grows with its width, so this
-// is the product's time in units of one column of one wave.
-inline int i8_tile_width(int rows, int cols, int sms = 148) {
-    const int mt = (rows + 127) / 128;
+// is the product's time in units of one column of one wave.  products: equal
+// products in one (grouped) launch.
+inline int i8_tile_width(int rows, int cols, int sms = 148, int products = 1) {
+    const int mt = (rows + 127) / 128 * products;
     int best_w = 64;
     long best = -1;
     for (int w : {64, 48, 32}) {
@@ -85,13 +91,25 @@ inline int i8_tile_width(int rows, int cols, int sms = 148) {
     }
     return best_w;
 }
+// The time step's width: i8_tile_width's, or 16 where its tiles would leave
+// at least half of the SMs without one (a small product is a chain of
+// k-blocks whose length is proportional to the width).  Measured per launch
+// with 64 / 48 / 32 / 16 columns: 768 x 1024 (rows x columns) 22.5 / 18.4 /
+// 27.4 / 36.4 us, 512 x 768 17.8 / 14.7 / 11.5 / 19.5, 384 x 512 13.5 / 11.1 /
+// 8.7 / 7.7, 256 x 384 11.6 / 9.6 / 7.5 / 6.5, 32 x 48 6.8 / 5.7 / 4.6 / 3.9.
+inline int i8_step_width(int rows, int cols, int sms = 148, int products = 1) {
+    const int w = i8_tile_width(rows, cols, sms, products);
+    const long ctas = static_cast<long>((rows + 127) / 128) * ((cols + w - 1) / w) * products;
+    return (w == 32 && 2 * ctas <= sms) ? 16 : w;
+}
 struct I8Plan {
     CUtensorMap map;
     int8_t *dig;
     double *scale;            // 2^e(row)
     long ldk;
     int rows_pad, rows, K;
-    int box;                  // rows per TMA box: 128 (A) or the output tile width (B: 48 or 64)
+    int box;                  // rows per TMA box: 128 (A) or the output tile width (B)
+    int slices;               // kI8S or kI8SPub
 };
 struct I8Out {
     double *out;
@@ -118,12 +136,12 @@ struct I8Task {
     const int *gate;
 };
 int i8_configure();
-// box_rows: 128 for the A operand, the output tile width (48 or 64) for B
-int i8_plan(I8Plan &p, int rows, int K, int box_rows);
-// digits of the column-major source A(r, k) = src[k * lds + r], r < R, k < K
-void launch_i8_split(const double *src, long lds, int R, int K, const I8Plan &p, cudaStream_t st);
-// the cut with the rows' maxima of |src| given in rmax (R entries); clear
-// (R entries, may be null) is zeroed for the next producer's maxima
+// box_rows: 128 for the A operand (one slice per copy), the output tile width
+// (64, 48, 32 or 16; all slices in one copy) for B
+int i8_plan(I8Plan &p, int rows, int K, int box_rows, int slices = kI8S);
+// digits of the column-major source A(r, k) = src[k * lds + r], r < R, k < K,
+// with the rows' maxima of |src| given in rmax (R entries); clear (R entries,
+// may be null) is zeroed for the next producer's maxima
 void launch_i8_cut_rows(const double *src, long lds, int R, int K, const I8Plan &p, const double *rmax,
                         double *clear, cudaStream_t st);
 // rmax[r] = max(rmax[r], max_k |src(r, k)|); rmax must start at zero

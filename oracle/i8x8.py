@@ -12,6 +12,10 @@ a = sum_i d_i 128^-(i+1); C = A B^T is then
     G_t = sum_{i+j=t} D_i E_j^T   (exact integer products, t < S),
 the G_t added in FP64 from t = S-1 down to 0, then the two power-of-two
 scales applied.
+
+The time step's transforms use S7 = 7 balanced digits of 8 bits instead
+(``balanced_digits``, ``gemm_balanced``): a 2^-e rounded to 55 bits,
+a = sum_i d_i 2^-(8 i + 7) with -128 <= d_i <= 127, and weights 2^-(8 t + 14).
 """
 from __future__ import annotations
 
@@ -45,4 +49,33 @@ def gemm(A: np.ndarray, B: np.ndarray, s: int = S) -> np.ndarray:
     for t in range(s - 1, -1, -1):
         G = sum(Da[i] @ Db[t - i].T for i in range(t + 1))
         acc = acc + G.astype(np.float64) * np.ldexp(1.0, -7 * (t + 2))
+    return (acc * np.ldexp(1.0, ea)[:, None]) * np.ldexp(1.0, eb)[None, :]
+
+
+S7 = 7
+
+
+def balanced_digits(X: np.ndarray):
+    """Row exponents e (|X[r]| <= 0.994 2^e[r]; 0 for a zero row) and the 7
+    balanced base-256 digit planes of rint(X 2^(55 - e))."""
+    X = np.asarray(X, dtype=np.float64)
+    m, e = np.frexp(np.abs(X).max(axis=1))
+    e = np.where(m > 0, e, 0).astype(np.int64) + (m > 0.994)
+    v = np.rint((X * np.ldexp(1.0, -e)[:, None]) * 2.0 ** 55).astype(np.int64)
+    bias = 0x0000808080808080          # 128 in each of the six lower digits
+    u = v + bias
+    return e, [u >> 48] + [((u >> (48 - 8 * i)) & 255) - 128 for i in range(1, S7)]
+
+
+def gemm_balanced(A: np.ndarray, B: np.ndarray) -> np.ndarray:
+    """C = A @ B.T as the time step's transforms compute it (same operations,
+    same order)."""
+    ea, Da = balanced_digits(A)
+    eb, Db = balanced_digits(B)
+    Da = [d.astype(np.float64) for d in Da]   # products and sums below 2^31: exact
+    Db = [d.astype(np.float64) for d in Db]
+    acc = np.zeros((A.shape[0], B.shape[0]), dtype=np.float64)
+    for t in range(S7 - 1, -1, -1):
+        G = sum(Da[i] @ Db[t - i].T for i in range(t + 1))
+        acc = acc + G * np.ldexp(1.0, -(8 * t + 14))
     return (acc * np.ldexp(1.0, ea)[:, None]) * np.ldexp(1.0, eb)[None, :]
