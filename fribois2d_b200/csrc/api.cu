@@ -930,7 +930,7 @@ int stage_impl(fb_ctx *c, int stage, int ns, int n) {
             fb::launch_mls_setup(d, st);
             fb::launch_spread_chains(d, st);
         }
-        fb::launch_mls_interp(d, st);
+        fb::launch_mls_interp(d, st, n == 1);
         fb::launch_mls_spread(d, st);
         break;
     case FB_ST_HELSOLVE:
@@ -1018,64 +1018,58 @@ int enqueue_fluid(fb_ctx *c, int ns) {
     const Dev &d = c->d;
     int r;
     if (c->vardt && (r = vardt_update(c, ns))) return r;
-    // The marker set-up of substep 1 (lgrdistribution, MLS weights) reads
-    // only marker data: it runs on a side branch while cfl, boucdq and the
+    // The marker set-up of substep 1 (nearest nodes, MLS weights, spreading
+    // chains) reads only marker data: it runs on a side branch while the
     // explicit terms run on the main stream.
     if (d.nlm) {
         CK(cudaEventRecord(c->ev_fork, c->stream));
         CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-        c->own_launches += 3;
-        fb::launch_lgrdist(d, c->side);
-        fb::launch_mls_setup(d, c->side);
+        c->own_launches += 2;
+        fb::launch_mls_setup(d, c->side, true);
         fb::launch_spread_chains(d, c->side);
         CK(cudaGetLastError());
         CK(cudaEventRecord(c->ev_join, c->side));
     }
-    if (!c->vardt && (r = stage_impl(c, FB_ST_CFL, ns, 1))) return r;
     c->beta = c->dt / c->hc.grid.ren * 0.5;
+    // boucdq and (fixed dt) cfl share nl_rhs's launch, boucqt and the CFL
+    // check divg's: a substep is a chain of launches that each wait for the
+    // one before, and these four depend on no step of it between those two.
     // RK3: pr_submean of substeps 1 and 2 is deferred; nl_rhs and updvp of
     // the next substep subtract the mean as they read pr, and the mean is
     // kept for the entries updvp does not rewrite, which the last pr_submean
-    // brings up to date.  boucqt and the next boucdq share one launch.
+    // brings up to date.
     const bool defer = (d.nsst == 3);
     for (int n = 1; n <= d.nsst; ++n) {
-        const bool pend = defer && n > 1;
+        const bool pend = defer && n > 1, cfl = (n == 1 && !c->vardt);
         double al, ga, ro;
         coefs(c, ns, n, al, ga, ro);
-        if (!pend && (r = stage_impl(c, FB_ST_BOUCDQ, ns, n))) return r;
-        if (pend) {
-            fb::launch_nl_rhs(d, al, ga, ro, c->stream, true, &c->nlmaps);
-            c->own_launches += 1;
-        } else if ((r = stage_impl(c, FB_ST_NL_RHS, ns, n))) {
-            return r;
-        }
+        c->al = al;
+        c->ga = ga;
+        c->ro = ro;
+        fb::launch_nl_rhs(d, al, ga, ro, c->stream, pend, &c->nlmaps, fb::kNlBoucdq | (cfl ? fb::kNlCfl : 0));
+        c->own_launches += 1;
         if (d.nlm) {
             if (n == 1) CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
             // the weights are ready: interpolation and spreading only
-            if ((r = stage_impl(c, FB_ST_FORCING, ns, n == 1 ? 2 : n))) return r;
+            fb::launch_mls_interp(d, c->stream, n == 1);
+            fb::launch_mls_spread(d, c->stream);
+            c->own_launches += 2;
         }
         if ((r = stage_impl(c, FB_ST_HELSOLVE, ns, n))) return r;
-        if ((r = stage_impl(c, FB_ST_DIVG, ns, n))) return r;
+        fb::launch_divg(d, c->usdtal[n - 1], c->stream,
+                        c->poisson_mode == FB_POISSON_INT8X8 ? c->i8max : nullptr,
+                        fb::kDivBoucqt | (cfl ? fb::kDivCfl : 0));
+        c->own_launches += 1;
         if ((r = stage_impl(c, FB_ST_PHCALC, ns, n))) return r;
-        if (pend) {
-            fb::launch_updvp_prcalc(d, al, al * c->beta, c->stream, true, &c->nlmaps);
-            c->own_launches += 1;
-        } else if ((r = stage_impl(c, FB_ST_UPDVP, ns, n))) {
-            return r;
-        }
-        if (defer && n < d.nsst) {
-            double al1, ga1, ro1;
-            coefs(c, ns, n + 1, al1, ga1, ro1);
-            fb::launch_substep_mid(d, n == 1 ? fb::S_PRAVG1 : fb::S_PRAVG2, ga1, ro1, c->stream);
-            c->own_launches += 1;
-        } else if (defer) {
-            fb::launch_submean_boucqt(d, c->stream, true);
-            c->own_launches += 1;
-        } else if ((r = stage_impl(c, FB_ST_PRSUBMEAN, ns, n))) {
-            return r;
-        }
+        fb::launch_updvp_prcalc(d, al, al * c->beta, c->stream, pend, &c->nlmaps,
+                                !defer || n == 3 ? -1 : n == 1 ? fb::S_PRAVG1 : fb::S_PRAVG2);
+        c->own_launches += 1;
         CK(cudaGetLastError());
     }
+    // (Adams-Bashforth: the two other means are zero and stay so)
+    fb::launch_submean_boucqt(d, c->stream, true);
+    c->own_launches += 1;
+    CK(cudaGetLastError());
     if (d.nlm && c->hc.deck.cbody && (r = stage_impl(c, FB_ST_LOADS, ns, 1))) return r;
     return FB_OK;
 }
@@ -2517,22 +2511,16 @@ int enqueue_group_fluid(BatchGroup *bg, int &k) {
     CK(cudaEventRecord(bg->fork, st));
     CK(cudaStreamWaitEvent(bg->side, bg->fork, 0));
     fb::glaunch_marker_setup(g, bg->side);
-    k += 3;
+    k += 2;
     CK(cudaEventRecord(bg->join, bg->side));
-    fb::glaunch_cfl(g, st);
-    k += 1;
     const double one = 1.0, zero = 0.0;
     double **p = bg->ptr;
-    for (int s = 0; s < 3; ++s) {   // pr_submean deferred as in enqueue_fluid
-        if (s == 0) {
-            fb::glaunch_boucdq(g, s, st);
-            k += 1;
-        }
-        fb::glaunch_nl_rhs(g, s, st, s > 0);
+    for (int s = 0; s < 3; ++s) {   // boucdq, cfl, boucqt and pr_submean as in enqueue_fluid
+        fb::glaunch_nl_rhs(g, s, st, s > 0, fb::kNlBoucdq | (s == 0 ? fb::kNlCfl : 0));
         if (s == 0) CK(cudaStreamWaitEvent(st, bg->join, 0));
-        fb::glaunch_forcing(g, st);
+        fb::glaunch_forcing(g, s, st);
         fb::glaunch_win_helsolve(g, s, st);
-        fb::glaunch_divg(g, s, st);
+        fb::glaunch_divg(g, s, st, fb::kDivBoucqt | (s == 0 ? fb::kDivCfl : 0));
         if (bg->tf32) {   // phcalc_tf32's launches, each over the whole group
             fb::launch_split_t_group(bg->sp, d.n2m, d.n3m, n, st);
             fb::launch_tf32x3_group(bg->gt, bg->plan_fwd, n, st);
@@ -2563,11 +2551,11 @@ int enqueue_group_fluid(BatchGroup *bg, int &k) {
                                   p + 4 * n, d.n3m, &zero, p + 5 * n, d.P, n));
             k += 1;
         }
-        fb::glaunch_updvp_prcalc(g, s, st, s > 0);
-        if (s < 2) fb::glaunch_substep_mid(g, s + 1, s == 0 ? fb::S_PRAVG1 : fb::S_PRAVG2, st);
-        else fb::glaunch_submean_boucqt(g, st, true);
-        k += 7;
+        fb::glaunch_updvp_prcalc(g, s, st, s > 0, s == 0 ? fb::S_PRAVG1 : s == 1 ? fb::S_PRAVG2 : -1);
+        k += 6;
     }
+    fb::glaunch_submean_boucqt(g, st, true);
+    k += 1;
     if (bg->cbody) {
         fb::glaunch_loads(g, st);
         k += 2;

@@ -186,16 +186,19 @@ __global__ void __launch_bounds__(256) k_cfl(Dev d) {
 
 // ------------------------------------------------------------ boundaries
 
-// iobcs.F90:5-77 (boucdq): radiative outflow increments + mass-flux correction
+// iobcs.F90:5-77 (boucdq): radiative outflow increments + mass-flux correction;
+// one block.  In the fused step it is a block of nl_rhs's launch: nl_rhs reads
+// the boundary values qb*, not their increments, which only helsolve needs.
 __device__ __forceinline__ void boucdq_body(const Dev &d, double ga, double ro) {
     __shared__ double sh[32];
     const int n3 = d.n3, n3m = d.n3m;
+    const int t = threadIdx.x + blockDim.x * threadIdx.y, nt = blockDim.x * blockDim.y;
     double qout = 0.0;
-    for (int j = threadIdx.x + 1; j <= d.n2; j += blockDim.x) {
+    for (int j = t + 1; j <= d.n2; j += nt) {
         d.dqb2s[j] = 0.0;
         d.dqb3s[j] = 0.0;
     }
-    for (int j = threadIdx.x + 1; j <= d.n2m; j += blockDim.x) {
+    for (int j = t + 1; j <= d.n2m; j += nt) {
         double dq2x2 = (d.qb2n[j] - Fv(d.q2, j, n3m)) * 2.0 * d.udx3c[n3];
         double dqb2n = -d.dt * (ga * dq2x2 + ro * d.dq2x2o[j]) * d.cou;
         double dq3x2 = (d.qb3n[j] - Fv(d.q3, j, n3m)) * d.udx3c[n3];
@@ -209,7 +212,7 @@ __device__ __forceinline__ void boucdq_body(const Dev &d, double ga, double ro) 
     double q = block_reduce_fast<false>(qout, sh);
     const double cor = (0.0 - q) / d.area_out;
     __syncthreads();
-    for (int j = threadIdx.x + 1; j <= d.n2m; j += blockDim.x) d.dqb3n[j] = d.dqb3n[j] + cor;
+    for (int j = t + 1; j <= d.n2m; j += nt) d.dqb3n[j] = d.dqb3n[j] + cor;
 }
 
 __global__ void __launch_bounds__(1024) k_boucdq(Dev d, double ga, double ro) {
@@ -371,6 +374,51 @@ __device__ __forceinline__ void nl_cell(const Dev &d, const Tile &t, int j0, int
 #undef S3
 #undef SP
 
+// cfl.F90 (fluid_tsch.F90:211-258) for one cell of a staged tile: the CFL sum
+// into mx and w times the cell's area (dz x dy) into sm, as cfl_body forms them
+template <int kC0, class Tile>
+__device__ __forceinline__ void cfl_cell(const Tile &t, int cj, int ck, double dz, double dy, double &mx, double &sm) {
+    const double a2 = t.q2[ck + 1][cj + kC0], b2 = t.q2[ck + 1][cj + 1 + kC0];
+    const double a3 = t.q3[ck + 1][cj + kC0], b3 = t.q3[ck + 2][cj + kC0];
+    const double q = fabs((a2 + b2) * 0.5 * t.udx2m[cj]) + fabs((a3 + b3) * 0.5 * t.udx3m[ck]);
+    mx = fmax(mx, (q == q) ? q : INFINITY);   // a NaN velocity reads as +inf
+    sm = sm + a3 * dz * dy;
+}
+
+// the block partials of nl_rhs's CFL number and mean w, combined by the last
+// of the nb tile blocks into S_CFLNEXT and S_Q3NEXT (divg of the substep makes
+// them the step's).  The partials lie in updvp's reduction slot, past its own.
+__device__ __forceinline__ void cfl_finish(const Dev &d, double mx, double sm, int nb) {
+    __shared__ double sh[32];
+    __shared__ bool last;
+    const int t = threadIdx.x + blockDim.x * threadIdx.y, nt = blockDim.x * blockDim.y;
+    double *rm = d.red + 2 * static_cast<size_t>(kRedSlot) + kRedSlot / 2, *rs = rm + kRedSlot / 4;
+    mx = block_reduce_fast<true>(mx, sh);
+    sm = block_reduce_fast<false>(sm, sh);
+    if (t == 0) {
+        rm[blockIdx.x] = mx;
+        rs[blockIdx.x] = sm;
+        __threadfence();
+        last = (atomicAdd(d.count, 1u) == static_cast<unsigned>(nb - 1));
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    mx = 1.0e-8;
+    sm = 0.0;
+    for (int i = t; i < nb; i += nt) {
+        mx = fmax(mx, __ldcg(rm + i));
+        sm = sm + __ldcg(rs + i);
+    }
+    mx = block_reduce_fast<true>(mx, sh);
+    sm = block_reduce_fast<false>(sm, sh);
+    if (t == 0) {
+        d.count[0] = 0u;
+        d.scal[S_CFLNEXT] = mx;
+        d.scal[S_Q3NEXT] = sm / (d.rext2 * d.alx3);
+    }
+}
+
 // the tile's coefficient vectors (cp.async), and the commit of the thread's
 // cp.async group
 template <class Tile>
@@ -440,9 +488,12 @@ __device__ __forceinline__ void nl_ru(const Dev &d, int tile, int ntj, double ro
 // pend: the previous substep's pressure mean (scal[S_PRAVG]) is still to be
 // subtracted from pr (the fused step defers pr_submean of RK3 substeps 1 and
 // 2): the staged tile gets pr - pravg, the value pr_submean would have stored.
-__device__ __forceinline__ void nl_rhs_body(const Dev &d, double al, double ga, double ro, NlTile *buf,
-                                            bool pend = false) {
+// nb: the launch's tile blocks.  kCfl: also the field's CFL number and mean w.
+template <bool kCfl>
+__device__ __forceinline__ void nl_rhs_body(const Dev &d, double al, double ga, double ro, NlTile *buf, bool pend,
+                                            int nb) {
     const double pravg = pend ? d.scal[S_PRAVG] : 0.0;
+    double cmx = 1.0e-8, csm = 0.0;
     const int ntj = (d.n2m + kNlJ - 1) / kNlJ, ntk = (d.n3m + kNlK - 1) / kNlK, ntiles = ntj * ntk;
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;
     int tile = blockIdx.x;
@@ -450,7 +501,7 @@ __device__ __forceinline__ void nl_rhs_body(const Dev &d, double al, double ga, 
     nl_prefetch(d, buf[0], tile, ntj, tid);
     double r2n[kNlK / 8], r3n[kNlK / 8];
     nl_ru(d, tile, ntj, ro, r2n, r3n);
-    for (int it = 0; tile < ntiles; ++it, tile += gridDim.x) {
+    for (int it = 0; tile < ntiles; ++it, tile += nb) {
         const NlTile &t = buf[it & 1];
         double r2[kNlK / 8], r3[kNlK / 8];
 #pragma unroll
@@ -458,7 +509,7 @@ __device__ __forceinline__ void nl_rhs_body(const Dev &d, double al, double ga, 
             r2[i] = r2n[i];
             r3[i] = r3n[i];
         }
-        const int nxt = tile + gridDim.x;
+        const int nxt = tile + nb;
         if (nxt < ntiles) {
             nl_prefetch(d, buf[(it + 1) & 1], nxt, ntj, tid);
             nl_ru(d, nxt, ntj, ro, r2n, r3n);
@@ -478,21 +529,24 @@ __device__ __forceinline__ void nl_rhs_body(const Dev &d, double al, double ga, 
         const int j0 = 1 + (tile % ntj) * kNlJ, k0 = 1 + (tile / ntj) * kNlK;
         const int jc = j0 + threadIdx.x;
         if (jc <= d.n2m) {
+            const double dy = kCfl ? d.rc[jc + 1] - d.rc[jc] : 0.0;
 #pragma unroll
             for (int i = 0; i < kNlK / 8; ++i) {
                 const int kc = k0 + (kNlK / 8) * threadIdx.y + i;
                 if (kc > d.n3m) break;
                 nl_cell<1>(d, t, j0, k0, jc, kc, al, ga, ro, r2[i], r3[i]);
+                if (kCfl) cfl_cell<1>(t, jc - j0, kc - k0, d.zz[kc + 1] - d.zz[kc], dy, cmx, csm);
             }
         }
         __syncthreads();   // this buffer is refilled two tiles on
     }
+    if (kCfl) cfl_finish(d, cmx, csm, nb);
 }
 
 __global__ void __launch_bounds__(256, kNlBlocksPerSM) k_nl_rhs(Dev d, double al, double ga, double ro, int pend) {
     extern __shared__ __align__(16) unsigned char nl_smem[];
     FB_GRID_WAIT();
-    nl_rhs_body(d, al, ga, ro, reinterpret_cast<NlTile *>(nl_smem), pend != 0);
+    nl_rhs_body<false>(d, al, ga, ro, reinterpret_cast<NlTile *>(nl_smem), pend != 0, gridDim.x);
 }
 
 // the three field boxes of a tile, issued by one thread on the buffer's
@@ -514,9 +568,11 @@ __device__ __forceinline__ void nl_issue_tma(const NlMaps &m, NlTileT &t, uint32
 // it / 2 of its buffer's mbarrier; the coefficient vectors stay cp.async.  A
 // wait that gives up (one second) records FB_ERR_TIMEOUT and ends the block's
 // tiles.
+template <bool kCfl>
 __device__ __forceinline__ void nl_rhs_tma_body(const Dev &d, const NlMaps &m, double al, double ga, double ro,
-                                                NlTileT *buf, uint64_t *bars, bool pend) {
+                                                NlTileT *buf, uint64_t *bars, bool pend, int nb) {
     const double pravg = pend ? d.scal[S_PRAVG] : 0.0;
+    double cmx = 1.0e-8, csm = 0.0;
     const int ntj = (d.n2m + kNlJ - 1) / kNlJ, ntk = (d.n3m + kNlK - 1) / kNlK, ntiles = ntj * ntk;
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;
     int tile = blockIdx.x;
@@ -535,7 +591,7 @@ __device__ __forceinline__ void nl_rhs_tma_body(const Dev &d, const NlMaps &m, d
     double r2n[kNlK / 8], r3n[kNlK / 8];
     nl_ru(d, tile, ntj, ro, r2n, r3n);
     __syncthreads();   // the barriers are initialised before any thread waits on them
-    for (int it = 0; tile < ntiles; ++it, tile += gridDim.x) {
+    for (int it = 0; tile < ntiles; ++it, tile += nb) {
         NlTileT &t = buf[it & 1];
         double r2[kNlK / 8], r3[kNlK / 8];
 #pragma unroll
@@ -543,7 +599,7 @@ __device__ __forceinline__ void nl_rhs_tma_body(const Dev &d, const NlMaps &m, d
             r2[i] = r2n[i];
             r3[i] = r3n[i];
         }
-        const int nxt = tile + gridDim.x;
+        const int nxt = tile + nb;
         if (nxt < ntiles) {
             if (tid == 0) nl_issue_tma(m, buf[(it + 1) & 1], (it & 1) ? bar0 : bar1, nxt, ntj);
             nl_prefetch_coef(d, buf[(it + 1) & 1], 1 + (nxt % ntj) * kNlJ, 1 + (nxt / ntj) * kNlK, tid);
@@ -555,7 +611,7 @@ __device__ __forceinline__ void nl_rhs_tma_body(const Dev &d, const NlMaps &m, d
         const bool landed = mbar_wait((it & 1) ? bar1 : bar0, static_cast<uint32_t>(it >> 1) & 1u);
         if (__syncthreads_or(!landed)) {
             if (tid == 0) atomicCAS(d.status, 0, FB_ERR_TIMEOUT);
-            return;
+            break;
         }
         if (pend) {
             for (int e = tid; e < kNlTH * kNlTW; e += 256) {
@@ -567,27 +623,40 @@ __device__ __forceinline__ void nl_rhs_tma_body(const Dev &d, const NlMaps &m, d
         const int j0 = 1 + (tile % ntj) * kNlJ, k0 = 1 + (tile / ntj) * kNlK;
         const int jc = j0 + threadIdx.x;
         if (jc <= d.n2m) {
+            const double dy = kCfl ? d.rc[jc + 1] - d.rc[jc] : 0.0;
 #pragma unroll
             for (int i = 0; i < kNlK / 8; ++i) {
                 const int kc = k0 + (kNlK / 8) * threadIdx.y + i;
                 if (kc > d.n3m) break;
                 nl_cell<2>(d, t, j0, k0, jc, kc, al, ga, ro, r2[i], r3[i]);
+                if (kCfl) cfl_cell<2>(t, jc - j0, kc - k0, d.zz[kc + 1] - d.zz[kc], dy, cmx, csm);
             }
         }
         __syncthreads();   // this buffer is refilled two tiles on
     }
+    if (kCfl) cfl_finish(d, cmx, csm, nb);
 }
 
+// extra (kernels.h): with kNlBoucdq the grid has one block more than the tiles
+template <bool kCfl>
 __global__ void __launch_bounds__(256, kNlBlocksPerSM)
     k_nl_rhs_tma(const __grid_constant__ Dev d, const __grid_constant__ NlMaps m, double al, double ga, double ro,
-                 int pend) {
+                 int pend, int extra) {
     extern __shared__ __align__(16) unsigned char nl_smem[];
     const uint32_t raw = smem_u32(nl_smem);
     unsigned char *base = nl_smem + ((128u - (raw & 127u)) & 127u);   // the tiles on 128-byte boundaries
     NlTileT *buf = reinterpret_cast<NlTileT *>(base);
     uint64_t *bars = reinterpret_cast<uint64_t *>(base + 2 * sizeof(NlTileT));
     FB_GRID_WAIT();
-    nl_rhs_tma_body(d, m, al, ga, ro, buf, bars, pend != 0);
+    int nb = gridDim.x;
+    if (extra & kNlBoucdq) {
+        --nb;
+        if (static_cast<int>(blockIdx.x) == nb) {
+            boucdq_body(d, ga, ro);
+            return;
+        }
+    }
+    nl_rhs_tma_body<kCfl>(d, m, al, ga, ro, buf, bars, pend != 0, nb);
 }
 
 // ------------------------------------------------------------ MLS forcing
@@ -821,6 +890,11 @@ __device__ __forceinline__ void sd_axes(const Dev &d, int idir, const double *&y
 // Marker set-up at substep 1: MLS_SD_ind + MLS_SF + momentum coefficient cl
 // (forcing_MLS.F90:57-94, MLSint.F90:115-166, compute_AB :284-338), and the
 // spreading keys.  One (marker, direction) per group of kNodeLanes lanes.
+// kFind: the group also finds its nearest y and z lines
+// (lgrdistribution.F90:189-267), one per lane, in place of a launch of its own
+// whose threads made the four searches of a marker one after another; the
+// spreading table is empty then (k_mls_interp empties it behind the chains).
+template <bool kFind>
 __device__ __forceinline__ void mls_setup_body(const Dev &d) {
     if (!d.nlm) return;
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
@@ -837,7 +911,34 @@ __device__ __forceinline__ void mls_setup_body(const Dev &d) {
     const bool stopped = __shfl_sync(0xffffffffu, static_cast<int>(*d.status != 0), base) != 0;
     const double pos[2] = {d.lmcc[2 * n], d.lmcc[2 * n + 1]};
     const bool ok = have && !stopped && (d.zz[1] < pos[1] && pos[1] < d.zz[d.n3]);
-    const int i0 = d.lmind[4 * n + 2 * (idir - 1)], k0 = d.lmind[4 * n + 2 * (idir - 1) + 1];
+    int *lmi = d.lmind + 4 * n + 2 * (idir - 1);   // nearest y line, nearest z line
+    int i0, k0;
+    if constexpr (kFind) {
+        int ind = -1;
+        if (have && m < 2) {
+            const double x = pos[m], far = (m == 0) ? d.rext2 : d.alx3;
+            const bool out = pos[0] > d.rext2 || pos[0] < 0.0 || pos[1] > d.alx3 || pos[1] < 0.0 ||
+                             !(pos[0] == pos[0]) || !(pos[1] == pos[1]);
+            if (out) {
+                if (m == 0) raise_status(d, FB_ERR_MARKER_OUT);
+            } else {
+                // cell-centred lines (zm of v, rm of w) keep a marker beyond
+                // their first or last one
+                const bool centred = (m == 1) == (idir == 1);
+                const double *a = (m == 0) ? (centred ? d.rm : d.rc) : (centred ? d.zm : d.zz);
+                const int hi = (m == 0) ? d.n2 : d.n3, mid = hi - 1;
+                if (centred && x < a[1] && x > 0.0) ind = 1;
+                else if (centred && x > a[mid] && x < far) ind = mid;
+                else ind = nearest_sorted(a, 1, hi, x, lmi[m]);
+            }
+            lmi[m] = ind;
+        }
+        i0 = __shfl_sync(0xffffffffu, ind, base);
+        k0 = __shfl_sync(0xffffffffu, ind, base + 1);
+    } else {
+        i0 = lmi[0];
+        k0 = lmi[1];
+    }
     // MLS_SD_ind: node m = 3 (j - 1) + (k - 1) of the 3 x 3 support, moved
     // inside the field
     const double *y, *z;
@@ -914,9 +1015,10 @@ __device__ __forceinline__ void mls_setup_body(const Dev &d) {
     raise_status(d, FB_ERR_UNSUPPORTED);   // more than kBucket x kBucketLevels boxes start in one cell
 }
 
+template <bool kFind>
 __global__ void k_mls_setup(Dev d) {
     FB_GRID_WAIT();
-    mls_setup_body(d);
+    mls_setup_body<kFind>(d);
 }
 
 // interp_spread (forcing_MLS.F90:135-182), interpolation half: the
@@ -925,13 +1027,24 @@ __global__ void k_mls_setup(Dev d) {
 // One (marker, direction) per 16 lanes, node m on lane m < kSD: the nine
 // support loads are independent, and each lane forms the sum of the nine
 // products in node order from the group's shuffles (the sequential sum).
+// clear (substep 1): the spreading table, read for the last time by
+// k_spread_chains, is emptied for the next step (every used entry is some
+// marker's own).
 constexpr int kInterpLanes = 16;
-__device__ __forceinline__ void mls_interp_body(const Dev &d) {
+__device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = T / kInterpLanes, m = T % kInterpLanes, lane = threadIdx.x & 31;
     const bool have = t < 2 * d.nlm;
     const bool stopped = (*d.status != 0);
     const int tt = have ? t : 0;
+    if (clear && have && m == kInterpLanes - 1) {   // (a lane without a node)
+        const int e = d.hslot[tt];
+        if (e) {
+            d.hkey[e - 1] = 0ull;
+            d.hcnt[e - 1] = 0;
+            d.hslot[tt] = 0;
+        }
+    }
     const int n = tt >> 1, idir = (tt & 1) + 1;
     const double pos2 = d.lmcc[2 * n + 1];
     const bool inside = (d.zz[1] < pos2 && pos2 < d.zz[d.n3]);
@@ -966,9 +1079,9 @@ __device__ __forceinline__ void mls_interp_body(const Dev &d) {
     c[m] = d.cl[tt] * phim * f;
 }
 
-__global__ void k_mls_interp(Dev d) {
+__global__ void k_mls_interp(Dev d, int clear) {
     FB_GRID_WAIT();
-    mls_interp_body(d);
+    mls_interp_body(d, clear != 0);
 }
 
 // interp_spread, spreading half, without atomics on the field.  Once per
@@ -978,20 +1091,12 @@ __global__ void k_mls_interp(Dev d) {
 // forcing_MLS.F90:51-104); the head of each chain is the lowest-index
 // toucher.  Every substep the heads then add their chain's sum fe*dt to rhs
 // (helsolve.F90:22,47).
-__device__ __forceinline__ void spread_chains_body(const Dev &d) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= 2 * d.nlm * kSD) return;
-    d.chead[g] = 0;
-    if (*d.status) return;
+// one slot's chain by one thread: dense marker clusters (more touchers than a
+// group's list holds, or cells with more than one table entry)
+__device__ __noinline__ void spread_chain_serial(const Dev &d, int g) {
     const int t = g / kSD, m = g % kSD, n = t >> 1, dir = t & 1;
-    const double pos2 = d.lmcc[2 * n + 1];
-    if (!(d.zz[1] < pos2 && pos2 < d.zz[d.n3])) return;
     const int *eu = d.eulins + static_cast<size_t>(t) * 2 * kSD;
     const int j = eu[m], k = eu[kSD + m];
-    // cells helsolve reads: v at j = 2..n2m, k = 1..n3m; w at j = 1..n2m, k = 2..n3m
-    const bool used = (dir == 0) ? (j >= 2 && j <= d.n2m && k >= 1 && k <= d.n3m)
-                                 : (j >= 1 && j <= d.n2m && k >= 2 && k <= d.n3m);
-    if (!used) return;
     const size_t plane = static_cast<size_t>(dir) * d.NK * d.P;
     // the cell's touchers are the markers registered at the 3 x 3 possible
     // box start cells (table lookups); a lower-index toucher means this slot
@@ -1054,7 +1159,98 @@ __device__ __forceinline__ void spread_chains_body(const Dev &d) {
     for (int p = 0; p < kHeadList; ++p) hl[p] = (p < L) ? ls[p] : g;
 }
 
-__global__ void k_spread_chains(Dev d) {
+// A slot's cell by a group of kNodeLanes lanes: lane q < 9 looks up the box
+// start cell q (the nine dependent chains of table reads side by side, where
+// one thread's went one after another), the touchers found go to the group's
+// list in shared memory, and each is placed by its rank among them.  Under ncu
+// 23.9 -> 9.5 us with 1200 markers, 17.6 -> 6.5 us with 302.
+constexpr int kChainThreads = 256;
+constexpr int kChainList = 64;   // touchers per group's list (9 boxes of up to 7 markers)
+__device__ __forceinline__ void spread_chains_body(const Dev &d) {
+    __shared__ int lists[kChainThreads / kNodeLanes][3][kChainList];   // marker, slot, slots in order
+    constexpr unsigned kAll = 0xffffffffu;
+    const int T = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g0 = T / kNodeLanes, m = T % kNodeLanes;
+    const int base = (threadIdx.x & 31) & ~(kNodeLanes - 1);
+    const bool have = g0 < 2 * d.nlm * kSD;
+    const int g = have ? g0 : 0;
+    if (have && m == 0) d.chead[g] = 0;
+    const int t = g / kSD, n = t >> 1, dir = t & 1;
+    const double pos2 = d.lmcc[2 * n + 1];
+    const int *eu = d.eulins + static_cast<size_t>(t) * 2 * kSD;
+    const int j = eu[g % kSD], k = eu[kSD + g % kSD];
+    // cells helsolve reads: v at j = 2..n2m, k = 1..n3m; w at j = 1..n2m, k = 2..n3m
+    const bool used = (dir == 0) ? (j >= 2 && j <= d.n2m && k >= 1 && k <= d.n3m)
+                                 : (j >= 1 && j <= d.n2m && k >= 2 && k <= d.n3m);
+    const bool stopped = __shfl_sync(kAll, static_cast<int>(*d.status != 0), base) != 0;
+    const bool act = have && !stopped && used && (d.zz[1] < pos2 && pos2 < d.zz[d.n3]);
+    // the cell's touchers are the markers registered at the 3 x 3 possible
+    // box start cells
+    int cnt = 0;
+    unsigned h = 0;
+    const int sj = j - m / 3, sk = k - m % 3;
+    if (act && m < kSD && sj >= 1 && sk >= 0) {
+        const unsigned mask = (1u << d.hlog) - 1u;
+        const unsigned long long key =
+            (static_cast<unsigned long long>(dir) * d.NK * d.P + fidx(d, sj, sk)) * kBucketLevels + 1;
+        h = bucket_hash(key, d.hlog);
+        unsigned long long kh = d.hkey[h];
+        cnt = d.hcnt[h];
+        for (unsigned probes = 0; kh != key && kh != 0ull && probes < mask; ++probes) {
+            h = (h + 1) & mask;
+            kh = d.hkey[h];
+            cnt = d.hcnt[h];
+        }
+        if (kh != key) cnt = 0;   // no boxes start in this cell
+    }
+    int off = cnt;   // inclusive sums over the group's lanes
+#pragma unroll
+    for (int o = 1; o < kNodeLanes; o <<= 1) {
+        const int x = __shfl_up_sync(kAll, off, o, kNodeLanes);
+        if (m >= o) off += x;
+    }
+    const int total = __shfl_sync(kAll, off, base + kNodeLanes - 1);
+    const bool serial = !group_none(cnt > kBucket, base) || total > kChainList;
+    int(&list)[3][kChainList] = lists[threadIdx.x / kNodeLanes];
+    bool lower = false;   // a lower-index toucher: this slot is not the head
+    if (!serial)
+        for (int e = 0; e < cnt; ++e) {
+            const int nn = d.hval[static_cast<size_t>(h) * kBucket + e];
+            lower = lower || nn < n;
+            list[0][off - cnt + e] = nn;
+            list[1][off - cnt + e] = (2 * nn + dir) * kSD + m;   // node (dj, dk) = (m / 3, m % 3) of marker nn
+        }
+    const bool head = group_none(lower, base) && act;
+    __syncwarp();
+    if (head && !serial) {
+        for (int i = m; i < total; i += kNodeLanes) {
+            const int nn = list[0][i];
+            if (nn == n) continue;
+            int r = -1;   // rank among the touchers after n (n itself is lower)
+            for (int p = 0; p < total; ++p) r += (list[0][p] < nn) ? 1 : 0;
+            list[2][r] = list[1][i];
+        }
+    }
+    __syncwarp();
+    if (!head) return;
+    if (serial) {
+        if (m == 0) spread_chain_serial(d, g);
+        return;
+    }
+    // this slot heads the cell's chain: link the touchers in marker order;
+    // the head also keeps the first kHeadList of them in line
+    const int L = total - 1;
+    for (int p = m; p <= L; p += kNodeLanes) d.chain[p ? list[2][p - 1] : g] = (p < L) ? list[2][p] : -1;
+    if (m < kHeadList) d.hlist[static_cast<size_t>(g) * kHeadList + m] = (m < L) ? list[2][m] : g;
+    if (m == 0) {
+        d.hlen[g] = L;
+        d.chead[g] = 1;
+    }
+}
+
+// (a grid constant: the call of the serial form takes its address, and a copy
+// of it on every thread's stack cost more than the kernel)
+__global__ void k_spread_chains(const __grid_constant__ Dev d) {
     FB_GRID_WAIT();
     spread_chains_body(d);
 }
@@ -1201,10 +1397,39 @@ __global__ void k_tri_z3(Dev d, SubDev s) {
 // and the rows k0 + y + 8 i.  rmax (may be null): the maxima of |dph| over
 // each row j (the rows of the INT8 transform's data operand) are accumulated
 // into rmax[j - 1], one atomic per block and row, for the digit cut that follows
+// extra (kernels.h): the grid has one row of blocks more (the first, so that it
+// is not the grid's tail), whose first block
+// runs boucqt (iobcs.F90:81-108; helsolve has used the increments, and nothing
+// reads the boundary values before the next nl_rhs) and publishes the CFL number
+// with the fixed-dt check of fluid_tsch.F90:49-55.
 constexpr int kDivK = 4;
-__device__ __forceinline__ void divg_body(const Dev &d, double usdtal, double *rmax = nullptr) {
+__device__ __forceinline__ void divg_extra(const Dev &d, int extra) {
+    const int t = threadIdx.x + blockDim.x * threadIdx.y, nt = blockDim.x * blockDim.y;
+    if (extra & kDivBoucqt)
+        for (int j = t + 1; j <= d.n2m; j += nt) {
+            const double a = d.qb2s[j] + d.dqb2s[j], b = d.qb3s[j] + d.dqb3s[j];
+            const double e = d.qb2n[j] + d.dqb2n[j], f = d.qb3n[j] + d.dqb3n[j];
+            d.qb2s[j] = a;   // (every load before the first store, which could alias them)
+            d.qb3s[j] = b;
+            d.qb2n[j] = e;
+            d.qb3n[j] = f;
+        }
+    if ((extra & kDivCfl) && t == 0) {
+        const double am = d.scal[S_CFLNEXT], cflm = am * d.dt;
+        d.scal[S_CFLM] = cflm;
+        d.scal[S_CFLRAW] = am;
+        d.scal[S_Q3AVG] = d.scal[S_Q3NEXT];
+        if (!(cflm <= d.cfllim)) raise_status(d, FB_ERR_CFL);
+    }
+}
+__device__ __forceinline__ void divg_body(const Dev &d, double usdtal, double *rmax, int extra) {
+    int by = blockIdx.y;
+    if (extra && by-- == 0) {
+        if (blockIdx.x == 0) divg_extra(d, extra);
+        return;
+    }
     const int jc = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int kb = blockIdx.y * blockDim.y * kDivK + threadIdx.y + 1;
+    const int kb = by * blockDim.y * kDivK + threadIdx.y + 1;
     double m = 0.0;
     if (jc <= d.n2m) {
 #pragma unroll
@@ -1228,9 +1453,9 @@ __device__ __forceinline__ void divg_body(const Dev &d, double usdtal, double *r
     }
 }
 
-__global__ void k_divg(Dev d, double usdtal, double *rmax) {
+__global__ void k_divg(Dev d, double usdtal, double *rmax, int extra) {
     FB_GRID_WAIT();
-    divg_body(d, usdtal, rmax);
+    divg_body(d, usdtal, rmax, extra);
 }
 
 // updvp.F90:5-59 (updvp) fused with updvp.F90:68-105 (prcalc) and the
@@ -1317,7 +1542,7 @@ __device__ __forceinline__ void up_own(const Dev &d, int tile, int ntj, double (
 // a wait that gives up records FB_ERR_TIMEOUT and ends the block's tiles (the
 // block still takes part in the mean)
 template <bool kTma, class Tile>
-__device__ __forceinline__ void updvp_prcalc_body(const Dev &d, double al, double be, Tile *buf, bool pend = false,
+__device__ __forceinline__ void updvp_prcalc_body(const Dev &d, double al, double be, Tile *buf, bool pend, int slot,
                                                   const NlMaps *m = nullptr, uint64_t *bars = nullptr) {
     __shared__ double sh[32];
     __shared__ bool last;
@@ -1428,31 +1653,34 @@ __device__ __forceinline__ void updvp_prcalc_body(const Dev &d, double al, doubl
     acc = block_reduce_fast<false>(acc, sh);
     if (t == 0) {
         d.count[2] = 0u;
-        d.scal[S_PRAVG] = acc / (d.rext2 * d.alx3);
+        const double avg = acc / (d.rext2 * d.alx3);
+        d.scal[S_PRAVG] = avg;
+        if (slot >= 0) d.scal[slot] = avg;
     }
 }
 
-__global__ void __launch_bounds__(256, kUpBlocksPerSM) k_updvp_prcalc(Dev d, double al, double be, int pend) {
+__global__ void __launch_bounds__(256, kUpBlocksPerSM) k_updvp_prcalc(Dev d, double al, double be, int pend, int slot) {
     extern __shared__ __align__(16) unsigned char up_smem[];
     FB_GRID_WAIT();
-    updvp_prcalc_body<false>(d, al, be, reinterpret_cast<UpTile *>(up_smem), pend != 0);
+    updvp_prcalc_body<false>(d, al, be, reinterpret_cast<UpTile *>(up_smem), pend != 0, slot);
 }
 
 __global__ void __launch_bounds__(256, kUpBlocksPerSM)
     k_updvp_prcalc_tma(const __grid_constant__ Dev d, const __grid_constant__ NlMaps m, double al, double be,
-                       int pend) {
+                       int pend, int slot) {
     extern __shared__ __align__(16) unsigned char up_smem[];
     const uint32_t raw = smem_u32(up_smem);
     unsigned char *base = up_smem + ((128u - (raw & 127u)) & 127u);   // the tiles on 128-byte boundaries
     FB_GRID_WAIT();
-    updvp_prcalc_body<true>(d, al, be, reinterpret_cast<UpTileT *>(base), pend != 0, &m,
+    updvp_prcalc_body<true>(d, al, be, reinterpret_cast<UpTileT *>(base), pend != 0, slot, &m,
                             reinterpret_cast<uint64_t *>(base + 2 * sizeof(UpTileT)));
 }
 
 // pr_submean (updvp.F90:336: the whole array) and boucqt (iobcs.F90:97-105)
 // deferred: the means of RK3 substeps 1 and 2 were applied to the cells that
 // updvp rewrites (j <= n2m, 1 <= k <= n3m) as it read them; the other
-// entries of the array get all three subtractions here, in order.
+// entries of the array get all three subtractions here, in order.  boucqt has
+// then run with divg.
 __device__ __forceinline__ void submean_boucqt_body(const Dev &d, bool deferred = false) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int k = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1462,7 +1690,7 @@ __device__ __forceinline__ void submean_boucqt_body(const Dev &d, bool deferred 
         if (deferred && (j > d.n2m || k < 1 || k > d.n3m)) p = (p - d.scal[S_PRAVG1]) - d.scal[S_PRAVG2];
         Fv(d.pr, j, k) = p - pravg;
     }
-    if (blockIdx.y == 0 && threadIdx.y == 0 && j <= d.n2m) {
+    if (!deferred && blockIdx.y == 0 && threadIdx.y == 0 && j <= d.n2m) {
         d.qb2s[j] = d.qb2s[j] + d.dqb2s[j];
         d.qb3s[j] = d.qb3s[j] + d.dqb3s[j];
         d.qb2n[j] = d.qb2n[j] + d.dqb2n[j];
@@ -1473,27 +1701,6 @@ __device__ __forceinline__ void submean_boucqt_body(const Dev &d, bool deferred 
 __global__ void k_submean_boucqt(Dev d, int deferred) {
     FB_GRID_WAIT();
     submean_boucqt_body(d, deferred != 0);
-}
-
-// The end of RK3 substep 1 or 2 in the fused step: boucqt (iobcs.F90:97-105),
-// the substep's pressure mean kept in slot for the final pr_submean, then
-// boucdq of the next substep (iobcs.F90:5-77) in the same block.  The mean
-// itself is subtracted by the next nl_rhs and updvp as they read pr.
-__device__ __forceinline__ void substep_mid_body(const Dev &d, int slot, double ga, double ro) {
-    for (int j = threadIdx.x + 1; j <= d.n2m; j += blockDim.x) {
-        d.qb2s[j] = d.qb2s[j] + d.dqb2s[j];
-        d.qb3s[j] = d.qb3s[j] + d.dqb3s[j];
-        d.qb2n[j] = d.qb2n[j] + d.dqb2n[j];
-        d.qb3n[j] = d.qb3n[j] + d.dqb3n[j];
-    }
-    if (threadIdx.x == 0) d.scal[slot] = d.scal[S_PRAVG];
-    __syncthreads();
-    boucdq_body(d, ga, ro);
-}
-
-__global__ void __launch_bounds__(1024) k_substep_mid(Dev d, int slot, double ga, double ro) {
-    FB_GRID_WAIT();
-    substep_mid_body(d, slot, ga, ro);
 }
 
 // ------------------------------------------------------------ loads
@@ -2174,36 +2381,28 @@ __global__ void __launch_bounds__(256) k_diag(Dev d, int hist_rows) {
 // staged in shared memory from the group's device array (the single-case
 // kernels take them by value).
 
-__global__ void __launch_bounds__(256) kg_cfl(const GroupCase *__restrict__ g) {
-    __shared__ Dev d;
-    if (!stage_case(g, &d)) return;
-    cfl_body(d);
-}
-
-__global__ void __launch_bounds__(1024) kg_boucdq(const GroupCase *__restrict__ g, int n) {
-    __shared__ Dev d;
-    __shared__ SubDev s;
-    if (!stage_case(g, &d, &s, n)) return;
-    boucdq_body(d, s.ga, s.ro);
-}
-
-__global__ void __launch_bounds__(256, kNlBlocksPerSM) kg_nl_rhs(const GroupCase *__restrict__ g, int n, int pend) {
+template <bool kCfl>
+__global__ void __launch_bounds__(256, kNlBlocksPerSM) kg_nl_rhs(const GroupCase *__restrict__ g, int n, int pend,
+                                                                 int extra) {
     extern __shared__ __align__(16) unsigned char nl_smem[];
     __shared__ Dev d;
     __shared__ SubDev s;
     if (!stage_case(g, &d, &s, n)) return;
-    nl_rhs_body(d, s.al, s.ga, s.ro, reinterpret_cast<NlTile *>(nl_smem), pend != 0);
-}
-__global__ void kg_lgrdist(const GroupCase *__restrict__ g) {
-    __shared__ Dev d;
-    if (!stage_case(g, &d)) return;
-    lgrdist_body(d);
+    int nb = gridDim.x;
+    if (extra & kNlBoucdq) {
+        --nb;
+        if (static_cast<int>(blockIdx.x) == nb) {
+            boucdq_body(d, s.ga, s.ro);
+            return;
+        }
+    }
+    nl_rhs_body<kCfl>(d, s.al, s.ga, s.ro, reinterpret_cast<NlTile *>(nl_smem), pend != 0, nb);
 }
 
 __global__ void kg_mls_setup(const GroupCase *__restrict__ g) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    mls_setup_body(d);
+    mls_setup_body<true>(d);
 }
 
 __global__ void kg_spread_chains(const GroupCase *__restrict__ g) {
@@ -2212,10 +2411,10 @@ __global__ void kg_spread_chains(const GroupCase *__restrict__ g) {
     spread_chains_body(d);
 }
 
-__global__ void kg_mls_interp(const GroupCase *__restrict__ g) {
+__global__ void kg_mls_interp(const GroupCase *__restrict__ g, int clear) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    mls_interp_body(d);
+    mls_interp_body(d, clear != 0);
 }
 
 __global__ void kg_mls_spread(const GroupCase *__restrict__ g) {
@@ -2224,34 +2423,26 @@ __global__ void kg_mls_spread(const GroupCase *__restrict__ g) {
     mls_spread_body(d);
 }
 
-__global__ void kg_divg(const GroupCase *__restrict__ g, int n) {
+__global__ void kg_divg(const GroupCase *__restrict__ g, int n, int extra) {
     __shared__ Dev d;
     __shared__ SubDev s;
     if (!stage_case(g, &d, &s, n)) return;
-    divg_body(d, s.usdtal);
+    divg_body(d, s.usdtal, nullptr, extra);
 }
 
 __global__ void __launch_bounds__(256, kUpBlocksPerSM) kg_updvp_prcalc(const GroupCase *__restrict__ g, int n,
-                                                                       int pend) {
+                                                                       int pend, int slot) {
     extern __shared__ __align__(16) unsigned char up_smem[];
     __shared__ Dev d;
     __shared__ SubDev s;
     if (!stage_case(g, &d, &s, n)) return;
-    updvp_prcalc_body<false>(d, s.al, s.al * s.beta, reinterpret_cast<UpTile *>(up_smem), pend != 0);
+    updvp_prcalc_body<false>(d, s.al, s.al * s.beta, reinterpret_cast<UpTile *>(up_smem), pend != 0, slot);
 }
 
 __global__ void kg_submean_boucqt(const GroupCase *__restrict__ g, int deferred) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
     submean_boucqt_body(d, deferred != 0);
-}
-
-// n: the next substep (0-based) whose boucdq runs here
-__global__ void __launch_bounds__(1024) kg_substep_mid(const GroupCase *__restrict__ g, int n, int slot) {
-    __shared__ Dev d;
-    __shared__ SubDev s;
-    if (!stage_case(g, &d, &s, n)) return;
-    substep_mid_body(d, slot, s.ga, s.ro);
 }
 
 __global__ void __launch_bounds__(kLoadThreads, 5) kg_loads_probe(const GroupCase *__restrict__ g) {
@@ -2304,10 +2495,15 @@ void launch_cfl(const Dev &d, cudaStream_t s) { pdl(k_cfl, dim3(std::min(d.n3m, 
 void launch_boucdq(const Dev &d, double ga, double ro, cudaStream_t s) { pdl(k_boucdq, dim3(1), dim3(1024), 0, s, d, ga, ro); }
 int nl_tiles(const Dev &d) { return ((d.n2m + kNlJ - 1) / kNlJ) * ((d.n3m + kNlK - 1) / kNlK); }
 
-void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend, const NlMaps *maps) {
-    const int blocks = std::min(nl_tiles(d), 148 * kNlBlocksPerSM);
-    if (maps) pdl(k_nl_rhs_tma, dim3(blocks), dim3(32, 8), kNlSmemT, s, d, *maps, al, ga, ro, pend ? 1 : 0);
-    else pdl(k_nl_rhs, dim3(blocks), dim3(32, 8), kNlSmem, s, d, al, ga, ro, pend ? 1 : 0);
+void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend, const NlMaps *maps,
+                   int extra) {
+    const int more = (extra & kNlBoucdq) ? 1 : 0;
+    const int blocks = std::min(nl_tiles(d), 148 * kNlBlocksPerSM - more) + more;   // all resident at once
+    if (maps)
+        pdl((extra & kNlCfl) ? k_nl_rhs_tma<true> : k_nl_rhs_tma<false>, dim3(blocks), dim3(32, 8), kNlSmemT, s, d,
+            *maps, al, ga, ro, pend ? 1 : 0, extra);
+    else
+        pdl(k_nl_rhs, dim3(blocks), dim3(32, 8), kNlSmem, s, d, al, ga, ro, pend ? 1 : 0);
 }
 
 // q2, q3, pr, dph as 2-D FP64 tensors: x = j - 1 (j = 1 .. n2), y = k (0 .. n3),
@@ -2341,15 +2537,17 @@ int encode_nl_maps(NlMaps *m, const Dev &d) {
 void launch_lgrdist(const Dev &d, cudaStream_t s) {
     if (d.nlm) pdl(k_lgrdist, dim3((d.nlm + 127) / 128), dim3(128), 0, s, d);
 }
-void launch_mls_setup(const Dev &d, cudaStream_t s) {
-    if (d.nlm) pdl(k_mls_setup, dim3((2 * d.nlm * kNodeLanes + 255) / 256), dim3(256), 0, s, d);
+void launch_mls_setup(const Dev &d, cudaStream_t s, bool find) {
+    if (d.nlm) pdl(find ? k_mls_setup<true> : k_mls_setup<false>, dim3((2 * d.nlm * kNodeLanes + 255) / 256), dim3(256), 0, s, d);
 }
-void launch_mls_interp(const Dev &d, cudaStream_t s) {
-    if (d.nlm) pdl(k_mls_interp, dim3((2 * d.nlm * kInterpLanes + 255) / 256), dim3(256), 0, s, d);
+void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear) {
+    if (d.nlm) pdl(k_mls_interp, dim3((2 * d.nlm * kInterpLanes + 255) / 256), dim3(256), 0, s, d, clear ? 1 : 0);
 }
+namespace {
+inline int chain_blocks(int nlm) { return (2 * nlm * kSD * kNodeLanes + kChainThreads - 1) / kChainThreads; }
+}  // namespace
 void launch_spread_chains(const Dev &d, cudaStream_t s) {
-    const int n = 2 * d.nlm * kSD;
-    if (n) pdl(k_spread_chains, dim3((n + 127) / 128), dim3(128), 0, s, d);
+    if (d.nlm) pdl(k_spread_chains, dim3(chain_blocks(d.nlm)), dim3(kChainThreads), 0, s, d);
 }
 void launch_mls_spread(const Dev &d, cudaStream_t s) {
     const int n = 2 * d.nlm * kSD;
@@ -2361,21 +2559,25 @@ void launch_helsolve(const Dev &d, const SubDev &sd, cudaStream_t s) {
     pdl(k_tri_y3, dim3((d.n3m + 63) / 64), dim3(64), 0, s, d, sd);
     pdl(k_tri_z3, dim3((d.n2m + 63) / 64), dim3(64), 0, s, d, sd);
 }
-void launch_divg(const Dev &d, double usdtal, cudaStream_t s, double *rmax) {
-    dim3 b(32, 8);   // the row maxima's reduction assumes these blocks
-    pdl(k_divg, dim3(grid2(d.n2m, (d.n3m + kDivK - 1) / kDivK, b)), dim3(b), 0, s, d, usdtal, rmax);
+namespace {
+inline dim3 divg_grid(const Dev &d, int extra) {
+    dim3 g = grid2(d.n2m, (d.n3m + kDivK - 1) / kDivK, dim3(32, 8));
+    if (extra) ++g.y;
+    return g;
 }
-void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, bool pend, const NlMaps *maps) {
+}  // namespace
+void launch_divg(const Dev &d, double usdtal, cudaStream_t s, double *rmax, int extra) {
+    // (the row maxima's reduction assumes these blocks)
+    pdl(k_divg, divg_grid(d, extra), dim3(32, 8), 0, s, d, usdtal, rmax, extra);
+}
+void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, bool pend, const NlMaps *maps, int slot) {
     const int blocks = std::min(nl_tiles(d), 148 * kUpBlocksPerSM);
-    if (maps) pdl(k_updvp_prcalc_tma, dim3(blocks), dim3(32, 8), kUpSmemT, s, d, *maps, al, be, pend ? 1 : 0);
-    else pdl(k_updvp_prcalc, dim3(blocks), dim3(32, 8), kUpSmem, s, d, al, be, pend ? 1 : 0);
+    if (maps) pdl(k_updvp_prcalc_tma, dim3(blocks), dim3(32, 8), kUpSmemT, s, d, *maps, al, be, pend ? 1 : 0, slot);
+    else pdl(k_updvp_prcalc, dim3(blocks), dim3(32, 8), kUpSmem, s, d, al, be, pend ? 1 : 0, slot);
 }
 void launch_submean_boucqt(const Dev &d, cudaStream_t s, bool deferred) {
     dim3 b(32, 8);
     pdl(k_submean_boucqt, dim3(grid2(d.n2, d.n3 + 1, b)), dim3(b), 0, s, d, deferred ? 1 : 0);
-}
-void launch_substep_mid(const Dev &d, int slot, double ga, double ro, cudaStream_t s) {
-    pdl(k_substep_mid, dim3(1), dim3(1024), 0, s, d, slot, ga, ro);
 }
 void launch_loads(const Dev &d, cudaStream_t s) {
     if (!d.nlm) return;
@@ -2411,65 +2613,54 @@ namespace {
 inline dim3 zgrid(dim3 g, const Group &gr) { return dim3(g.x, g.y, static_cast<unsigned>(gr.n)); }
 }  // namespace
 
-void glaunch_cfl(const Group &g, cudaStream_t s) {
-    pdl(kg_cfl, zgrid(dim3(std::max(1, std::min(g.rep.n3m, (2 * 148 * 8 + g.n - 1) / g.n))), g), dim3(256), 0, s,
-        g.cases);
-}
-void glaunch_boucdq(const Group &g, int n, cudaStream_t s) {
-    pdl(kg_boucdq, zgrid(dim3(1), g), dim3(1024), 0, s, g.cases, n);
-}
-void glaunch_nl_rhs(const Group &g, int n, cudaStream_t s, bool pend) {
+void glaunch_nl_rhs(const Group &g, int n, cudaStream_t s, bool pend, int extra) {
     // about two waves of resident blocks over the whole group
-    const int per_case = std::max(1, std::min(nl_tiles(g.rep), (2 * 148 * kNlBlocksPerSM + g.n - 1) / g.n));
-    pdl(kg_nl_rhs, zgrid(dim3(per_case), g), dim3(32, 8), kNlSmem, s, g.cases, n, pend ? 1 : 0);
+    const int per_case = std::max(1, std::min(nl_tiles(g.rep), (2 * 148 * kNlBlocksPerSM + g.n - 1) / g.n)) +
+                         ((extra & kNlBoucdq) ? 1 : 0);
+    pdl((extra & kNlCfl) ? kg_nl_rhs<true> : kg_nl_rhs<false>, zgrid(dim3(per_case), g), dim3(32, 8), kNlSmem, s,
+        g.cases, n, pend ? 1 : 0, extra);
 }
 
 cudaError_t kernels_configure() {
-    cudaError_t e = cudaFuncSetAttribute(k_nl_rhs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(kNlSmem));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_nl_rhs_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kNlSmemT));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_updvp_prcalc_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kUpSmemT));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kg_nl_rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kNlSmem));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_updvp_prcalc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kUpSmem));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kg_updvp_prcalc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kUpSmem));
+    cudaError_t e = cudaSuccess;
+    auto allow = [&](auto kern, size_t smem) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    };
+    allow(k_nl_rhs, kNlSmem);
+    allow(k_nl_rhs_tma<false>, kNlSmemT);
+    allow(k_nl_rhs_tma<true>, kNlSmemT);
+    allow(kg_nl_rhs<false>, kNlSmem);
+    allow(kg_nl_rhs<true>, kNlSmem);
+    allow(k_updvp_prcalc, kUpSmem);
+    allow(k_updvp_prcalc_tma, kUpSmemT);
+    allow(kg_updvp_prcalc, kUpSmem);
     return e;
 }
 void glaunch_marker_setup(const Group &g, cudaStream_t s) {
     const Dev &d = g.rep;
     if (!d.nlm) return;
-    pdl(kg_lgrdist, zgrid(dim3((d.nlm + 127) / 128), g), dim3(128), 0, s, g.cases);
     pdl(kg_mls_setup, zgrid(dim3((2 * d.nlm * kNodeLanes + 255) / 256), g), dim3(256), 0, s, g.cases);
-    pdl(kg_spread_chains, zgrid(dim3((2 * d.nlm * kSD + 127) / 128), g), dim3(128), 0, s, g.cases);
+    pdl(kg_spread_chains, zgrid(dim3(chain_blocks(d.nlm)), g), dim3(kChainThreads), 0, s, g.cases);
 }
-void glaunch_forcing(const Group &g, cudaStream_t s) {
+void glaunch_forcing(const Group &g, int n, cudaStream_t s) {
     const Dev &d = g.rep;
     if (!d.nlm) return;
-    pdl(kg_mls_interp, zgrid(dim3((2 * d.nlm * kInterpLanes + 255) / 256), g), dim3(256), 0, s, g.cases);
+    pdl(kg_mls_interp, zgrid(dim3((2 * d.nlm * kInterpLanes + 255) / 256), g), dim3(256), 0, s, g.cases,
+        n == 0 ? 1 : 0);
     pdl(kg_mls_spread, zgrid(dim3((2 * d.nlm * kSD + 127) / 128), g), dim3(128), 0, s, g.cases);
 }
-void glaunch_divg(const Group &g, int n, cudaStream_t s) {
-    dim3 b(32, 8);
-    pdl(kg_divg, zgrid(grid2(g.rep.n2m, (g.rep.n3m + kDivK - 1) / kDivK, b), g), dim3(b), 0, s, g.cases, n);
+void glaunch_divg(const Group &g, int n, cudaStream_t s, int extra) {
+    pdl(kg_divg, zgrid(divg_grid(g.rep, extra), g), dim3(32, 8), 0, s, g.cases, n, extra);
 }
-void glaunch_updvp_prcalc(const Group &g, int n, cudaStream_t s, bool pend) {
+void glaunch_updvp_prcalc(const Group &g, int n, cudaStream_t s, bool pend, int slot) {
     const int per_case = std::max(1, std::min(nl_tiles(g.rep), (2 * 148 * kUpBlocksPerSM + g.n - 1) / g.n));
-    pdl(kg_updvp_prcalc, zgrid(dim3(per_case), g), dim3(32, 8), kUpSmem, s, g.cases, n, pend ? 1 : 0);
+    pdl(kg_updvp_prcalc, zgrid(dim3(per_case), g), dim3(32, 8), kUpSmem, s, g.cases, n, pend ? 1 : 0,
+        slot);
 }
 void glaunch_submean_boucqt(const Group &g, cudaStream_t s, bool deferred) {
     dim3 b(32, 8);
     pdl(kg_submean_boucqt, zgrid(grid2(g.rep.n2, g.rep.n3 + 1, b), g), dim3(b), 0, s, g.cases, deferred ? 1 : 0);
-}
-void glaunch_substep_mid(const Group &g, int n_next, int slot, cudaStream_t s) {
-    pdl(kg_substep_mid, zgrid(dim3(1), g), dim3(1024), 0, s, g.cases, n_next, slot);
 }
 void glaunch_loads(const Group &g, cudaStream_t s) {
     const Dev &d = g.rep;

@@ -21,24 +21,34 @@ struct alignas(64) NlMaps {
 };
 int encode_nl_maps(NlMaps *m, const Dev &d);   // FB_OK, or an error (no maps)
 // pend / deferred: the fused step's deferred pr_submean of RK3 substeps 1 and 2.
-// maps: stage the tiles with TMA (the single-case step); null: cp.async
+// maps: stage the tiles with TMA (the single-case step); null: cp.async.
+// extra: the fused step's work on the same launch (kNlBoucdq: boucdq of this
+// substep in a block of its own; kNlCfl: the CFL number and the mean w of the
+// field the tiles hold)
+constexpr int kNlBoucdq = 1, kNlCfl = 2;
 void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend = false,
-                   const NlMaps *maps = nullptr);
+                   const NlMaps *maps = nullptr, int extra = 0);
 void launch_lgrdist(const Dev &d, cudaStream_t s);
-void launch_mls_setup(const Dev &d, cudaStream_t s);
-void launch_mls_interp(const Dev &d, cudaStream_t s);
+// find: the nearest nodes (lgrdistribution) in the same launch
+void launch_mls_setup(const Dev &d, cudaStream_t s, bool find = false);
+// clear: empty the spreading table behind k_spread_chains (substep 1)
+void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear);
 void launch_mls_spread(const Dev &d, cudaStream_t s);
 void launch_spread_chains(const Dev &d, cudaStream_t s);
 void launch_helsolve(const Dev &d, const SubDev &sd, cudaStream_t s);
 // rmax (may be null): n2m row maxima of |dph| accumulated for the INT8 digit cut
-void launch_divg(const Dev &d, double usdtal, cudaStream_t s, double *rmax = nullptr);
+// extra: the fused step's work on the same launch (kDivBoucqt: boucqt;
+// kDivCfl: the CFL number of nl_rhs made the step's, and its check)
+constexpr int kDivBoucqt = 1, kDivCfl = 2;
+void launch_divg(const Dev &d, double usdtal, cudaStream_t s, double *rmax = nullptr, int extra = 0);
+// slot: a scalar slot that keeps the pressure mean beside S_PRAVG (-1: none)
 void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, bool pend = false,
-                         const NlMaps *maps = nullptr);
+                         const NlMaps *maps = nullptr, int slot = -1);
 // mbox[0] = *d.status, mbox[1..8] = d.forces[0..7] (when forces); mbox in
 // mapped host memory
 void launch_publish(const Dev &d, bool forces, double *mbox, cudaStream_t s);
+// deferred: the end of the fused step (boucqt has run with divg)
 void launch_submean_boucqt(const Dev &d, cudaStream_t s, bool deferred = false);
-void launch_substep_mid(const Dev &d, int slot, double ga, double ro, cudaStream_t s);  // boucqt + next boucdq
 void launch_loads(const Dev &d, cudaStream_t s);
 void launch_diag(const Dev &d, int hist_rows, cudaStream_t s);
 enum RigidMode { RIGID_STEP = 0, RIGID_PLACE = 1, RIGID_FORCES = 2, RIGID_COMMIT = 3 };
@@ -48,15 +58,12 @@ void launch_rigid(const Dev &d, int hist_rows, cudaStream_t s, int mode = RIGID_
                   double *mbox = nullptr);
 
 // grouped forms (one launch over a group of cases; substep n 0-based)
-void glaunch_cfl(const Group &g, cudaStream_t s);
-void glaunch_boucdq(const Group &g, int n, cudaStream_t s);
-void glaunch_nl_rhs(const Group &g, int n, cudaStream_t s, bool pend = false);
-void glaunch_marker_setup(const Group &g, cudaStream_t s);   // lgrdist, MLS weights, spreading chains
-void glaunch_forcing(const Group &g, cudaStream_t s);        // interpolation and spreading
-void glaunch_divg(const Group &g, int n, cudaStream_t s);
-void glaunch_updvp_prcalc(const Group &g, int n, cudaStream_t s, bool pend = false);
+void glaunch_nl_rhs(const Group &g, int n, cudaStream_t s, bool pend, int extra);
+void glaunch_marker_setup(const Group &g, cudaStream_t s);   // nearest nodes and MLS weights, spreading chains
+void glaunch_forcing(const Group &g, int n, cudaStream_t s); // interpolation and spreading
+void glaunch_divg(const Group &g, int n, cudaStream_t s, int extra);
+void glaunch_updvp_prcalc(const Group &g, int n, cudaStream_t s, bool pend, int slot);
 void glaunch_submean_boucqt(const Group &g, cudaStream_t s, bool deferred = false);
-void glaunch_substep_mid(const Group &g, int n_next, int slot, cudaStream_t s);
 void glaunch_loads(const Group &g, cudaStream_t s);
 void glaunch_rigid(const Group &g, cudaStream_t s, int mode = RIGID_STEP);
 void glaunch_diag(const Group &g, cudaStream_t s);
