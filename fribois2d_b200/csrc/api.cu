@@ -868,7 +868,7 @@ int setup_i8(fb_ctx *c) {
         p.ldk = ldk;
         p.rows_pad = (rows + 127) / 128 * 128;
         int r;
-        if ((r = dnew(c, &p.dig, static_cast<size_t>(fb::kI8S) * p.rows_pad * ldk))) return r;
+        if ((r = dnew(c, &p.dig, static_cast<size_t>(fb::kI8Step) * p.rows_pad * ldk))) return r;
         if ((r = dnew(c, &p.scale, static_cast<size_t>(p.rows_pad)))) return r;
         return fb::i8_plan(p, rows, d.n3m, box);
     };
@@ -3259,8 +3259,8 @@ int fb_gemm_i8x8(int device, int M, int N, int K, const double *A, const double 
     double *dA = static_cast<double *>(alloc(sizeof(double) * M * K));
     double *dB = static_cast<double *>(alloc(sizeof(double) * N * K));
     double *dC = static_cast<double *>(alloc(sizeof(double) * M * N));
-    pa.dig = static_cast<int8_t *>(alloc(static_cast<size_t>(fb::kI8SPub) * pa.rows_pad * ldk));
-    pb.dig = static_cast<int8_t *>(alloc(static_cast<size_t>(fb::kI8SPub) * pb.rows_pad * ldk));
+    pa.dig = static_cast<int8_t *>(alloc(static_cast<size_t>(fb::kI8S) * pa.rows_pad * ldk));
+    pb.dig = static_cast<int8_t *>(alloc(static_cast<size_t>(fb::kI8S) * pb.rows_pad * ldk));
     pa.scale = static_cast<double *>(alloc(sizeof(double) * pa.rows_pad));
     pb.scale = static_cast<double *>(alloc(sizeof(double) * pb.rows_pad));
     int *status = static_cast<int *>(alloc(sizeof(int)));
@@ -3275,8 +3275,8 @@ int fb_gemm_i8x8(int device, int M, int N, int K, const double *A, const double 
                 cudaMemset(mxA, 0, sizeof(double) * M) != cudaSuccess ||
                 cudaMemset(mxB, 0, sizeof(double) * N) != cudaSuccess))
         st = FB_ERR_CUDA;
-    if (!st) st = fb::i8_plan(pa, M, K, 128, fb::kI8SPub);
-    if (!st) st = fb::i8_plan(pb, N, K, fb::kI8BN, fb::kI8SPub);
+    if (!st) st = fb::i8_plan(pa, M, K, 128, fb::kI8S);
+    if (!st) st = fb::i8_plan(pb, N, K, fb::kI8BN, fb::kI8S);
     if (!st) {
         // row maxima, then the cut of each operand (the step's kernels)
         fb::launch_i8_rowmax(dA, M, M, K, mxA, nullptr);

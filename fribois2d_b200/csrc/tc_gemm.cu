@@ -679,7 +679,7 @@ __device__ __forceinline__ int i8_row_exp(double mm) {
     int e = 0;
     if (mm > 0.0) {
         const double m = frexp(mm, &e);   // mm = m 2^e, m < 1
-        if (S == kI8S && m > 0.994) ++e;
+        if (S == kI8Step && m > 0.994) ++e;
     }
     return e;
 }
@@ -704,7 +704,7 @@ __device__ __forceinline__ void i8_cut_emit(const double (&a)[V / 4][4], double 
     constexpr int kP = V / 4;   // 32-bit words (four columns) per thread and slice
     const bool live = c0 < ldk;   // ldk is a multiple of 128, so a run is inside or wholly past it
     int8_t *out = dig + static_cast<size_t>(r) * ldk + c0;
-    if constexpr (S == kI8S) {
+    if constexpr (S == kI8Step) {
         // a s 2^55 rounded to an integer v = sum_i d_i 256^(6 - i), |d_i| <= 128:
         // with 128 added to each of the six lower digits (one 64-bit addition)
         // every digit is a byte of the sum, biased by 128; the exclusive or
@@ -809,12 +809,12 @@ __device__ __forceinline__ void i8_cut_body(const double *__restrict__ src, long
     if (w == 0) {
         double mm = 0.0;
         for (int q = 0; q < kCutCl; ++q) mm = fmax(mm, *cl.map_shared_rank(&part[lane], q));
-        const int e = i8_row_exp<kI8S>(mm);
+        const int e = i8_row_exp<kI8Step>(mm);
         sc[lane] = ldexp(1.0, -e);
         if (rank == 0 && r < R) rowscale[r] = ldexp(1.0, e);
     }
     cl.sync();   // no CTA leaves while another still reads its maxima
-    i8_cut_emit<V, kI8S>(a, sc[lane], r, c0, dig, ldk, plane);
+    i8_cut_emit<V, kI8Step>(a, sc[lane], r, c0, dig, ldk, plane);
 }
 
 // The cut with the rows' maxima of |a| given (accumulated by the operand's
@@ -899,7 +899,7 @@ struct I8Cfg {
     // D s32 (2), A and B signed 8-bit (1), both K-major, M = 128; N set per MMA
     static constexpr uint32_t kIdescBase = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(128 >> 4) << 24);
     // weight class t: 2^-(kShift t + kW0)
-    static constexpr int kShift = (S == kI8S) ? 8 : 7, kW0 = 14;
+    static constexpr int kShift = (S == kI8Step) ? 8 : 7, kW0 = 14;
     static_assert(S * BN <= 512, "TMEM columns");
     static_assert(BN % 16 == 0 && BN <= 256, "MMA N: a multiple of 16, at most 256");
     static_assert(kBSlice % 1024 == 0, "B slices start on swizzle atoms");
@@ -1137,7 +1137,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) kg_i8x8_gemm(const I8Task *__re
     const I8Task &tk = t[blockIdx.z];
     if (tk.gate && !*tk.gate) return;
     const I8Out o = tk.o;
-    i8x8_body<kI8S, BN, true>(&tk.a, &tk.b, o, tk.K, tk.status);
+    i8x8_body<kI8Step, BN, true>(&tk.a, &tk.b, o, tk.K, tk.status);
 }
 
 void launch_poisson_residual(const Dev &d, const double *phi, const SplitPlane &dst, cudaStream_t st,
@@ -1276,7 +1276,7 @@ void launch_split_t(const double *src, long lds, int R, int C, const SplitPlane 
 int i8_plan(I8Plan &p, int rows, int K, int box_rows, int slices) {
     if (K > kI8MaxK) return FB_ERR_UNSUPPORTED;   // the int32 class sums would overflow
     if (box_rows != 128 && box_rows != 64 && box_rows != 48 && box_rows != 32 && box_rows != 16) return FB_ERR_STATE;
-    if (slices != kI8S && (slices != kI8SPub || (box_rows != 128 && box_rows != kI8BN))) return FB_ERR_STATE;
+    if (slices != kI8Step && (slices != kI8S || (box_rows != 128 && box_rows != kI8BN))) return FB_ERR_STATE;
     if (!p.dig || (p.ldk % 128) || p.rows_pad < rows) return FB_ERR_STATE;
     if (!g_encode) {
         void *fn = nullptr;
@@ -1310,10 +1310,10 @@ int i8_configure() {
         ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) ==
                        cudaSuccess;
     };
-    allow(k_i8x8_gemm<kI8SPub, kI8BN>, I8Cfg<kI8SPub, kI8BN>::kSmem);
+    allow(k_i8x8_gemm<kI8S, kI8BN>, I8Cfg<kI8S, kI8BN>::kSmem);
 #define FB_I8_ALLOW(BN)                                 \
-    allow(k_i8x8_gemm<kI8S, BN>, I8Cfg<kI8S, BN>::kSmem); \
-    allow(kg_i8x8_gemm<BN>, I8Cfg<kI8S, BN>::kSmem);
+    allow(k_i8x8_gemm<kI8Step, BN>, I8Cfg<kI8Step, BN>::kSmem); \
+    allow(kg_i8x8_gemm<BN>, I8Cfg<kI8Step, BN>::kSmem);
     FB_I8_ALLOW(64) FB_I8_ALLOW(48) FB_I8_ALLOW(32) FB_I8_ALLOW(16)
 #undef FB_I8_ALLOW
     return ok ? FB_OK : FB_ERR_CUDA;
@@ -1332,17 +1332,17 @@ void launch_i8_split_group(const I8SplitTask *tasks, const I8Plan &rep, int R, i
 
 void launch_i8x8_group(const I8Task *tasks, int M, int N, int n, int bn, cudaStream_t st) {
     const dim3 grid((M + 127) / 128, (N + bn - 1) / bn, n);
-    if (bn == 48) pdl(kg_i8x8_gemm<48>, grid, dim3(kI8Threads), I8Cfg<kI8S, 48>::kSmem, st, tasks);
-    else if (bn == 32) pdl(kg_i8x8_gemm<32>, grid, dim3(kI8Threads), I8Cfg<kI8S, 32>::kSmem, st, tasks);
-    else if (bn == 16) pdl(kg_i8x8_gemm<16>, grid, dim3(kI8Threads), I8Cfg<kI8S, 16>::kSmem, st, tasks);
-    else pdl(kg_i8x8_gemm<64>, grid, dim3(kI8Threads), I8Cfg<kI8S, 64>::kSmem, st, tasks);
+    if (bn == 48) pdl(kg_i8x8_gemm<48>, grid, dim3(kI8Threads), I8Cfg<kI8Step, 48>::kSmem, st, tasks);
+    else if (bn == 32) pdl(kg_i8x8_gemm<32>, grid, dim3(kI8Threads), I8Cfg<kI8Step, 32>::kSmem, st, tasks);
+    else if (bn == 16) pdl(kg_i8x8_gemm<16>, grid, dim3(kI8Threads), I8Cfg<kI8Step, 16>::kSmem, st, tasks);
+    else pdl(kg_i8x8_gemm<64>, grid, dim3(kI8Threads), I8Cfg<kI8Step, 64>::kSmem, st, tasks);
 }
 
 void launch_i8_cut_rows(const double *src, long lds, int R, int K, const I8Plan &p, const double *rmax,
                         double *clear, cudaStream_t st) {
     const dim3 grid(p.rows_pad / 32, static_cast<unsigned>(p.ldk / 128));
     const long plane = p.ldk * static_cast<long>(p.rows_pad);
-    pdl(p.slices == kI8SPub ? k_i8_cut_rows<kI8SPub> : k_i8_cut_rows<kI8S>, grid, dim3(256), 0, st, src, lds, R, K,
+    pdl(p.slices == kI8S ? k_i8_cut_rows<kI8S> : k_i8_cut_rows<kI8Step>, grid, dim3(256), 0, st, src, lds, R, K,
         p.dig, p.ldk, plane, p.scale, rmax, clear);
 }
 
@@ -1359,11 +1359,11 @@ void launch_i8x8(const I8Plan &a, const I8Plan &b, double *out, long ldo, int *s
     auto go = [&](auto kern, size_t smem) {
         pdl(kern, grid, dim3(kI8Threads), smem, st, a.map, b.map, o, a.K, status);
     };
-    if (b.slices == kI8SPub) go(k_i8x8_gemm<kI8SPub, kI8BN>, I8Cfg<kI8SPub, kI8BN>::kSmem);
-    else if (b.box == 48) go(k_i8x8_gemm<kI8S, 48>, I8Cfg<kI8S, 48>::kSmem);
-    else if (b.box == 32) go(k_i8x8_gemm<kI8S, 32>, I8Cfg<kI8S, 32>::kSmem);
-    else if (b.box == 16) go(k_i8x8_gemm<kI8S, 16>, I8Cfg<kI8S, 16>::kSmem);
-    else go(k_i8x8_gemm<kI8S, 64>, I8Cfg<kI8S, 64>::kSmem);
+    if (b.slices == kI8S) go(k_i8x8_gemm<kI8S, kI8BN>, I8Cfg<kI8S, kI8BN>::kSmem);
+    else if (b.box == 48) go(k_i8x8_gemm<kI8Step, 48>, I8Cfg<kI8Step, 48>::kSmem);
+    else if (b.box == 32) go(k_i8x8_gemm<kI8Step, 32>, I8Cfg<kI8Step, 32>::kSmem);
+    else if (b.box == 16) go(k_i8x8_gemm<kI8Step, 16>, I8Cfg<kI8Step, 16>::kSmem);
+    else go(k_i8x8_gemm<kI8Step, 64>, I8Cfg<kI8Step, 64>::kSmem);
 }
 
 }  // namespace fb

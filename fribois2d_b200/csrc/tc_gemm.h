@@ -62,8 +62,8 @@ struct ResidualTask {    // one Poisson residual: phi -> hi, lo (ldd), row facto
 // their slices per operand: 7 balanced 8-bit digits (28 digit pairs; the time
 // step) and 8 sign-magnitude 7-bit digits (36 pairs; the public product
 // fb_gemm_i8x8, whose digits and summation order are its documented result).
-constexpr int kI8S = 7;       // digit slices per operand of the time step
-constexpr int kI8SPub = 8;    // ... of fb_gemm_i8x8
+constexpr int kI8Step = 7;       // digit slices per operand of the time step
+constexpr int kI8S = 8;    // ... of fb_gemm_i8x8
 constexpr int kI8BK = 128;    // K bytes per k-block (one 128-byte swizzle row)
 constexpr int kI8BN = 64;     // widest output tile
 // Largest K of one product: the last weight class sums S digit pairs (7 of at
@@ -109,7 +109,7 @@ struct I8Plan {
     long ldk;
     int rows_pad, rows, K;
     int box;                  // rows per TMA box: 128 (A) or the output tile width (B)
-    int slices;               // kI8S or kI8SPub
+    int slices;               // kI8Step or kI8S
 };
 struct I8Out {
     double *out;
@@ -138,7 +138,7 @@ struct I8Task {
 int i8_configure();
 // box_rows: 128 for the A operand (one slice per copy), the output tile width
 // (64, 48, 32 or 16; all slices in one copy) for B
-int i8_plan(I8Plan &p, int rows, int K, int box_rows, int slices = kI8S);
+int i8_plan(I8Plan &p, int rows, int K, int box_rows, int slices = kI8Step);
 // digits of the column-major source A(r, k) = src[k * lds + r], r < R, k < K,
 // with the rows' maxima of |src| given in rmax (R entries); clear (R entries,
 // may be null) is zeroed for the next producer's maxima
