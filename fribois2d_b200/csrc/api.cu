@@ -63,8 +63,12 @@ struct fb_ctx {
     double usdtal[3] = {0, 0, 0};
     std::vector<void *> allocs;
     int hist_cap = 0;
-    cudaGraph_t graph = nullptr;
+    cudaGraph_t graph = nullptr;              // a coupled step
     cudaGraphExec_t graph_exec = nullptr;
+    // fb_advance, loose coupling: the first step up to its last updvp, the end
+    // of a step beside the start of the next one up to that one's last updvp,
+    // the end of the last step
+    cudaGraphExec_t head_exec = nullptr, next_exec = nullptr, tail_exec = nullptr;
     cudaGraph_t fgraph = nullptr;             // fluid step alone (fb_fluid_tsch), fixed dt
     cudaGraphExec_t fgraph_exec = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1014,39 +1018,39 @@ int vardt_update(fb_ctx *c, int ns) {
     return FB_OK;
 }
 
-int enqueue_fluid(fb_ctx *c, int ns) {
+// the marker set-up of substep 1 (nearest nodes, MLS weights, spreading
+// chains) on the side branch; it reads only marker data
+void enqueue_marker_setup(fb_ctx *c) {
+    c->own_launches += 2;
+    fb::launch_mls_setup(c->d, c->side, true);
+    fb::launch_spread_chains(c->d, c->side);
+}
+
+// The substeps of one step, from nl_rhs to the last updvp, beside the side
+// branch that ends with ev_join (the marker set-up): the explicit terms of
+// substep 1 need no markers.  follows: the step before has not subtracted its
+// last pressure mean(s) yet.
+int enqueue_substeps(fb_ctx *c, int ns, bool follows) {
     const Dev &d = c->d;
     int r;
-    if (c->vardt && (r = vardt_update(c, ns))) return r;
-    // The marker set-up of substep 1 (nearest nodes, MLS weights, spreading
-    // chains) reads only marker data: it runs on a side branch while the
-    // explicit terms run on the main stream.
-    if (d.nlm) {
-        CK(cudaEventRecord(c->ev_fork, c->stream));
-        CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-        c->own_launches += 2;
-        fb::launch_mls_setup(d, c->side, true);
-        fb::launch_spread_chains(d, c->side);
-        CK(cudaGetLastError());
-        CK(cudaEventRecord(c->ev_join, c->side));
-    }
     c->beta = c->dt / c->hc.grid.ren * 0.5;
     // boucdq and (fixed dt) cfl share nl_rhs's launch, boucqt and the CFL
     // check divg's: a substep is a chain of launches that each wait for the
     // one before, and these four depend on no step of it between those two.
-    // RK3: pr_submean of substeps 1 and 2 is deferred; nl_rhs and updvp of
-    // the next substep subtract the mean as they read pr, and the mean is
-    // kept for the entries updvp does not rewrite, which the last pr_submean
-    // brings up to date.
+    // RK3: pr_submean of substeps 1 and 2 is deferred (follows: and that of the
+    // step before); nl_rhs and updvp of the next substep subtract the mean as
+    // they read pr, and the mean is kept for the entries updvp does not rewrite,
+    // which the last pr_submean (follows: nl_rhs) brings up to date.
     const bool defer = (d.nsst == 3);
     for (int n = 1; n <= d.nsst; ++n) {
-        const bool pend = defer && n > 1, cfl = (n == 1 && !c->vardt);
+        const bool pend = (n == 1) ? follows : defer, cfl = (n == 1 && !c->vardt);
         double al, ga, ro;
         coefs(c, ns, n, al, ga, ro);
         c->al = al;
         c->ga = ga;
         c->ro = ro;
-        fb::launch_nl_rhs(d, al, ga, ro, c->stream, pend, &c->nlmaps, fb::kNlBoucdq | (cfl ? fb::kNlCfl : 0));
+        fb::launch_nl_rhs(d, al, ga, ro, c->stream, pend, &c->nlmaps,
+                          fb::kNlBoucdq | (cfl ? fb::kNlCfl : 0) | (n == 1 && follows ? fb::kNlMeans : 0));
         c->own_launches += 1;
         if (d.nlm) {
             if (n == 1) CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
@@ -1066,17 +1070,51 @@ int enqueue_fluid(fb_ctx *c, int ns) {
         c->own_launches += 1;
         CK(cudaGetLastError());
     }
-    // (Adams-Bashforth: the two other means are zero and stay so)
-    fb::launch_submean_boucqt(d, c->stream, true);
-    c->own_launches += 1;
-    CK(cudaGetLastError());
-    if (d.nlm && c->hc.deck.cbody && (r = stage_impl(c, FB_ST_LOADS, ns, 1))) return r;
     return FB_OK;
 }
 
-int enqueue_report(fb_ctx *c) {
+// the pressure mean(s) of the step, then its loads
+int enqueue_fluid_end(fb_ctx *c, int ns) {
+    // (Adams-Bashforth: the two other means are zero and stay so)
+    fb::launch_submean_boucqt(c->d, c->stream, true);
+    c->own_launches += 1;
+    int r;
+    if (c->d.nlm && c->hc.deck.cbody && (r = stage_impl(c, FB_ST_LOADS, ns, 1))) return r;
+    CK(cudaGetLastError());
+    return FB_OK;
+}
+
+int fork_side(fb_ctx *c) {
+    CK(cudaEventRecord(c->ev_fork, c->stream));
+    CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
+    return FB_OK;
+}
+int end_side(fb_ctx *c) {
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(c->ev_join, c->side));
+    return FB_OK;
+}
+
+// the fluid step up to its last updvp
+int enqueue_fluid_start(fb_ctx *c, int ns) {
+    int r;
+    if (c->vardt && (r = vardt_update(c, ns))) return r;
+    if (c->d.nlm) {
+        if ((r = fork_side(c))) return r;
+        enqueue_marker_setup(c);
+        if ((r = end_side(c))) return r;
+    }
+    return enqueue_substeps(c, ns, false);
+}
+
+int enqueue_fluid(fb_ctx *c, int ns) {
+    const int r = enqueue_fluid_start(c, ns);
+    return r ? r : enqueue_fluid_end(c, ns);
+}
+
+int enqueue_report(fb_ctx *c, cudaStream_t st = nullptr) {
     if (!c->report || !c->d.nlm) return FB_OK;
-    fb::launch_diag(c->d, c->hist_cap, c->stream);
+    fb::launch_diag(c->d, c->hist_cap, st ? st : c->stream);
     c->own_launches += 1;
     return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
@@ -1091,7 +1129,30 @@ int enqueue_step(fb_ctx *c, int ns) {
     return FB_OK;
 }
 
+// The end of a step (loads, rigid, report: markers and one field pass) beside
+// the start of the next one.  nl_rhs of the next step needs nothing of it, and
+// its chain of small launches, followed by the next step's marker set-up, is
+// the longer of the two branches.
+int enqueue_next_step(fb_ctx *c) {
+    int r;
+    if ((r = fork_side(c))) return r;
+    if (c->hc.deck.cbody) {
+        fb::launch_loads(c->d, c->side, true);
+        c->own_launches += 2;
+    }
+    fb::launch_rigid(c->d, c->hist_cap, c->side);
+    c->own_launches += 1;
+    if ((r = enqueue_report(c, c->side))) return r;
+    enqueue_marker_setup(c);
+    if ((r = end_side(c))) return r;
+    return enqueue_substeps(c, 1, true);
+}
+
 void drop_graph(fb_ctx *c) {
+    for (cudaGraphExec_t *e : {&c->head_exec, &c->next_exec, &c->tail_exec}) {
+        if (*e) cudaGraphExecDestroy(*e);
+        *e = nullptr;
+    }
     if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
     if (c->graph) cudaGraphDestroy(c->graph);
     if (c->fgraph_exec) cudaGraphExecDestroy(c->fgraph_exec);
@@ -1115,22 +1176,39 @@ void host_clock(fb_ctx *c, int nsteps) {
 
 int capture_coupled(fb_ctx *c);
 
-int capture_step(fb_ctx *c) {
-    if (c->graph_exec) return FB_OK;
-    if (c->coupling != FB_COUPLING_LOOSE) return capture_coupled(c);
+// captures what fn enqueues on the context's stream into exec (kept if it is there)
+template <class F>
+int capture_exec(fb_ctx *c, cudaGraphExec_t *exec, F fn) {
+    if (*exec) return FB_OK;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    c->own_launches = 0;
-    int r = enqueue_step(c, 1);
-    c->step_kernels = c->own_launches;
+    const int r = fn();
     cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-    if (r) {
-        if (g) cudaGraphDestroy(g);
-        return r;
+    const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+    cudaError_t ei = cudaSuccess;
+    if (!r && e == cudaSuccess) ei = cudaGraphInstantiate(exec, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (r) return r;
+    CK(e);
+    CK(ei);
+    return FB_OK;
+}
+
+// the graphs of fb_advance: steps > 1 also needs the joint of two steps
+int capture_step(fb_ctx *c, int steps = 1) {
+    if (c->coupling != FB_COUPLING_LOOSE) return c->graph_exec ? FB_OK : capture_coupled(c);
+    int r;
+    if (!c->head_exec || !c->tail_exec) {
+        c->own_launches = 0;
+        if ((r = capture_exec(c, &c->head_exec, [&] { return enqueue_fluid_start(c, 1); })) ||
+            (r = capture_exec(c, &c->tail_exec, [&] {
+                 int q;
+                 if ((q = enqueue_fluid_end(c, 1)) || (q = stage_impl(c, FB_ST_RIGID, 1, 1))) return q;
+                 return enqueue_report(c);
+             })))
+            return r;
+        c->step_kernels = c->own_launches;
     }
-    if (e != cudaSuccess) return FB_ERR_CUDA;
-    c->graph = g;
-    CK(cudaGraphInstantiate(&c->graph_exec, g, 0));
+    if (steps > 1) return capture_exec(c, &c->next_exec, [&] { return enqueue_next_step(c); });
     return FB_OK;
 }
 
@@ -1606,13 +1684,19 @@ int fb_advance(fb_ctx *c, int ns0, int nsteps, double *hist) {
     } else if (done == 0) {
         c->last_ms = 0.0;
     }
-    if ((r = capture_step(c))) return r;
+    if ((r = capture_step(c, std::min(nsteps - done, c->hist_cap)))) return r;
     while (done < nsteps) {
         const int chunk = std::min(nsteps - done, c->hist_cap);
         double row0;
         CK(cudaMemcpyAsync(&row0, c->d.scal + fb::S_STEP, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaEventRecord(c->ev0, c->stream));
-        for (int i = 0; i < chunk; ++i) CK(cudaGraphLaunch(c->graph_exec, c->stream));
+        if (c->coupling == FB_COUPLING_LOOSE) {
+            CK(cudaGraphLaunch(c->head_exec, c->stream));
+            for (int i = 1; i < chunk; ++i) CK(cudaGraphLaunch(c->next_exec, c->stream));
+            CK(cudaGraphLaunch(c->tail_exec, c->stream));
+        } else {
+            for (int i = 0; i < chunk; ++i) CK(cudaGraphLaunch(c->graph_exec, c->stream));
+        }
         CK(cudaEventRecord(c->ev1, c->stream));
         if ((r = read_status(c, &status))) return r;
         float ms = 0.f;

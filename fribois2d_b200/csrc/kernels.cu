@@ -215,6 +215,28 @@ __device__ __forceinline__ void boucdq_body(const Dev &d, double ga, double ro) 
     for (int j = t + 1; j <= d.n2m; j += nt) d.dqb3n[j] = d.dqb3n[j] + cor;
 }
 
+// pr_submean (updvp.F90:336) of a step's three pressure means, in order, for
+// the entries of pr that updvp never rewrites and no stencil reads (j = n2,
+// k = 0, k = n3); one block
+__device__ __forceinline__ void edge_means_body(const Dev &d) {
+    const int t = threadIdx.x + blockDim.x * threadIdx.y, nt = blockDim.x * blockDim.y;
+    const double m1 = d.scal[S_PRAVG1], m2 = d.scal[S_PRAVG2], m3 = d.scal[S_PRAVG];
+    const int n = (d.n3 + 1) + 2 * d.n2m;   // column j = n2, then rows k = 0 and n3
+    constexpr int kU = 4;
+    for (int i0 = t; i0 < n; i0 += kU * nt) {
+        double *p[kU], v[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {   // every load before the first store
+            const int i = min(i0 + u * nt, n - 1), e = i - (d.n3 + 1);
+            p[u] = d.pr + (e < 0 ? fidx(d, d.n2, i) : e < d.n2m ? fidx(d, e + 1, 0) : fidx(d, e - d.n2m + 1, d.n3));
+            v[u] = *p[u];
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+            if (i0 + u * nt < n) *p[u] = ((v[u] - m1) - m2) - m3;
+    }
+}
+
 __global__ void __launch_bounds__(1024) k_boucdq(Dev d, double ga, double ro) {
     FB_GRID_WAIT();
     boucdq_body(d, ga, ro);
@@ -637,7 +659,11 @@ __device__ __forceinline__ void nl_rhs_tma_body(const Dev &d, const NlMaps &m, d
     if (kCfl) cfl_finish(d, cmx, csm, nb);
 }
 
-// extra (kernels.h): with kNlBoucdq the grid has one block more than the tiles
+// the blocks of nl_rhs's launch beyond the tiles' (kernels.h: extra)
+__host__ __device__ inline int nl_more(int extra) {
+    return ((extra & kNlBoucdq) ? 1 : 0) + ((extra & kNlMeans) ? 1 : 0);
+}
+
 template <bool kCfl>
 __global__ void __launch_bounds__(256, kNlBlocksPerSM)
     k_nl_rhs_tma(const __grid_constant__ Dev d, const __grid_constant__ NlMaps m, double al, double ga, double ro,
@@ -648,13 +674,11 @@ __global__ void __launch_bounds__(256, kNlBlocksPerSM)
     NlTileT *buf = reinterpret_cast<NlTileT *>(base);
     uint64_t *bars = reinterpret_cast<uint64_t *>(base + 2 * sizeof(NlTileT));
     FB_GRID_WAIT();
-    int nb = gridDim.x;
-    if (extra & kNlBoucdq) {
-        --nb;
-        if (static_cast<int>(blockIdx.x) == nb) {
-            boucdq_body(d, ga, ro);
-            return;
-        }
+    const int nb = gridDim.x - nl_more(extra);
+    if (static_cast<int>(blockIdx.x) >= nb) {
+        if ((extra & kNlBoucdq) && static_cast<int>(blockIdx.x) == nb) boucdq_body(d, ga, ro);
+        else edge_means_body(d);
+        return;
     }
     nl_rhs_tma_body<kCfl>(d, m, al, ga, ro, buf, bars, pend != 0, nb);
 }
@@ -1718,7 +1742,9 @@ constexpr int kLoadLanes = kNodeLanes;
 constexpr int kLoadMk = 2;   // markers per block: the three groups of a marker in one block
 constexpr int kLoadThreads = 3 * kLoadMk * kLoadLanes;
 
-__device__ __forceinline__ void loads_probe_body(const Dev &d) {
+// pend: the step's last pressure mean is still to be subtracted from pr; the
+// value is the one pr_submean would have stored.
+__device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend) {
     constexpr unsigned kAll = 0xffffffffu;
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1806,9 +1832,10 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d) {
     double f0 = 0.0, fym = 0.0, fzm = 0.0, g2r = 1.0, g3r = 1.0;
     if (act) {
         const double *f = (idir == 1) ? d.q2 : (idir == 2 ? d.q3 : d.pr);
-        f0 = Fv(f, ej, ek);
-        fym = Fv(f, ej - 1, ek);
-        fzm = Fv(f, ej, ek - 1);
+        const double mean = (pend && idir == 3) ? d.scal[S_PRAVG] : 0.0;   // (x - 0.0 is x)
+        f0 = Fv(f, ej, ek) - mean;
+        fym = Fv(f, ej - 1, ek) - mean;
+        fzm = Fv(f, ej, ek - 1) - mean;
         g2r = d.g2rc[ej];
         g3r = d.g3rc[ek];
     }
@@ -1903,9 +1930,9 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d) {
 
 // the probes of kLoadMk markers per block, then each probed marker's own
 // tangent (loads_transfer.F90:177-185) from its first two probes
-__device__ __forceinline__ void loads_probe_tan_body(const Dev &d) {
+__device__ __forceinline__ void loads_probe_tan_body(const Dev &d, bool pend) {
     if (!d.nlm) return;
-    loads_probe_body(d);
+    loads_probe_body(d, pend);
     __syncthreads();
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = T / kLoadLanes;
@@ -1927,9 +1954,9 @@ __device__ __forceinline__ void loads_probe_tan_body(const Dev &d) {
     }
 }
 
-__global__ void __launch_bounds__(kLoadThreads, 5) k_loads_probe(Dev d) {
+__global__ void __launch_bounds__(kLoadThreads, 5) k_loads_probe(Dev d, int pend) {
     FB_GRID_WAIT();
-    loads_probe_tan_body(d);
+    loads_probe_tan_body(d, pend != 0);
 }
 
 // loads_transfer_c (loads_transfer.F90:187-214): the tangent carries over
@@ -2388,13 +2415,11 @@ __global__ void __launch_bounds__(256, kNlBlocksPerSM) kg_nl_rhs(const GroupCase
     __shared__ Dev d;
     __shared__ SubDev s;
     if (!stage_case(g, &d, &s, n)) return;
-    int nb = gridDim.x;
-    if (extra & kNlBoucdq) {
-        --nb;
-        if (static_cast<int>(blockIdx.x) == nb) {
-            boucdq_body(d, s.ga, s.ro);
-            return;
-        }
+    const int nb = gridDim.x - nl_more(extra);
+    if (static_cast<int>(blockIdx.x) >= nb) {
+        if ((extra & kNlBoucdq) && static_cast<int>(blockIdx.x) == nb) boucdq_body(d, s.ga, s.ro);
+        else edge_means_body(d);
+        return;
     }
     nl_rhs_body<kCfl>(d, s.al, s.ga, s.ro, reinterpret_cast<NlTile *>(nl_smem), pend != 0, nb);
 }
@@ -2445,10 +2470,10 @@ __global__ void kg_submean_boucqt(const GroupCase *__restrict__ g, int deferred)
     submean_boucqt_body(d, deferred != 0);
 }
 
-__global__ void __launch_bounds__(kLoadThreads, 5) kg_loads_probe(const GroupCase *__restrict__ g) {
+__global__ void __launch_bounds__(kLoadThreads, 5) kg_loads_probe(const GroupCase *__restrict__ g, int pend) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    loads_probe_tan_body(d);
+    loads_probe_tan_body(d, pend != 0);
 }
 
 __global__ void __launch_bounds__(kLoadFin) kg_loads_finish(const GroupCase *__restrict__ g) {
@@ -2497,7 +2522,7 @@ int nl_tiles(const Dev &d) { return ((d.n2m + kNlJ - 1) / kNlJ) * ((d.n3m + kNlK
 
 void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend, const NlMaps *maps,
                    int extra) {
-    const int more = (extra & kNlBoucdq) ? 1 : 0;
+    const int more = nl_more(extra);
     const int blocks = std::min(nl_tiles(d), 148 * kNlBlocksPerSM - more) + more;   // all resident at once
     if (maps)
         pdl((extra & kNlCfl) ? k_nl_rhs_tma<true> : k_nl_rhs_tma<false>, dim3(blocks), dim3(32, 8), kNlSmemT, s, d,
@@ -2579,9 +2604,9 @@ void launch_submean_boucqt(const Dev &d, cudaStream_t s, bool deferred) {
     dim3 b(32, 8);
     pdl(k_submean_boucqt, dim3(grid2(d.n2, d.n3 + 1, b)), dim3(b), 0, s, d, deferred ? 1 : 0);
 }
-void launch_loads(const Dev &d, cudaStream_t s) {
+void launch_loads(const Dev &d, cudaStream_t s, bool pend) {
     if (!d.nlm) return;
-    pdl(k_loads_probe, dim3((d.nlm + kLoadMk - 1) / kLoadMk), dim3(kLoadThreads), 0, s, d);
+    pdl(k_loads_probe, dim3((d.nlm + kLoadMk - 1) / kLoadMk), dim3(kLoadThreads), 0, s, d, pend ? 1 : 0);
     pdl(k_loads_finish, dim3((d.nlm + kLoadFin - 1) / kLoadFin), dim3(kLoadFin), 0, s, d);
 }
 void launch_diag(const Dev &d, int hist_rows, cudaStream_t s) {
@@ -2616,7 +2641,7 @@ inline dim3 zgrid(dim3 g, const Group &gr) { return dim3(g.x, g.y, static_cast<u
 void glaunch_nl_rhs(const Group &g, int n, cudaStream_t s, bool pend, int extra) {
     // about two waves of resident blocks over the whole group
     const int per_case = std::max(1, std::min(nl_tiles(g.rep), (2 * 148 * kNlBlocksPerSM + g.n - 1) / g.n)) +
-                         ((extra & kNlBoucdq) ? 1 : 0);
+                         nl_more(extra);
     pdl((extra & kNlCfl) ? kg_nl_rhs<true> : kg_nl_rhs<false>, zgrid(dim3(per_case), g), dim3(32, 8), kNlSmem, s,
         g.cases, n, pend ? 1 : 0, extra);
 }
@@ -2662,10 +2687,11 @@ void glaunch_submean_boucqt(const Group &g, cudaStream_t s, bool deferred) {
     dim3 b(32, 8);
     pdl(kg_submean_boucqt, zgrid(grid2(g.rep.n2, g.rep.n3 + 1, b), g), dim3(b), 0, s, g.cases, deferred ? 1 : 0);
 }
-void glaunch_loads(const Group &g, cudaStream_t s) {
+void glaunch_loads(const Group &g, cudaStream_t s, bool pend) {
     const Dev &d = g.rep;
     if (!d.nlm) return;
-    pdl(kg_loads_probe, zgrid(dim3((d.nlm + kLoadMk - 1) / kLoadMk), g), dim3(kLoadThreads), 0, s, g.cases);
+    pdl(kg_loads_probe, zgrid(dim3((d.nlm + kLoadMk - 1) / kLoadMk), g), dim3(kLoadThreads), 0, s, g.cases,
+        pend ? 1 : 0);
     pdl(kg_loads_finish, zgrid(dim3((d.nlm + kLoadFin - 1) / kLoadFin), g), dim3(kLoadFin), 0, s, g.cases);
 }
 void glaunch_rigid(const Group &g, cudaStream_t s, int mode) {

@@ -24,8 +24,10 @@ int encode_nl_maps(NlMaps *m, const Dev &d);   // FB_OK, or an error (no maps)
 // maps: stage the tiles with TMA (the single-case step); null: cp.async.
 // extra: the fused step's work on the same launch (kNlBoucdq: boucdq of this
 // substep in a block of its own; kNlCfl: the CFL number and the mean w of the
-// field the tiles hold)
-constexpr int kNlBoucdq = 1, kNlCfl = 2;
+// field the tiles hold; kNlMeans: the step before left all its pressure means to
+// be subtracted, and a block of its own brings the entries of pr that updvp does
+// not rewrite up to date)
+constexpr int kNlBoucdq = 1, kNlCfl = 2, kNlMeans = 4;
 void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend = false,
                    const NlMaps *maps = nullptr, int extra = 0);
 void launch_lgrdist(const Dev &d, cudaStream_t s);
@@ -49,7 +51,8 @@ void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, boo
 void launch_publish(const Dev &d, bool forces, double *mbox, cudaStream_t s);
 // deferred: the end of the fused step (boucqt has run with divg)
 void launch_submean_boucqt(const Dev &d, cudaStream_t s, bool deferred = false);
-void launch_loads(const Dev &d, cudaStream_t s);
+// pend: pr still lacks the subtraction of its mean (S_PRAVG)
+void launch_loads(const Dev &d, cudaStream_t s, bool pend = false);
 void launch_diag(const Dev &d, int hist_rows, cudaStream_t s);
 enum RigidMode { RIGID_STEP = 0, RIGID_PLACE = 1, RIGID_FORCES = 2, RIGID_COMMIT = 3 };
 // mbox (mapped host memory, may be null; RIGID_STEP and RIGID_COMMIT): the status
@@ -64,7 +67,7 @@ void glaunch_forcing(const Group &g, int n, cudaStream_t s); // interpolation an
 void glaunch_divg(const Group &g, int n, cudaStream_t s, int extra);
 void glaunch_updvp_prcalc(const Group &g, int n, cudaStream_t s, bool pend, int slot);
 void glaunch_submean_boucqt(const Group &g, cudaStream_t s, bool deferred = false);
-void glaunch_loads(const Group &g, cudaStream_t s);
+void glaunch_loads(const Group &g, cudaStream_t s, bool pend = false);
 void glaunch_rigid(const Group &g, cudaStream_t s, int mode = RIGID_STEP);
 void glaunch_diag(const Group &g, cudaStream_t s);
 

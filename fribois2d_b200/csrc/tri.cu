@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "device.cuh"
 #include "pdl.h"
@@ -176,10 +177,17 @@ __device__ __forceinline__ void warp_line(double (&v)[M], int i0, int cnt, const
     bwd_apply(v, c, cnt, x);
 }
 
+// the barrier of one line's G warps (bar > 0: a named one), or the block's
+template <int G>
+__device__ __forceinline__ void line_sync(int bar) {
+    if (bar) asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(32 * G) : "memory");
+    else __syncthreads();
+}
+
 // G consecutive warps share one line (lane chunks in warp-major order);
 // warps exchange their chunk composites through sh (2 * G doubles per line).
 template <int M, int G, class Co>
-__device__ __forceinline__ void group_line(double (&v)[M], int i0, int cnt, const Co &co, double *sh) {
+__device__ __forceinline__ void group_line(double (&v)[M], int i0, int cnt, const Co &co, double *sh, int bar = 0) {
     const int lane = threadIdx.x & 31, gw = (threadIdx.x >> 5) % G;
     double c[M], A, C;
     co.loadA(c, i0, cnt);
@@ -201,14 +209,14 @@ __device__ __forceinline__ void group_line(double (&v)[M], int i0, int cnt, cons
         Aex = 1.0;
         Cex = 0.0;
     }
-    __syncthreads();
+    line_sync<G>(bar);
     double PC = 0.0;
     for (int q = 0; q < gw; ++q) PC = fma(sh[2 * q], PC, sh[2 * q + 1]);
     fwd_apply(v, c, cnt, fma(Aex, PC, Cex));
     co.loadG(c, i0, cnt);
     scale(v, c, cnt);
     co.loadE(c, i0, cnt);
-    __syncthreads();
+    line_sync<G>(bar);
     bwd_compose(v, c, cnt, A, C);
 #pragma unroll
     for (int dd = 1; dd < 32; dd <<= 1) {
@@ -228,7 +236,7 @@ __device__ __forceinline__ void group_line(double (&v)[M], int i0, int cnt, cons
         Aex = 1.0;
         Cex = 0.0;
     }
-    __syncthreads();
+    line_sync<G>(bar);
     double SC = 0.0;
     for (int q = G - 1; q > gw; --q) SC = fma(sh[2 * q], SC, sh[2 * q + 1]);
     bwd_apply(v, c, cnt, fma(Aex, SC, Cex));
@@ -402,84 +410,33 @@ __global__ void __launch_bounds__(kYLines * W * 32) k_ylines(Dev d, ScanSys s2, 
 
 // ---------------------------------------------------------------- Poisson modes
 
-// The per-mode y solves of phcalc (phcalc_outflow.F90:34-56): one warp per
-// mode.  The block copies the y off-diagonals once and each warp its mode's
-// right-hand side (a row of hmn) and reciprocal pivots to its own
+// The per-mode y solves of phcalc (phcalc_outflow.F90:34-56): W warps per
+// mode.  The block copies the y off-diagonals once and each mode's warps its
+// right-hand side (a row of hmn) and reciprocal pivots to the mode's own
 // shared-memory rows, all with cp.async in flight together (one wait instead
-// of a round trip per element group), then solves with lane chunks of
-// an odd length m (conflict-free 8-byte shared accesses): each lane composes
-// its chunk of the forward recurrence y(i) = a(i) y(i-1) + b(i),
-// a(i) = -amphj(i+1) g(i-1), the warp scans the composites, the lanes apply
-// them, scale by g(i), and do the same backward with
-// e(i) = -apphj(i+1) g(i); only warp-level synchronisation inside the
-// solve.  nw warps (modes) per block, as many as the shared memory holds.
-// one warp's mode: the forward and backward recurrences of the staged line
-// (in place), then the line stored to its row of hmn
-__device__ __forceinline__ void ymodes_solve(int n, int lane, const double *am, const double *ap, double *line,
-                                             const double *piv, double *row) {
-    const int m = ((n + 31) / 32) | 1;
-    const int i0 = min(lane * m, n), cnt = min(m, n - i0);
-    // forward: composite of the chunk, y_out = A y_in + C
-    double A = 1.0, C = 0.0;
-    for (int t = 0; t < cnt; ++t) {
-        const int i = i0 + t;
-        const double a = (i == 0) ? 0.0 : -(am[i + 1] * piv[i - 1]);
-        C = fma(a, C, line[i]);
-        A *= a;
-    }
-#pragma unroll
-    for (int dd = 1; dd < 32; dd <<= 1) {
-        const double Ao = __shfl_up_sync(kFull, A, dd), Co = __shfl_up_sync(kFull, C, dd);
-        if (lane >= dd) {
-            C = fma(A, Co, C);
-            A *= Ao;
-        }
-    }
-    double y = __shfl_up_sync(kFull, C, 1);
-    if (lane == 0) y = 0.0;
-    for (int t = 0; t < cnt; ++t) {
-        const int i = i0 + t;
-        const double a = (i == 0) ? 0.0 : -(am[i + 1] * piv[i - 1]);
-        y = fma(a, y, line[i]);
-        line[i] = piv[i] * y;   // g(i) y(i)
-    }
-    // backward: x(i) = e(i) x(i+1) + g(i) y(i)
-    A = 1.0;
-    C = 0.0;
-    for (int t = cnt - 1; t >= 0; --t) {
-        const int i = i0 + t;
-        const double e = (i == n - 1) ? 0.0 : -(ap[i + 1] * piv[i]);
-        C = fma(e, C, line[i]);
-        A *= e;
-    }
-#pragma unroll
-    for (int dd = 1; dd < 32; dd <<= 1) {
-        const double Ao = __shfl_down_sync(kFull, A, dd), Co = __shfl_down_sync(kFull, C, dd);
-        if (lane + dd < 32) {
-            C = fma(A, Co, C);
-            A *= Ao;
-        }
-    }
-    double x = __shfl_down_sync(kFull, C, 1);
-    if (lane == 31) x = 0.0;
-    for (int t = cnt - 1; t >= 0; --t) {
-        const int i = i0 + t;
-        const double e = (i == n - 1) ? 0.0 : -(ap[i + 1] * piv[i]);
-        x = fma(e, x, line[i]);
-        line[i] = x;
-    }
-    __syncwarp();
-    for (int i = lane; i < n; i += 32) row[i] = line[i];
-}
+// of a round trip per element group), then solves with lane chunks of an odd
+// length m (conflict-free 8-byte shared accesses): the forward recurrence
+// y(i) = a(i) y(i-1) + b(i), a(i) = -amphj(i+1) g(i-1), scaled by g(i), and the
+// backward one with e(i) = -apphj(i+1) g(i), each composed per chunk, scanned
+// over the chunks and applied.  A chunk and its coefficients stay in registers
+// (M >= m of them, every loop unrolled), so a step of a chain is one
+// dependent FMA: with the chunk in shared memory a step also waited for its
+// loads behind the step before's store, ~100 cycles, and the solve took 8.7 of
+// the 14.5 us between the launches before and after it at 1024 x 768 (9.9 us
+// now); W = 2 where one warp's chunk would not fit the registers.  nw modes
+// per block, as many as the shared memory holds.
 
 // rmax (may be null): the maxima of |hmn| over each row j (over the modes:
 // the rows of the INT8 transform's data operand) are accumulated into rmax[j]
 // from the block's modes, for the digit cut that follows
+template <int M, int W>
 __device__ __forceinline__ void ymodes_body(const Dev &d, int nw, double *rmax = nullptr) {
     extern __shared__ double sm[];
-    const int n = d.n2m, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __shared__ double shx[8][2 * W];
+    const int n = d.n2m, w = threadIdx.x / (32 * W), tl = threadIdx.x % (32 * W);
     double *am = sm, *ap = sm + (n + 2);                       // 1-based off-diagonals
-    double *line = sm + 2 * (n + 2) + static_cast<size_t>(w) * 2 * (n + 1);
+    double *lines = sm + 2 * (n + 2);
+    double *line = lines + static_cast<size_t>(w) * 2 * (n + 1);
     double *piv = line + (n + 1);
     // every copy of the block in flight at once (cp.async), one wait
     for (int i = threadIdx.x; i <= n + 1; i += blockDim.x) {
@@ -487,38 +444,58 @@ __device__ __forceinline__ void ymodes_body(const Dev &d, int nw, double *rmax =
         cp8(ap + i, d.apphj + i);
     }
     const int r = blockIdx.x * nw + w;
-    const bool live = (w < nw) && (r < d.n3m);
-    double *row = live ? d.hmn + static_cast<size_t>(r) * d.ldh : nullptr;
+    const bool live = r < d.n3m;
     if (live) {
-        const double *pgr = d.pg + static_cast<size_t>(r) * d.ldh;
-        for (int i = lane; i < n; i += 32) {
+        const double *row = d.hmn + static_cast<size_t>(r) * d.ldh, *pgr = d.pg + static_cast<size_t>(r) * d.ldh;
+        for (int i = tl; i < n; i += 32 * W) {
             cp8(line + i, row + i);
             cp8(piv + i, pgr + i);
         }
     }
     cp_wait();
     __syncthreads();   // the off-diagonals (and every line) are staged
-    if (live) ymodes_solve(n, lane, am, ap, line, piv, row);
-    if (!rmax) return;
-    __syncthreads();   // every live warp's solved line is in shared memory
-    const int nlive = max(0, min(nw, d.n3m - blockIdx.x * nw));
+    if (live) {
+        const int m = ((n + 32 * W - 1) / (32 * W)) | 1;
+        const int i0 = min(tl * m, n), cnt = min(m, n - i0);
+        double v[M];
+#pragma unroll
+        for (int t = 0; t < M; ++t)
+            if (t < cnt) v[t] = line[i0 + t];
+        const CoefModeS co{piv, am, ap, n};
+        if constexpr (W == 1) warp_line<M>(v, i0, cnt, co);
+        else group_line<M, W>(v, i0, cnt, co, shx[w], w + 1);
+#pragma unroll
+        for (int t = 0; t < M; ++t)
+            if (t < cnt) line[i0 + t] = v[t];
+    }
+    __syncthreads();   // every live mode's solved line is in shared memory
+    const int nlive = max(0, min(nw, d.n3m - static_cast<int>(blockIdx.x) * nw));
+    double *row0 = d.hmn + static_cast<size_t>(blockIdx.x) * nw * d.ldh;
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
         double mx = 0.0;
-        for (int q = 0; q < nlive; ++q)
-            mx = fmax(mx, fabs(sm[2 * (n + 2) + static_cast<size_t>(q) * 2 * (n + 1) + j]));
-        if (mx > 0.0) atomic_max_nonneg(rmax + j, mx);
+#pragma unroll 4
+        for (int q = 0; q < nlive; ++q) {
+            const double x = lines[static_cast<size_t>(q) * 2 * (n + 1) + j];
+            row0[static_cast<size_t>(q) * d.ldh + j] = x;
+            mx = fmax(mx, fabs(x));
+        }
+        if (rmax && mx > 0.0) atomic_max_nonneg(rmax + j, mx);
     }
 }
 
-__global__ void __launch_bounds__(256) k_ymodes(Dev d, int nw, double *rmax) {
+constexpr int ymodes_threads(int M, int W) { return W == 1 ? 256 : M <= 25 ? 512 : 384; }
+
+template <int M, int W>
+__global__ void __launch_bounds__(ymodes_threads(M, W), 1) k_ymodes(Dev d, int nw, double *rmax) {
     FB_GRID_WAIT();
-    ymodes_body(d, nw, rmax);
+    ymodes_body<M, W>(d, nw, rmax);
 }
 
-__global__ void __launch_bounds__(256) kg_ymodes(const GroupCase *__restrict__ g, int nw) {
+template <int M, int W>
+__global__ void __launch_bounds__(ymodes_threads(M, W), 1) kg_ymodes(const GroupCase *__restrict__ g, int nw) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    ymodes_body(d, nw);
+    ymodes_body<M, W>(d, nw);
 }
 
 // ---------------------------------------------------------------- z lines
@@ -944,6 +921,10 @@ cudaError_t allow_smem(K kern) {
 
 }  // namespace
 
+// shared memory of the mode solves: the 227 KB opt-in less the static arrays
+// (the grouped kernel's Dev, the warps' composites)
+constexpr int kYmSmem = 225 * 1024;
+
 cudaError_t scan_configure() {
     cudaError_t e;
 #define AL(K)                                  \
@@ -957,9 +938,14 @@ cudaError_t scan_configure() {
     AL((kg_helsolve_win<12, 32>)) AL((kg_helsolve_win<12, 64>))
     AL((kg_helsolve_win<16, 32>)) AL((kg_helsolve_win<16, 64>))
     AL((kg_helsolve_win<kWinMax, 32>)) AL((kg_helsolve_win<kWinMax, 64>))
-    if ((e = cudaFuncSetAttribute(k_ymodes, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(kg_ymodes, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024)) != cudaSuccess)
+#define YM(M, W)                                                                                                \
+    if ((e = cudaFuncSetAttribute(k_ymodes<M, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kYmSmem)) !=      \
+            cudaSuccess ||                                                                                      \
+        (e = cudaFuncSetAttribute(kg_ymodes<M, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kYmSmem)) !=     \
+            cudaSuccess)                                                                                        \
         return e;
+    YM(9, 1) YM(17, 1) YM(25, 1) YM(17, 2) YM(25, 2) YM(33, 2)
+#undef YM
 #undef AL
     return cudaSuccess;
 }
@@ -994,22 +980,37 @@ void launch_scan_helsolve(const Dev &d, const SubDev &s, cudaStream_t st) {
 }
 
 namespace {
-// modes per block and shared bytes of k_ymodes: as many warps as fit (<= 8)
-int ymodes_shape(const Dev &d, size_t *smem) {
+// modes per block and shared bytes of k_ymodes: as many as fit (<= 8, and the
+// thread limit of the chunk length's kernel)
+int ymodes_shape(const Dev &d, int M, int W, size_t *smem) {
     const size_t shared = 2 * static_cast<size_t>(d.n2m + 2) * sizeof(double);
     const size_t per = 2 * static_cast<size_t>(d.n2m + 1) * sizeof(double);
-    const size_t cap = 225u * 1024u;   // the 227 KB opt-in less the grouped kernel's static Dev
-    int nw = static_cast<int>(std::min<size_t>(8, (cap - shared) / per));
-    if (nw < 1) nw = 1;
+    int nw = static_cast<int>(std::min<size_t>(8, (kYmSmem - shared) / per));
+    nw = std::max(1, std::min(nw, ymodes_threads(M, W) / (32 * W)));
     *smem = shared + per * static_cast<size_t>(nw);
     return nw;
+}
+
+// calls go(M, W) as integral constants: chunks of M values on W warps per mode
+template <class F>
+void ymodes_form(const Dev &d, F go) {
+    const int n = d.n2m;
+    using std::integral_constant;
+    if (n <= 32 * 9) go(integral_constant<int, 9>{}, integral_constant<int, 1>{});
+    else if (n <= 32 * 17) go(integral_constant<int, 17>{}, integral_constant<int, 1>{});
+    else if (n <= 32 * 25) go(integral_constant<int, 25>{}, integral_constant<int, 1>{});
+    else if (n <= 64 * 17) go(integral_constant<int, 17>{}, integral_constant<int, 2>{});
+    else if (n <= 64 * 25) go(integral_constant<int, 25>{}, integral_constant<int, 2>{});
+    else go(integral_constant<int, 33>{}, integral_constant<int, 2>{});
 }
 }  // namespace
 
 void launch_scan_poisson(const Dev &d, cudaStream_t st, double *rmax) {
-    size_t smem = 0;
-    const int nw = ymodes_shape(d, &smem);
-    pdl(k_ymodes, dim3((d.n3m + nw - 1) / nw), dim3(32 * nw), smem, st, d, nw, rmax);
+    ymodes_form(d, [&](auto M, auto W) {
+        size_t smem = 0;
+        const int nw = ymodes_shape(d, M, W, &smem);
+        pdl(k_ymodes<M, W>, dim3((d.n3m + nw - 1) / nw), dim3(32 * W * nw), smem, st, d, nw, rmax);
+    });
 }
 
 template <int TK>
@@ -1038,9 +1039,11 @@ void glaunch_win_helsolve(const Group &g, int n, cudaStream_t st) {
 
 void glaunch_scan_poisson(const Group &g, cudaStream_t st) {
     const Dev &d = g.rep;
-    size_t smem = 0;
-    const int nw = ymodes_shape(d, &smem);
-    pdl(kg_ymodes, dim3((d.n3m + nw - 1) / nw, 1, g.n), dim3(32 * nw), smem, st, g.cases, nw);
+    ymodes_form(d, [&](auto M, auto W) {
+        size_t smem = 0;
+        const int nw = ymodes_shape(d, M, W, &smem);
+        pdl(kg_ymodes<M, W>, dim3((d.n3m + nw - 1) / nw, 1, g.n), dim3(32 * W * nw), smem, st, g.cases, nw);
+    });
 }
 
 }  // namespace fb
