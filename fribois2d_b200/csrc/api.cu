@@ -903,7 +903,9 @@ int phcalc_i8(fb_ctx *c) {
     // dph's row maxima come from divg, hmn's from the mode solves
     double *mx_dph = c->i8max, *mx_hmn = c->i8max + d.ldh;
     fb::launch_i8_cut_rows(d.dph + d.P, d.P, d.n2m, d.n3m, c->i8a, mx_dph, mx_hmn, st);
-    fb::launch_i8x8(c->i8a, c->i8f, d.hmn, d.ldh, d.status, st, true);   // i8f, i8b: cut once at set-up
+    // (i8f, i8b: cut once at set-up; the pivots for the mode solves that follow)
+    fb::launch_i8x8(c->i8a, c->i8f, d.hmn, d.ldh, d.status, st, true, d.pg,
+                    static_cast<size_t>(d.n3m) * d.ldh * sizeof(double));
     fb::launch_scan_poisson(d, st, mx_hmn);
     fb::launch_i8_cut_rows(d.hmn, d.ldh, d.n2m, d.n3m, c->i8a, mx_hmn, mx_dph, st);
     fb::launch_i8x8(c->i8a, c->i8b, d.dph + d.P, d.P, d.status, st, true);
@@ -1019,17 +1021,29 @@ int vardt_update(fb_ctx *c, int ns) {
 }
 
 // the marker set-up of substep 1 (nearest nodes, MLS weights, spreading
-// chains) on the side branch; it reads only marker data
-void enqueue_marker_setup(fb_ctx *c) {
+// chains); it reads only marker data
+void enqueue_marker_setup(fb_ctx *c, cudaStream_t st) {
     c->own_launches += 2;
-    fb::launch_mls_setup(c->d, c->side, true);
-    fb::launch_spread_chains(c->d, c->side);
+    fb::launch_mls_setup(c->d, st, true);
+    fb::launch_spread_chains(c->d, st);
 }
 
-// The substeps of one step, from nl_rhs to the last updvp, beside the side
-// branch that ends with ev_join (the marker set-up): the explicit terms of
-// substep 1 need no markers.  follows: the step before has not subtracted its
-// last pressure mean(s) yet.
+// the explicit terms of substep n, with boucdq and (substep 1 at fixed dt) cfl
+// on the same launch.  follows: the first substep of a step whose predecessor
+// has not subtracted its last pressure mean(s) yet.
+void enqueue_nl_rhs(fb_ctx *c, int ns, int n, bool follows, cudaStream_t st) {
+    double al, ga, ro;
+    coefs(c, ns, n, al, ga, ro);
+    const bool pend = (n == 1) ? follows : c->d.nsst == 3;
+    fb::launch_nl_rhs(c->d, al, ga, ro, st, pend, &c->nlmaps,
+                      fb::kNlBoucdq | (n == 1 && !c->vardt ? fb::kNlCfl : 0) | (follows ? fb::kNlMeans : 0));
+    c->own_launches += 1;
+}
+
+// The substeps of one step up to the last updvp, from nl_rhs of substep 1 on;
+// follows (as above): from the forcing of substep 1 on.  The side branch that
+// ends with ev_join (the marker set-up; follows: nl_rhs) joins before the
+// forcing of substep 1.
 int enqueue_substeps(fb_ctx *c, int ns, bool follows) {
     const Dev &d = c->d;
     int r;
@@ -1049,9 +1063,7 @@ int enqueue_substeps(fb_ctx *c, int ns, bool follows) {
         c->al = al;
         c->ga = ga;
         c->ro = ro;
-        fb::launch_nl_rhs(d, al, ga, ro, c->stream, pend, &c->nlmaps,
-                          fb::kNlBoucdq | (cfl ? fb::kNlCfl : 0) | (n == 1 && follows ? fb::kNlMeans : 0));
-        c->own_launches += 1;
+        if (n > 1 || !follows) enqueue_nl_rhs(c, ns, n, false, c->stream);
         if (d.nlm) {
             if (n == 1) CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
             // the weights are ready: interpolation and spreading only
@@ -1101,7 +1113,7 @@ int enqueue_fluid_start(fb_ctx *c, int ns) {
     if (c->vardt && (r = vardt_update(c, ns))) return r;
     if (c->d.nlm) {
         if ((r = fork_side(c))) return r;
-        enqueue_marker_setup(c);
+        enqueue_marker_setup(c, c->side);
         if ((r = end_side(c))) return r;
     }
     return enqueue_substeps(c, ns, false);
@@ -1112,9 +1124,9 @@ int enqueue_fluid(fb_ctx *c, int ns) {
     return r ? r : enqueue_fluid_end(c, ns);
 }
 
-int enqueue_report(fb_ctx *c, cudaStream_t st = nullptr) {
+int enqueue_report(fb_ctx *c) {
     if (!c->report || !c->d.nlm) return FB_OK;
-    fb::launch_diag(c->d, c->hist_cap, st ? st : c->stream);
+    fb::launch_diag(c->d, c->hist_cap, c->stream);
     c->own_launches += 1;
     return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
@@ -1129,22 +1141,42 @@ int enqueue_step(fb_ctx *c, int ns) {
     return FB_OK;
 }
 
-// The end of a step (loads, rigid, report: markers and one field pass) beside
-// the start of the next one.  nl_rhs of the next step needs nothing of it, and
-// its chain of small launches, followed by the next step's marker set-up, is
-// the longer of the two branches.
-int enqueue_next_step(fb_ctx *c) {
+// The end of a step behind its last updvp (loads, rigid update, report), the
+// next one's explicit terms (next) on the side branch behind the rigid update.
+// pend: the step's last pressure mean is still to be subtracted.
+int enqueue_step_end(fb_ctx *c, bool pend, bool next) {
+    const Dev &d = c->d;
+    const bool close = c->hc.deck.cbody && fb::step_closes(d.nlm);
     int r;
-    if ((r = fork_side(c))) return r;
-    if (c->hc.deck.cbody) {
-        fb::launch_loads(c->d, c->side, true);
+    if (close) {
+        fb::launch_loads_probe(d, c->stream, pend, true);
+        c->own_launches += 1;
+    } else if (c->hc.deck.cbody) {
+        fb::launch_loads(d, c->stream, pend);
         c->own_launches += 2;
     }
-    fb::launch_rigid(c->d, c->hist_cap, c->side);
+    if (close) fb::launch_step_close(d, c->hist_cap, c->stream);
+    else fb::launch_rigid(d, c->hist_cap, c->stream);
     c->own_launches += 1;
-    if ((r = enqueue_report(c, c->side))) return r;
-    enqueue_marker_setup(c);
-    if ((r = end_side(c))) return r;
+    if (next) {
+        if ((r = fork_side(c))) return r;
+        enqueue_nl_rhs(c, 1, 1, true, c->side);
+        if ((r = end_side(c))) return r;
+    }
+    CK(cudaGetLastError());
+    return enqueue_report(c);
+}
+
+// The end of a step and the next one up to its last updvp.  nl_rhs of the next
+// step needs nothing of the markers; it runs beside the next marker set-up.
+// (Beside the probes and the rigid update it held them up: its persistent
+// blocks kept the probes waiting, 28.9 us instead of 10 at 1024 x 768, and the
+// rigid update's one block, sharing its SM with them, took 19.6 us instead of 8.)
+int enqueue_next_step(fb_ctx *c) {
+    const int r = enqueue_step_end(c, true, true);
+    if (r) return r;
+    enqueue_marker_setup(c, c->stream);
+    CK(cudaGetLastError());
     return enqueue_substeps(c, 1, true);
 }
 
@@ -1201,9 +1233,10 @@ int capture_step(fb_ctx *c, int steps = 1) {
         c->own_launches = 0;
         if ((r = capture_exec(c, &c->head_exec, [&] { return enqueue_fluid_start(c, 1); })) ||
             (r = capture_exec(c, &c->tail_exec, [&] {
-                 int q;
-                 if ((q = enqueue_fluid_end(c, 1)) || (q = stage_impl(c, FB_ST_RIGID, 1, 1))) return q;
-                 return enqueue_report(c);
+                 // (Adams-Bashforth: the two other means are zero and stay so)
+                 fb::launch_submean_boucqt(c->d, c->stream, true);
+                 c->own_launches += 1;
+                 return enqueue_step_end(c, false, false);
              })))
             return r;
         c->step_kernels = c->own_launches;

@@ -355,7 +355,7 @@ __device__ __forceinline__ void nl_cell(const Dev &d, const Tile &t, int j0, int
         // alias the shared-memory tile and reuses the tile loads across the
         // thread's consecutive cells
         __stcg(d.rhs2 + i, (ga * dph + ro * ru + alre * dcq2 - dpx22) * dt);
-        __stcg(d.ru2 + i, dph);
+        __stcs(d.ru2 + i, dph);
     }
 
     // ---- w momentum at (jc, kc), kc = 2..n3m
@@ -389,7 +389,7 @@ __device__ __forceinline__ void nl_cell(const Dev &d, const Tile &t, int j0, int
         const size_t i = fidx(d, jc, kc);
         const double ru = ru3v;
         __stcg(d.rhs3 + i, (ga * qcap + ro * ru + alre * dcq3 - dpx33) * dt);
-        __stcg(d.ru3 + i, qcap);
+        __stcs(d.ru3 + i, qcap);
     }
 }
 #undef S2
@@ -492,7 +492,10 @@ __device__ __forceinline__ void nl_prefetch(const Dev &d, NlTile &t, int tile, i
     nl_prefetch_coef(d, t, j0, k0, tid);
 }
 
-// ru2/ru3 at this thread's cells of a tile (0 when ro = 0)
+// ru2/ru3 at this thread's cells of a tile (0 when ro = 0); read once per
+// substep and written once (nl_cell), both as streams, so that they do not push
+// the fields the next launches share out of L2 (with the pivots' prefetch in
+// the transform before the mode solves: 438 -> 435 us per step at 1024 x 768)
 __device__ __forceinline__ void nl_ru(const Dev &d, int tile, int ntj, double ro, double (&r2)[kNlK / 8],
                                       double (&r3)[kNlK / 8]) {
     const int jc = 1 + (tile % ntj) * kNlJ + threadIdx.x, k0 = 1 + (tile / ntj) * kNlK;
@@ -501,8 +504,8 @@ __device__ __forceinline__ void nl_ru(const Dev &d, int tile, int ntj, double ro
         const int kc = k0 + (kNlK / 8) * threadIdx.y + i;
         const bool ok = jc <= d.n2m && kc <= d.n3m && ro != 0.0;
         const size_t x = fidx(d, min(jc, d.n2m), min(kc, d.n3m));
-        r2[i] = ok ? d.ru2[x] : 0.0;
-        r3[i] = ok ? d.ru3[x] : 0.0;
+        r2[i] = ok ? __ldcs(d.ru2 + x) : 0.0;
+        r3[i] = ok ? __ldcs(d.ru3 + x) : 0.0;
     }
 }
 
@@ -759,67 +762,87 @@ __global__ void k_lgrdist(Dev d) {
     lgrdist_body(d);
 }
 
-// utils_math.f90:637-725 (GEsolve), n = 3, scaled partial pivoting
-__device__ __forceinline__ bool gesolve3(const double ai[3][3], const double bi[3], double x[3]) {
-    // every loop unrolled and the row exchange written per candidate row, so
-    // that the matrix stays in registers
-    double a[3][3], b[3], s[3];
+// utils_math.f90:637-725 (GEsolve), n = 3, scaled partial pivoting: the
+// elimination of the matrix, whose multipliers and row exchanges are kept so
+// that further right-hand sides take the same operations without repeating it
+// (the same results).  Every loop is unrolled and the row exchange written per
+// candidate row, so that the matrix stays in registers.
+struct GeLu {
+    double a[3][3];   // upper triangle
+    double c[2][3];   // multipliers c[k][i], i > k
+    int l[2];         // row exchanged with row k
+    bool ok;
+};
+
+__device__ __forceinline__ void ge_factor(const double ai[3][3], GeLu &f) {
+    f.ok = true;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        b[i] = bi[i];
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) a[i][j] = ai[i][j];
-    }
+        for (int j = 0; j < 3; ++j) f.a[i][j] = ai[i][j];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
+        double s[3];
 #pragma unroll
         for (int i = k; i < 3; ++i) {
             s[i] = 0.0;
 #pragma unroll
-            for (int j = k; j < 3; ++j) s[i] = fmax(s[i], fabs(a[i][j]));
+            for (int j = k; j < 3; ++j) s[i] = fmax(s[i], fabs(f.a[i][j]));
         }
-        double pivot = fabs(a[k][k] / s[k]);
+        double pivot = fabs(f.a[k][k] / s[k]);
         int l = k;
 #pragma unroll
         for (int j = k + 1; j < 3; ++j) {
-            double q = fabs(a[j][k] / s[j]);
+            const double q = fabs(f.a[j][k] / s[j]);
             if (q > pivot) {
                 pivot = q;
                 l = j;
             }
         }
-        if (pivot == 0.0) return false;
+        if (pivot == 0.0) f.ok = false;
+        f.l[k] = l;
 #pragma unroll
         for (int r = k + 1; r < 3; ++r) {
             if (l != r) continue;
 #pragma unroll
             for (int j = k; j < 3; ++j) {
-                double t = a[k][j];
-                a[k][j] = a[r][j];
-                a[r][j] = t;
+                const double t = f.a[k][j];
+                f.a[k][j] = f.a[r][j];
+                f.a[r][j] = t;
             }
-            double t = b[k];
+        }
+#pragma unroll
+        for (int i = k + 1; i < 3; ++i) {
+            const double c = f.a[i][k] / f.a[k][k];
+            f.c[k][i] = c;
+#pragma unroll
+            for (int j = k + 1; j < 3; ++j) f.a[i][j] = f.a[i][j] - c * f.a[k][j];
+        }
+    }
+}
+
+__device__ __forceinline__ void ge_apply(const GeLu &f, const double bi[3], double x[3]) {
+    double b[3] = {bi[0], bi[1], bi[2]};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+#pragma unroll
+        for (int r = k + 1; r < 3; ++r) {
+            if (f.l[k] != r) continue;
+            const double t = b[k];
             b[k] = b[r];
             b[r] = t;
         }
 #pragma unroll
-        for (int i = k + 1; i < 3; ++i) {
-            double c = a[i][k] / a[k][k];
-            a[i][k] = 0.0;
-            b[i] = b[i] - c * b[k];
-#pragma unroll
-            for (int j = k + 1; j < 3; ++j) a[i][j] = a[i][j] - c * a[k][j];
-        }
+        for (int i = k + 1; i < 3; ++i) b[i] = b[i] - f.c[k][i] * b[k];
     }
-    x[2] = b[2] / a[2][2];
+    x[2] = b[2] / f.a[2][2];
 #pragma unroll
     for (int i = 1; i >= 0; --i) {
         double c = 0.0;
 #pragma unroll
-        for (int j = i + 1; j < 3; ++j) c = c + a[i][j] * x[j];
-        x[i] = (b[i] - c) / a[i][i];
+        for (int j = i + 1; j < 3; ++j) c = c + f.a[i][j] * x[j];
+        x[i] = (b[i] - c) / f.a[i][i];
     }
-    return true;
 }
 
 // MLSint.F90:406-486 (one axis of the weight function) and its derivative
@@ -869,12 +892,31 @@ __device__ void wkernel(int wfun, double difc, double sdds, double &wc, double &
 // carries on with its loads and stores switched off.
 constexpr int kNodeLanes = 16;
 
-// x summed over the group's first kSD lanes in lane order, on every lane
-__device__ __forceinline__ double group_sum_nodes(double x, int base) {
-    double s = 0.0;
+// N sums over the group's nodes through shared memory (buf: 10 N doubles of the
+// group's own): lane i forms sums i, i + kNodeLanes, ... from the nine terms the nodes
+// left there, in node order, and every lane reads them back.  One shuffle and
+// addition after another per sum (18 of them for a probe) was most of the
+// instructions of these latency-bound kernels.
+template <int N>
+__device__ __forceinline__ void group_sums(double (&x)[N], int m, double *buf) {
+    __syncwarp();   // (the buffer's earlier values are read)
+    if (m < kSD)
 #pragma unroll
-    for (int mm = 0; mm < kSD; ++mm) s = s + __shfl_sync(0xffffffffu, x, base + mm);
-    return s;
+        for (int i = 0; i < N; ++i) buf[i * kSD + m] = x[i];
+    __syncwarp();
+#pragma unroll
+    for (int i0 = 0; i0 < N; i0 += kNodeLanes) {
+        const int i = i0 + m;
+        if (i < N) {
+            double s = 0.0;
+#pragma unroll
+            for (int q = 0; q < kSD; ++q) s = s + buf[i * kSD + q];
+            buf[N * kSD + i] = s;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = buf[N * kSD + i];
 }
 
 // the group's lane index of the least v, the first of equal values (as a
@@ -918,12 +960,15 @@ __device__ __forceinline__ void sd_axes(const Dev &d, int idir, const double *&y
 // (lgrdistribution.F90:189-267), one per lane, in place of a launch of its own
 // whose threads made the four searches of a marker one after another; the
 // spreading table is empty then (k_mls_interp empties it behind the chains).
+constexpr int kSetupThreads = 128;
 template <bool kFind>
 __device__ __forceinline__ void mls_setup_body(const Dev &d) {
     if (!d.nlm) return;
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = T / kNodeLanes, m = T % kNodeLanes;
     const int base = (threadIdx.x & 31) & ~(kNodeLanes - 1);
+    __shared__ double bufs[kSetupThreads / kNodeLanes][10 * 6];
+    double *buf = bufs[threadIdx.x / kNodeLanes];
     const bool have = t < 2 * d.nlm;
     const int tt = have ? t : 0;
     const int n = tt >> 1, idir = (tt & 1) + 1;
@@ -987,26 +1032,30 @@ __device__ __forceinline__ void mls_setup_body(const Dev &d) {
         w = wc0 * wc1;
     }
     const double pk[3] = {1.0, sc0, sc1};
-    double A[3][3];
+    double mom[6];   // pk[a] pk[b] = pk[b] pk[a]: the same terms, the same sums
+    int q = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int b = 0; b < 3; ++b)   // pk[a] pk[b] = pk[b] pk[a]: the same terms, the same sums
-            A[a][b] = (b < a) ? A[b][a] : group_sum_nodes(w * (pk[a] * pk[b]), base);
+        for (int b = a; b < 3; ++b) mom[q++] = w * (pk[a] * pk[b]);
+    group_sums<6>(mom, m, buf);
+    const double A[3][3] = {{mom[0], mom[1], mom[2]}, {mom[1], mom[3], mom[4]}, {mom[2], mom[4], mom[5]}};
     const double gps[3] = {1.0, pos[0], pos[1]};
     double ptA[3];
-    gesolve3(A, gps, ptA);
+    GeLu lu;
+    ge_factor(A, lu);
+    ge_apply(lu, gps, ptA);
     const double B0 = 1.0 * w, B1 = sc0 * w, B2 = sc1 * w;
     double ph = 0.0;
     ph = ph + ptA[0] * B0;
     ph = ph + ptA[1] * B1;
     ph = ph + ptA[2] * B2;
-    const double sumphi = group_sum_nodes(ph, base);
-    if (good && m == 0 && !(fabs(1.0 - fabs(sumphi)) <= 1.0e-10)) raise_status(d, FB_ERR_MLS);
     const double vol = sd0 * sd1;
-    const double dvel = group_sum_nodes(ph * vol, base);
-    const double lgr_h = group_sum_nodes(1.0 / 2.0 * ph * (sd0 + sd1), base);
-    if (!good) return;   // (after the group's last shuffle)
+    double sums[3] = {ph, ph * vol, 1.0 / 2.0 * ph * (sd0 + sd1)};
+    group_sums<3>(sums, m, buf);
+    const double sumphi = sums[0], dvel = sums[1], lgr_h = sums[2];
+    if (good && m == 0 && !(fabs(1.0 - fabs(sumphi)) <= 1.0e-10)) raise_status(d, FB_ERR_MLS);
+    if (!good) return;   // (after the group's last exchange)
     if (node) {
         phi[m] = ph;
         eu[m] = ej;
@@ -1744,12 +1793,15 @@ constexpr int kLoadThreads = 3 * kLoadMk * kLoadLanes;
 
 // pend: the step's last pressure mean is still to be subtracted from pr; the
 // value is the one pr_submean would have stored.
-__device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend) {
+// vals (may be null): the block's markers' values in shared memory, 24 each
+__device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double *vals) {
     constexpr unsigned kAll = 0xffffffffu;
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = T / kLoadLanes, m = T % kLoadLanes;
     const int base = (threadIdx.x & 31) & ~(kLoadLanes - 1);
+    __shared__ double bufs[3 * kLoadMk][10 * 18];
+    double *buf = bufs[threadIdx.x / kLoadLanes];
     const bool have = t < 3 * d.nlm;
     const int tt = have ? t : 0;
     const int n = tt / 3, idir = tt % 3 + 1;
@@ -1760,6 +1812,7 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend) {
     if (have && m == 0) {
         if (idir == 1) {
             pb[23] = inside ? 0.0 : -1.0;
+            if (vals) vals[24 * (threadIdx.x / (3 * kLoadLanes)) + 23] = inside ? 0.0 : -1.0;
             d.bcerrv[n] = 0.0;
         }
         if (idir == 2) d.bcerrw[n] = 0.0;
@@ -1774,11 +1827,6 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend) {
         const int *eu = d.eulins + static_cast<size_t>(t2) * 2 * kSD;
         const double *q = (idir == 1) ? d.q2 : d.q3;
         prod = d.phi[static_cast<size_t>(t2) * kSD + m] * q[fidx(d, eu[m], eu[kSD + m])];
-    }
-    const double u = group_sum_nodes(prod, base);
-    if (ok && idir <= 2 && m == 0) {
-        if (idir == 1) d.bcerrv[n] = d.lmvel[2 * n] - u;
-        else d.bcerrw[n] = d.lmvel[2 * n + 1] - u;
     }
 
     const double hpr = d.ddmin * d.kprobe;
@@ -1854,47 +1902,50 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend) {
         w2 = wc[0] * dw[1];
     }
     const double pk[3] = {1.0, sc0, sc1};
-    double A[3][3][3];
+    // the moments of the weights and of their two derivatives; pk[a] pk[b] =
+    // pk[b] pk[a]: the same terms, the same sums
+    double mom[18];
+    int q = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            if (b < a) {   // pk[a] pk[b] = pk[b] pk[a]: the same terms, the same sums
-#pragma unroll
-                for (int l = 0; l < 3; ++l) A[a][b][l] = A[b][a][l];
-                continue;
-            }
+        for (int b = a; b < 3; ++b) {
             const double pp = pk[a] * pk[b];
-            A[a][b][0] = group_sum_nodes(w0 * pp, base);
-            A[a][b][1] = group_sum_nodes(w1 * pp, base);
-            A[a][b][2] = group_sum_nodes(w2 * pp, base);
+            mom[q] = w0 * pp;
+            mom[6 + q] = w1 * pp;
+            mom[12 + q] = w2 * pp;
+            ++q;
         }
-    double Aa[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) Aa[a][b] = A[a][b][0];
+    group_sums<18>(mom, m, buf);
+    const double Aa[3][3] = {{mom[0], mom[1], mom[2]}, {mom[1], mom[3], mom[4]}, {mom[2], mom[4], mom[5]}};
+    GeLu lu;
+    ge_factor(Aa, lu);
     double gam[3][3];
     const double gps[3] = {1.0, probe[0], probe[1]};
     double g0[3];
-    gesolve3(Aa, gps, g0);
-#pragma unroll
-    for (int l = 1; l <= 2; ++l) {
+    ge_apply(lu, gps, g0);
+    {
+        // the two derivatives' systems on the group's two halves
+        const int l = (m < kNodeLanes / 2) ? 1 : 2;
+        const double *ml = buf + 18 * kSD + 6 * l;   // (the sums, where group_sums left them)
+        const double Al[3][3] = {{ml[0], ml[1], ml[2]}, {ml[1], ml[3], ml[4]}, {ml[2], ml[4], ml[5]}};
         double C[3], gx[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             double acc = 0.0;
 #pragma unroll
-            for (int b = 0; b < 3; ++b) acc = acc + A[a][b][l] * g0[b];
+            for (int b = 0; b < 3; ++b) acc = acc + Al[a][b] * g0[b];
             const double gpl = (a == l) ? 1.0 : 0.0;
             C[a] = gpl - acc;
         }
-        gesolve3(Aa, C, gx);
+        ge_apply(lu, C, gx);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) gam[a][l] = gx[a];
+        for (int a = 0; a < 3; ++a) {
+            gam[a][0] = g0[a];
+            gam[a][1] = __shfl_sync(kAll, gx[a], base);
+            gam[a][2] = __shfl_sync(kAll, gx[a], base + kNodeLanes / 2);
+        }
     }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) gam[a][0] = g0[a];
     double p0 = 0.0, p1 = 0.0, p2 = 0.0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -1903,11 +1954,9 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend) {
         p1 = p1 + gam[a][1] * B0 + gam[a][0] * B1;
         p2 = p2 + gam[a][2] * B0 + gam[a][0] * B2;
     }
-    const double sumphi = group_sum_nodes(p0, base);
-    if (good && m == 0 && !(fabs(1.0 - fabs(sumphi)) <= 1.0e-10)) raise_status(d, FB_ERR_MLS);
-
-    // getpbup (loads_transfer.F90:285-357) for this quantity
-    double o[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    // getpbup (loads_transfer.F90:285-357) for this quantity; the last two: the
+    // partition of unity and checkbcs's velocity
+    double o[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, p0, prod};
     if (act) {
         const double uk1 = (f0 - fym) * d.dx2 / g2r;
         const double uk2 = (f0 - fzm) * d.dx3 / g3r;
@@ -1919,44 +1968,103 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend) {
         o[5] = p2 * uk1;
         o[6] = p2 * uk2;
     }
-    double res = 0.0;
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        const double s = group_sum_nodes(o[i], base);
-        if (m == i) res = s;
+    group_sums<9>(o, m, buf);
+    if (good && m == 0 && !(fabs(1.0 - fabs(o[7])) <= 1.0e-10)) raise_status(d, FB_ERR_MLS);
+    if (ok && idir <= 2 && m == 0) {
+        if (idir == 1) d.bcerrv[n] = d.lmvel[2 * n] - o[8];
+        else d.bcerrw[n] = d.lmvel[2 * n + 1] - o[8];
     }
-    if (good && m < 7) pb[7 * (idir - 1) + m] = res;
+    const double res = buf[9 * kSD + min(m, 8)];   // sum m
+    if (good && m < 7) {
+        pb[7 * (idir - 1) + m] = res;
+        if (vals) vals[24 * (threadIdx.x / (3 * kLoadLanes)) + 7 * (idir - 1) + m] = res;
+    }
+}
+
+// loads_transfer.F90:187-214 for marker n with probe values pb (ucy, ucz, pc of
+// seven each) and tangent (tany, tanz): pressure extrapolation (Wang et al.
+// 2019 eq. 20) and wall shear (eq. 26)
+__device__ __forceinline__ void finish_marker(const Dev &d, int n, const double *pb, double tany, double tanz,
+                                              double &press, double (&tau)[2]) {
+    const double hpr = d.ddmin * d.kprobe, visc = d.visc;
+    const double *ucy = pb, *ucz = pb + 7, *pc = pb + 14;
+    const double nory = d.lmnor[2 * n], norz = d.lmnor[2 * n + 1];
+    double dpdnw = d.lmacc[2 * n] * nory + d.lmacc[2 * n + 1] * norz;
+    dpdnw = -1.0 * dpdnw;
+    const double dpdne = pc[1] * nory + pc[2] * norz;
+    press = pc[0] - 0.5 * (dpdnw + dpdne) * hpr;
+    const double ducdn = (ucy[1] * tany * nory + ucy[2] * tany * norz + ucz[1] * tanz * nory +
+                          ucz[2] * tanz * norz);
+    const double d3ucdn3 = (pc[3] * nory * nory + pc[4] * nory * norz + pc[5] * norz * nory +
+                            pc[6] * norz * norz) * 1.0 / visc;
+    const double d2ucdn2 = (ucy[3] * tany * nory * nory + ucy[4] * tany * nory * norz +
+                            ucy[5] * tany * norz * nory + ucy[6] * tany * norz * norz +
+                            ucz[3] * tanz * nory * nory + ucz[4] * tanz * nory * norz +
+                            ucz[5] * tanz * norz * nory + ucz[6] * tanz * norz * norz);
+    const double ducdnm = ducdn - d2ucdn2 * hpr - 0.5 * d3ucdn3 * (hpr * hpr);
+    tau[0] = visc * ducdnm * tany;
+    tau[1] = visc * ducdnm * tanz;
+}
+
+// the tangent of the last marker up to n that has one of its own (zero if none)
+__device__ __forceinline__ void carried_tangent(const Dev &d, int n, double &tany, double &tanz) {
+    for (int m = n; m >= 0; --m) {
+        const double *pm = d.probe + static_cast<size_t>(m) * 24;
+        if (pm[23] > 0.5) {
+            tany = pm[21];
+            tanz = pm[22];
+            return;
+        }
+    }
 }
 
 // the probes of kLoadMk markers per block, then each probed marker's own
-// tangent (loads_transfer.F90:177-185) from its first two probes
+// tangent (loads_transfer.F90:177-185) from its first two probes.  kFinish: a
+// marker with a tangent of its own is finished here (press, tau), one outside
+// the channel gets zeros, and only those whose tangent carries over from
+// another marker are left to the launch that sums the loads.
+template <bool kFinish>
 __device__ __forceinline__ void loads_probe_tan_body(const Dev &d, bool pend) {
     if (!d.nlm) return;
-    loads_probe_body(d, pend);
+    __shared__ double vals[kLoadMk][24];
+    loads_probe_body(d, pend, kFinish ? &vals[0][0] : nullptr);
     __syncthreads();
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = T / kLoadLanes;
     if (t >= 3 * d.nlm || t % 3 != 0 || T % kLoadLanes != 0 || *d.status) return;
     const int n = t / 3;
     double *pb = d.probe + static_cast<size_t>(n) * 24;
-    if (pb[23] < 0.0) return;
-    const double nory = d.lmnor[2 * n], norz = d.lmnor[2 * n + 1];
-    const double vel0 = pb[0], vel1 = pb[7];
-    const double veln_md = vel0 * nory + vel1 * norz;
-    const double velt0 = vel0 - veln_md * nory, velt1 = vel1 - veln_md * norz;
-    const double velt_md = sqrt(velt0 * velt0 + velt1 * velt1);
-    if (velt_md != 0.0) {
-        pb[21] = velt0 / sqrt(velt0 * velt0 + velt1 * velt1);
-        pb[22] = velt1 / sqrt(velt0 * velt0 + velt1 * velt1);
-        pb[23] = 1.0;
-    } else {
-        pb[23] = 0.0;
+    const double *pv = kFinish ? vals[threadIdx.x / (3 * kLoadLanes)] : pb;
+    double press = 0.0, tau[2] = {0.0, 0.0};
+    bool done = true;
+    if (pv[23] >= 0.0) {
+        const double nory = d.lmnor[2 * n], norz = d.lmnor[2 * n + 1];
+        const double vel0 = pv[0], vel1 = pv[7];
+        const double veln_md = vel0 * nory + vel1 * norz;
+        const double velt0 = vel0 - veln_md * nory, velt1 = vel1 - veln_md * norz;
+        const double velt_md = sqrt(velt0 * velt0 + velt1 * velt1);
+        if (velt_md != 0.0) {
+            const double tany = velt0 / velt_md, tanz = velt1 / velt_md;
+            pb[21] = tany;
+            pb[22] = tanz;
+            pb[23] = 1.0;
+            if (kFinish) finish_marker(d, n, pv, tany, tanz, press, tau);
+        } else {
+            pb[23] = 0.0;
+            done = false;
+        }
+    }
+    if (kFinish && done) {
+        d.press[n] = press;
+        d.tau[2 * n] = tau[0];
+        d.tau[2 * n + 1] = tau[1];
     }
 }
 
+template <bool kFinish>
 __global__ void __launch_bounds__(kLoadThreads, 5) k_loads_probe(Dev d, int pend) {
     FB_GRID_WAIT();
-    loads_probe_tan_body(d, pend != 0);
+    loads_probe_tan_body<kFinish>(d, pend != 0);
 }
 
 // loads_transfer_c (loads_transfer.F90:187-214): the tangent carries over
@@ -1966,43 +2074,20 @@ __global__ void __launch_bounds__(kLoadThreads, 5) k_loads_probe(Dev d, int pend
 __device__ __forceinline__ void loads_finish_body(const Dev &d) {
     __shared__ double sh[32];
     __shared__ bool last;
-    const double hpr = d.ddmin * d.kprobe, visc = d.visc;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     double sv = 0.0, sw = 0.0;
     if (n < d.nlm) {
         const double *pb = d.probe + static_cast<size_t>(n) * 24;
         if (*d.status == 0) {
-            d.press[n] = 0.0;
-            d.tau[2 * n] = 0.0;
-            d.tau[2 * n + 1] = 0.0;
+            double press = 0.0, tau[2] = {0.0, 0.0};
             if (pb[23] >= 0.0) {
                 double tany = 0.0, tanz = 0.0;
-                for (int m = n; m >= 0; --m) {   // the last marker up to n with a tangent of its own
-                    const double *pm = d.probe + static_cast<size_t>(m) * 24;
-                    if (pm[23] > 0.5) {
-                        tany = pm[21];
-                        tanz = pm[22];
-                        break;
-                    }
-                }
-                const double *ucy = pb, *ucz = pb + 7, *pc = pb + 14;
-                const double nory = d.lmnor[2 * n], norz = d.lmnor[2 * n + 1];
-                double dpdnw = d.lmacc[2 * n] * nory + d.lmacc[2 * n + 1] * norz;
-                dpdnw = -1.0 * dpdnw;
-                const double dpdne = pc[1] * nory + pc[2] * norz;
-                d.press[n] = pc[0] - 0.5 * (dpdnw + dpdne) * hpr;
-                const double ducdn = (ucy[1] * tany * nory + ucy[2] * tany * norz + ucz[1] * tanz * nory +
-                                      ucz[2] * tanz * norz);
-                const double d3ucdn3 = (pc[3] * nory * nory + pc[4] * nory * norz + pc[5] * norz * nory +
-                                        pc[6] * norz * norz) * 1.0 / visc;
-                const double d2ucdn2 = (ucy[3] * tany * nory * nory + ucy[4] * tany * nory * norz +
-                                        ucy[5] * tany * norz * nory + ucy[6] * tany * norz * norz +
-                                        ucz[3] * tanz * nory * nory + ucz[4] * tanz * nory * norz +
-                                        ucz[5] * tanz * norz * nory + ucz[6] * tanz * norz * norz);
-                const double ducdnm = ducdn - d2ucdn2 * hpr - 0.5 * d3ucdn3 * (hpr * hpr);
-                d.tau[2 * n] = visc * ducdnm * tany;
-                d.tau[2 * n + 1] = visc * ducdnm * tanz;
+                carried_tangent(d, n, tany, tanz);
+                finish_marker(d, n, pb, tany, tanz, press, tau);
             }
+            d.press[n] = press;
+            d.tau[2 * n] = tau[0];
+            d.tau[2 * n + 1] = tau[1];
         }
         sv = d.bcerrv[n] * d.bcerrv[n];
         sw = d.bcerrw[n] * d.bcerrw[n];
@@ -2055,6 +2140,155 @@ __device__ void modfn(double K[6], const double t[6], const double FF[6], const 
     }
 }
 
+// explicit RK4 (kinem_RK4) with loads frozen over the stages: the three degrees
+// of freedom i (y, z, rotation) are independent (modfn); xns[i], xns[3 + i] are
+// the new displacement and velocity
+__device__ __forceinline__ void rigid_rk4(const Dev &d, int i, const double *rs, double Fy, double Fz, double M,
+                                          double *xns) {
+    const double dt = d.dt;
+    const double csp = (i == 0) ? d.cmposi0 : (i == 1 ? d.cmposi1 : d.cmroti);
+    double FFi, Mii;
+    if (i == 0) {
+        if (d.rtcoup) {
+            FFi = Fy + M / d.rrr;
+            Mii = 1.0 / ((d.rba1 / (d.rrr * d.rrr) + d.rba0) * d.rbden);
+        } else {
+            FFi = Fy;
+            Mii = 1.0 / (d.rba0 * d.rbden);
+        }
+    } else if (i == 1) {
+        FFi = Fz;
+        Mii = 1.0 / (d.rba0 * d.rbden);
+    } else {
+        FFi = M;
+        Mii = 1.0 / (d.rba1 * d.rbden);
+    }
+    const double kk = d.kk[i], cc = d.cc[i], kk3 = d.kk3[i];
+    // modfn (rigid.F90) for component i: K_x = v, K_v = Mi (-kk x + -cc v + -kk3 x^3 + F)
+    auto mod = [&](double x, double v, double &kx, double &kv) {
+        const double cube = x * x * x;
+        const double lin = -kk * x + -cc * v;
+        const double rhs = lin + -kk3 * cube + FFi;
+        kx = v;
+        kv = Mii * rhs;
+    };
+    const double xo = rs[i] - csp, vo = rs[3 + i];
+    double k1x, k1v, k2x, k2v, k3x, k3v, k4x, k4v;
+    mod(xo, vo, k1x, k1v);
+    mod(xo + k1x * dt / 2.0, vo + k1v * dt / 2.0, k2x, k2v);
+    mod(xo + k2x * dt / 2.0, vo + k2v * dt / 2.0, k3x, k3v);
+    mod(xo + k3x * dt, vo + k3v * dt, k4x, k4v);
+    xns[i] = xo + dt * (k1x / 6.0 + k2x / 3.0 + k3x / 3.0 + k4x / 6.0);
+    xns[3 + i] = vo + dt * (k1v / 6.0 + k2v / 3.0 + k3v / 3.0 + k4v / 6.0);
+}
+
+// the body's state cm[0..17] (rigid layout) after the RK4 update xn, and the
+// rotation matrix of the step (get_rotmat); one thread
+__device__ __forceinline__ void rigid_state(const Dev &d, const double *rs, const double *xns, const double *kin,
+                                            const int *mcon, double *cm, double *rot) {
+    const double dt = d.dt;
+    const double csp[3] = {d.cmposi0, d.cmposi1, d.cmroti};
+    double xn[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) xn[i] = xns[i];
+    // P1, V1, A1 (rigid[9..17]) formed in shared memory (cm)
+    for (int i = 0; i < 18; ++i) cm[i] = rs[i];
+    double *P1 = cm + 9, *V1 = cm + 12, *A1 = cm + 15;
+    if (!d.rtcoup) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            P1[i] = csp[i] + xn[i];
+            V1[i] = xn[3 + i];
+            A1[i] = (V1[i] - rs[3 + i]) / dt;
+        }
+    } else {
+        P1[0] = csp[0] + xn[0];
+        V1[0] = xn[3];
+        A1[0] = (V1[0] - rs[3]) / dt;
+        P1[1] = csp[1];
+        V1[1] = 0.0;
+        A1[1] = 0.0;
+        P1[2] = csp[2] + xn[0] / d.rrr;
+        V1[2] = V1[0] / d.rrr;
+        A1[2] = A1[2] / d.rrr;  // as rigid.F90:296 (incoming value / rr)
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (mcon[i] == 1) {
+            P1[i] = kin[i];
+            V1[i] = kin[3 + i];
+            A1[i] = kin[6 + i];
+        }
+    const double cmrot = P1[2] - rs[2];
+    double sn, cs;
+    sincos(cmrot, &sn, &cs);
+    rot[0] = cs;
+    rot[1] = -sn;
+    rot[2] = sn;
+    rot[3] = cs;
+}
+
+// a marker (y, z) carried by the body's motion P0 -> P1 (kinematics of
+// rigid.F90:75-108): new position, velocity, acceleration
+__device__ __forceinline__ void move_marker(const double *cm, const double *rot, double y, double z, double (&pos)[2],
+                                            double (&vel)[2], double (&acc)[2]) {
+    const double *P0 = cm, *P1 = cm + 9, *V1 = cm + 12, *A1 = cm + 15;
+    const double rho0 = y - P0[0], rho1 = z - P0[1];
+    const double c10 = -V1[2] * rho1, c11 = V1[2] * rho0;
+    const double c20 = -A1[2] * rho1, c21 = A1[2] * rho0;
+    const double c30 = -V1[2] * c11, c31 = V1[2] * c10;
+    pos[0] = P1[0] + (rot[0] * rho0 + rot[1] * rho1);
+    pos[1] = P1[1] + (rot[2] * rho0 + rot[3] * rho1);
+    vel[0] = V1[0] + c10;
+    vel[1] = V1[1] + c11;
+    acc[0] = A1[0] + c20 + c30;
+    acc[1] = A1[1] + c21 + c31;
+}
+
+// a vertex rotated about the updated centre (rigid.F90:110-121)
+__device__ __forceinline__ void move_vertex(const double *cm, const double *rot, const double *v, double (&o)[2]) {
+    const double *P1 = cm + 9;
+    const double rho0 = v[0] - P1[0], rho1 = v[1] - P1[1];
+    o[0] = P1[0] + (rot[0] * rho0 + rot[1] * rho1);
+    o[1] = P1[1] + (rot[2] * rho0 + rot[3] * rho1);
+}
+
+// createnorm (rigid.F90:468-495): the normal of the segment a -> b
+__device__ __forceinline__ void segment_normal(const double *a, const double *b, double (&nor)[2]) {
+    const double v1[3] = {0.0 - 0.0, b[0] - a[0], b[1] - a[1]};
+    const double v2[3] = {-1.0 - 0.0, (a[0] + b[0]) * 0.5 - a[0], (a[1] + b[1]) * 0.5 - a[1]};
+    const double c0 = v1[1] * v2[2] - v1[2] * v2[1];
+    const double c1 = v1[2] * v2[0] - v1[0] * v2[2];
+    const double c2 = v1[0] * v2[1] - v1[1] * v2[0];
+    const double den = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
+    nor[0] = c1 / den;
+    nor[1] = c2 / den;
+}
+
+// the end of a step (one thread): body state, clock (main.F90:92), history row
+__device__ __forceinline__ void commit_step(const Dev &d, int hist_rows, const double *cm, const double (&fv)[8],
+                                            double t0, double stepd, double nbcv, double nbcw, double cflm,
+                                            double solves) {
+    for (int i = 0; i < 9; ++i) d.rigid[i] = cm[9 + i];
+    const double t1 = t0 + d.dt;
+    d.scal[S_TIME] = t1;
+    const int row = static_cast<int>(stepd);
+    if (hist_rows > 0) {
+        double *h = d.hist + static_cast<size_t>(row % hist_rows) * FB_HIST_COLS;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h[i] = fv[i];
+        h[8] = t1;
+        for (int i = 0; i < 9; ++i) h[9 + i] = cm[9 + i];
+        h[18] = nbcv;
+        h[19] = nbcw;
+        h[20] = cflm;
+        h[21] = d.dt;
+        for (int i = 22; i < FB_HIST_COLS; ++i) h[i] = 0.0;  // diagnostics, when enabled
+        h[30] = solves;
+    }
+    d.scal[S_STEP] = static_cast<double>(row + 1);
+}
+
 // rigid.F90:4-138 (rigid) with int_stress :373-464, kinem_RK4 :165-228 /
 // kinem_RK4i :233-299, get_rotmat :142-161, createnorm :468-495; then the
 // clock update of main.F90:92 and one history row.  Single block.
@@ -2103,7 +2337,7 @@ __device__ __forceinline__ void rigid_body(const Dev &d, int hist_rows, int mode
         mom = f[4];
     }
     // the loads of the step (every thread forms the same values)
-    const double time = d.scal[S_TIME], dt = d.dt;
+    const double time = d.scal[S_TIME];
     double Fy, Fz, M;
     if (from_loads) {
         const double fy = fyp + fyv, fz = fzp + fzv;
@@ -2127,84 +2361,10 @@ __device__ __forceinline__ void rigid_body(const Dev &d, int hist_rows, int mode
         d.forces[6] = fyv;
         d.forces[7] = fzv;
     }
-    // explicit RK4 with loads frozen over the stages: the three degrees of
-    // freedom (y, z, rotation) are independent (modfn), one thread each
-    if (tid < 3) {
-        const int i = tid;
-        const double csp = (i == 0) ? d.cmposi0 : (i == 1 ? d.cmposi1 : d.cmroti);
-        double FFi, Mii;
-        if (i == 0) {
-            if (d.rtcoup) {
-                FFi = Fy + M / d.rrr;
-                Mii = 1.0 / ((d.rba1 / (d.rrr * d.rrr) + d.rba0) * d.rbden);
-            } else {
-                FFi = Fy;
-                Mii = 1.0 / (d.rba0 * d.rbden);
-            }
-        } else if (i == 1) {
-            FFi = Fz;
-            Mii = 1.0 / (d.rba0 * d.rbden);
-        } else {
-            FFi = M;
-            Mii = 1.0 / (d.rba1 * d.rbden);
-        }
-        const double kk = d.kk[i], cc = d.cc[i], kk3 = d.kk3[i];
-        // modfn (rigid.F90) for component i: K_x = v, K_v = Mi (-kk x + -cc v + -kk3 x^3 + F)
-        auto mod = [&](double x, double v, double &kx, double &kv) {
-            const double cube = x * x * x;
-            const double lin = -kk * x + -cc * v;
-            const double rhs = lin + -kk3 * cube + FFi;
-            kx = v;
-            kv = Mii * rhs;
-        };
-        const double xo = rs[i] - csp, vo = rs[3 + i];
-        double k1x, k1v, k2x, k2v, k3x, k3v, k4x, k4v;
-        mod(xo, vo, k1x, k1v);
-        mod(xo + k1x * dt / 2.0, vo + k1v * dt / 2.0, k2x, k2v);
-        mod(xo + k2x * dt / 2.0, vo + k2v * dt / 2.0, k3x, k3v);
-        mod(xo + k3x * dt, vo + k3v * dt, k4x, k4v);
-        xns[i] = xo + dt * (k1x / 6.0 + k2x / 3.0 + k3x / 3.0 + k4x / 6.0);
-        xns[3 + i] = vo + dt * (k1v / 6.0 + k2v / 3.0 + k3v / 3.0 + k4v / 6.0);
-    }
+    if (tid < 3) rigid_rk4(d, tid, rs, Fy, Fz, M, xns);
     __syncthreads();
     if (tid == 0) {
-        const double csp[3] = {d.cmposi0, d.cmposi1, d.cmroti};
-        double xn[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) xn[i] = xns[i];
-        // P1, V1, A1 (rigid[9..17]) formed in shared memory (cm), then stored
-        for (int i = 0; i < 18; ++i) cm[i] = rs[i];
-        double *P1 = cm + 9, *V1 = cm + 12, *A1 = cm + 15;
-        if (!d.rtcoup) {
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                P1[i] = csp[i] + xn[i];
-                V1[i] = xn[3 + i];
-                A1[i] = (V1[i] - rs[3 + i]) / dt;
-            }
-        } else {
-            P1[0] = csp[0] + xn[0];
-            V1[0] = xn[3];
-            A1[0] = (V1[0] - rs[3]) / dt;
-            P1[1] = csp[1];
-            V1[1] = 0.0;
-            A1[1] = 0.0;
-            P1[2] = csp[2] + xn[0] / d.rrr;
-            V1[2] = V1[0] / d.rrr;
-            A1[2] = A1[2] / d.rrr;  // as rigid.F90:296 (incoming value / rr)
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            if (mcon[i] == 1) {
-                P1[i] = kin[i];
-                V1[i] = kin[3 + i];
-                A1[i] = kin[6 + i];
-            }
-        const double cmrot = P1[2] - rs[2];
-        rot[0] = cos(cmrot);
-        rot[1] = -sin(cmrot);
-        rot[2] = sin(cmrot);
-        rot[3] = cos(cmrot);
+        rigid_state(d, rs, xns, kin, mcon, cm, rot);
         for (int i = 9; i < 18; ++i) R[i] = cm[i];
     }
     __syncthreads();
@@ -2213,7 +2373,6 @@ __device__ __forceinline__ void rigid_body(const Dev &d, int hist_rows, int mode
     // stores could alias the next loads, so a load after a store would wait
     // for the store's round trip.
     constexpr int kRgU = 4;
-    const double *P0 = cm, *P1 = cm + 9, *V1 = cm + 12, *A1 = cm + 15;
     for (int i0 = tid; i0 < nlm; i0 += kRgU * nt) {
         double y[kRgU], z[kRgU];
 #pragma unroll
@@ -2226,16 +2385,14 @@ __device__ __forceinline__ void rigid_body(const Dev &d, int hist_rows, int mode
         for (int u = 0; u < kRgU; ++u) {
             const int i = i0 + u * nt;
             if (i >= nlm) break;
-            const double rho0 = y[u] - P0[0], rho1 = z[u] - P0[1];
-            const double c10 = -V1[2] * rho1, c11 = V1[2] * rho0;
-            const double c20 = -A1[2] * rho1, c21 = A1[2] * rho0;
-            const double c30 = -V1[2] * c11, c31 = V1[2] * c10;
-            d.lmcc[2 * i] = P1[0] + (rot[0] * rho0 + rot[1] * rho1);
-            d.lmcc[2 * i + 1] = P1[1] + (rot[2] * rho0 + rot[3] * rho1);
-            d.lmvel[2 * i] = V1[0] + c10;
-            d.lmvel[2 * i + 1] = V1[1] + c11;
-            d.lmacc[2 * i] = A1[0] + c20 + c30;
-            d.lmacc[2 * i + 1] = A1[1] + c21 + c31;
+            double pos[2], vel[2], acc[2];
+            move_marker(cm, rot, y[u], z[u], pos, vel, acc);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                d.lmcc[2 * i + q] = pos[q];
+                d.lmvel[2 * i + q] = vel[q];
+                d.lmacc[2 * i + q] = acc[q];
+            }
         }
     }
     // vertices rotate about the updated centre (rigid.F90:110-121)
@@ -2251,9 +2408,11 @@ __device__ __forceinline__ void rigid_body(const Dev &d, int hist_rows, int mode
         for (int u = 0; u < kRgU; ++u) {
             const int i = i0 + u * nt;
             if (i > nlm) break;
-            const double rho0 = y[u] - P1[0], rho1 = z[u] - P1[1];
-            d.vert[2 * i] = P1[0] + (rot[0] * rho0 + rot[1] * rho1);
-            d.vert[2 * i + 1] = P1[1] + (rot[2] * rho0 + rot[3] * rho1);
+            const double v[2] = {y[u], z[u]};
+            double o[2];
+            move_vertex(cm, rot, v, o);
+            d.vert[2 * i] = o[0];
+            d.vert[2 * i + 1] = o[1];
         }
     }
     __syncthreads();
@@ -2269,15 +2428,10 @@ __device__ __forceinline__ void rigid_body(const Dev &d, int hist_rows, int mode
         for (int u = 0; u < kRgU; ++u) {
             const int i = i0 + u * nt;
             if (i >= nlm) break;
-            const double *a = va[u], *b = va[u] + 2;
-            const double v1[3] = {0.0 - 0.0, b[0] - a[0], b[1] - a[1]};
-            const double v2[3] = {-1.0 - 0.0, (a[0] + b[0]) * 0.5 - a[0], (a[1] + b[1]) * 0.5 - a[1]};
-            const double c0 = v1[1] * v2[2] - v1[2] * v2[1];
-            const double c1 = v1[2] * v2[0] - v1[0] * v2[2];
-            const double c2 = v1[0] * v2[1] - v1[1] * v2[0];
-            const double den = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-            d.lmnor[2 * i] = c1 / den;
-            d.lmnor[2 * i + 1] = c2 / den;
+            double nor[2];
+            segment_normal(va[u], va[u] + 2, nor);
+            d.lmnor[2 * i] = nor[0];
+            d.lmnor[2 * i + 1] = nor[1];
         }
     }
     if (mode == RIGID_PLACE) return;     // markers at the trial state; nothing committed
@@ -2289,24 +2443,7 @@ __device__ __forceinline__ void rigid_body(const Dev &d, int hist_rows, int mode
 #pragma unroll
         for (int i = 0; i < 8; ++i) fv[i] = d.forces[i];
         const double solves = (mode == RIGID_COMMIT) ? fin[3] : 1.0;   // fluid solves this step
-        for (int i = 0; i < 9; ++i) R[i] = cm[9 + i];
-        const double t1 = t0 + d.dt;
-        d.scal[S_TIME] = t1;
-        const int row = static_cast<int>(stepd);
-        if (hist_rows > 0) {
-            double *h = d.hist + static_cast<size_t>(row % hist_rows) * FB_HIST_COLS;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) h[i] = fv[i];
-            h[8] = t1;
-            for (int i = 0; i < 9; ++i) h[9 + i] = cm[9 + i];
-            h[18] = nbcv;
-            h[19] = nbcw;
-            h[20] = cflm;
-            h[21] = d.dt;
-            for (int i = 22; i < FB_HIST_COLS; ++i) h[i] = 0.0;  // diagnostics, when enabled
-            h[30] = solves;
-        }
-        d.scal[S_STEP] = static_cast<double>(row + 1);
+        commit_step(d, hist_rows, cm, fv, t0, stepd, nbcv, nbcw, cflm, solves);
         if (mbox) {   // the synchronous call's status and forcecomp row, into mapped host memory
             volatile double *m = mbox;
             m[0] = static_cast<double>(*d.status);
@@ -2320,6 +2457,104 @@ __device__ __forceinline__ void rigid_body(const Dev &d, int hist_rows, int mode
 __global__ void __launch_bounds__(512) k_rigid(Dev d, int hist_rows, int mode, const double *fin, double *mbox) {
     FB_GRID_WAIT();
     rigid_body(d, hist_rows, mode, fin, mbox);
+}
+
+// The end of a loosely coupled step behind k_loads_probe<true> in one block:
+// the markers whose tangent carries over (loads_transfer.F90:187-214), the
+// checkbcs norms, then rigid (RIGID_STEP).  It replaces two launches of the
+// step's serial end; its marker and vertex arrays are staged at once and the
+// normals formed from the vertices in registers, so that it makes one round
+// trip to global memory where the two launches made seven.  In the step, 5.4 +
+// 6.0 -> 6.0 us with 40 markers; the probes in front of it 9.7 -> 7.0 us.
+constexpr int kCloseThreads = 512;
+constexpr int kCloseMax = 2048;   // markers: a single block's worth (beyond, the two launches)
+inline size_t close_smem(int nlm) { return static_cast<size_t>(4 * nlm + 2) * sizeof(double); }
+
+__device__ __forceinline__ void close_body(const Dev &d, int hist_rows) {
+    extern __shared__ __align__(16) double close_sm[];
+    __shared__ double sh[32 * 7];
+    __shared__ double cm[18], rot[4], xns[6], rs[18], kin[9];
+    __shared__ int mcon[3];
+    const int tid = threadIdx.x, nt = blockDim.x, nlm = d.nlm;
+    double *pos0 = close_sm, *ver0 = close_sm + 2 * nlm;   // markers and vertices at the start
+    for (int i = tid; i < 2 * nlm; i += nt) cp8(pos0 + i, d.lmcc + i);
+    for (int i = tid; i < 2 * nlm + 2; i += nt) cp8(ver0 + i, d.vert + i);
+    if (tid < 18) rs[tid] = d.rigid[tid];
+    else if (tid >= 32 && tid < 41) kin[tid - 32] = d.kinori[tid - 32];
+    else if (tid >= 64 && tid < 67) mcon[tid - 64] = d.rbmcon[tid - 64];
+    const double time = d.scal[S_TIME], stepd = d.scal[S_STEP], cflm = d.scal[S_CFLM];
+    const double c0 = d.rigid[0], c1 = d.rigid[1];
+    const bool good = *d.status == 0;
+    double f[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // fyp, fzp, fyv, fzv, mom, the checkbcs sums
+    for (int i = tid; i < nlm; i += nt) {
+        double p = d.press[i], tau[2] = {d.tau[2 * i], d.tau[2 * i + 1]};
+        const double A = d.lmA[i], ny = d.lmnor[2 * i], nz = d.lmnor[2 * i + 1];
+        const double y = d.lmcc[2 * i], z = d.lmcc[2 * i + 1], ev = d.bcerrv[i], ew = d.bcerrw[i];
+        const double *pb = d.probe + static_cast<size_t>(i) * 24;
+        if (good && pb[23] == 0.0) {   // no tangent of its own
+            double tany = 0.0, tanz = 0.0;
+            carried_tangent(d, i, tany, tanz);
+            finish_marker(d, i, pb, tany, tanz, p, tau);
+            d.press[i] = p;
+            d.tau[2 * i] = tau[0];
+            d.tau[2 * i + 1] = tau[1];
+        }
+        const double Fp1 = -p * ny * A, Fp2 = -p * nz * A;
+        const double Fv1 = tau[0] * A, Fv2 = tau[1] * A;
+        f[0] = f[0] + Fp1;
+        f[1] = f[1] + Fp2;
+        f[2] = f[2] + Fv1;
+        f[3] = f[3] + Fv2;
+        const double r1 = y - c0, r2 = z - c1;
+        f[4] = f[4] + (r1 * (Fp2 + Fv2) - r2 * (Fp1 + Fv1));
+        f[5] = f[5] + ev * ev;
+        f[6] = f[6] + ew * ew;
+    }
+    cp_wait();
+    block_sum_n<7>(f, sh);   // (its barriers also publish the staged arrays)
+    const double fy = f[0] + f[2], fz = f[1] + f[3];
+    const double g0 = (1.0 - 1.0 / d.rbden) * d.rba0 * d.rbgravF0;
+    const double g1 = (1.0 - 1.0 / d.rbden) * d.rba0 * d.rbgravF1;
+    const double Fy = fy + g0, Fz = fz + g1, M = f[4];
+    if (tid < 32) {
+        if (tid < 3) rigid_rk4(d, tid, rs, Fy, Fz, M, xns);
+        __syncwarp();
+        if (tid == 0) rigid_state(d, rs, xns, kin, mcon, cm, rot);
+    }
+    __syncthreads();
+    for (int i = tid; i <= nlm; i += nt) {
+        double o[2];
+        move_vertex(cm, rot, ver0 + 2 * i, o);
+        d.vert[2 * i] = o[0];
+        d.vert[2 * i + 1] = o[1];
+        if (i == nlm) break;
+        double b[2], nor[2], pos[2], vel[2], acc[2];
+        move_vertex(cm, rot, ver0 + 2 * i + 2, b);
+        segment_normal(o, b, nor);
+        move_marker(cm, rot, pos0[2 * i], pos0[2 * i + 1], pos, vel, acc);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            d.lmnor[2 * i + q] = nor[q];
+            d.lmcc[2 * i + q] = pos[q];
+            d.lmvel[2 * i + q] = vel[q];
+            d.lmacc[2 * i + q] = acc[q];
+        }
+    }
+    if (tid == nt - 1) {
+        const double nbcv = sqrt(f[5]) / static_cast<double>(nlm), nbcw = sqrt(f[6]) / static_cast<double>(nlm);
+        d.scal[S_NBCV] = nbcv;
+        d.scal[S_NBCW] = nbcw;
+        const double fv[8] = {time, Fy, Fz, M, f[0], f[1], f[2], f[3]};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d.forces[i] = fv[i];
+        for (int i = 9; i < 18; ++i) d.rigid[i] = cm[i];
+        commit_step(d, hist_rows, cm, fv, time, stepd, nbcv, nbcw, cflm, 1.0);
+    }
+}
+
+__global__ void __launch_bounds__(kCloseThreads, 2) k_step_close(Dev d, int hist_rows) {
+    FB_GRID_WAIT();
+    close_body(d, hist_rows);
 }
 
 // ------------------------------------------------------------ diagnostics
@@ -2470,10 +2705,11 @@ __global__ void kg_submean_boucqt(const GroupCase *__restrict__ g, int deferred)
     submean_boucqt_body(d, deferred != 0);
 }
 
+template <bool kFinish>
 __global__ void __launch_bounds__(kLoadThreads, 5) kg_loads_probe(const GroupCase *__restrict__ g, int pend) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    loads_probe_tan_body(d, pend != 0);
+    loads_probe_tan_body<kFinish>(d, pend != 0);
 }
 
 __global__ void __launch_bounds__(kLoadFin) kg_loads_finish(const GroupCase *__restrict__ g) {
@@ -2523,7 +2759,12 @@ int nl_tiles(const Dev &d) { return ((d.n2m + kNlJ - 1) / kNlJ) * ((d.n3m + kNlK
 void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend, const NlMaps *maps,
                    int extra) {
     const int more = nl_more(extra);
-    const int blocks = std::min(nl_tiles(d), 148 * kNlBlocksPerSM - more) + more;   // all resident at once
+    // all resident at once; beside the marker set-up of the step (kNlMeans) a
+    // sixteenth of the slots is left to its small blocks, which otherwise waited
+    // for these persistent ones (none, 20, 37, 74 or 148 slots left: 1568, 1559,
+    // 1562, 1572, 1592 us per step at 2048 x 1536)
+    const int slots = 148 * kNlBlocksPerSM - more - ((extra & kNlMeans) ? 148 * kNlBlocksPerSM / 16 : 0);
+    const int blocks = std::min(nl_tiles(d), slots) + more;
     if (maps)
         pdl((extra & kNlCfl) ? k_nl_rhs_tma<true> : k_nl_rhs_tma<false>, dim3(blocks), dim3(32, 8), kNlSmemT, s, d,
             *maps, al, ga, ro, pend ? 1 : 0, extra);
@@ -2562,8 +2803,12 @@ int encode_nl_maps(NlMaps *m, const Dev &d) {
 void launch_lgrdist(const Dev &d, cudaStream_t s) {
     if (d.nlm) pdl(k_lgrdist, dim3((d.nlm + 127) / 128), dim3(128), 0, s, d);
 }
+namespace {
+inline int setup_blocks(int nlm) { return (2 * nlm * kNodeLanes + kSetupThreads - 1) / kSetupThreads; }
+}  // namespace
 void launch_mls_setup(const Dev &d, cudaStream_t s, bool find) {
-    if (d.nlm) pdl(find ? k_mls_setup<true> : k_mls_setup<false>, dim3((2 * d.nlm * kNodeLanes + 255) / 256), dim3(256), 0, s, d);
+    if (d.nlm) pdl(find ? k_mls_setup<true> : k_mls_setup<false>, dim3(setup_blocks(d.nlm)), dim3(kSetupThreads),
+                   0, s, d);
 }
 void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear) {
     if (d.nlm) pdl(k_mls_interp, dim3((2 * d.nlm * kInterpLanes + 255) / 256), dim3(256), 0, s, d, clear ? 1 : 0);
@@ -2604,9 +2849,17 @@ void launch_submean_boucqt(const Dev &d, cudaStream_t s, bool deferred) {
     dim3 b(32, 8);
     pdl(k_submean_boucqt, dim3(grid2(d.n2, d.n3 + 1, b)), dim3(b), 0, s, d, deferred ? 1 : 0);
 }
+void launch_loads_probe(const Dev &d, cudaStream_t s, bool pend, bool finish) {
+    pdl(finish ? k_loads_probe<true> : k_loads_probe<false>, dim3((d.nlm + kLoadMk - 1) / kLoadMk),
+        dim3(kLoadThreads), 0, s, d, pend ? 1 : 0);
+}
+bool step_closes(int nlm) { return nlm > 0 && nlm <= kCloseMax; }
+void launch_step_close(const Dev &d, int hist_rows, cudaStream_t s) {
+    pdl(k_step_close, dim3(1), dim3(kCloseThreads), close_smem(d.nlm), s, d, hist_rows);
+}
 void launch_loads(const Dev &d, cudaStream_t s, bool pend) {
     if (!d.nlm) return;
-    pdl(k_loads_probe, dim3((d.nlm + kLoadMk - 1) / kLoadMk), dim3(kLoadThreads), 0, s, d, pend ? 1 : 0);
+    launch_loads_probe(d, s, pend, false);
     pdl(k_loads_finish, dim3((d.nlm + kLoadFin - 1) / kLoadFin), dim3(kLoadFin), 0, s, d);
 }
 void launch_diag(const Dev &d, int hist_rows, cudaStream_t s) {
@@ -2660,12 +2913,13 @@ cudaError_t kernels_configure() {
     allow(k_updvp_prcalc, kUpSmem);
     allow(k_updvp_prcalc_tma, kUpSmemT);
     allow(kg_updvp_prcalc, kUpSmem);
+    allow(k_step_close, close_smem(kCloseMax));
     return e;
 }
 void glaunch_marker_setup(const Group &g, cudaStream_t s) {
     const Dev &d = g.rep;
     if (!d.nlm) return;
-    pdl(kg_mls_setup, zgrid(dim3((2 * d.nlm * kNodeLanes + 255) / 256), g), dim3(256), 0, s, g.cases);
+    pdl(kg_mls_setup, zgrid(dim3(setup_blocks(d.nlm)), g), dim3(kSetupThreads), 0, s, g.cases);
     pdl(kg_spread_chains, zgrid(dim3(chain_blocks(d.nlm)), g), dim3(kChainThreads), 0, s, g.cases);
 }
 void glaunch_forcing(const Group &g, int n, cudaStream_t s) {
@@ -2690,7 +2944,7 @@ void glaunch_submean_boucqt(const Group &g, cudaStream_t s, bool deferred) {
 void glaunch_loads(const Group &g, cudaStream_t s, bool pend) {
     const Dev &d = g.rep;
     if (!d.nlm) return;
-    pdl(kg_loads_probe, zgrid(dim3((d.nlm + kLoadMk - 1) / kLoadMk), g), dim3(kLoadThreads), 0, s, g.cases,
+    pdl(kg_loads_probe<false>, zgrid(dim3((d.nlm + kLoadMk - 1) / kLoadMk), g), dim3(kLoadThreads), 0, s, g.cases,
         pend ? 1 : 0);
     pdl(kg_loads_finish, zgrid(dim3((d.nlm + kLoadFin - 1) / kLoadFin), g), dim3(kLoadFin), 0, s, g.cases);
 }

@@ -51,6 +51,13 @@ void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, boo
 void launch_publish(const Dev &d, bool forces, double *mbox, cudaStream_t s);
 // deferred: the end of the fused step (boucqt has run with divg)
 void launch_submean_boucqt(const Dev &d, cudaStream_t s, bool deferred = false);
+// the probes alone; finish: with press and tau of every marker that has a
+// tangent of its own, for launch_step_close
+void launch_loads_probe(const Dev &d, cudaStream_t s, bool pend, bool finish);
+// the rest of the loads and the rigid update of a loosely coupled step in one
+// launch, for the marker counts that step_closes
+bool step_closes(int nlm);
+void launch_step_close(const Dev &d, int hist_rows, cudaStream_t s);
 // pend: pr still lacks the subtraction of its mean (S_PRAVG)
 void launch_loads(const Dev &d, cudaStream_t s, bool pend = false);
 void launch_diag(const Dev &d, int hist_rows, cudaStream_t s);

@@ -819,7 +819,10 @@ __device__ __forceinline__ void i8_cut_body(const double *__restrict__ src, long
 
 // The cut with the rows' maxima of |a| given (accumulated by the operand's
 // producer, or by k_i8_rowmax): no exchange between blocks.  Block (x, y):
-// rows 32 x .. 32 x + 31 (lane = row), columns 128 y + 16 w .. (warp w).  Column group 0 stores the row scales and, for
+// rows 32 x .. 32 x + 31, columns 128 y .. 128 y + 127; a warp holds 16 rows of
+// 32 columns, 16 of them per thread, so that one store instruction writes whole
+// 32-byte sectors (half sectors of digit planes that had left L2 since their
+// last use were filled from memory first).  Column group 0 stores the row scales and, for
 // the next producer, clears its maxima (clear, may be null).
 template <int S>
 __global__ void __launch_bounds__(256)
@@ -828,19 +831,19 @@ __global__ void __launch_bounds__(256)
     FB_GRID_WAIT();
     constexpr int V = 16, kP = V / 4;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int r = blockIdx.x * 32 + lane;
-    const int c0 = blockIdx.y * 8 * V + V * w;
+    const int r = blockIdx.x * 32 + 16 * (w & 1) + (lane & 15);
+    const int c0 = blockIdx.y * 128 + 32 * (w >> 1) + V * (lane >> 4);
     double a[kP][4];
 #pragma unroll
     for (int p = 0; p < kP; ++p)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int k = c0 + 4 * p + q;   // each load coalesced over the warp's 32 rows
+            const int k = c0 + 4 * p + q;   // each load: 128 bytes of two columns
             a[p][q] = (r < R && k < K) ? src[static_cast<size_t>(k) * lds + r] : 0.0;
         }
     const double mm = (r < R) ? rmax[r] : 0.0;
     const int e = i8_row_exp<S>(mm);
-    if (blockIdx.y == 0 && w == 0 && r < R) {
+    if (blockIdx.y == 0 && w < 2 && lane < 16 && r < R) {
         rowscale[r] = ldexp(1.0, e);
         if (clear) clear[r] = 0.0;
     }
@@ -964,6 +967,17 @@ __device__ __forceinline__ void i8x8_body(const CUtensorMap *ma, const CUtensorM
     // of a B operand that was in place before it (the eigenvector planes), so
     // that they are in flight while the previous kernel drains.
     const bool producer = (warp == 0 && lane == 0);
+    if (!kGlobalMaps && o.pf && warp == 2 && lane == 0) {
+        // this CTA's share of the next kernel's constant operand (nothing
+        // writes it, so it need not wait); DRAM is idle meanwhile
+        const size_t ctas = static_cast<size_t>(gridDim.x) * gridDim.y, me = blockIdx.y * gridDim.x + blockIdx.x;
+        const size_t share = (o.pf_bytes / ctas + 16) / 16 * 16;
+        const size_t from = me * share;
+        if (from < o.pf_bytes) {
+            const uint32_t n = static_cast<uint32_t>(o.pf_bytes - from < share ? o.pf_bytes - from : share);
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(o.pf + from), "r"(n) : "memory");
+        }
+    }
     if (!kGlobalMaps && !producer) FB_GRID_WAIT();
     // the epilogue's scales: this row's, and columns n0 + lane, n0 + 32 + lane
     const int quarter = warp & 3;
@@ -1353,8 +1367,8 @@ void launch_i8_rowmax(const double *src, long lds, int R, int K, double *rmax, c
 
 // the tile width is the B operand's box height (i8_plan)
 void launch_i8x8(const I8Plan &a, const I8Plan &b, double *out, long ldo, int *status, cudaStream_t st,
-                 bool b_const) {
-    I8Out o{out, ldo, a.scale, b.scale, a.rows, b.rows, b_const ? 1 : 0};
+                 bool b_const, const void *pf, size_t pf_bytes) {
+    I8Out o{out, ldo, a.scale, b.scale, a.rows, b.rows, b_const ? 1 : 0, static_cast<const char *>(pf), pf_bytes};
     const dim3 grid((a.rows + 127) / 128, (b.rows + b.box - 1) / b.box);
     auto go = [&](auto kern, size_t smem) {
         pdl(kern, grid, dim3(kI8Threads), smem, st, a.map, b.map, o, a.K, status);
