@@ -3,6 +3,7 @@
 #include <cublasLt.h>
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
+#include <omp.h>
 
 #include <algorithm>
 #include <array>
@@ -44,6 +45,10 @@ struct fb_ctx {
     // stage_ev (recorded after their copies) has completed
     double *stage_h = nullptr;
     cudaEvent_t stage_ev = nullptr;
+    // fb_get_array: pinned staging of large fields, two chunks (copy_out)
+    char *out_h = nullptr;
+    size_t out_chunk = 0;
+    cudaEvent_t out_ev[2] = {nullptr, nullptr};
     // fb_fluid_tsch / fb_rigid: status and forcecomp row written by the GPU
     // into mapped host memory (k_publish), read after the stream sync
     double *mbox_h = nullptr, *mbox_d = nullptr;
@@ -1245,6 +1250,75 @@ int capture_step(fb_ctx *c, int steps = 1) {
     return FB_OK;
 }
 
+// A pitched field to the caller's (pageable, often untouched) memory, ordered on
+// the context's stream and waited for.  Large fields go through two pinned
+// chunks: the copy engine fills one while several host threads empty the other
+// into the caller's array, whose first-touch page faults they share.  (The
+// driver's own staging copied 4.3 GB/s: 18 of the 108 ms of 50 steps at 2048 x
+// 1536 with three fields read at the end.)
+int copy_out(fb_ctx *c, double *host, const double *dev, size_t pitch, size_t width, size_t rows) {
+    constexpr size_t kDirect = 512u << 10, kChunk = 1u << 20;
+    bool staged = rows * width > kDirect && width <= kChunk;
+    if (staged && !c->out_h) {   // (without pinned memory to be had: the direct copy)
+        int cur = 0;
+        CK(cudaGetDevice(&cur));
+        CK(cudaSetDevice(c->device));
+        for (cudaEvent_t &e : c->out_ev)
+            if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) staged = false;
+        if (staged && cudaMallocHost(&c->out_h, 2 * kChunk) != cudaSuccess) {
+            c->out_h = nullptr;
+            staged = false;
+        }
+        if (!staged) cudaGetLastError();
+        c->out_chunk = kChunk;
+        CK(cudaSetDevice(cur));
+    }
+    if (!staged) {
+        CK(cudaMemcpy2DAsync(host, width, dev, pitch, width, rows, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        return FB_OK;
+    }
+    const size_t per = c->out_chunk / width, n = (rows + per - 1) / per;   // rows per chunk, chunks
+    auto issue = [&](size_t i) -> int {
+        const size_t r0 = i * per, nr = std::min(per, rows - r0);
+        CK(cudaMemcpy2DAsync(c->out_h + (i & 1) * c->out_chunk, width,
+                             reinterpret_cast<const char *>(dev) + r0 * pitch, pitch, width, nr,
+                             cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaEventRecord(c->out_ev[i & 1], c->stream));
+        return FB_OK;
+    };
+    int r;
+    if ((r = issue(0))) return r;
+    const int threads = std::max(1, std::min(8, omp_get_num_procs()));
+    for (size_t i = 0; i < n; ++i) {
+        if (i + 1 < n && (r = issue(i + 1))) return r;   // (its chunk was emptied in the round before)
+        CK(cudaEventSynchronize(c->out_ev[i & 1]));
+        const size_t bytes = std::min(per, rows - i * per) * width;
+        char *dst = reinterpret_cast<char *>(host) + i * per * width;
+        const char *src = c->out_h + (i & 1) * c->out_chunk;
+#pragma omp parallel for num_threads(threads) schedule(static)
+        for (int t = 0; t < threads; ++t) {
+            const size_t a = bytes / 64 * t / threads * 64, b = t + 1 == threads ? bytes : bytes / 64 * (t + 1) / threads * 64;
+            std::memcpy(dst + a, src + a, b - a);
+        }
+    }
+    return FB_OK;
+}
+
+// n history rows from ring row row0 on into the caller's array
+int copy_history(fb_ctx *c, double *hist, int row0, int n) {
+    const size_t w = FB_HIST_COLS * sizeof(double);
+    for (int done = 0; done < n;) {   // at most two runs (n <= hist_cap)
+        const int from = (row0 + done) % c->hist_cap, run = std::min(n - done, c->hist_cap - from);
+        CK(cudaMemcpyAsync(hist + static_cast<size_t>(done) * FB_HIST_COLS,
+                           c->d.hist + static_cast<size_t>(from) * FB_HIST_COLS, static_cast<size_t>(run) * w,
+                           cudaMemcpyDeviceToHost, c->stream));
+        done += run;
+    }
+    CK(cudaStreamSynchronize(c->stream));
+    return FB_OK;
+}
+
 // field (j, k) <-> host (k, j) dense copies
 int field_ptr(fb_ctx *c, int id, double **p) {
     Dev &d = c->d;
@@ -1363,6 +1437,9 @@ int fb_destroy(fb_ctx *c) {
     if (c->coef_pini) cudaFreeHost(c->coef_pini);
     if (c->stage_h) cudaFreeHost(c->stage_h);
     if (c->mbox_h) cudaFreeHost(c->mbox_h);
+    if (c->out_h) cudaFreeHost(c->out_h);
+    for (cudaEvent_t e : c->out_ev)
+        if (e) cudaEventDestroy(e);
     if (c->stage_ev) cudaEventDestroy(c->stage_ev);
     if (c->blas) cublasDestroy(c->blas);
     for (cublasLtMatrixLayout_t l : c->lt_l)
@@ -1736,12 +1813,8 @@ int fb_advance(fb_ctx *c, int ns0, int nsteps, double *hist) {
         CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
         c->last_ms += ms;
         if (hist) {
-            for (int i = 0; i < chunk; ++i) {
-                int row = (static_cast<int>(row0) + i) % c->hist_cap;
-                CK(cudaMemcpy(hist + static_cast<size_t>(done + i) * FB_HIST_COLS,
-                              c->d.hist + static_cast<size_t>(row) * FB_HIST_COLS, FB_HIST_COLS * sizeof(double),
-                              cudaMemcpyDeviceToHost));
-            }
+            if ((r = copy_history(c, hist + static_cast<size_t>(done) * FB_HIST_COLS, static_cast<int>(row0), chunk)))
+                return r;
         }
         host_clock(c, chunk);
         done += chunk;
@@ -2010,10 +2083,7 @@ int fb_get_array(fb_ctx *c, int id, double *host, int64_t n) {
     // writes the array, and waited for before returning
     if (field_ptr(c, id, &p) == FB_OK) {
         if (n != static_cast<int64_t>(d.NK) * d.n2) return FB_ERR_STATE;
-        CK(cudaMemcpy2DAsync(host, d.n2 * sizeof(double), p, d.P * sizeof(double), d.n2 * sizeof(double), d.NK,
-                             cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        return FB_OK;
+        return copy_out(c, host, p, d.P * sizeof(double), d.n2 * sizeof(double), static_cast<size_t>(d.NK));
     }
     if (id == FB_SCALARS) {
         if (n != 13) return FB_ERR_STATE;
