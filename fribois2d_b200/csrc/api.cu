@@ -108,7 +108,7 @@ struct fb_ctx {
     fb_mlp *mlp = nullptr;
     float *mlp_norm_d = nullptr;               // x mean, x std, t mean, t std
     bool cond_graph = true;                    // coupled step as a graph WHILE node (else a host loop)
-    int tune_tk = 64;         // windowed helsolve tile height (autotuned per grid size)
+    int tune_tk = 64;         // windowed helsolve tile height (by grid size; autotuned)
     int tune_bn = 128;        // 3xTF32 GEMM tile width (autotuned per grid size)
     int tune_i8bn = fb::kI8BN;  // INT8 digit-product tile width, 16, 32, 48 or 64 (by grid size)
     bool i8_fixed = false;      // the width set by FRIBOIS2D_I8_TILE: not tuned
@@ -619,6 +619,7 @@ int create_impl(const char *dir, int device, fb_ctx *c) {
     for (int i = 0; i < 9; ++i) d.kinori[i] = c->hc.kinori[i];
     d.rtcoup = dk.rtcoup ? 1 : 0;
 
+    c->tune_tk = fb::win_tile_rows(d.n2m, d.n3m);
     if ((st = build_substeps(c))) return st;
     CK(cudaStreamSynchronize(c->stream));
     c->beta = c->dt / g.ren * 0.5;

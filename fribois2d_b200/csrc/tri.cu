@@ -586,80 +586,74 @@ __global__ void __launch_bounds__(kMaxThreads) k_zlines(Dev d, SubDev sd, int nb
 // multipliers a(i) (forward) and e(i) (backward) fall below 2^-56 for a
 // window K that the host measures from the factors of each substep
 // (overlapped, truncated partitions: the truncated-SPIKE idea of Polizzi and
-// Sameh for diagonally dominant banded systems).  A thread computes a
-// segment of kWSeg values of one recurrence exactly as the sequential
-// recurrence would, except that it starts K positions early from zero;
-// segments need no communication.  A tile runs four phases through shared
-// memory: forward and backward y recurrences over the tile's rows plus a
-// halo of K rows on either side in k, then forward and backward z
-// recurrences over its columns, adding the result to q2/q3.  rhs2/rhs3 are
-// read once and q2/q3 read and written once; the recurrence coefficients of
-// the tile are staged in shared memory with it.
-constexpr int kWTj = 32;        // tile columns (j): one lane each in the z phases
-constexpr int kWSeg = 16;       // values per thread segment
-constexpr int kWSegY = 24;      // values per forward-y segment (2 cover a tile row and its halo)
-constexpr int kWThreads = 256;
+// Sameh for diagonally dominant banded systems).  A thread computes a segment
+// of kWSeg unknowns exactly as the sequential recurrences would, except that it
+// starts the forward one K positions before the segment, from zero, and the
+// backward one K positions behind it; the forward values stay in registers
+// between the two, and segments need no communication.  A tile runs two phases
+// through shared memory: the y solves of its rows plus a halo of K rows on
+// either side in k, then the z solves of its columns, added to q2/q3.
+// rhs2/rhs3 are read once and q2/q3 read and written once; the tile of q and
+// the recurrence coefficients are staged in shared memory with the right-hand
+// side, all of it in flight at once.
+//
+// What bounds it: shared-memory reads and the latency of the chains.  As four
+// phases (forward and backward recurrences apart, their values exchanged
+// through shared memory) a tile of 32 x 64 made 53 thousand 8-byte accesses and
+// three blocks of 72 KB fitted an SM; the fused segments make 28 thousand
+// (coefficients in pairs) and 51 KB.  20.4 -> 15.9 us at 1024 x 768, 88.7 -> 70.9 at
+// 2048 x 1536 (K = 15), 8.2 -> 5.8 at 384 x 256, 7.0 -> 5.4 at 48 x 32 (32 rows).
+constexpr int kWTj = 32;        // tile columns (j): one lane each in the z phase
+constexpr int kWSeg = 16;       // unknowns per thread segment
+constexpr int kWThreads = 192;  // six warps: the y segments of a 32 x 64 tile with K <= 16
 constexpr int kWXp = kWTj + 1;  // row stride of the z right-hand side tile (odd: conflict-free column stores)
 
 namespace {
 
-// y(i) = a(i) y(i-1) + F(i) for the TS positions from s, started from zero K
-// positions earlier; a and F are indexed relative to the segment start
-// (a[u], F(u) for u = -K .. TS-1).  Positions at or past nmax are not set.
-template <int TS, int KM, class FA, class FF>
-__device__ __forceinline__ void seg_fwd(const FA &A, const FF &F, int K, int lo, int nmax, double (&y)[TS]) {
-    double v = 0.0;
+// One segment: x(i) for the kWSeg positions from s on, i = s + t, from
+//   y(i) = a(i) y(i-1) + F(i)   (positions from s - K on, and from line index 0)
+//   x(i) = e(i) x(i+1) + g(i) y(i)   (positions below s + kWSeg + K)
+// A(u), F(u), EG(u) are indexed relative to s; lo: line index 0 relative to s;
+// positions at or past nmax are outside the line (x stays 0).
+template <int KM, class FA, class FE>
+__device__ __forceinline__ void win_segment(const FA &AF, const FE &EG, int K, int lo, int nmax, double (&x)[kWSeg]) {
+    double y[kWSeg + KM], v = 0.0;
 #pragma unroll
     for (int u = -KM; u < 0; ++u)
-        if (u >= -K && u >= lo) v = fma(A(u), v, F(u));
+        if (u >= -K && u >= lo) v = AF(u, v);
 #pragma unroll
-    for (int t = 0; t < TS; ++t) {
+    for (int t = 0; t < kWSeg + KM; ++t) {
         y[t] = 0.0;
-        if (t < nmax) {
-            v = fma(A(t), v, F(t));
+        if (t < kWSeg + K && t < nmax) {
+            v = AF(t, v);
             y[t] = v;
         }
     }
-}
-
-// x(i) = e(i) x(i+1) + g(i) Y(i) for the TS positions from s, started from
-// zero K positions after the segment; positions at or past nmax are not used
-template <int TS, int KM, class FE, class FG, class FY>
-__device__ __forceinline__ void seg_bwd(const FE &E, const FG &G, const FY &Y, int K, int nmax, double (&x)[TS]) {
-    double v = 0.0;
+    v = 0.0;
 #pragma unroll
-    for (int u = TS + KM - 1; u >= TS; --u)
-        if (u < TS + K && u < nmax) v = fma(E(u), v, G(u) * Y(u));
-#pragma unroll
-    for (int t = TS - 1; t >= 0; --t) {
-        x[t] = 0.0;
-        if (t < nmax) {
-            v = fma(E(t), v, G(t) * Y(t));
-            x[t] = v;
+    for (int t = kWSeg + KM - 1; t >= 0; --t) {
+        if (t < kWSeg + K && t < nmax) {
+            const double2 c = EG(t);
+            v = fma(c.x, v, c.y * y[t]);
         }
+        if (t < kWSeg) x[t] = (t < nmax) ? v : 0.0;
     }
 }
 
 template <int kWTk>
 struct WinShape {            // shared-memory layout of one tile of kWTk rows (in doubles)
-    int nyf, cols, pitch, rows;  // forward y segments per row; rhs tile rows x cols (stride pitch, odd)
-    int ypitch, nzf;             // row stride of the forward y values; forward z segments per column
-    int ncy, ncz;                // staged coefficient counts (y: a e g; z: a e g)
-    int a_size, b_size, c_size;  // regions A (rhs, then z rhs), B (y, then z partials), C (coefficients)
+    int rows, cols, pitch;   // right-hand side tile (row stride pitch, odd)
+    int ncz;                 // staged z coefficients
+    int a_size, q_size, c_size;   // regions A (rhs, then z rhs), Q (the tile of q), C (coefficients)
     __host__ __device__ WinShape(int Ky, int Kz) {
-        nyf = (kWTj + Ky + kWSegY - 1) / kWSegY;
-        cols = nyf * kWSegY + Ky;  // every forward y segment reads inside its row
-        pitch = cols | 1;
         rows = kWTk + 2 * Kz;
-        ypitch = (nyf * kWSegY) | 1;
-        nzf = (kWTk + Kz + kWSeg - 1) / kWSeg;
-        ncy = cols;
-        ncz = nzf * kWSeg + Kz;
+        cols = kWTj + 2 * Ky;
+        pitch = cols | 1;
+        ncz = kWTk + 2 * Kz;
         const int a1 = rows * pitch, a2 = rows * kWXp;
-        a_size = a1 > a2 ? a1 : a2;
-        const int b1 = rows * ypitch, b2 = nzf * kWSeg * kWTj;
-        b_size = b1 > b2 ? b1 : b2;
-        c_size = 4 * ncy + 3 * ncz;   // y: a e g and the row normalisers; z: a e g
+        a_size = ((a1 > a2 ? a1 : a2) + 1) & ~1;   // (the pairs behind it 16-byte aligned)
+        q_size = kWTk * kWTj;
+        c_size = 4 * cols + 2 * ncz + ncz;   // pairs (a, s) and (e, g) of y, (e, g) of z, a of z
     }
 };
 
@@ -669,9 +663,9 @@ struct WinShape {            // shared-memory layout of one tile of kWTk rows (i
 // blockIdx.x = tile (tj fastest).
 template <int KM, int kWTk>
 __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd, int ntj, int Ky, int Kz) {
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];
     const WinShape<kWTk> sh(Ky, Kz);
-    double *A = sm, *B = sm + sh.a_size, *C = B + sh.b_size;
+    double *A = sm, *Q = sm + sh.a_size, *C = Q + sh.q_size;
     const int fld = blockIdx.y;
     const int tj = blockIdx.x % ntj, tk = blockIdx.x / ntj;
     const int j0 = 1 + tj * kWTj, k0 = 1 + tk * kWTk;
@@ -686,40 +680,37 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
     const int jlo = fld ? 1 : 2;          // columns with a right-hand side
     const int klo = fld ? 2 : 1;          // rows whose y lines are solved
     const int rows = sh.rows, cols = sh.cols;
-    const int iy0 = j0 - 1 - Ky;          // y line index of tile column 0
-    const int iz0 = k0 - 1 - Kz;          // z line index of tile row 0
-    double *cya = C, *cye = C + sh.ncy, *cyg = C + 2 * sh.ncy, *cys = C + 3 * sh.ncy;
-    double *cza = C + 4 * sh.ncy, *cze = cza + sh.ncz, *czg = cza + 2 * sh.ncz;
+    double *cas = C, *ceg = C + 2 * cols;                              // (a, normaliser), (e, g) of y by tile column
+    double *zeg = C + 4 * cols, *za = zeg + 2 * sh.ncz;                // (e, g), a of z by tile row
 
-    // 1. coefficients, the y row normalisers of the tile's columns (cys) and
-    //    the right-hand side tile; A[r * pitch + c] holds (j0 - Ky + c, k0 - Kz + r).
-    //    All of the tile's copies are issued at once (cp.async); the forward
-    //    y recurrences scale the right-hand side as they read it
-    for (int c = threadIdx.x; c < sh.ncy; c += kWThreads) {
-        const int i = iy0 + c;
+    // 1. coefficients, the y row normalisers, the right-hand side tile
+    //    (A[r * pitch + c] holds (j0 - Ky + c, k0 - Kz + r)) and the tile of q:
+    //    all copies issued at once (cp.async); the forward y recurrence scales
+    //    the right-hand side as it reads it
+    for (int c = threadIdx.x; c < cols; c += kWThreads) {
+        const int i = j0 - 1 - Ky + c, jc = i + 1;   // line index, column
         if (i >= 0 && i < ny) {
-            cp8(cya + c, sy.a + i);
-            cp8(cye + c, sy.e + i);
-            cp8(cyg + c, sy.g + i);
+            cp8(cas + 2 * c, sy.a + i);
+            cp8(ceg + 2 * c, sy.e + i);
+            cp8(ceg + 2 * c + 1, sy.g + i);
         } else {
-            cya[c] = cye[c] = cyg[c] = 0.0;
+            cas[2 * c] = ceg[2 * c] = ceg[2 * c + 1] = 0.0;
         }
-        const int jc = j0 - Ky + c;
-        if (c < cols && jc >= jlo && jc <= d.n2m) cp8(cys + c, by + jc);
-        else cys[c] = 0.0;
+        if (jc >= jlo && jc <= d.n2m) cp8(cas + 2 * c + 1, by + jc);
+        else cas[2 * c + 1] = 0.0;
     }
     for (int c = threadIdx.x; c < sh.ncz; c += kWThreads) {
-        const int i = iz0 + c;
+        const int i = k0 - 1 - Kz + c;
         if (i >= 0 && i < nz) {
-            cp8(cza + c, sz.a + i);
-            cp8(cze + c, sz.e + i);
-            cp8(czg + c, sz.g + i);
+            cp8(za + c, sz.a + i);
+            cp8(zeg + 2 * c, sz.e + i);
+            cp8(zeg + 2 * c + 1, sz.g + i);
         } else {
-            cza[c] = cze[c] = czg[c] = 0.0;
+            za[c] = zeg[2 * c] = zeg[2 * c + 1] = 0.0;
         }
     }
     {
-        constexpr int kCC = 3;   // column chunks of 32 (cols <= 96)
+        constexpr int kCC = 3;   // column chunks of 32 (cols <= 80)
         int jc[kCC];
         bool okc[kCC];
 #pragma unroll
@@ -739,119 +730,114 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
                 else *dst = 0.0;
             }
         }
-        cp_wait();
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const int j = j0 + lane;
+    const bool jlive = (j >= jlo && j <= d.n2m);
+    if (jlive)
+        for (int r = w; r < kWTk && k0 + r <= d.n3m; r += kWarps) cp8(Q + r * kWTj + lane, q + fidx(d, j, k0 + r));
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");   // all but q
     __syncthreads();
 
-    // 2. forward y recurrences: lanes = rows, warps = (row group, segment);
-    //    B[r * ypitch + c] = y at tile column c (j = j0 + c), c < nyf * kWSegY
-    const int nrg = (rows + 31) / 32;
-    for (int task = w; task < nrg * sh.nyf; task += kWarps) {
-        const int rg = task / sh.nyf, sg = task - rg * sh.nyf;
-        const int r = rg * 32 + lane, rr = min(r, rows - 1);
-        const int c0 = Ky + sg * kWSegY;  // coefficient/rhs column of the segment start
+    // 2. y solves: lanes = rows, one segment per warp task; the results go to A
+    //    as the z right-hand side once every thread has read its inputs:
+    //    A[r * kWXp + c] = f at (j0 + c, k0 - Kz + r), scaled by the z row normalisers
+    constexpr int kSegs = kWTj / kWSeg;
+    constexpr int kTasks = (kWTk + 2 * KM + 31) / 32 * kSegs;
+    constexpr int kRounds = (kTasks + kWarps - 1) / kWarps;
+    double xs[kRounds][kWSeg];
+    const int ntask = (rows + 31) / 32 * kSegs;
+#pragma unroll
+    for (int it = 0; it < kRounds; ++it) {
+        const int task = w + it * kWarps;
+        if (task >= ntask) break;
+        const int sg = task % kSegs, rr = min(task / kSegs * 32 + lane, rows - 1);
+        const int c0 = Ky + sg * kWSeg;   // tile column of the segment's start
         const double *arow = A + rr * sh.pitch + c0;
-        const int lo = -(j0 - 1 + sg * kWSegY);  // line index 0 relative to the segment start
-        double y[kWSegY];
-        seg_fwd<kWSegY, KM>([&](int u) { return cya[c0 + u]; }, [&](int u) { return arow[u] * cys[c0 + u]; }, Ky,
-                           lo, ny - (j0 - 1 + sg * kWSegY), y);
-        if (r < rows) {
-#pragma unroll
-            for (int t = 0; t < kWSegY; ++t) B[r * sh.ypitch + sg * kWSegY + t] = y[t];
-        }
+        const double2 *as = reinterpret_cast<const double2 *>(cas) + c0;
+        const double2 *eg = reinterpret_cast<const double2 *>(ceg) + c0;
+        const int s0 = j0 - 1 + sg * kWSeg;   // line index of the segment's start
+        win_segment<KM>(
+            [&](int u, double v) {
+                const double2 c = as[u];
+                return fma(c.x, v, arow[u] * c.y);
+            },
+            [&](int u) { return eg[u]; }, Ky, -s0, ny - s0, xs[it]);
     }
     __syncthreads();
-
-    // 3. backward y recurrences over the tile's columns, then the z right-hand
-    //    side: A[r * kWXp + c] = f at (j0 + c, k0 - Kz + r), scaled by the z
-    //    row normalisers, with the inflow/outflow terms (solve_fluid.F90:208-209,
-    //    266-275)
-    for (int task = w; task < nrg * (kWTj / kWSeg); task += kWarps) {
-        const int rg = task / (kWTj / kWSeg), sg = task - rg * (kWTj / kWSeg);
-        const int r = rg * 32 + lane, rr = min(r, rows - 1);
-        const int k = k0 - Kz + r;
-        const bool live = (r < rows) && k >= klo && k <= d.n3m;
-        const int c0 = Ky + sg * kWSeg;
-        const double *brow = B + rr * sh.ypitch + sg * kWSeg;
-        double x[kWSeg];
-        seg_bwd<kWSeg, KM>([&](int u) { return cye[c0 + u]; }, [&](int u) { return cyg[c0 + u]; },
-                           [&](int u) { return brow[u]; }, Ky, ny - (j0 - 1 + sg * kWSeg), x);
-        if (r < rows) {
-            const double bzk = (k >= 1 && k <= nz) ? __ldg(bz + k) : 0.0;
-            double *arow = A + r * kWXp + sg * kWSeg;
-            if (k != 1 && k != nz) {   // interior rows: no inflow/outflow term
 #pragma unroll
-                for (int t = 0; t < kWSeg; ++t) arow[t] = live ? x[t] * bzk : 0.0;
-            } else {
+    for (int it = 0; it < kRounds; ++it) {
+        const int task = w + it * kWarps;
+        if (task >= ntask) break;
+        const int sg = task % kSegs, r = task / kSegs * 32 + lane, k = k0 - Kz + r;
+        if (r >= rows) continue;
+        const bool live = k >= klo && k <= d.n3m;
+        const double bzk = (k >= 1 && k <= nz) ? __ldg(bz + k) : 0.0;
+        double *arow = A + r * kWXp + sg * kWSeg;
 #pragma unroll
-                for (int t = 0; t < kWSeg; ++t) {
-                    const int j = j0 + sg * kWSeg + t;
-                    const int jj = min(max(j, 1), d.n2m);
-                    double f = live ? x[t] * bzk : 0.0;
-                    if (fld == 0) {
-                        if (k == 1) f = f + d.dqb2s[jj] * sd.ugkks;
-                        if (k == nz) f = f + d.dqb2n[jj] * sd.ugkkn;
-                    } else {
-                        if (k == 1) f = d.dqb3s[jj];
-                        if (k == nz) f = d.dqb3n[jj];
-                    }
-                    arow[t] = f;
-                }
+        for (int t = 0; t < kWSeg; ++t) arow[t] = live ? xs[it][t] * bzk : 0.0;
+    }
+    // the inflow/outflow terms of rows k = 1 and nz (solve_fluid.F90:208-209,
+    // 266-275), where the tile or its halo holds them; one lane per column
+    const int rs = 1 - (k0 - Kz), rn = nz - (k0 - Kz);   // their tile rows
+    const bool ends = (rs >= 0 && rs < rows) || (rn >= 0 && rn < rows);
+    if (ends) {
+        const int jj = min(max(j, 1), d.n2m);
+        double fs = 0.0, fn = 0.0;
+        if (w == 0) {
+            fs = fld ? d.dqb3s[jj] : d.dqb2s[jj];
+            fn = fld ? d.dqb3n[jj] : d.dqb2n[jj];
+        }
+        __syncthreads();
+        if (w == 0) {
+            if (rs >= 0 && rs < rows) {
+                double &f = A[rs * kWXp + lane];
+                f = fld ? fs : f + fs * sd.ugkks;
+            }
+            if (rn >= 0 && rn < rows) {
+                double &f = A[rn * kWXp + lane];
+                f = fld ? fn : f + fn * sd.ugkkn;
             }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");   // q
     __syncthreads();
 
-    // 4. forward z recurrences: lanes = columns, warps = segments of rows;
-    //    B[c * kWTj + lane] = z partial at tile row c from k0, c < nzf * kWSeg
-    const int j = j0 + lane;
-    const bool jlive = (j >= jlo && j <= d.n2m);
-    const double *acol = A + lane;
-    for (int sg = w; sg < sh.nzf; sg += kWarps) {
-        const int c0 = Kz + sg * kWSeg;  // tile row and coefficient index of the segment start
-        double y[kWSeg];
-        // rows past the tile's halo (c0 + u >= rows, last segment only) read
-        // whatever region A holds there, inside its allocation ((rows + 15) x
-        // kWXp < rows x pitch): they feed only positions past the halo, which
-        // the backward z phase never reads
-        seg_fwd<kWSeg, KM>([&](int u) { return cza[c0 + u]; }, [&](int u) { return acol[(c0 + u) * kWXp]; }, Kz,
-                           -(k0 - 1 + sg * kWSeg), nz - (k0 - 1 + sg * kWSeg), y);
-#pragma unroll
-        for (int t = 0; t < kWSeg; ++t) B[(sg * kWSeg + t) * kWTj + lane] = y[t];
-    }
-    __syncthreads();
-
-    // 5. backward z recurrences over the tile's rows; q += result
+    // 3. z solves: lanes = columns, warps = segments of rows; q += result
     for (int sg = w; sg < kWTk / kWSeg; sg += kWarps) {
-        const int s = k0 - 1 + sg * kWSeg;
-        if (s >= d.n3m) continue;
-        const int c0 = Kz + sg * kWSeg;
-        const double *bcol = B + sg * kWSeg * kWTj + lane;
+        const int s0 = k0 - 1 + sg * kWSeg;   // line index of the segment's start
+        if (s0 >= d.n3m) continue;
+        const int c0 = Kz + sg * kWSeg;       // its tile row
+        const double *acol = A + c0 * kWXp + lane;
+        const double *a = za + c0;
+        const double2 *eg = reinterpret_cast<const double2 *>(zeg) + c0;
         double x[kWSeg];
-        seg_bwd<kWSeg, KM>([&](int u) { return cze[c0 + u]; }, [&](int u) { return czg[c0 + u]; },
-                           [&](int u) { return bcol[u * kWTj]; }, Kz, nz - s, x);
+        win_segment<KM>([&](int u, double v) { return fma(a[u], v, acol[u * kWXp]); }, [&](int u) { return eg[u]; },
+                        Kz, -s0, nz - s0, x);
         if (jlive) {
-            double qv[kWSeg];
+            const double *qc = Q + sg * kWSeg * kWTj + lane;
 #pragma unroll
             for (int t = 0; t < kWSeg; ++t)
-                if (s + 1 + t <= d.n3m) qv[t] = __ldcg(q + fidx(d, j, s + 1 + t));
-#pragma unroll
-            for (int t = 0; t < kWSeg; ++t)
-                if (s + 1 + t <= d.n3m) q[fidx(d, j, s + 1 + t)] = qv[t] + x[t];
+                if (s0 + 1 + t <= d.n3m) q[fidx(d, j, s0 + 1 + t)] = qc[t * kWTj] + x[t];
         }
     }
-    if (fld == 1 && jlive && w == 0 && k0 <= d.n3m && k0 + kWTk > d.n3m)
-        Fv(q, j, d.n3) = Fv(q, j, d.n3) + d.dqb3n[j];
-    if (fld == 0 && blockIdx.x == 0) {  // helsolve.F90:35-36: wall values of v
-        for (int k = threadIdx.x; k <= d.n3; k += kWThreads) {
-            Fv(d.q2, 1, k) = 0.0;
-            Fv(d.q2, d.n2, k) = 0.0;
-        }
+    if (w != kWarps - 1) return;   // the last warp, without a segment, does the edges
+    const bool top = k0 + kWTk > d.n3m;
+    if (fld == 1 && jlive && top) Fv(q, j, d.n3) = Fv(q, j, d.n3) + d.dqb3n[j];
+    if (fld == 0) {   // helsolve.F90:35-36: wall values of v, each tile its rows
+        const int ka = (tk == 0) ? 0 : k0, kb = top ? d.n3 : k0 + kWTk - 1;
+        if (tj == 0)
+            for (int k = ka + lane; k <= kb; k += 32) Fv(d.q2, 1, k) = 0.0;
+        if (tj == ntj - 1)
+            for (int k = ka + lane; k <= kb; k += 32) Fv(d.q2, d.n2, k) = 0.0;
     }
 }
 
+// resident blocks per SM that the registers of the window's segments allow
+constexpr int win_blocks(int KM) { return KM <= 8 ? 4 : KM <= 16 ? 3 : 2; }
+
 template <int KM, int kWTk>
-__global__ void __launch_bounds__(kWThreads, 3) k_helsolve_win(Dev d, SubDev sd, int ntj, int Ky, int Kz) {
+__global__ void __launch_bounds__(kWThreads, win_blocks(KM)) k_helsolve_win(Dev d, SubDev sd, int ntj, int Ky, int Kz) {
     FB_GRID_WAIT();
     helsolve_win_body<KM, kWTk>(d, sd, ntj, Ky, Kz);
 }
@@ -859,7 +845,7 @@ __global__ void __launch_bounds__(kWThreads, 3) k_helsolve_win(Dev d, SubDev sd,
 // grouped forms (blockIdx.z = case; substep n 0-based): each case keeps its
 // own windows, the group's shared memory fits the largest
 template <int KM, int kWTk>
-__global__ void __launch_bounds__(kWThreads, 3) kg_helsolve_win(const GroupCase *__restrict__ g, int n, int ntj) {
+__global__ void __launch_bounds__(kWThreads, win_blocks(KM)) kg_helsolve_win(const GroupCase *__restrict__ g, int n, int ntj) {
     __shared__ Dev d;
     __shared__ SubDev s;
     if (!stage_case(g, &d, &s, n)) return;
@@ -930,11 +916,11 @@ cudaError_t scan_configure() {
 #define AL(K)                                  \
     if ((e = allow_smem(K)) != cudaSuccess) return e;
     AL((k_ylines<9, 0>)) AL((k_ylines<17, 0>)) AL((k_ylines<33, 0>))
-    AL((k_helsolve_win<9, 32>)) AL((k_helsolve_win<9, 64>))
+    AL((k_helsolve_win<8, 32>)) AL((k_helsolve_win<8, 64>))
     AL((k_helsolve_win<12, 32>)) AL((k_helsolve_win<12, 64>))
     AL((k_helsolve_win<16, 32>)) AL((k_helsolve_win<16, 64>))
     AL((k_helsolve_win<kWinMax, 32>)) AL((k_helsolve_win<kWinMax, 64>))
-    AL((kg_helsolve_win<9, 32>)) AL((kg_helsolve_win<9, 64>))
+    AL((kg_helsolve_win<8, 32>)) AL((kg_helsolve_win<8, 64>))
     AL((kg_helsolve_win<12, 32>)) AL((kg_helsolve_win<12, 64>))
     AL((kg_helsolve_win<16, 32>)) AL((kg_helsolve_win<16, 64>))
     AL((kg_helsolve_win<kWinMax, 32>)) AL((kg_helsolve_win<kWinMax, 64>))
@@ -955,12 +941,12 @@ void win_launch(const Dev &d, const SubDev &s, cudaStream_t st) {
     const int ntj = (d.n2m + kWTj - 1) / kWTj, ntk = (d.n3m + TK - 1) / TK;
     const dim3 grid(ntj * ntk, 2);
     const WinShape<TK> sh(s.win_y, s.win_z);
-    const size_t smem = static_cast<size_t>(sh.a_size + sh.b_size + sh.c_size) * sizeof(double);
+    const size_t smem = static_cast<size_t>(sh.a_size + sh.q_size + sh.c_size) * sizeof(double);
     // the warm-up of every segment runs KM predicated steps: the smallest
     // instantiated KM that covers both windows
     const int km = std::max(s.win_y, s.win_z);
-    if (km <= 9)
-        pdl(k_helsolve_win<9, TK>, dim3(grid), dim3(kWThreads), smem, st, d, s, ntj, s.win_y, s.win_z);
+    if (km <= 8)
+        pdl(k_helsolve_win<8, TK>, dim3(grid), dim3(kWThreads), smem, st, d, s, ntj, s.win_y, s.win_z);
     else if (km <= 12)
         pdl(k_helsolve_win<12, TK>, dim3(grid), dim3(kWThreads), smem, st, d, s, ntj, s.win_y, s.win_z);
     else if (km <= 16)
@@ -1020,10 +1006,10 @@ void gwin_launch(const Group &g, int n, cudaStream_t st) {
     const dim3 grid(ntj * ntk, 2, g.n);
     const int ky = g.win_ky[n], kz = g.win_kz[n];
     const WinShape<TK> sh(ky, kz);   // sizes grow with the windows: fits every case
-    const size_t smem = static_cast<size_t>(sh.a_size + sh.b_size + sh.c_size) * sizeof(double);
+    const size_t smem = static_cast<size_t>(sh.a_size + sh.q_size + sh.c_size) * sizeof(double);
     const int km = std::max(ky, kz);
-    if (km <= 9)
-        pdl(kg_helsolve_win<9, TK>, grid, dim3(kWThreads), smem, st, g.cases, n, ntj);
+    if (km <= 8)
+        pdl(kg_helsolve_win<8, TK>, grid, dim3(kWThreads), smem, st, g.cases, n, ntj);
     else if (km <= 12)
         pdl(kg_helsolve_win<12, TK>, grid, dim3(kWThreads), smem, st, g.cases, n, ntj);
     else if (km <= 16)
