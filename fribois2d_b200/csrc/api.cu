@@ -45,10 +45,9 @@ struct fb_ctx {
     // stage_ev (recorded after their copies) has completed
     double *stage_h = nullptr;
     cudaEvent_t stage_ev = nullptr;
-    // fb_get_array: pinned staging of large fields, two chunks (copy_out)
-    char *out_h = nullptr;
-    size_t out_chunk = 0;
+    // fb_get_array: the events of the two pinned chunks (copy_out)
     cudaEvent_t out_ev[2] = {nullptr, nullptr};
+    bool out_user = false;
     // fb_fluid_tsch / fb_rigid: status and forcecomp row written by the GPU
     // into mapped host memory (k_publish), read after the stream sync
     double *mbox_h = nullptr, *mbox_d = nullptr;
@@ -1251,6 +1250,41 @@ int capture_step(fb_ctx *c, int steps = 1) {
     return FB_OK;
 }
 
+// The pinned chunks of copy_out, one pair for all contexts of the process that
+// read fields (pinning memory is slow, and a context would hold its own for a
+// few reads): made by the first read, given back with the last context that
+// has used them.  A read that finds them in use by another thread goes without.
+struct OutChunks {
+    static constexpr size_t kBytes = 1u << 20;   // one chunk
+    std::mutex mu;     // users, buf
+    std::mutex busy;   // held while the chunks are in use
+    int users = 0;
+    char *buf = nullptr;
+    // the chunks for a context that registers as a user (null: none to be had)
+    char *get(bool &registered) {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!buf && cudaHostAlloc(&buf, 2 * kBytes, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            buf = nullptr;
+        }
+        if (buf && !registered) {
+            registered = true;
+            ++users;
+        }
+        return buf;
+    }
+    void release(bool &registered) {
+        if (!registered) return;
+        std::lock_guard<std::mutex> lk(mu);
+        registered = false;
+        if (--users == 0) {
+            cudaFreeHost(buf);
+            buf = nullptr;
+        }
+    }
+};
+OutChunks g_out;
+
 // A pitched field to the caller's (pageable, often untouched) memory, ordered on
 // the context's stream and waited for.  Large fields go through two pinned
 // chunks: the copy engine fills one while several host threads empty the other
@@ -1258,33 +1292,30 @@ int capture_step(fb_ctx *c, int steps = 1) {
 // driver's own staging copied 4.3 GB/s: 18 of the 108 ms of 50 steps at 2048 x
 // 1536 with three fields read at the end.)
 int copy_out(fb_ctx *c, double *host, const double *dev, size_t pitch, size_t width, size_t rows) {
-    constexpr size_t kDirect = 512u << 10, kChunk = 1u << 20;
-    bool staged = rows * width > kDirect && width <= kChunk;
-    if (staged && !c->out_h) {   // (without pinned memory to be had: the direct copy)
+    constexpr size_t kDirect = 512u << 10, kChunk = OutChunks::kBytes;
+    std::unique_lock<std::mutex> busy(g_out.busy, std::defer_lock);
+    char *buf = nullptr;
+    if (rows * width > kDirect && width <= kChunk) {
+        CK(cudaStreamSynchronize(c->stream));   // (the chunks are not held while the GPU works)
+        if (busy.try_lock()) buf = g_out.get(c->out_user);
+    }
+    if (buf && !c->out_ev[0]) {
         int cur = 0;
         CK(cudaGetDevice(&cur));
         CK(cudaSetDevice(c->device));
-        for (cudaEvent_t &e : c->out_ev)
-            if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) staged = false;
-        if (staged && cudaMallocHost(&c->out_h, 2 * kChunk) != cudaSuccess) {
-            c->out_h = nullptr;
-            staged = false;
-        }
-        if (!staged) cudaGetLastError();
-        c->out_chunk = kChunk;
+        for (cudaEvent_t &e : c->out_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         CK(cudaSetDevice(cur));
     }
-    if (!staged) {
+    if (!buf) {
         CK(cudaMemcpy2DAsync(host, width, dev, pitch, width, rows, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         return FB_OK;
     }
-    const size_t per = c->out_chunk / width, n = (rows + per - 1) / per;   // rows per chunk, chunks
+    const size_t per = kChunk / width, n = (rows + per - 1) / per;   // rows per chunk, chunks
     auto issue = [&](size_t i) -> int {
         const size_t r0 = i * per, nr = std::min(per, rows - r0);
-        CK(cudaMemcpy2DAsync(c->out_h + (i & 1) * c->out_chunk, width,
-                             reinterpret_cast<const char *>(dev) + r0 * pitch, pitch, width, nr,
-                             cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpy2DAsync(buf + (i & 1) * kChunk, width, reinterpret_cast<const char *>(dev) + r0 * pitch, pitch,
+                             width, nr, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaEventRecord(c->out_ev[i & 1], c->stream));
         return FB_OK;
     };
@@ -1296,7 +1327,7 @@ int copy_out(fb_ctx *c, double *host, const double *dev, size_t pitch, size_t wi
         CK(cudaEventSynchronize(c->out_ev[i & 1]));
         const size_t bytes = std::min(per, rows - i * per) * width;
         char *dst = reinterpret_cast<char *>(host) + i * per * width;
-        const char *src = c->out_h + (i & 1) * c->out_chunk;
+        const char *src = buf + (i & 1) * kChunk;
 #pragma omp parallel for num_threads(threads) schedule(static)
         for (int t = 0; t < threads; ++t) {
             const size_t a = bytes / 64 * t / threads * 64, b = t + 1 == threads ? bytes : bytes / 64 * (t + 1) / threads * 64;
@@ -1438,7 +1469,7 @@ int fb_destroy(fb_ctx *c) {
     if (c->coef_pini) cudaFreeHost(c->coef_pini);
     if (c->stage_h) cudaFreeHost(c->stage_h);
     if (c->mbox_h) cudaFreeHost(c->mbox_h);
-    if (c->out_h) cudaFreeHost(c->out_h);
+    g_out.release(c->out_user);
     for (cudaEvent_t e : c->out_ev)
         if (e) cudaEventDestroy(e);
     if (c->stage_ev) cudaEventDestroy(c->stage_ev);
