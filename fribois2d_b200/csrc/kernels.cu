@@ -596,18 +596,15 @@ __device__ __forceinline__ void nl_issue_tma(const NlMaps &m, NlTileT &t, uint32
 template <bool kCfl>
 __device__ __forceinline__ void nl_rhs_tma_body(const Dev &d, const NlMaps &m, double al, double ga, double ro,
                                                 NlTileT *buf, uint64_t *bars, bool pend, int nb) {
-    const double pravg = pend ? d.scal[S_PRAVG] : 0.0;
     double cmx = 1.0e-8, csm = 0.0;
     const int ntj = (d.n2m + kNlJ - 1) / kNlJ, ntk = (d.n3m + kNlK - 1) / kNlK, ntiles = ntj * ntk;
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;
     int tile = blockIdx.x;
-    if (tile >= ntiles) return;
     const uint32_t bar0 = smem_u32(bars), bar1 = smem_u32(bars + 1);
     if (tid == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar1, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        nl_issue_tma(m, buf[0], bar0, tile, ntj);
     }
     {
         const int j0 = 1 + (tile % ntj) * kNlJ, k0 = 1 + (tile / ntj) * kNlK;
@@ -615,6 +612,9 @@ __device__ __forceinline__ void nl_rhs_tma_body(const Dev &d, const NlMaps &m, d
     }
     double r2n[kNlK / 8], r3n[kNlK / 8];
     nl_ru(d, tile, ntj, ro, r2n, r3n);
+    FB_GRID_WAIT();   // (updvp before it writes q2, q3, pr and the mean)
+    const double pravg = pend ? d.scal[S_PRAVG] : 0.0;
+    if (tid == 0) nl_issue_tma(m, buf[0], bar0, tile, ntj);
     __syncthreads();   // the barriers are initialised before any thread waits on them
     for (int it = 0; tile < ntiles; ++it, tile += nb) {
         NlTileT &t = buf[it & 1];
@@ -676,9 +676,9 @@ __global__ void __launch_bounds__(256, kNlBlocksPerSM)
     unsigned char *base = nl_smem + ((128u - (raw & 127u)) & 127u);   // the tiles on 128-byte boundaries
     NlTileT *buf = reinterpret_cast<NlTileT *>(base);
     uint64_t *bars = reinterpret_cast<uint64_t *>(base + 2 * sizeof(NlTileT));
-    FB_GRID_WAIT();
-    const int nb = gridDim.x - nl_more(extra);
+    const int nb = gridDim.x - nl_more(extra);   // (at most one block per tile)
     if (static_cast<int>(blockIdx.x) >= nb) {
+        FB_GRID_WAIT();
         if ((extra & kNlBoucdq) && static_cast<int>(blockIdx.x) == nb) boucdq_body(d, ga, ro);
         else edge_means_body(d);
         return;
@@ -1104,12 +1104,37 @@ __global__ void k_mls_setup(Dev d) {
 // k_spread_chains, is emptied for the next step (every used entry is some
 // marker's own).
 constexpr int kInterpLanes = 16;
+// kWait: the body waits for the kernel before it (nl_rhs, which writes
+// rhs2/rhs3, or the spreading chains) with everything else loaded.
+template <bool kWait>
 __device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = T / kInterpLanes, m = T % kInterpLanes, lane = threadIdx.x & 31;
     const bool have = t < 2 * d.nlm;
-    const bool stopped = (*d.status != 0);
     const int tt = have ? t : 0;
+    const int n = tt >> 1, idir = (tt & 1) + 1;
+    const double pos2 = d.lmcc[2 * n + 1], vel = d.lmvel[2 * n + idir - 1], cl = d.cl[tt];
+    const bool inside = (d.zz[1] < pos2 && pos2 < d.zz[d.n3]);
+    const bool node = have && inside && m < kSD;
+    double phim = 0.0, qv = 0.0;
+    const double *rp = nullptr;
+    if (node) {
+        const int *eu = d.eulins + static_cast<size_t>(tt) * 2 * kSD;
+        const double *q = (idir == 1) ? d.q2 : d.q3;
+        phim = d.phi[static_cast<size_t>(tt) * kSD + m];
+        const int j = eu[m], k = eu[kSD + m];
+        // q2f/q3f are written only where invtr2/invtr3 write them; elsewhere
+        // the reference reads storage that was never set (zero here)
+        const bool written = (idir == 1) ? (j >= 2 && j <= d.n2m && k >= 1 && k <= d.n3m)
+                                         : (j >= 1 && j <= d.n2m && k >= 2 && k <= d.n3m);
+        if (written) {
+            const size_t i = fidx(d, j, k);
+            qv = __ldcg(q + i);
+            rp = ((idir == 1) ? d.rhs2 : d.rhs3) + i;
+        }
+    }
+    if (kWait) FB_GRID_WAIT();
+    const bool stopped = (*d.status != 0);
     if (clear && have && m == kInterpLanes - 1) {   // (a lane without a node)
         const int e = d.hslot[tt];
         if (e) {
@@ -1118,27 +1143,7 @@ __device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
             d.hslot[tt] = 0;
         }
     }
-    const int n = tt >> 1, idir = (tt & 1) + 1;
-    const double pos2 = d.lmcc[2 * n + 1];
-    const bool inside = (d.zz[1] < pos2 && pos2 < d.zz[d.n3]);
-    double phim = 0.0, prod = 0.0;
-    if (have && inside && m < kSD) {
-        const int *eu = d.eulins + static_cast<size_t>(tt) * 2 * kSD;
-        const double *q = (idir == 1) ? d.q2 : d.q3;
-        const double *r = (idir == 1) ? d.rhs2 : d.rhs3;
-        phim = d.phi[static_cast<size_t>(tt) * kSD + m];
-        const int j = eu[m], k = eu[kSD + m];
-        // q2f/q3f are written only where invtr2/invtr3 write them; elsewhere
-        // the reference reads storage that was never set (zero here)
-        const bool written = (idir == 1) ? (j >= 2 && j <= d.n2m && k >= 1 && k <= d.n3m)
-                                         : (j >= 1 && j <= d.n2m && k >= 2 && k <= d.n3m);
-        double qf = 0.0;
-        if (written) {
-            const size_t i = fidx(d, j, k);
-            qf = q[i] + r[i];
-        }
-        prod = phim * qf;
-    }
+    const double prod = rp ? phim * (qv + *rp) : phim * 0.0;
     double u = 0.0;
 #pragma unroll
     for (int mm = 0; mm < kSD; ++mm) u = u + __shfl_sync(0xffffffffu, prod, (lane & ~(kInterpLanes - 1)) + mm);
@@ -1148,14 +1153,11 @@ __device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
         c[m] = 0.0;
         return;
     }
-    const double f = (d.lmvel[2 * n + idir - 1] - u) / d.dt;
-    c[m] = d.cl[tt] * phim * f;
+    const double f = (vel - u) / d.dt;
+    c[m] = cl * phim * f;
 }
 
-__global__ void k_mls_interp(Dev d, int clear) {
-    FB_GRID_WAIT();
-    mls_interp_body(d, clear != 0);
-}
+__global__ void k_mls_interp(Dev d, int clear) { mls_interp_body<true>(d, clear != 0); }
 
 // interp_spread, spreading half, without atomics on the field.  Once per
 // step (the supports are fixed for the three substeps) every cell's touchers
@@ -1328,20 +1330,30 @@ __global__ void k_spread_chains(const __grid_constant__ Dev d) {
     spread_chains_body(d);
 }
 
+// kWait: the body waits for the kernel before it (k_mls_interp, which writes
+// contrib) with the slot's chain and its cell's right-hand side loaded.
+template <bool kWait>
 __device__ __forceinline__ void mls_spread_body(const Dev &d) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= 2 * d.nlm * kSD) return;
-    if (*d.status) return;
-    if (!d.chead[g]) return;  // not the head of a cell's chain
-    const int t = g / kSD, dir = t & 1;
-    const int *eu = d.eulins + static_cast<size_t>(t) * 2 * kSD;
-    const int m = g % kSD;
-    // the head's in-line list gives the first kHeadList members at once
-    // (independent loads); a longer chain continues along chain[]; the sum
-    // runs in chain order
-    const int L = d.hlen[g];
-    const int4 *hl = reinterpret_cast<const int4 *>(d.hlist + static_cast<size_t>(g) * kHeadList);
-    const int4 h0 = hl[0], h1 = hl[1];
+    const bool head = g < 2 * d.nlm * kSD && d.chead[g] != 0;   // the head of a cell's chain
+    int L = 0;
+    int4 h0{}, h1{};
+    double *r = nullptr, rv = 0.0;
+    if (head) {
+        const int t = g / kSD, dir = t & 1, m = g % kSD;
+        const int *eu = d.eulins + static_cast<size_t>(t) * 2 * kSD;
+        // the head's in-line list gives the first kHeadList members at once
+        // (independent loads); a longer chain continues along chain[]; the sum
+        // runs in chain order
+        L = d.hlen[g];
+        const int4 *hl = reinterpret_cast<const int4 *>(d.hlist + static_cast<size_t>(g) * kHeadList);
+        h0 = hl[0];
+        h1 = hl[1];
+        r = ((dir == 0) ? d.rhs2 : d.rhs3) + fidx(d, eu[m], eu[kSD + m]);
+        rv = __ldcg(r);
+    }
+    if (kWait) FB_GRID_WAIT();
+    if (!head || *d.status) return;
     const int idx[kHeadList] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
     double cv[kHeadList];
 #pragma unroll
@@ -1353,15 +1365,10 @@ __device__ __forceinline__ void mls_spread_body(const Dev &d) {
         if (p < L) fe = fe + cv[p];
     if (L > kHeadList)
         for (int s = d.chain[idx[kHeadList - 1]]; s >= 0; s = d.chain[s]) fe = fe + d.contrib[s];
-    double *r = (dir == 0) ? d.rhs2 : d.rhs3;
-    const size_t i = fidx(d, eu[m], eu[kSD + m]);
-    r[i] = r[i] + fe * d.dt;
+    *r = rv + fe * d.dt;
 }
 
-__global__ void k_mls_spread(Dev d) {
-    FB_GRID_WAIT();
-    mls_spread_body(d);
-}
+__global__ void k_mls_spread(Dev d) { mls_spread_body<true>(d); }
 
 // ------------------------------------------------------------ tridiagonal
 
@@ -1614,6 +1621,8 @@ __device__ __forceinline__ void up_own(const Dev &d, int tile, int ntj, double (
 // mean).  kTma: the dph tiles are TMA boxes on the mbarriers bars (maps m);
 // a wait that gives up records FB_ERR_TIMEOUT and ends the block's tiles (the
 // block still takes part in the mean)
+// (kTma: the single-case kernel; it waits here for the kernel before it, the
+// transform that writes dph, with everything but dph of its first tile loaded)
 template <bool kTma, class Tile>
 __device__ __forceinline__ void updvp_prcalc_body(const Dev &d, double al, double be, Tile *buf, bool pend, int slot,
                                                   const NlMaps *m = nullptr, uint64_t *bars = nullptr) {
@@ -1633,19 +1642,21 @@ __device__ __forceinline__ void updvp_prcalc_body(const Dev &d, double al, doubl
         bar0 = smem_u32(bars);
         bar1 = smem_u32(bars + 1);
     }
-    if (tile < ntiles) {
-        if constexpr (kTma) {
+    if constexpr (kTma) {
+        if (tile < ntiles) {
             if (t == 0) {
                 mbar_init(bar0, 1);
                 mbar_init(bar1, 1);
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-                up_issue_tma(*m, buf[0], bar0, tile, ntj);
             }
             up_prefetch_coef(d, buf[0], 1 + (tile % ntj) * kNlJ, 1 + (tile / ntj) * kNlK, t);
-            __syncthreads();   // the barriers are initialised before any thread waits on them
-        } else {
-            up_prefetch(d, buf[0], tile, ntj, t);
+            up_own(d, tile, ntj, q2n, q3n, prn);
         }
+        FB_GRID_WAIT();
+        if (tile < ntiles && t == 0) up_issue_tma(*m, buf[0], bar0, tile, ntj);
+        __syncthreads();   // the barriers are initialised before any thread waits on them
+    } else if (tile < ntiles) {
+        up_prefetch(d, buf[0], tile, ntj, t);
         up_own(d, tile, ntj, q2n, q3n, prn);
     }
     for (int it = 0; tile < ntiles; ++it, tile += gridDim.x) {
@@ -1744,7 +1755,6 @@ __global__ void __launch_bounds__(256, kUpBlocksPerSM)
     extern __shared__ __align__(16) unsigned char up_smem[];
     const uint32_t raw = smem_u32(up_smem);
     unsigned char *base = up_smem + ((128u - (raw & 127u)) & 127u);   // the tiles on 128-byte boundaries
-    FB_GRID_WAIT();
     updvp_prcalc_body<true>(d, al, be, reinterpret_cast<UpTileT *>(base), pend != 0, slot, &m,
                             reinterpret_cast<uint64_t *>(base + 2 * sizeof(UpTileT)));
 }
@@ -1794,6 +1804,7 @@ constexpr int kLoadThreads = 3 * kLoadMk * kLoadLanes;
 // pend: the step's last pressure mean is still to be subtracted from pr; the
 // value is the one pr_submean would have stored.
 // vals (may be null): the block's markers' values in shared memory, 24 each
+template <bool kWait>
 __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double *vals) {
     constexpr unsigned kAll = 0xffffffffu;
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
@@ -1820,14 +1831,6 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
     const bool stopped = __shfl_sync(kAll, static_cast<int>(*d.status != 0), base) != 0;
     const bool ok = have && !stopped && inside;
 
-    // checkbcs: the velocity at the marker from the substep-1 weights
-    double prod = 0.0;
-    if (ok && idir <= 2 && node) {
-        const int t2 = 2 * n + idir - 1;
-        const int *eu = d.eulins + static_cast<size_t>(t2) * 2 * kSD;
-        const double *q = (idir == 1) ? d.q2 : d.q3;
-        prod = d.phi[static_cast<size_t>(t2) * kSD + m] * q[fidx(d, eu[m], eu[kSD + m])];
-    }
 
     const double hpr = d.ddmin * d.kprobe;
     const double probe[2] = {pos[0] + d.lmnor[2 * n] * hpr, pos[1] + d.lmnor[2 * n + 1] * hpr};
@@ -1874,19 +1877,6 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
     const bool good = supported && ej0 >= 2;
     if (ok && !good && m == 0) raise_status(d, FB_ERR_MARKER_OUT);
     const bool act = good && node;
-
-    // the field values that getpbup reads, requested before the MLS algebra
-    // so that their latency overlaps it
-    double f0 = 0.0, fym = 0.0, fzm = 0.0, g2r = 1.0, g3r = 1.0;
-    if (act) {
-        const double *f = (idir == 1) ? d.q2 : (idir == 2 ? d.q3 : d.pr);
-        const double mean = (pend && idir == 3) ? d.scal[S_PRAVG] : 0.0;   // (x - 0.0 is x)
-        f0 = Fv(f, ej, ek) - mean;
-        fym = Fv(f, ej - 1, ek) - mean;
-        fzm = Fv(f, ej, ek - 1) - mean;
-        g2r = d.g2rc[ej];
-        g3r = d.g3rc[ek];
-    }
 
     // MLS_SF_d (MLSint.F90:173-258) with compute_AB_d (:342-402)
     double sc0 = 0.0, sc1 = 0.0, w0 = 0.0, w1 = 0.0, w2 = 0.0;
@@ -1953,6 +1943,27 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
         p0 = p0 + gam[a][0] * B0;
         p1 = p1 + gam[a][1] * B0 + gam[a][0] * B1;
         p2 = p2 + gam[a][2] * B0 + gam[a][0] * B2;
+    }
+    // All of the above depends on the markers alone: kWait waits only here for
+    // the kernel before it (updvp or pr_submean, which write q2, q3 and pr)
+    if (kWait) FB_GRID_WAIT();
+    // checkbcs: the velocity at the marker from the substep-1 weights
+    double prod = 0.0;
+    if (ok && idir <= 2 && node) {
+        const int t2 = 2 * n + idir - 1;
+        const int *eu = d.eulins + static_cast<size_t>(t2) * 2 * kSD;
+        const double *q = (idir == 1) ? d.q2 : d.q3;
+        prod = d.phi[static_cast<size_t>(t2) * kSD + m] * q[fidx(d, eu[m], eu[kSD + m])];
+    }
+    double f0 = 0.0, fym = 0.0, fzm = 0.0, g2r = 1.0, g3r = 1.0;
+    if (act) {
+        const double *f = (idir == 1) ? d.q2 : (idir == 2 ? d.q3 : d.pr);
+        const double mean = (pend && idir == 3) ? d.scal[S_PRAVG] : 0.0;   // (x - 0.0 is x)
+        f0 = Fv(f, ej, ek) - mean;
+        fym = Fv(f, ej - 1, ek) - mean;
+        fzm = Fv(f, ej, ek - 1) - mean;
+        g2r = d.g2rc[ej];
+        g3r = d.g3rc[ek];
     }
     // getpbup (loads_transfer.F90:285-357) for this quantity; the last two: the
     // partition of unity and checkbcs's velocity
@@ -2023,11 +2034,11 @@ __device__ __forceinline__ void carried_tangent(const Dev &d, int n, double &tan
 // marker with a tangent of its own is finished here (press, tau), one outside
 // the channel gets zeros, and only those whose tangent carries over from
 // another marker are left to the launch that sums the loads.
-template <bool kFinish>
+template <bool kFinish, bool kWait>
 __device__ __forceinline__ void loads_probe_tan_body(const Dev &d, bool pend) {
     if (!d.nlm) return;
     __shared__ double vals[kLoadMk][24];
-    loads_probe_body(d, pend, kFinish ? &vals[0][0] : nullptr);
+    loads_probe_body<kWait>(d, pend, kFinish ? &vals[0][0] : nullptr);
     __syncthreads();
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = T / kLoadLanes;
@@ -2063,8 +2074,7 @@ __device__ __forceinline__ void loads_probe_tan_body(const Dev &d, bool pend) {
 
 template <bool kFinish>
 __global__ void __launch_bounds__(kLoadThreads, 5) k_loads_probe(Dev d, int pend) {
-    FB_GRID_WAIT();
-    loads_probe_tan_body<kFinish>(d, pend != 0);
+    loads_probe_tan_body<kFinish, true>(d, pend != 0);
 }
 
 // loads_transfer_c (loads_transfer.F90:187-214): the tangent carries over
@@ -2484,6 +2494,7 @@ __device__ __forceinline__ void close_body(const Dev &d, int hist_rows) {
     else if (tid >= 64 && tid < 67) mcon[tid - 64] = d.rbmcon[tid - 64];
     const double time = d.scal[S_TIME], stepd = d.scal[S_STEP], cflm = d.scal[S_CFLM];
     const double c0 = d.rigid[0], c1 = d.rigid[1];
+    FB_GRID_WAIT();   // (the probes before it write press, tau, bcerrv, bcerrw, probe)
     const bool good = *d.status == 0;
     double f[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // fyp, fzp, fyv, fzv, mom, the checkbcs sums
     for (int i = tid; i < nlm; i += nt) {
@@ -2553,7 +2564,6 @@ __device__ __forceinline__ void close_body(const Dev &d, int hist_rows) {
 }
 
 __global__ void __launch_bounds__(kCloseThreads, 2) k_step_close(Dev d, int hist_rows) {
-    FB_GRID_WAIT();
     close_body(d, hist_rows);
 }
 
@@ -2674,13 +2684,13 @@ __global__ void kg_spread_chains(const GroupCase *__restrict__ g) {
 __global__ void kg_mls_interp(const GroupCase *__restrict__ g, int clear) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    mls_interp_body(d, clear != 0);
+    mls_interp_body<false>(d, clear != 0);
 }
 
 __global__ void kg_mls_spread(const GroupCase *__restrict__ g) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    mls_spread_body(d);
+    mls_spread_body<false>(d);
 }
 
 __global__ void kg_divg(const GroupCase *__restrict__ g, int n, int extra) {
@@ -2709,7 +2719,7 @@ template <bool kFinish>
 __global__ void __launch_bounds__(kLoadThreads, 5) kg_loads_probe(const GroupCase *__restrict__ g, int pend) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    loads_probe_tan_body<kFinish>(d, pend != 0);
+    loads_probe_tan_body<kFinish, false>(d, pend != 0);
 }
 
 __global__ void __launch_bounds__(kLoadFin) kg_loads_finish(const GroupCase *__restrict__ g) {

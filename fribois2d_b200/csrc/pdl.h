@@ -20,6 +20,14 @@
 // block triggers only once it is running, the next grid launches after all of
 // this grid's blocks have started: a waiting grid never holds slots that this
 // one still needs.
+//
+// What a kernel may read before its wait: the kernel before it has triggered,
+// that is, every block of it has passed its own wait, so everything earlier is
+// complete and visible; only what the kernel directly before it writes is not.
+// The kernels of the time step use that: they load the operands that come from
+// further back, and do the work that depends on them alone, ahead of their wait
+// (marked there with what the kernel before them writes).  Nothing is stored
+// ahead of it that an earlier kernel still running could read.
 #define FB_GRID_WAIT() asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory")
 
 namespace fb {

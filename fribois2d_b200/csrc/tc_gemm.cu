@@ -894,9 +894,10 @@ struct I8Cfg {
     static constexpr uint32_t kATile = 128 * kI8BK;                 // one A digit slice: 128 rows x 128 B
     static constexpr uint32_t kBSlice = BN * kI8BK;                 // one B digit slice
     static constexpr uint32_t kBStage = S * BN * kI8BK;             // all B slices of a k-block
-    // as many A slots (in pairs) as the shared memory holds beside two B stages, at most 10
+    // as many A slots (in pairs) as the shared memory holds beside two B stages, at
+    // most 8: what small products leave lets the next kernel's blocks start early
     static constexpr int kAFit = static_cast<int>((227u * 1024u - 1280u - 2u * kBStage) / kATile);
-    static constexpr int kASlots = (kAFit < 10 ? kAFit : 10) / 2 * 2;
+    static constexpr int kASlots = (kAFit < 8 ? kAFit : 8) / 2 * 2;
     static constexpr size_t kSmem = 2 * kBStage + kASlots * kATile + 1024 + 256;
     static constexpr uint32_t kTmemCols = (S * BN > 256) ? 512 : (S * BN > 128) ? 256 : 128;   // S class accumulators of BN columns
     // D s32 (2), A and B signed 8-bit (1), both K-major, M = 128; N set per MMA

@@ -429,7 +429,9 @@ __global__ void __launch_bounds__(kYLines * W * 32) k_ylines(Dev d, ScanSys s2, 
 // rmax (may be null): the maxima of |hmn| over each row j (over the modes:
 // the rows of the INT8 transform's data operand) are accumulated into rmax[j]
 // from the block's modes, for the digit cut that follows
-template <int M, int W>
+// kWait: the body waits for the kernel before it (the transform, which writes
+// hmn) once the constant operands are under way.
+template <int M, int W, bool kWait>
 __device__ __forceinline__ void ymodes_body(const Dev &d, int nw, double *rmax = nullptr) {
     extern __shared__ double sm[];
     __shared__ double shx[8][2 * W];
@@ -446,11 +448,13 @@ __device__ __forceinline__ void ymodes_body(const Dev &d, int nw, double *rmax =
     const int r = blockIdx.x * nw + w;
     const bool live = r < d.n3m;
     if (live) {
-        const double *row = d.hmn + static_cast<size_t>(r) * d.ldh, *pgr = d.pg + static_cast<size_t>(r) * d.ldh;
-        for (int i = tl; i < n; i += 32 * W) {
-            cp8(line + i, row + i);
-            cp8(piv + i, pgr + i);
-        }
+        const double *pgr = d.pg + static_cast<size_t>(r) * d.ldh;
+        for (int i = tl; i < n; i += 32 * W) cp8(piv + i, pgr + i);
+    }
+    if (kWait) FB_GRID_WAIT();
+    if (live) {
+        const double *row = d.hmn + static_cast<size_t>(r) * d.ldh;
+        for (int i = tl; i < n; i += 32 * W) cp8(line + i, row + i);
     }
     cp_wait();
     __syncthreads();   // the off-diagonals (and every line) are staged
@@ -487,15 +491,14 @@ constexpr int ymodes_threads(int M, int W) { return W == 1 ? 256 : M <= 25 ? 512
 
 template <int M, int W>
 __global__ void __launch_bounds__(ymodes_threads(M, W), 1) k_ymodes(Dev d, int nw, double *rmax) {
-    FB_GRID_WAIT();
-    ymodes_body<M, W>(d, nw, rmax);
+    ymodes_body<M, W, true>(d, nw, rmax);
 }
 
 template <int M, int W>
 __global__ void __launch_bounds__(ymodes_threads(M, W), 1) kg_ymodes(const GroupCase *__restrict__ g, int nw) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    ymodes_body<M, W>(d, nw);
+    ymodes_body<M, W, false>(d, nw);
 }
 
 // ---------------------------------------------------------------- z lines
@@ -661,7 +664,9 @@ struct WinShape {            // shared-memory layout of one tile of kWTk rows (i
 
 // blockIdx.y = 0: v (solq2j + solq2k + walls), 1: w (solq3j + solq3k);
 // blockIdx.x = tile (tj fastest).
-template <int KM, int kWTk>
+// kWait: the body waits for the kernel before it, which writes rhs2/rhs3 (the
+// spreading, or nl_rhs): the coefficients and the tile of q are under way then.
+template <int KM, int kWTk, bool kWait>
 __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd, int ntj, int Ky, int Kz) {
     extern __shared__ __align__(16) double sm[];
     const WinShape<kWTk> sh(Ky, Kz);
@@ -709,6 +714,11 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
             za[c] = zeg[2 * c] = zeg[2 * c + 1] = 0.0;
         }
     }
+    const int j = j0 + lane;
+    const bool jlive = (j >= jlo && j <= d.n2m);
+    if (jlive)
+        for (int r = w; r < kWTk && k0 + r <= d.n3m; r += kWarps) cp8(Q + r * kWTj + lane, q + fidx(d, j, k0 + r));
+    if (kWait) FB_GRID_WAIT();
     {
         constexpr int kCC = 3;   // column chunks of 32 (cols <= 80)
         int jc[kCC];
@@ -731,12 +741,7 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
             }
         }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const int j = j0 + lane;
-    const bool jlive = (j >= jlo && j <= d.n2m);
-    if (jlive)
-        for (int r = w; r < kWTk && k0 + r <= d.n3m; r += kWarps) cp8(Q + r * kWTj + lane, q + fidx(d, j, k0 + r));
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");   // all but q
+    cp_wait();
     __syncthreads();
 
     // 2. y solves: lanes = rows, one segment per warp task; the results go to A
@@ -800,7 +805,6 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
             }
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");   // q
     __syncthreads();
 
     // 3. z solves: lanes = columns, warps = segments of rows; q += result
@@ -838,8 +842,7 @@ constexpr int win_blocks(int KM) { return KM <= 8 ? 4 : KM <= 16 ? 3 : 2; }
 
 template <int KM, int kWTk>
 __global__ void __launch_bounds__(kWThreads, win_blocks(KM)) k_helsolve_win(Dev d, SubDev sd, int ntj, int Ky, int Kz) {
-    FB_GRID_WAIT();
-    helsolve_win_body<KM, kWTk>(d, sd, ntj, Ky, Kz);
+    helsolve_win_body<KM, kWTk, true>(d, sd, ntj, Ky, Kz);
 }
 
 // grouped forms (blockIdx.z = case; substep n 0-based): each case keeps its
@@ -849,7 +852,7 @@ __global__ void __launch_bounds__(kWThreads, win_blocks(KM)) kg_helsolve_win(con
     __shared__ Dev d;
     __shared__ SubDev s;
     if (!stage_case(g, &d, &s, n)) return;
-    helsolve_win_body<KM, kWTk>(d, s, ntj, s.win_y, s.win_z);
+    helsolve_win_body<KM, kWTk, false>(d, s, ntj, s.win_y, s.win_z);
 }
 
 
