@@ -796,7 +796,7 @@ int phcalc_tf32(fb_ctx *c) {
     // phi_0 = Z T^-1 Z^-1 dph into pw
     fb::launch_split_t(d.dph + d.P, d.P, d.n2m, d.n3m, c->pl_a, st, c->zsinv_d);
     fb::launch_tf32x3(c->plan_fwd, d.hmn, d.ldh, nullptr, 0, d.status, st);
-    fb::launch_scan_poisson(d, st);
+    fb::launch_scan_poisson(d, st, nullptr, true);
     fb::launch_split_t(d.hmn, d.ldh, d.n2m, d.n3m, c->pl_a2, st);
     fb::launch_tf32x3(c->plan_bwd, c->pw + d.P, d.P, nullptr, 0, d.status, st, c->zs_d);
     // refinement sweeps: phi += Z T^-1 Z^-1 (dph - L phi); the last lands in dph
@@ -804,7 +804,7 @@ int phcalc_tf32(fb_ctx *c) {
         const bool last = (sw == c->tf32_sweeps);
         fb::launch_poisson_residual(d, c->pw, c->pl_a, st, c->zsinv_d);
         fb::launch_tf32x3(c->plan_fwd, d.hmn, d.ldh, nullptr, 0, d.status, st);
-        fb::launch_scan_poisson(d, st);
+        fb::launch_scan_poisson(d, st, nullptr, true);
         fb::launch_split_t(d.hmn, d.ldh, d.n2m, d.n3m, c->pl_a2, st);
         fb::launch_tf32x3(c->plan_bwd, (last ? d.dph : c->pw) + d.P, d.P, c->pw + d.P, d.P, d.status, st, c->zs_d);
     }
@@ -946,7 +946,7 @@ int stage_impl(fb_ctx *c, int stage, int ns, int n) {
         break;
     case FB_ST_HELSOLVE:
         if (s.win_y > 0) {
-            fb::launch_win_helsolve(d, s, st);
+            fb::launch_win_helsolve(d, s, st, c->poisson_mode == FB_POISSON_TF32X3);
             c->own_launches -= 3;
         } else if (s.scan_ok) {
             fb::launch_scan_helsolve(d, s, st);
@@ -2558,9 +2558,9 @@ int group_helsolve_tile(BatchGroup *bg) {
     for (int cand : {32, 64}) {
         if (r) break;
         bg->g.win_tk = cand;
-        fb::glaunch_win_helsolve(bg->g, 0, bg->st);
+        fb::glaunch_win_helsolve(bg->g, 0, bg->st, bg->tf32);
         cudaEventRecord(e0, bg->st);
-        for (int k = 0; k < 3; ++k) fb::glaunch_win_helsolve(bg->g, 0, bg->st);
+        for (int k = 0; k < 3; ++k) fb::glaunch_win_helsolve(bg->g, 0, bg->st, bg->tf32);
         cudaEventRecord(e1, bg->st);
         float ms = 0.f;
         if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
@@ -2738,18 +2738,18 @@ int enqueue_group_fluid(BatchGroup *bg, int &k) {
         fb::glaunch_nl_rhs(g, s, st, s > 0, fb::kNlBoucdq | (s == 0 ? fb::kNlCfl : 0));
         if (s == 0) CK(cudaStreamWaitEvent(st, bg->join, 0));
         fb::glaunch_forcing(g, s, st);
-        fb::glaunch_win_helsolve(g, s, st);
+        fb::glaunch_win_helsolve(g, s, st, bg->tf32);
         fb::glaunch_divg(g, s, st, fb::kDivBoucqt | (s == 0 ? fb::kDivCfl : 0));
         if (bg->tf32) {   // phcalc_tf32's launches, each over the whole group
             fb::launch_split_t_group(bg->sp, d.n2m, d.n3m, n, st);
             fb::launch_tf32x3_group(bg->gt, bg->plan_fwd, n, st);
-            fb::glaunch_scan_poisson(g, st);
+            fb::glaunch_scan_poisson(g, st, true);
             fb::launch_split_t_group(bg->sp + n, d.n2m, d.n3m, n, st);
             fb::launch_tf32x3_group(bg->gt + n, bg->plan_bwd, n, st);
             for (int sw = 1; sw <= bg->sweeps; ++sw) {   // the last sweep lands in dph
                 fb::launch_poisson_residual_group(g, bg->rt, st);
                 fb::launch_tf32x3_group(bg->gt, bg->plan_fwd, n, st);
-                fb::glaunch_scan_poisson(g, st);
+                fb::glaunch_scan_poisson(g, st, true);
                 fb::launch_split_t_group(bg->sp + n, d.n2m, d.n3m, n, st);
                 fb::launch_tf32x3_group(bg->gt + (sw == bg->sweeps ? 2 : 3) * n, bg->plan_bwd, n, st);
             }

@@ -418,13 +418,77 @@ __global__ void __launch_bounds__(kYLines * W * 32) k_ylines(Dev d, ScanSys s2, 
 // length m (conflict-free 8-byte shared accesses): the forward recurrence
 // y(i) = a(i) y(i-1) + b(i), a(i) = -amphj(i+1) g(i-1), scaled by g(i), and the
 // backward one with e(i) = -apphj(i+1) g(i), each composed per chunk, scanned
-// over the chunks and applied.  A chunk and its coefficients stay in registers
-// (M >= m of them, every loop unrolled), so a step of a chain is one
-// dependent FMA: with the chunk in shared memory a step also waited for its
-// loads behind the step before's store, ~100 cycles, and the solve took 8.7 of
-// the 14.5 us between the launches before and after it at 1024 x 768 (9.9 us
-// now); W = 2 where one warp's chunk would not fit the registers.  nw modes
-// per block, as many as the shared memory holds.
+// over the chunks and applied.  A chunk and its coefficients are held in
+// registers (M >= m of them, every loop unrolled), so a step of a chain is one
+// dependent FMA: with the chunk in shared memory a step also waits for its loads
+// behind the store of the step before, ~100 cycles, and the solve took 8.7 of
+// the 14.5 us between the launches before and after it at 1024 x 768 (8.4 us
+// now).  A longer chunk does not fit the registers: up to 1088 unknowns two warps
+// share a mode (1500 x 1000: 19.5 -> 16.6 us), above that the chunk stays in
+// shared memory (M = 0; 1536 unknowns: 26.2 us, 30.4 with two and 31.7 with three
+// warps, whose registers spill, 39.5 with the chunk in two register parts).  The
+// split-precision form (one_warp) never takes two: a scan over more lanes rounds
+// differently, and its TF32 roundings turn a last bit into 1e-8 of the pressure.
+// nw modes per block, as many as the shared memory holds.
+
+constexpr int kYmModes = 8;   // modes per block at most
+
+// one warp's mode with its chunks in shared memory (solved in place)
+__device__ __forceinline__ void ymodes_loop(int n, const double *am, const double *ap, double *line,
+                                            const double *piv) {
+    const int lane = threadIdx.x & 31;
+    const int m = ((n + 31) / 32) | 1;
+    const int i0 = min(lane * m, n), cnt = min(m, n - i0);
+    // forward: composite of the chunk, y_out = A y_in + C
+    double A = 1.0, C = 0.0;
+    for (int t = 0; t < cnt; ++t) {
+        const int i = i0 + t;
+        const double a = (i == 0) ? 0.0 : -(am[i + 1] * piv[i - 1]);
+        C = fma(a, C, line[i]);
+        A *= a;
+    }
+#pragma unroll
+    for (int dd = 1; dd < 32; dd <<= 1) {
+        const double Ao = __shfl_up_sync(kFull, A, dd), Co = __shfl_up_sync(kFull, C, dd);
+        if (lane >= dd) {
+            C = fma(A, Co, C);
+            A *= Ao;
+        }
+    }
+    double y = __shfl_up_sync(kFull, C, 1);
+    if (lane == 0) y = 0.0;
+    for (int t = 0; t < cnt; ++t) {
+        const int i = i0 + t;
+        const double a = (i == 0) ? 0.0 : -(am[i + 1] * piv[i - 1]);
+        y = fma(a, y, line[i]);
+        line[i] = piv[i] * y;   // g(i) y(i)
+    }
+    // backward: x(i) = e(i) x(i+1) + g(i) y(i)
+    A = 1.0;
+    C = 0.0;
+    for (int t = cnt - 1; t >= 0; --t) {
+        const int i = i0 + t;
+        const double e = (i == n - 1) ? 0.0 : -(ap[i + 1] * piv[i]);
+        C = fma(e, C, line[i]);
+        A *= e;
+    }
+#pragma unroll
+    for (int dd = 1; dd < 32; dd <<= 1) {
+        const double Ao = __shfl_down_sync(kFull, A, dd), Co = __shfl_down_sync(kFull, C, dd);
+        if (lane + dd < 32) {
+            C = fma(A, Co, C);
+            A *= Ao;
+        }
+    }
+    double x = __shfl_down_sync(kFull, C, 1);
+    if (lane == 31) x = 0.0;
+    for (int t = cnt - 1; t >= 0; --t) {
+        const int i = i0 + t;
+        const double e = (i == n - 1) ? 0.0 : -(ap[i + 1] * piv[i]);
+        x = fma(e, x, line[i]);
+        line[i] = x;
+    }
+}
 
 // rmax (may be null): the maxima of |hmn| over each row j (over the modes:
 // the rows of the INT8 transform's data operand) are accumulated into rmax[j]
@@ -434,7 +498,7 @@ __global__ void __launch_bounds__(kYLines * W * 32) k_ylines(Dev d, ScanSys s2, 
 template <int M, int W, bool kWait>
 __device__ __forceinline__ void ymodes_body(const Dev &d, int nw, double *rmax = nullptr) {
     extern __shared__ double sm[];
-    __shared__ double shx[8][2 * W];
+    __shared__ double shx[kYmModes][2 * W];
     const int n = d.n2m, w = threadIdx.x / (32 * W), tl = threadIdx.x % (32 * W);
     double *am = sm, *ap = sm + (n + 2);                       // 1-based off-diagonals
     double *lines = sm + 2 * (n + 2);
@@ -459,18 +523,22 @@ __device__ __forceinline__ void ymodes_body(const Dev &d, int nw, double *rmax =
     cp_wait();
     __syncthreads();   // the off-diagonals (and every line) are staged
     if (live) {
-        const int m = ((n + 32 * W - 1) / (32 * W)) | 1;
-        const int i0 = min(tl * m, n), cnt = min(m, n - i0);
-        double v[M];
+        if constexpr (M == 0) {
+            ymodes_loop(n, am, ap, line, piv);
+        } else {
+            const int m = ((n + 32 * W - 1) / (32 * W)) | 1;
+            const int i0 = min(tl * m, n), cnt = min(m, n - i0);
+            double v[M];
 #pragma unroll
-        for (int t = 0; t < M; ++t)
-            if (t < cnt) v[t] = line[i0 + t];
-        const CoefModeS co{piv, am, ap, n};
-        if constexpr (W == 1) warp_line<M>(v, i0, cnt, co);
-        else group_line<M, W>(v, i0, cnt, co, shx[w], w + 1);
+            for (int t = 0; t < M; ++t)
+                if (t < cnt) v[t] = line[i0 + t];
+            const CoefModeS co{piv, am, ap, n};
+            if constexpr (W == 1) warp_line<M>(v, i0, cnt, co);
+            else group_line<M, W>(v, i0, cnt, co, shx[w], w + 1);
 #pragma unroll
-        for (int t = 0; t < M; ++t)
-            if (t < cnt) line[i0 + t] = v[t];
+            for (int t = 0; t < M; ++t)
+                if (t < cnt) line[i0 + t] = v[t];
+        }
     }
     __syncthreads();   // every live mode's solved line is in shared memory
     const int nlive = max(0, min(nw, d.n3m - static_cast<int>(blockIdx.x) * nw));
@@ -487,15 +555,13 @@ __device__ __forceinline__ void ymodes_body(const Dev &d, int nw, double *rmax =
     }
 }
 
-constexpr int ymodes_threads(int M, int W) { return W == 1 ? 256 : M <= 25 ? 512 : 384; }
-
 template <int M, int W>
-__global__ void __launch_bounds__(ymodes_threads(M, W), 1) k_ymodes(Dev d, int nw, double *rmax) {
+__global__ void __launch_bounds__(32 * W * kYmModes, 1) k_ymodes(Dev d, int nw, double *rmax) {
     ymodes_body<M, W, true>(d, nw, rmax);
 }
 
 template <int M, int W>
-__global__ void __launch_bounds__(ymodes_threads(M, W), 1) kg_ymodes(const GroupCase *__restrict__ g, int nw) {
+__global__ void __launch_bounds__(32 * W * kYmModes, 1) kg_ymodes(const GroupCase *__restrict__ g, int nw) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
     ymodes_body<M, W, false>(d, nw);
@@ -618,16 +684,32 @@ namespace {
 //   x(i) = e(i) x(i+1) + g(i) y(i)   (positions below s + kWSeg + K)
 // A(u), F(u), EG(u) are indexed relative to s; lo: line index 0 relative to s;
 // positions at or past nmax are outside the line (x stays 0).
-template <int KM, class FA, class FE>
-__device__ __forceinline__ void win_segment(const FA &AF, const FE &EG, int K, int lo, int nmax, double (&x)[kWSeg]) {
+// kB > 0: the forward recurrence starts anew, K positions early and from zero, at
+// the positions that are multiples of kB from the tile's edge (b0: the last of
+// them at or before s, relative to s) instead of once before s.  The values
+// differ by less than 2^-56 of their influence.  The split-precision Poisson
+// form takes it, with the blocks of 24 (y) and 16 (z) positions that its results
+// have always been computed with: its TF32 roundings turn a last bit of the
+// right-hand side into 1e-8 of the pressure.
+template <int KM, int kB, class FA, class FE>
+__device__ __forceinline__ void win_segment(const FA &AF, const FE &EG, int K, int lo, int nmax, int b0,
+                                            double (&x)[kWSeg]) {
     double y[kWSeg + KM], v = 0.0;
+    if constexpr (kB == 0) {
 #pragma unroll
-    for (int u = -KM; u < 0; ++u)
-        if (u >= -K && u >= lo) v = AF(u, v);
+        for (int u = -KM; u < 0; ++u)
+            if (u >= -K && u >= lo) v = AF(u, v);
+    } else {
+        for (int u = max(b0 - K, lo); u < 0; ++u) v = AF(u, v);
+    }
 #pragma unroll
     for (int t = 0; t < kWSeg + KM; ++t) {
         y[t] = 0.0;
         if (t < kWSeg + K && t < nmax) {
+            if (kB > 0 && t > 0 && (t - b0) % (kB > 0 ? kB : 1) == 0) {
+                v = 0.0;
+                for (int u = max(t - K, lo); u < t; ++u) v = AF(u, v);
+            }
             v = AF(t, v);
             y[t] = v;
         }
@@ -666,7 +748,8 @@ struct WinShape {            // shared-memory layout of one tile of kWTk rows (i
 // blockIdx.x = tile (tj fastest).
 // kWait: the body waits for the kernel before it, which writes rhs2/rhs3 (the
 // spreading, or nl_rhs): the coefficients and the tile of q are under way then.
-template <int KM, int kWTk, bool kWait>
+// kBlk: the forward recurrences in blocks (win_segment's kB).
+template <int KM, int kWTk, bool kBlk, bool kWait>
 __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd, int ntj, int Ky, int Kz) {
     extern __shared__ __align__(16) double sm[];
     const WinShape<kWTk> sh(Ky, Kz);
@@ -762,12 +845,12 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
         const double2 *as = reinterpret_cast<const double2 *>(cas) + c0;
         const double2 *eg = reinterpret_cast<const double2 *>(ceg) + c0;
         const int s0 = j0 - 1 + sg * kWSeg;   // line index of the segment's start
-        win_segment<KM>(
+        win_segment<KM, kBlk ? 24 : 0>(
             [&](int u, double v) {
                 const double2 c = as[u];
                 return fma(c.x, v, arow[u] * c.y);
             },
-            [&](int u) { return eg[u]; }, Ky, -s0, ny - s0, xs[it]);
+            [&](int u) { return eg[u]; }, Ky, -s0, ny - s0, -sg * kWSeg, xs[it]);
     }
     __syncthreads();
 #pragma unroll
@@ -816,8 +899,8 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
         const double *a = za + c0;
         const double2 *eg = reinterpret_cast<const double2 *>(zeg) + c0;
         double x[kWSeg];
-        win_segment<KM>([&](int u, double v) { return fma(a[u], v, acol[u * kWXp]); }, [&](int u) { return eg[u]; },
-                        Kz, -s0, nz - s0, x);
+        win_segment<KM, kBlk ? 16 : 0>([&](int u, double v) { return fma(a[u], v, acol[u * kWXp]); },
+                                       [&](int u) { return eg[u]; }, Kz, -s0, nz - s0, 0, x);
         if (jlive) {
             const double *qc = Q + sg * kWSeg * kWTj + lane;
 #pragma unroll
@@ -840,19 +923,19 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
 // resident blocks per SM that the registers of the window's segments allow
 constexpr int win_blocks(int KM) { return KM <= 8 ? 4 : KM <= 16 ? 3 : 2; }
 
-template <int KM, int kWTk>
+template <int KM, int kWTk, bool kBlk>
 __global__ void __launch_bounds__(kWThreads, win_blocks(KM)) k_helsolve_win(Dev d, SubDev sd, int ntj, int Ky, int Kz) {
-    helsolve_win_body<KM, kWTk, true>(d, sd, ntj, Ky, Kz);
+    helsolve_win_body<KM, kWTk, kBlk, true>(d, sd, ntj, Ky, Kz);
 }
 
 // grouped forms (blockIdx.z = case; substep n 0-based): each case keeps its
 // own windows, the group's shared memory fits the largest
-template <int KM, int kWTk>
+template <int KM, int kWTk, bool kBlk>
 __global__ void __launch_bounds__(kWThreads, win_blocks(KM)) kg_helsolve_win(const GroupCase *__restrict__ g, int n, int ntj) {
     __shared__ Dev d;
     __shared__ SubDev s;
     if (!stage_case(g, &d, &s, n)) return;
-    helsolve_win_body<KM, kWTk, false>(d, s, ntj, s.win_y, s.win_z);
+    helsolve_win_body<KM, kWTk, kBlk, false>(d, s, ntj, s.win_y, s.win_z);
 }
 
 
@@ -911,7 +994,7 @@ cudaError_t allow_smem(K kern) {
 }  // namespace
 
 // shared memory of the mode solves: the 227 KB opt-in less the static arrays
-// (the grouped kernel's Dev, the warps' composites)
+// (the grouped kernel's Dev)
 constexpr int kYmSmem = 225 * 1024;
 
 cudaError_t scan_configure() {
@@ -919,48 +1002,51 @@ cudaError_t scan_configure() {
 #define AL(K)                                  \
     if ((e = allow_smem(K)) != cudaSuccess) return e;
     AL((k_ylines<9, 0>)) AL((k_ylines<17, 0>)) AL((k_ylines<33, 0>))
-    AL((k_helsolve_win<8, 32>)) AL((k_helsolve_win<8, 64>))
-    AL((k_helsolve_win<12, 32>)) AL((k_helsolve_win<12, 64>))
-    AL((k_helsolve_win<16, 32>)) AL((k_helsolve_win<16, 64>))
-    AL((k_helsolve_win<kWinMax, 32>)) AL((k_helsolve_win<kWinMax, 64>))
-    AL((kg_helsolve_win<8, 32>)) AL((kg_helsolve_win<8, 64>))
-    AL((kg_helsolve_win<12, 32>)) AL((kg_helsolve_win<12, 64>))
-    AL((kg_helsolve_win<16, 32>)) AL((kg_helsolve_win<16, 64>))
-    AL((kg_helsolve_win<kWinMax, 32>)) AL((kg_helsolve_win<kWinMax, 64>))
+#define WN(KM)                                                                                  \
+    AL((k_helsolve_win<KM, 32, false>)) AL((k_helsolve_win<KM, 64, false>))                     \
+    AL((k_helsolve_win<KM, 32, true>)) AL((k_helsolve_win<KM, 64, true>))                       \
+    AL((kg_helsolve_win<KM, 32, false>)) AL((kg_helsolve_win<KM, 64, false>))                   \
+    AL((kg_helsolve_win<KM, 32, true>)) AL((kg_helsolve_win<KM, 64, true>))
+    WN(8) WN(12) WN(16) WN(kWinMax)
+#undef WN
 #define YM(M, W)                                                                                                \
     if ((e = cudaFuncSetAttribute(k_ymodes<M, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kYmSmem)) !=      \
             cudaSuccess ||                                                                                      \
         (e = cudaFuncSetAttribute(kg_ymodes<M, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kYmSmem)) !=     \
             cudaSuccess)                                                                                        \
         return e;
-    YM(9, 1) YM(17, 1) YM(25, 1) YM(17, 2) YM(25, 2) YM(33, 2)
+    YM(9, 1) YM(17, 1) YM(25, 1) YM(0, 1) YM(17, 2)
 #undef YM
 #undef AL
     return cudaSuccess;
 }
 
-template <int TK>
-void win_launch(const Dev &d, const SubDev &s, cudaStream_t st) {
-    const int ntj = (d.n2m + kWTj - 1) / kWTj, ntk = (d.n3m + TK - 1) / TK;
-    const dim3 grid(ntj * ntk, 2);
-    const WinShape<TK> sh(s.win_y, s.win_z);
-    const size_t smem = static_cast<size_t>(sh.a_size + sh.q_size + sh.c_size) * sizeof(double);
-    // the warm-up of every segment runs KM predicated steps: the smallest
-    // instantiated KM that covers both windows
-    const int km = std::max(s.win_y, s.win_z);
-    if (km <= 8)
-        pdl(k_helsolve_win<8, TK>, dim3(grid), dim3(kWThreads), smem, st, d, s, ntj, s.win_y, s.win_z);
-    else if (km <= 12)
-        pdl(k_helsolve_win<12, TK>, dim3(grid), dim3(kWThreads), smem, st, d, s, ntj, s.win_y, s.win_z);
-    else if (km <= 16)
-        pdl(k_helsolve_win<16, TK>, dim3(grid), dim3(kWThreads), smem, st, d, s, ntj, s.win_y, s.win_z);
-    else
-        pdl(k_helsolve_win<kWinMax, TK>, dim3(grid), dim3(kWThreads), smem, st, d, s, ntj, s.win_y, s.win_z);
+namespace {
+// calls go with the smallest instantiated warm-up length that covers the window
+template <class F>
+void win_form(int km, F go) {
+    using std::integral_constant;
+    if (km <= 8) go(integral_constant<int, 8>{});
+    else if (km <= 12) go(integral_constant<int, 12>{});
+    else if (km <= 16) go(integral_constant<int, 16>{});
+    else go(integral_constant<int, kWinMax>{});
 }
 
-void launch_win_helsolve(const Dev &d, const SubDev &s, cudaStream_t st) {
-    if (s.win_tk == 32) win_launch<32>(d, s, st);
-    else win_launch<64>(d, s, st);
+template <int TK>
+void win_launch(const Dev &d, const SubDev &s, cudaStream_t st, bool blocks) {
+    const int ntj = (d.n2m + kWTj - 1) / kWTj, ntk = (d.n3m + TK - 1) / TK;
+    const WinShape<TK> sh(s.win_y, s.win_z);
+    const size_t smem = static_cast<size_t>(sh.a_size + sh.q_size + sh.c_size) * sizeof(double);
+    win_form(std::max(s.win_y, s.win_z), [&](auto KM) {
+        pdl(blocks ? k_helsolve_win<KM, TK, true> : k_helsolve_win<KM, TK, false>, dim3(ntj * ntk, 2), dim3(kWThreads),
+            smem, st, d, s, ntj, s.win_y, s.win_z);
+    });
+}
+}  // namespace
+
+void launch_win_helsolve(const Dev &d, const SubDev &s, cudaStream_t st, bool blocks) {
+    if (s.win_tk == 32) win_launch<32>(d, s, st, blocks);
+    else win_launch<64>(d, s, st, blocks);
 }
 
 void launch_scan_helsolve(const Dev &d, const SubDev &s, cudaStream_t st) {
@@ -969,68 +1055,62 @@ void launch_scan_helsolve(const Dev &d, const SubDev &s, cudaStream_t st) {
 }
 
 namespace {
-// modes per block and shared bytes of k_ymodes: as many as fit (<= 8, and the
-// thread limit of the chunk length's kernel)
-int ymodes_shape(const Dev &d, int M, int W, size_t *smem) {
+// modes per block and shared bytes of k_ymodes: as many as fit
+int ymodes_shape(const Dev &d, size_t *smem) {
     const size_t shared = 2 * static_cast<size_t>(d.n2m + 2) * sizeof(double);
     const size_t per = 2 * static_cast<size_t>(d.n2m + 1) * sizeof(double);
-    int nw = static_cast<int>(std::min<size_t>(8, (kYmSmem - shared) / per));
-    nw = std::max(1, std::min(nw, ymodes_threads(M, W) / (32 * W)));
+    const int nw = std::max(1, static_cast<int>(std::min<size_t>(kYmModes, (kYmSmem - shared) / per)));
     *smem = shared + per * static_cast<size_t>(nw);
     return nw;
 }
 
-// calls go(M, W) as integral constants: chunks of M values on W warps per mode
+// calls go(M, W) as integral constants: lane chunks of M values (0: in shared
+// memory), W warps per mode
 template <class F>
-void ymodes_form(const Dev &d, F go) {
-    const int n = d.n2m;
+void ymodes_form(const Dev &d, bool one_warp, F go) {
     using std::integral_constant;
-    if (n <= 32 * 9) go(integral_constant<int, 9>{}, integral_constant<int, 1>{});
-    else if (n <= 32 * 17) go(integral_constant<int, 17>{}, integral_constant<int, 1>{});
-    else if (n <= 32 * 25) go(integral_constant<int, 25>{}, integral_constant<int, 1>{});
-    else if (n <= 64 * 17) go(integral_constant<int, 17>{}, integral_constant<int, 2>{});
-    else if (n <= 64 * 25) go(integral_constant<int, 25>{}, integral_constant<int, 2>{});
-    else go(integral_constant<int, 33>{}, integral_constant<int, 2>{});
+    const int m = ((d.n2m + 31) / 32) | 1;   // one warp's lane chunk
+    if (m <= 9) go(integral_constant<int, 9>{}, integral_constant<int, 1>{});
+    else if (m <= 17) go(integral_constant<int, 17>{}, integral_constant<int, 1>{});
+    else if (m <= 25) go(integral_constant<int, 25>{}, integral_constant<int, 1>{});
+    else if (d.n2m <= 64 * 17 && !one_warp) go(integral_constant<int, 17>{}, integral_constant<int, 2>{});
+    else go(integral_constant<int, 0>{}, integral_constant<int, 1>{});
 }
 }  // namespace
 
-void launch_scan_poisson(const Dev &d, cudaStream_t st, double *rmax) {
-    ymodes_form(d, [&](auto M, auto W) {
+void launch_scan_poisson(const Dev &d, cudaStream_t st, double *rmax, bool one_warp) {
+    ymodes_form(d, one_warp, [&](auto M, auto W) {
         size_t smem = 0;
-        const int nw = ymodes_shape(d, M, W, &smem);
+        const int nw = ymodes_shape(d, &smem);
         pdl(k_ymodes<M, W>, dim3((d.n3m + nw - 1) / nw), dim3(32 * W * nw), smem, st, d, nw, rmax);
     });
 }
 
+namespace {
 template <int TK>
-void gwin_launch(const Group &g, int n, cudaStream_t st) {
+void gwin_launch(const Group &g, int n, cudaStream_t st, bool blocks) {
     const Dev &d = g.rep;
     const int ntj = (d.n2m + kWTj - 1) / kWTj, ntk = (d.n3m + TK - 1) / TK;
-    const dim3 grid(ntj * ntk, 2, g.n);
     const int ky = g.win_ky[n], kz = g.win_kz[n];
     const WinShape<TK> sh(ky, kz);   // sizes grow with the windows: fits every case
     const size_t smem = static_cast<size_t>(sh.a_size + sh.q_size + sh.c_size) * sizeof(double);
-    const int km = std::max(ky, kz);
-    if (km <= 8)
-        pdl(kg_helsolve_win<8, TK>, grid, dim3(kWThreads), smem, st, g.cases, n, ntj);
-    else if (km <= 12)
-        pdl(kg_helsolve_win<12, TK>, grid, dim3(kWThreads), smem, st, g.cases, n, ntj);
-    else if (km <= 16)
-        pdl(kg_helsolve_win<16, TK>, grid, dim3(kWThreads), smem, st, g.cases, n, ntj);
-    else
-        pdl(kg_helsolve_win<kWinMax, TK>, grid, dim3(kWThreads), smem, st, g.cases, n, ntj);
+    win_form(std::max(ky, kz), [&](auto KM) {
+        pdl(blocks ? kg_helsolve_win<KM, TK, true> : kg_helsolve_win<KM, TK, false>, dim3(ntj * ntk, 2, g.n),
+            dim3(kWThreads), smem, st, g.cases, n, ntj);
+    });
+}
+}  // namespace
+
+void glaunch_win_helsolve(const Group &g, int n, cudaStream_t st, bool blocks) {
+    if (g.win_tk == 32) gwin_launch<32>(g, n, st, blocks);
+    else gwin_launch<64>(g, n, st, blocks);
 }
 
-void glaunch_win_helsolve(const Group &g, int n, cudaStream_t st) {
-    if (g.win_tk == 32) gwin_launch<32>(g, n, st);
-    else gwin_launch<64>(g, n, st);
-}
-
-void glaunch_scan_poisson(const Group &g, cudaStream_t st) {
+void glaunch_scan_poisson(const Group &g, cudaStream_t st, bool one_warp) {
     const Dev &d = g.rep;
-    ymodes_form(d, [&](auto M, auto W) {
+    ymodes_form(d, one_warp, [&](auto M, auto W) {
         size_t smem = 0;
-        const int nw = ymodes_shape(d, M, W, &smem);
+        const int nw = ymodes_shape(d, &smem);
         pdl(kg_ymodes<M, W>, dim3((d.n3m + nw - 1) / nw, 1, g.n), dim3(32 * W * nw), smem, st, g.cases, nw);
     });
 }

@@ -23,12 +23,14 @@ inline int win_tile_rows(int n2m, int n3m, int sms = 148) {
 }
 
 cudaError_t scan_configure();
-void launch_win_helsolve(const Dev &d, const SubDev &s, cudaStream_t st);
+// blocks: forward recurrences in blocks (the split-precision Poisson form)
+void launch_win_helsolve(const Dev &d, const SubDev &s, cudaStream_t st, bool blocks);
 void launch_scan_helsolve(const Dev &d, const SubDev &s, cudaStream_t st);
 // rmax (may be null): n2m row maxima of |hmn| (over the modes) accumulated for
-// the INT8 digit cut
-void launch_scan_poisson(const Dev &d, cudaStream_t st, double *rmax = nullptr);
-void glaunch_win_helsolve(const Group &g, int n, cudaStream_t st);  // substep n (0-based)
-void glaunch_scan_poisson(const Group &g, cudaStream_t st);
+// the INT8 digit cut; one_warp: one warp per mode at any size (the
+// split-precision form)
+void launch_scan_poisson(const Dev &d, cudaStream_t st, double *rmax = nullptr, bool one_warp = false);
+void glaunch_win_helsolve(const Group &g, int n, cudaStream_t st, bool blocks);  // substep n (0-based)
+void glaunch_scan_poisson(const Group &g, cudaStream_t st, bool one_warp = false);
 
 }  // namespace fb
