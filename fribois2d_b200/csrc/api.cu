@@ -908,9 +908,7 @@ int phcalc_i8(fb_ctx *c) {
     // dph's row maxima come from divg, hmn's from the mode solves
     double *mx_dph = c->i8max, *mx_hmn = c->i8max + d.ldh;
     fb::launch_i8_cut_rows(d.dph + d.P, d.P, d.n2m, d.n3m, c->i8a, mx_dph, mx_hmn, st);
-    // (i8f, i8b: cut once at set-up; the pivots for the mode solves that follow)
-    fb::launch_i8x8(c->i8a, c->i8f, d.hmn, d.ldh, d.status, st, true, d.pg,
-                    static_cast<size_t>(d.n3m) * d.ldh * sizeof(double));
+    fb::launch_i8x8(c->i8a, c->i8f, d.hmn, d.ldh, d.status, st, true);   // i8f, i8b: cut once at set-up
     fb::launch_scan_poisson(d, st, mx_hmn);
     fb::launch_i8_cut_rows(d.hmn, d.ldh, d.n2m, d.n3m, c->i8a, mx_hmn, mx_dph, st);
     fb::launch_i8x8(c->i8a, c->i8b, d.dph + d.P, d.P, d.status, st, true);

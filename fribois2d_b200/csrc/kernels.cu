@@ -355,7 +355,7 @@ __device__ __forceinline__ void nl_cell(const Dev &d, const Tile &t, int j0, int
         // alias the shared-memory tile and reuses the tile loads across the
         // thread's consecutive cells
         __stcg(d.rhs2 + i, (ga * dph + ro * ru + alre * dcq2 - dpx22) * dt);
-        __stcs(d.ru2 + i, dph);
+        __stcg(d.ru2 + i, dph);
     }
 
     // ---- w momentum at (jc, kc), kc = 2..n3m
@@ -389,7 +389,7 @@ __device__ __forceinline__ void nl_cell(const Dev &d, const Tile &t, int j0, int
         const size_t i = fidx(d, jc, kc);
         const double ru = ru3v;
         __stcg(d.rhs3 + i, (ga * qcap + ro * ru + alre * dcq3 - dpx33) * dt);
-        __stcs(d.ru3 + i, qcap);
+        __stcg(d.ru3 + i, qcap);
     }
 }
 #undef S2
@@ -492,10 +492,7 @@ __device__ __forceinline__ void nl_prefetch(const Dev &d, NlTile &t, int tile, i
     nl_prefetch_coef(d, t, j0, k0, tid);
 }
 
-// ru2/ru3 at this thread's cells of a tile (0 when ro = 0); read once per
-// substep and written once (nl_cell), both as streams, so that they do not push
-// the fields the next launches share out of L2 (with the pivots' prefetch in
-// the transform before the mode solves: 438 -> 435 us per step at 1024 x 768)
+// ru2/ru3 at this thread's cells of a tile (0 when ro = 0)
 __device__ __forceinline__ void nl_ru(const Dev &d, int tile, int ntj, double ro, double (&r2)[kNlK / 8],
                                       double (&r3)[kNlK / 8]) {
     const int jc = 1 + (tile % ntj) * kNlJ + threadIdx.x, k0 = 1 + (tile / ntj) * kNlK;
@@ -504,8 +501,8 @@ __device__ __forceinline__ void nl_ru(const Dev &d, int tile, int ntj, double ro
         const int kc = k0 + (kNlK / 8) * threadIdx.y + i;
         const bool ok = jc <= d.n2m && kc <= d.n3m && ro != 0.0;
         const size_t x = fidx(d, min(jc, d.n2m), min(kc, d.n3m));
-        r2[i] = ok ? __ldcs(d.ru2 + x) : 0.0;
-        r3[i] = ok ? __ldcs(d.ru3 + x) : 0.0;
+        r2[i] = ok ? d.ru2[x] : 0.0;
+        r3[i] = ok ? d.ru3[x] : 0.0;
     }
 }
 

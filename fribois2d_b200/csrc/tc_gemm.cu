@@ -968,17 +968,6 @@ __device__ __forceinline__ void i8x8_body(const CUtensorMap *ma, const CUtensorM
     // of a B operand that was in place before it (the eigenvector planes), so
     // that they are in flight while the previous kernel drains.
     const bool producer = (warp == 0 && lane == 0);
-    if (!kGlobalMaps && o.pf && warp == 2 && lane == 0) {
-        // this CTA's share of the next kernel's constant operand (nothing
-        // writes it, so it need not wait); DRAM is idle meanwhile
-        const size_t ctas = static_cast<size_t>(gridDim.x) * gridDim.y, me = blockIdx.y * gridDim.x + blockIdx.x;
-        const size_t share = (o.pf_bytes / ctas + 16) / 16 * 16;
-        const size_t from = me * share;
-        if (from < o.pf_bytes) {
-            const uint32_t n = static_cast<uint32_t>(o.pf_bytes - from < share ? o.pf_bytes - from : share);
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(o.pf + from), "r"(n) : "memory");
-        }
-    }
     if (!kGlobalMaps && !producer) FB_GRID_WAIT();
     // the epilogue's scales: this row's, and columns n0 + lane, n0 + 32 + lane
     const int quarter = warp & 3;
@@ -1368,8 +1357,8 @@ void launch_i8_rowmax(const double *src, long lds, int R, int K, double *rmax, c
 
 // the tile width is the B operand's box height (i8_plan)
 void launch_i8x8(const I8Plan &a, const I8Plan &b, double *out, long ldo, int *status, cudaStream_t st,
-                 bool b_const, const void *pf, size_t pf_bytes) {
-    I8Out o{out, ldo, a.scale, b.scale, a.rows, b.rows, b_const ? 1 : 0, static_cast<const char *>(pf), pf_bytes};
+                 bool b_const) {
+    I8Out o{out, ldo, a.scale, b.scale, a.rows, b.rows, b_const ? 1 : 0};
     const dim3 grid((a.rows + 127) / 128, (b.rows + b.box - 1) / b.box);
     auto go = [&](auto kern, size_t smem) {
         pdl(kern, grid, dim3(kI8Threads), smem, st, a.map, b.map, o, a.K, status);

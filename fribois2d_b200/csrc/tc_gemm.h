@@ -117,10 +117,6 @@ struct I8Out {
     const double *rowscale, *colscale;
     int M, N;
     int b_const = 0;   // B's digit planes and scales were written before the previous kernel ran
-    // a constant array that the next kernel reads, brought into L2 while this
-    // one multiplies (16-byte aligned; bytes a multiple of 16)
-    const char *pf = nullptr;
-    size_t pf_bytes = 0;
 };
 // grouped launches (blockIdx.z = case): per-case split sources and products
 struct I8SplitTask {
@@ -154,9 +150,8 @@ void launch_i8_rowmax(const double *src, long lds, int R, int K, double *rmax, c
 // b_const: b's planes and scales were written before the previous kernel in
 // the stream started (the constant eigenvector operand), so its first copies
 // may be issued before waiting for that kernel
-// pf: a constant array of pf_bytes to bring into L2 meanwhile (null: none)
 void launch_i8x8(const I8Plan &a, const I8Plan &b, double *out, long ldo, int *status, cudaStream_t st,
-                 bool b_const = false, const void *pf = nullptr, size_t pf_bytes = 0);
+                 bool b_const = false);
 // the same over n cases of one shape (rep: geometry of the split)
 void launch_i8_split_group(const I8SplitTask *tasks, const I8Plan &rep, int R, int K, int n, cudaStream_t st);
 void launch_i8x8_group(const I8Task *tasks, int M, int N, int n, int bn, cudaStream_t st);
