@@ -2604,8 +2604,9 @@ int group_setup_i8(BatchGroup *bg) {
         const size_t k = static_cast<size_t>(i), m = static_cast<size_t>(n);
         const fb::I8Plan &a = c->i8a;
         const int *gate = couple_gate(c);
-        sp[k] = {d.dph + d.P, d.P, a.dig, a.ldk, a.scale, a.rows_pad, gate};
-        sp[m + k] = {d.hmn, d.ldh, a.dig, a.ldk, a.scale, a.rows_pad, gate};
+        double *mx_dph = c->i8max, *mx_hmn = c->i8max + d.ldh;   // as phcalc_i8
+        sp[k] = {d.dph + d.P, d.P, a.dig, a.ldk, a.scale, a.rows_pad, gate, mx_dph, mx_hmn};
+        sp[m + k] = {d.hmn, d.ldh, a.dig, a.ldk, a.scale, a.rows_pad, gate, mx_hmn, mx_dph};
         gt[k] = {a.map, f.map, fb::I8Out{d.hmn, d.ldh, a.scale, f.scale, d.n2m, d.n3m}, d.n3m, d.status, gate};
         gt[m + k] = {a.map, b.map, fb::I8Out{d.dph + d.P, d.P, a.scale, b.scale, d.n2m, d.n3m}, d.n3m, d.status,
                      gate};
@@ -2691,6 +2692,8 @@ int group_setup(BatchGroup *bg) {
         gc.gate = couple_gate(c);
         gc.fin = c->coupling != FB_COUPLING_LOOSE ? couple_fin(const_cast<fb_ctx *>(c)) : nullptr;
         const Dev &d = c->d;
+        gc.rmax_dph = (c->poisson_mode == FB_POISSON_INT8X8) ? c->i8max : nullptr;
+        gc.rmax_hmn = gc.rmax_dph ? c->i8max + d.ldh : nullptr;
         ptr[static_cast<size_t>(0 * n + i)] = d.dph + d.P;
         ptr[static_cast<size_t>(1 * n + i)] = c->zmmt;
         ptr[static_cast<size_t>(2 * n + i)] = d.hmn;

@@ -99,6 +99,9 @@ struct GroupCase {
     // *gate is non-zero (null: always); fin is its trial load for k_rigid
     const int *gate;
     const double *fin;
+    // row maxima of the INT8 transforms' data operand (null in the other forms):
+    // dph's, accumulated by divg, and hmn's, accumulated by the mode solves
+    double *rmax_dph, *rmax_hmn;
 };
 
 #ifdef __CUDACC__

@@ -2694,7 +2694,7 @@ __global__ void kg_divg(const GroupCase *__restrict__ g, int n, int extra) {
     __shared__ Dev d;
     __shared__ SubDev s;
     if (!stage_case(g, &d, &s, n)) return;
-    divg_body(d, s.usdtal, nullptr, extra);
+    divg_body(d, s.usdtal, g[blockIdx.z].rmax_dph, extra);
 }
 
 __global__ void __launch_bounds__(256, kUpBlocksPerSM) kg_updvp_prcalc(const GroupCase *__restrict__ g, int n,

@@ -13,7 +13,6 @@
 // the accumulator back with tcgen05.ld and store FP64 results.  Every
 // mbarrier wait gives up after one second, records FB_ERR_TIMEOUT and lets
 // the CTA finish (waiting for its own copies and MMAs, freeing its TMEM).
-#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
@@ -655,21 +654,15 @@ __global__ void __launch_bounds__(256) kg_poisson_residual(const GroupCase *__re
 // Per launch, S = 8 -> S = 7: 768 x 1024 22.8 -> 18.4 us (48 columns), 256 x
 // 384 8.7 -> 7.5 us (32 columns; 6.5 with 16).
 
-// Two forms of the digit cut.  k_i8_cut_rows (the single-case step, the
-// eigenvector operands, the public product) takes each row's maximum from an
-// array that the operand's producer (or k_i8_rowmax) accumulated, so its
-// blocks are independent.  kg_i8_cut (the batched launches) finds the maxima
-// itself: a cluster of kCutCl CTAs per 32 rows, each CTA over its own range
-// of 8 V columns, whose row maxima go to the cluster through distributed
-// shared memory.  In both, thread (lane, warp w) holds V consecutive columns
-// of row lane in registers, all its loads in flight at once (each load
-// coalesced over the 32 rows), turns its values into integers (one
-// conversion each), takes the digits from them four columns to a 32-bit word,
-// and stores each slice's V digit bytes of its row with 16-byte stores.  The
-// operand is read once.  Columns past K and rows past R get zero digits, up
-// to ldk and rows_pad.  k_i8_cut_rows has V = 16 for every K: with V = 32 at
-// K = 1500 a thread's two rounds of loads and half as many blocks took 13.3 us.
-constexpr int kCutCl = 8;
+// The digit cut takes each row's maximum from an array that the operand's
+// producer (or k_i8_rowmax) accumulated, so its blocks are independent (finding
+// the maxima itself, a cluster of eight CTAs per 32 rows, it took 13.5 us per
+// launch over groups of two to eight cases of up to 768 x 512; 8.3 us so).  A
+// thread holds 16 consecutive columns of a row in registers, all its loads in
+// flight at once, turns its values into integers (one conversion each), takes the
+// digits from them four columns to a 32-bit word, and stores each slice's 16
+// digit bytes of its row with one store.  The operand is read once.  Columns past
+// K and rows past R get zero digits, up to ldk and rows_pad.
 
 // The exponent of a row whose largest |a| is mm: its digits are those of
 // a 2^-e.  8 slices: |a| 2^-e < 1.  7 slices: at most 0.994, so that the
@@ -772,63 +765,16 @@ __device__ __forceinline__ void i8_cut_emit(const double (&a)[V / 4][4], double 
     }
 }
 
-template <int V>
-__device__ __forceinline__ void i8_cut_body(const double *__restrict__ src, long lds, int R, int K, int8_t *dig,
-                                            long ldk, long plane, double *rowscale) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    constexpr int kP = V / 4;   // 32-bit words (four columns) per thread and slice
-    static_assert(V % 16 == 0, "a thread's run of columns is whole 16-byte stores");
-    __shared__ double part[32];
-    __shared__ double mx[8][32];
-    __shared__ double sc[32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int rank = static_cast<int>(cl.block_rank());
-    const int r0 = (blockIdx.x / kCutCl) * 32, r = r0 + lane;
-    const int c0 = rank * 8 * V + V * w;   // this thread's V consecutive columns of row r
-    double a[kP][4];
-    double m = 0.0;
-#pragma unroll
-    for (int p = 0; p < kP; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int k = c0 + 4 * p + q;   // each load coalesced over the warp's 32 rows
-            a[p][q] = (r < R && k < K) ? src[static_cast<size_t>(k) * lds + r] : 0.0;
-        }
-#pragma unroll
-    for (int p = 0; p < kP; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) m = fmax(m, fabs(a[p][q]));
-    mx[w][lane] = m;
-    __syncthreads();
-    if (w == 0) {
-        for (int q = 1; q < 8; ++q) m = fmax(m, mx[q][lane]);
-        part[lane] = m;
-    }
-    cl.sync();   // every CTA's maxima are written
-    if (w == 0) {
-        double mm = 0.0;
-        for (int q = 0; q < kCutCl; ++q) mm = fmax(mm, *cl.map_shared_rank(&part[lane], q));
-        const int e = i8_row_exp<kI8Step>(mm);
-        sc[lane] = ldexp(1.0, -e);
-        if (rank == 0 && r < R) rowscale[r] = ldexp(1.0, e);
-    }
-    cl.sync();   // no CTA leaves while another still reads its maxima
-    i8_cut_emit<V, kI8Step>(a, sc[lane], r, c0, dig, ldk, plane);
-}
-
-// The cut with the rows' maxima of |a| given (accumulated by the operand's
-// producer, or by k_i8_rowmax): no exchange between blocks.  Block (x, y):
-// rows 32 x .. 32 x + 31, columns 128 y .. 128 y + 127; a warp holds 16 rows of
-// 32 columns, 16 of them per thread, so that one store instruction writes whole
-// 32-byte sectors (half sectors of digit planes that had left L2 since their
-// last use were filled from memory first).  Column group 0 stores the row scales and, for
-// the next producer, clears its maxima (clear, may be null).
+// Block (x, y): rows 32 x .. 32 x + 31, columns 128 y .. 128 y + 127; a warp
+// holds 16 rows of 32 columns, 16 of them per thread, so that one store
+// instruction writes whole 32-byte sectors (half sectors of digit planes that had
+// left L2 since their last use were filled from memory first).  Column group 0
+// stores the row scales and, for the next producer, clears its maxima (clear, may
+// be null).
 template <int S>
-__global__ void __launch_bounds__(256)
-    k_i8_cut_rows(const double *__restrict__ src, long lds, int R, int K, int8_t *dig, long ldk, long plane,
-                  double *rowscale, const double *__restrict__ rmax, double *clear) {
-    FB_GRID_WAIT();
+__device__ __forceinline__ void i8_cut_rows_body(const double *__restrict__ src, long lds, int R, int K, int8_t *dig,
+                                                 long ldk, long plane, double *rowscale,
+                                                 const double *__restrict__ rmax, double *clear) {
     constexpr int V = 16, kP = V / 4;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int r = blockIdx.x * 32 + 16 * (w & 1) + (lane & 15);
@@ -848,6 +794,23 @@ __global__ void __launch_bounds__(256)
         if (clear) clear[r] = 0.0;
     }
     i8_cut_emit<V, S>(a, ldexp(1.0, -e), r, c0, dig, ldk, plane);
+}
+
+template <int S>
+__global__ void __launch_bounds__(256)
+    k_i8_cut_rows(const double *__restrict__ src, long lds, int R, int K, int8_t *dig, long ldk, long plane,
+                  double *rowscale, const double *__restrict__ rmax, double *clear) {
+    FB_GRID_WAIT();
+    i8_cut_rows_body<S>(src, lds, R, K, dig, ldk, plane, rowscale, rmax, clear);
+}
+
+// grouped (blockIdx.z = case)
+__global__ void __launch_bounds__(256) kg_i8_cut_rows(const I8SplitTask *__restrict__ tk, int R, int K) {
+    const I8SplitTask t = tk[blockIdx.z];
+    FB_GRID_WAIT();
+    if (t.gate && !*t.gate) return;
+    i8_cut_rows_body<kI8Step>(t.src, t.lds, R, K, t.dig, t.ldk, t.ldk * static_cast<long>(t.rows_pad), t.scale, t.rmax,
+                              t.clear);
 }
 
 // rmax[r] = max(rmax[r], max_k |src[k lds + r]|) for rows r < R, columns k < K
@@ -870,22 +833,6 @@ __global__ void __launch_bounds__(256) k_i8_rowmax(const double *__restrict__ sr
 }
 
 // grouped (blockIdx.z = case; a cluster never spans two cases)
-template <int V>
-__global__ void __cluster_dims__(kCutCl, 1, 1) __launch_bounds__(256)
-    kg_i8_cut(const I8SplitTask *__restrict__ tk, int R, int K) {
-    const I8SplitTask t = tk[blockIdx.z];
-    FB_GRID_WAIT();
-    if (t.gate && !*t.gate) return;   // the whole cluster: one case
-    i8_cut_body<V>(t.src, t.lds, R, K, t.dig, t.ldk, t.ldk * static_cast<long>(t.rows_pad), t.scale);
-}
-
-// columns per thread: the CTA's share of ldk over its 8 warps
-inline int cut_values(long ldk) {
-    const long per = (ldk + 8 * kCutCl - 1) / (8 * kCutCl);
-    // at least 16: whole 16-byte stores per slice and thread
-    return per <= 16 ? 16 : per <= 32 ? 32 : 64;
-}
-
 // S: digit slices; BN: output tile width, 64, 48, 32 or 16 (a 128 x 48 tile
 // puts 132 CTAs on a 768 x 1024 product where 128 x 64 tiles leave a third of
 // the 148 SMs idle; 32 and 16 spread small products over more SMs)
@@ -1324,14 +1271,8 @@ int i8_configure() {
 }
 
 void launch_i8_split_group(const I8SplitTask *tasks, const I8Plan &rep, int R, int K, int n, cudaStream_t st) {
-    const dim3 grid(rep.rows_pad / 32 * kCutCl, 1, n);
-    switch (cut_values(rep.ldk)) {
-#define FB_CUT_CASE(V) \
-    case V: pdl(kg_i8_cut<V>, grid, dim3(256), 0, st, tasks, R, K); break;
-        FB_CUT_CASE(16) FB_CUT_CASE(32)
-#undef FB_CUT_CASE
-    default: pdl(kg_i8_cut<64>, grid, dim3(256), 0, st, tasks, R, K); break;
-    }
+    pdl(kg_i8_cut_rows, dim3(rep.rows_pad / 32, static_cast<unsigned>(rep.ldk / 128), n), dim3(256), 0, st, tasks, R,
+        K);
 }
 
 void launch_i8x8_group(const I8Task *tasks, int M, int N, int n, int bn, cudaStream_t st) {

@@ -127,6 +127,8 @@ struct I8SplitTask {
     double *scale;
     int rows_pad;
     const int *gate;
+    const double *rmax;       // the rows' maxima, and the array to clear (launch_i8_cut_rows)
+    double *clear;
 };
 struct I8Task {
     CUtensorMap a, b;

@@ -564,7 +564,7 @@ template <int M, int W>
 __global__ void __launch_bounds__(32 * W * kYmModes, 1) kg_ymodes(const GroupCase *__restrict__ g, int nw) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    ymodes_body<M, W, false>(d, nw);
+    ymodes_body<M, W, false>(d, nw, g[blockIdx.z].rmax_hmn);
 }
 
 // ---------------------------------------------------------------- z lines
