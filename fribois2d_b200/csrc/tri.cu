@@ -920,8 +920,10 @@ __device__ __forceinline__ void helsolve_win_body(const Dev &d, const SubDev &sd
     }
 }
 
-// resident blocks per SM that the registers of the window's segments allow
-constexpr int win_blocks(int KM) { return KM <= 8 ? 4 : KM <= 16 ? 3 : 2; }
+// resident blocks per SM that the registers of the window's segments allow (10 rows:
+// the four blocks of 8 with 80 registers; a 20-case batch takes 93.1 ms per 50
+// steps so, 94.4 with its 9 and 10 row windows in the form of 12)
+constexpr int win_blocks(int KM) { return KM <= 10 ? 4 : KM <= 16 ? 3 : 2; }
 
 template <int KM, int kWTk, bool kBlk>
 __global__ void __launch_bounds__(kWThreads, win_blocks(KM)) k_helsolve_win(Dev d, SubDev sd, int ntj, int Ky, int Kz) {
@@ -1007,7 +1009,7 @@ cudaError_t scan_configure() {
     AL((k_helsolve_win<KM, 32, true>)) AL((k_helsolve_win<KM, 64, true>))                       \
     AL((kg_helsolve_win<KM, 32, false>)) AL((kg_helsolve_win<KM, 64, false>))                   \
     AL((kg_helsolve_win<KM, 32, true>)) AL((kg_helsolve_win<KM, 64, true>))
-    WN(8) WN(12) WN(16) WN(kWinMax)
+    WN(8) WN(10) WN(12) WN(16) WN(kWinMax)
 #undef WN
 #define YM(M, W)                                                                                                \
     if ((e = cudaFuncSetAttribute(k_ymodes<M, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kYmSmem)) !=      \
@@ -1027,6 +1029,7 @@ template <class F>
 void win_form(int km, F go) {
     using std::integral_constant;
     if (km <= 8) go(integral_constant<int, 8>{});
+    else if (km <= 10) go(integral_constant<int, 10>{});
     else if (km <= 12) go(integral_constant<int, 12>{});
     else if (km <= 16) go(integral_constant<int, 16>{});
     else go(integral_constant<int, kWinMax>{});
