@@ -92,6 +92,11 @@ struct fb_ctx {
     std::vector<std::pair<const double **, size_t>> coef_fix;
     std::vector<std::pair<const int **, size_t>> coef_fixi;
     size_t coef_cap = 0, coef_capi = 0;
+    // variable dt: where each substep's coefficients start in the two images
+    // (one more than substeps), the dt they were built for, their upload
+    size_t coef_off[fb::kMaxSub + 1] = {}, coef_offi[fb::kMaxSub + 1] = {};
+    double coef_dt[fb::kMaxSub] = {};
+    cudaEvent_t ev_coef = nullptr;
     bool vardt = false;       // idtv = .false.: dt from the CFL number every step
     // strong fluid-structure coupling (fb_set_coupling), iterated on the device
     int coupling = FB_COUPLING_LOOSE;
@@ -338,36 +343,62 @@ int build_substep(fb_ctx *c, int n, double al) {
     return FB_OK;
 }
 
-// (Re)builds the coefficients of every substep for the current dt and
-// uploads them: allocated on the first call, then refreshed in place with one
-// asynchronous copy on the context stream (ordered before the next kernels).
-int build_substeps(fb_ctx *c) {
+void coef_clear(fb_ctx *c) {
     c->coef_h.clear();
     c->coef_hi.clear();
     c->coef_fix.clear();
     c->coef_fixi.clear();
+}
+
+// Builds the coefficients of every substep for the deck's dt and uploads them
+// with one asynchronous copy on the context stream (ordered before the next kernels).
+int build_substeps(fb_ctx *c) {
+    coef_clear(c);
     const int nsst = c->hc.deck.nsst;
     int st;
     for (int n = 0; n < nsst; ++n) {
         const double al = (nsst == 3) ? c->hc.alm[n] : 1.0;
         if ((st = build_substep(c, n, al))) return st;
+        c->coef_dt[n] = c->dt;
+        c->coef_off[n + 1] = c->coef_h.size();
+        c->coef_offi[n + 1] = c->coef_hi.size();
     }
     const size_t nd = c->coef_h.size(), ni = std::max<size_t>(c->coef_hi.size(), 1);
-    if (!c->coef_d) {
-        if ((st = dnew(c, &c->coef_d, nd))) return st;
-        if ((st = dnew(c, &c->coef_di, ni))) return st;
-        CK(cudaMallocHost(&c->coef_pin, nd * sizeof(double)));
-        CK(cudaMallocHost(&c->coef_pini, ni * sizeof(int)));
-        c->coef_cap = nd;
-        c->coef_capi = ni;
-    }
-    if (nd != c->coef_cap || ni != c->coef_capi) return FB_ERR_STATE;  // sizes never change with dt
+    if ((st = dnew(c, &c->coef_d, nd))) return st;
+    if ((st = dnew(c, &c->coef_di, ni))) return st;
+    CK(cudaMallocHost(&c->coef_pin, (nd + 2) * sizeof(double)));   // + the CFL number and the status of a step
+    CK(cudaMallocHost(&c->coef_pini, ni * sizeof(int)));
+    c->coef_cap = nd;
+    c->coef_capi = ni;
     for (auto &f : c->coef_fix) *f.first = c->coef_d + f.second;
     for (auto &f : c->coef_fixi) *f.first = c->coef_di + f.second;
     std::memcpy(c->coef_pin, c->coef_h.data(), nd * sizeof(double));
     if (!c->coef_hi.empty()) std::memcpy(c->coef_pini, c->coef_hi.data(), c->coef_hi.size() * sizeof(int));
     CK(cudaMemcpyAsync(c->coef_d, c->coef_pin, nd * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->coef_di, c->coef_pini, ni * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    return FB_OK;
+}
+
+// The coefficients of substep n (from 0) for the current dt, refreshed in place.
+// The host has waited for the CFL number of this step, so the kernels and copies
+// of the step before are done with both images; the copies run on the side
+// stream, and the context stream waits for them before its next launch.
+int rebuild_substep(fb_ctx *c, int n) {
+    coef_clear(c);
+    const int st = build_substep(c, n, c->hc.deck.nsst == 3 ? c->hc.alm[n] : 1.0);
+    if (st) return st;
+    const size_t o = c->coef_off[n], oi = c->coef_offi[n], nd = c->coef_h.size(), ni = c->coef_hi.size();
+    if (nd != c->coef_off[n + 1] - o || ni != c->coef_offi[n + 1] - oi) return FB_ERR_STATE;  // sizes never change with dt
+    for (auto &f : c->coef_fix) *f.first = c->coef_d + o + f.second;
+    for (auto &f : c->coef_fixi) *f.first = c->coef_di + oi + f.second;
+    std::memcpy(c->coef_pin + o, c->coef_h.data(), nd * sizeof(double));
+    if (ni) std::memcpy(c->coef_pini + oi, c->coef_hi.data(), ni * sizeof(int));
+    CK(cudaMemcpyAsync(c->coef_d + o, c->coef_pin + o, nd * sizeof(double), cudaMemcpyHostToDevice, c->side));
+    if (ni)
+        CK(cudaMemcpyAsync(c->coef_di + oi, c->coef_pini + oi, ni * sizeof(int), cudaMemcpyHostToDevice, c->side));
+    CK(cudaEventRecord(c->ev_coef, c->side));
+    CK(cudaStreamWaitEvent(c->stream, c->ev_coef, 0));
+    c->coef_dt[n] = c->dt;
     return FB_OK;
 }
 
@@ -453,6 +484,7 @@ int create_impl(const char *dir, int device, fb_ctx *c) {
     CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&c->ev_coef, cudaEventDisableTiming));
     CK(cudaEventCreate(&c->ev0));
     CK(cudaEventCreate(&c->ev1));
     CB(cublasCreate(&c->blas));
@@ -1000,27 +1032,26 @@ int stage_impl(fb_ctx *c, int stage, int ns, int n) {
     return FB_OK;
 }
 
-// fluid_tsch.F90:30-182 enqueued on the context stream (no host sync)
 // variable dt (fluid_tsch.F90:34-48): the CFL number of the current field
-// sets dt = cflmax / cflm (at most dtmax) from the second step on; the
-// substep coefficients are rebuilt for it.  Runs cfl and waits for it.
-int vardt_update(fb_ctx *c, int ns) {
+// sets dt = cflmax / cflm (at most dtmax) from the second step on.  Runs cfl and
+// waits for it; before is the status word ahead of this step.
+int vardt_update(fb_ctx *c, int ns, int *before) {
     int r;
     if ((r = stage_impl(c, FB_ST_CFL, ns, 1))) return r;
-    double am = 0.0;
-    CK(cudaMemcpyAsync(&am, c->d.scal + fb::S_CFLRAW, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    double *am = c->coef_pin + c->coef_cap;
+    int *status = reinterpret_cast<int *>(am + 1);
+    CK(cudaMemcpyAsync(am, c->d.scal + fb::S_CFLRAW, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    if (before) CK(cudaMemcpyAsync(status, c->d.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (before && (*before = *status)) return FB_OK;
     double dt = c->dt;
     if (ns > 0) {
-        dt = c->hc.deck.cflmax / am;
+        dt = c->hc.deck.cflmax / *am;
         if (dt > c->hc.deck.dtmax) dt = c->hc.deck.dtmax;
     }
     if (!(dt >= 1.0e-8)) return FB_ERR_CFL;
-    if (dt != c->dt) {
-        c->dt = dt;
-        c->d.dt = dt;
-        if ((r = build_substeps(c))) return r;
-    }
+    c->dt = dt;
+    c->d.dt = dt;
     return FB_OK;
 }
 
@@ -1075,6 +1106,9 @@ int enqueue_substeps(fb_ctx *c, int ns, bool follows) {
             fb::launch_mls_spread(d, c->stream);
             c->own_launches += 2;
         }
+        // variable dt: the host builds the coefficients beside the kernels above
+        // (and the substep before)
+        if (c->vardt && c->coef_dt[n - 1] != c->dt && (r = rebuild_substep(c, n - 1))) return r;
         if ((r = stage_impl(c, FB_ST_HELSOLVE, ns, n))) return r;
         fb::launch_divg(d, c->usdtal[n - 1], c->stream,
                         c->poisson_mode == FB_POISSON_INT8X8 ? c->i8max : nullptr,
@@ -1111,21 +1145,23 @@ int end_side(fb_ctx *c) {
     return FB_OK;
 }
 
-// the fluid step up to its last updvp
-int enqueue_fluid_start(fb_ctx *c, int ns) {
+// The fluid step (fluid_tsch.F90:30-182) up to its last updvp.  Variable dt: the
+// marker set-up needs no dt and runs beside cfl and the host's wait for it; with
+// before, a status raised by an earlier step ends the step here.
+int enqueue_fluid_start(fb_ctx *c, int ns, int *before = nullptr) {
     int r;
-    if (c->vardt && (r = vardt_update(c, ns))) return r;
     if (c->d.nlm) {
         if ((r = fork_side(c))) return r;
         enqueue_marker_setup(c, c->side);
         if ((r = end_side(c))) return r;
     }
+    if (c->vardt && ((r = vardt_update(c, ns, before)) || (before && *before))) return r;
     return enqueue_substeps(c, ns, false);
 }
 
-int enqueue_fluid(fb_ctx *c, int ns) {
-    const int r = enqueue_fluid_start(c, ns);
-    return r ? r : enqueue_fluid_end(c, ns);
+int enqueue_fluid(fb_ctx *c, int ns, int *before = nullptr) {
+    const int r = enqueue_fluid_start(c, ns, before);
+    return r || (before && *before) ? r : enqueue_fluid_end(c, ns);
 }
 
 int enqueue_report(fb_ctx *c) {
@@ -1135,9 +1171,9 @@ int enqueue_report(fb_ctx *c) {
     return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
 
-int enqueue_step(fb_ctx *c, int ns) {
-    int r = enqueue_fluid(c, ns);
-    if (r) return r;
+int enqueue_step(fb_ctx *c, int ns, int *before = nullptr) {
+    int r = enqueue_fluid(c, ns, before);
+    if (r || (before && *before)) return r;
     if (c->d.nlm) {
         if ((r = stage_impl(c, FB_ST_RIGID, ns, 1))) return r;
         return enqueue_report(c);
@@ -1510,6 +1546,7 @@ int fb_destroy(fb_ctx *c) {
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
+    if (c->ev_coef) cudaEventDestroy(c->ev_coef);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return FB_OK;
@@ -1816,20 +1853,39 @@ int fb_advance(fb_ctx *c, int ns0, int nsteps, double *hist) {
         if (done == nsteps) return FB_OK;
     }
     if (c->vardt) {   // dt changes every step: eager launches, no captured graph
+        // One wait per step, for its CFL number and the status the steps before
+        // it have left; the history rows are read once per ring.  The launches
+        // that need no coefficients go before their building (60 steps on
+        // 501 x 333, dt following the CFL number: 11.2 ms; with the coefficients
+        // built before the first launch and a wait and two copies at the end of
+        // each step 15.1 ms).
         c->last_ms = 0.0;
-        for (; done < nsteps; ++done) {
-            CK(cudaEventRecord(c->ev0, c->stream));
-            if ((r = enqueue_step(c, ns0 + done))) return r;
-            CK(cudaEventRecord(c->ev1, c->stream));
-            if ((r = read_status(c, &status))) return r;
-            float ms = 0.f;
-            CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-            c->last_ms += ms;
-            if (hist && (r = fb_last_history(c, hist + static_cast<size_t>(done) * FB_HIST_COLS))) return r;
+        if (!nsteps) return FB_OK;
+        double row0;
+        CK(cudaMemcpyAsync(&row0, c->d.scal + fb::S_STEP, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        int read = 0;
+        auto rows = [&] {
+            if (!hist || read == done) return static_cast<int>(FB_OK);
+            const int e = copy_history(c, hist + static_cast<size_t>(read) * FB_HIST_COLS, static_cast<int>(row0) + read,
+                                       done - read);
+            read = done;
+            return e;
+        };
+        CK(cudaEventRecord(c->ev0, c->stream));
+        int e = FB_OK;
+        while (done < nsteps && !status && !e) {
+            if ((e = enqueue_step(c, ns0 + done, done ? &status : nullptr)) || status) break;
             host_clock(c, 1);
-            if (status) return status;
+            ++done;
+            if (done - read == c->hist_cap) e = rows();
         }
-        return FB_OK;
+        CK(cudaEventRecord(c->ev1, c->stream));
+        int last = 0;
+        if ((r = read_status(c, &last)) || (r = rows())) return r;
+        float ms = 0.f;
+        CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+        c->last_ms = ms;
+        return status ? status : e ? e : last;
     }
     // the first Adams-Bashforth step has its own coefficients: run it eagerly
     if (c->coupling == FB_COUPLING_LOOSE && c->hc.deck.nsst == 1 && ns0 == 0 && nsteps > 0) {
