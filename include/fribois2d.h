@@ -306,7 +306,7 @@ int fb_kernel_count(fb_ctx *ctx, int32_t *per_step);
 #define FB_POISSON_TF32X3 1
 /* FB_POISSON_INT8X8 (the default): the two FP64 eigen transforms computed
  * exactly in integer arithmetic on the INT8 tensor cores (rows scaled by
- * powers of two and cut into 8 signed 8-bit digits; the digit products summed
+ * powers of two and cut into 7 balanced 8-bit digits; the digit products summed
  * in FP64): FP64-level accuracy (~2e-16 of sum |a||b| at K = 1024, as DGEMM),
  * no refinement sweep; K (= n3 - 1) at most 16384. */
 #define FB_POISSON_INT8X8 2
