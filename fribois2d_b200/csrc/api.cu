@@ -1145,9 +1145,23 @@ int end_side(fb_ctx *c) {
     return FB_OK;
 }
 
+// Takes back the marker set-up on the side branch of a step that ends before its
+// forcing: the branch joins (nothing of the step still runs when the caller next
+// writes the markers), and the spreading table is empty for the next set-up.
+int undo_marker_setup(fb_ctx *c) {
+    if (!c->d.nlm) return FB_OK;
+    CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+    fb::launch_table_clear(c->d, c->stream);
+    c->own_launches += 1;
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(c->stream));
+    return FB_OK;
+}
+
 // The fluid step (fluid_tsch.F90:30-182) up to its last updvp.  Variable dt: the
-// marker set-up needs no dt and runs beside cfl and the host's wait for it; with
-// before, a status raised by an earlier step ends the step here.
+// marker set-up needs no dt and runs beside cfl and the host's wait for it, and
+// is taken back where dt is refused; with before, a status raised by an earlier
+// step ends the step here.
 int enqueue_fluid_start(fb_ctx *c, int ns, int *before = nullptr) {
     int r;
     if (c->d.nlm) {
@@ -1155,7 +1169,10 @@ int enqueue_fluid_start(fb_ctx *c, int ns, int *before = nullptr) {
         enqueue_marker_setup(c, c->side);
         if ((r = end_side(c))) return r;
     }
-    if (c->vardt && ((r = vardt_update(c, ns, before)) || (before && *before))) return r;
+    if (c->vardt && ((r = vardt_update(c, ns, before)) || (before && *before))) {
+        const int u = undo_marker_setup(c);
+        return r ? r : u;
+    }
     return enqueue_substeps(c, ns, false);
 }
 

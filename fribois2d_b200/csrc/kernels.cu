@@ -719,21 +719,21 @@ __device__ __forceinline__ unsigned bucket_hash(unsigned long long key, int hlog
     return static_cast<unsigned>((key * 0x9E3779B97F4A7C15ull) >> (64 - hlog));
 }
 
+// empties the spreading-table entry that (marker, direction) tt filled.  Every
+// used entry is some marker's own, so all of them together empty the table.
+__device__ __forceinline__ void clear_entry(const Dev &d, int tt) {
+    const int e = d.hslot[tt];
+    if (!e) return;
+    d.hkey[e - 1] = 0ull;
+    d.hcnt[e - 1] = 0;
+    d.hslot[tt] = 0;
+}
+
 // lgrdistribution.F90:189-267: nearest nodes per marker and direction
 __device__ __forceinline__ void lgrdist_body(const Dev &d) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.nlm) return;
-    // empty the spreading-table entries this marker filled at the previous
-    // step: every used entry is some marker's own entry, so the table is
-    // empty again before the set-up fills it
-    for (int dir = 0; dir < 2; ++dir) {
-        const int e = d.hslot[2 * i + dir];
-        if (e) {
-            d.hkey[e - 1] = 0ull;
-            d.hcnt[e - 1] = 0;
-            d.hslot[2 * i + dir] = 0;
-        }
-    }
+    for (int dir = 0; dir < 2; ++dir) clear_entry(d, 2 * i + dir);   // empty before the set-up fills it
     const double y = d.lmcc[2 * i], z = d.lmcc[2 * i + 1];
     if (y > d.rext2 || y < 0.0 || z > d.alx3 || z < 0.0 || !(y == y) || !(z == z)) {
         raise_status(d, FB_ERR_MARKER_OUT);
@@ -956,7 +956,8 @@ __device__ __forceinline__ void sd_axes(const Dev &d, int idir, const double *&y
 // kFind: the group also finds its nearest y and z lines
 // (lgrdistribution.F90:189-267), one per lane, in place of a launch of its own
 // whose threads made the four searches of a marker one after another; the
-// spreading table is empty then (k_mls_interp empties it behind the chains).
+// spreading table has to be empty then: k_mls_interp empties it behind the
+// chains, k_table_clear where a step ends before it.
 constexpr int kSetupThreads = 128;
 template <bool kFind>
 __device__ __forceinline__ void mls_setup_body(const Dev &d) {
@@ -1098,8 +1099,7 @@ __global__ void k_mls_setup(Dev d) {
 // support loads are independent, and each lane forms the sum of the nine
 // products in node order from the group's shuffles (the sequential sum).
 // clear (substep 1): the spreading table, read for the last time by
-// k_spread_chains, is emptied for the next step (every used entry is some
-// marker's own).
+// k_spread_chains, is emptied for the next step.
 constexpr int kInterpLanes = 16;
 // kWait: the body waits for the kernel before it (nl_rhs, which writes
 // rhs2/rhs3, or the spreading chains) with everything else loaded.
@@ -1132,14 +1132,7 @@ __device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
     }
     if (kWait) FB_GRID_WAIT();
     const bool stopped = (*d.status != 0);
-    if (clear && have && m == kInterpLanes - 1) {   // (a lane without a node)
-        const int e = d.hslot[tt];
-        if (e) {
-            d.hkey[e - 1] = 0ull;
-            d.hcnt[e - 1] = 0;
-            d.hslot[tt] = 0;
-        }
-    }
+    if (clear && have && m == kInterpLanes - 1) clear_entry(d, tt);   // (a lane without a node)
     const double prod = rp ? phim * (qv + *rp) : phim * 0.0;
     double u = 0.0;
 #pragma unroll
@@ -1155,6 +1148,14 @@ __device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
 }
 
 __global__ void k_mls_interp(Dev d, int clear) { mls_interp_body<true>(d, clear != 0); }
+
+// the spreading table emptied on its own: a step that ends between its marker
+// set-up and its interpolation (a refused dt)
+__global__ void k_table_clear(Dev d) {
+    FB_GRID_WAIT();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 2 * d.nlm) clear_entry(d, t);
+}
 
 // interp_spread, spreading half, without atomics on the field.  Once per
 // step (the supports are fixed for the three substeps) every cell's touchers
@@ -2819,6 +2820,9 @@ void launch_mls_setup(const Dev &d, cudaStream_t s, bool find) {
 }
 void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear) {
     if (d.nlm) pdl(k_mls_interp, dim3((2 * d.nlm * kInterpLanes + 255) / 256), dim3(256), 0, s, d, clear ? 1 : 0);
+}
+void launch_table_clear(const Dev &d, cudaStream_t s) {
+    if (d.nlm) pdl(k_table_clear, dim3((2 * d.nlm + 127) / 128), dim3(128), 0, s, d);
 }
 namespace {
 inline int chain_blocks(int nlm) { return (2 * nlm * kSD * kNodeLanes + kChainThreads - 1) / kChainThreads; }

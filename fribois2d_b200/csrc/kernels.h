@@ -35,6 +35,8 @@ void launch_lgrdist(const Dev &d, cudaStream_t s);
 void launch_mls_setup(const Dev &d, cudaStream_t s, bool find = false);
 // clear: empty the spreading table behind k_spread_chains (substep 1)
 void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear);
+// empty the spreading table behind a set-up that no interpolation follows
+void launch_table_clear(const Dev &d, cudaStream_t s);
 void launch_mls_spread(const Dev &d, cudaStream_t s);
 void launch_spread_chains(const Dev &d, cudaStream_t s);
 void launch_helsolve(const Dev &d, const SubDev &sd, cudaStream_t s);
