@@ -366,7 +366,8 @@ int build_substeps(fb_ctx *c) {
     const size_t nd = c->coef_h.size(), ni = std::max<size_t>(c->coef_hi.size(), 1);
     if ((st = dnew(c, &c->coef_d, nd))) return st;
     if ((st = dnew(c, &c->coef_di, ni))) return st;
-    CK(cudaMallocHost(&c->coef_pin, (nd + 2) * sizeof(double)));   // + the CFL number and the status of a step
+    // + the CFL number of a step, the scalars and status ahead of it
+    CK(cudaMallocHost(&c->coef_pin, (nd + 1 + fb::kScalStatus + 1) * sizeof(double)));
     CK(cudaMallocHost(&c->coef_pini, ni * sizeof(int)));
     c->coef_cap = nd;
     c->coef_capi = ni;
@@ -625,12 +626,12 @@ int create_impl(const char *dir, int device, fb_ctx *c) {
     if ((st = dnew(c, &d.rigid, 18))) return st;
     if ((st = h2d(c, d.rigid, c->hc.rigid, 18 * sizeof(double)))) return st;
     if ((st = dnew(c, &d.forces, 8))) return st;
-    if ((st = dnew(c, &d.scal, fb::S_SLOTS))) return st;
+    if ((st = dnew(c, &d.scal, fb::kScalStatus + 1))) return st;
+    d.status = reinterpret_cast<int *>(d.scal + fb::kScalStatus);
     c->hist_cap = 4096;
     if ((st = dnew(c, &d.hist, static_cast<size_t>(c->hist_cap) * FB_HIST_COLS))) return st;
     if ((st = dnew(c, &d.red, static_cast<size_t>(3) * fb::kRedSlot))) return st;
     if ((st = dnew(c, &d.count, 4))) return st;
-    if ((st = dnew(c, &d.status, 1))) return st;
     const size_t gridblocks = static_cast<size_t>((d.n2m + 31) / 32) * ((d.n3m + 7) / 8);
     if (gridblocks > static_cast<size_t>(fb::kRedSlot)) return FB_ERR_UNSUPPORTED;
     d.rbden = dk.rbden;
@@ -1034,16 +1035,20 @@ int stage_impl(fb_ctx *c, int stage, int ns, int n) {
 
 // variable dt (fluid_tsch.F90:34-48): the CFL number of the current field
 // sets dt = cflmax / cflm (at most dtmax) from the second step on.  Runs cfl and
-// waits for it; before is the status word ahead of this step.
-int vardt_update(fb_ctx *c, int ns, int *before) {
-    int r;
-    if ((r = stage_impl(c, FB_ST_CFL, ns, 1))) return r;
+// waits for it; before is the status word ahead of this step (h: note_state's
+// copy), which ends it here when it is set.
+int vardt_update(fb_ctx *c, int ns, const double *h, int *before) {
+    fb::launch_cfl(c->d, c->stream);
+    c->own_launches += 1;
+    CK(cudaGetLastError());
     double *am = c->coef_pin + c->coef_cap;
-    int *status = reinterpret_cast<int *>(am + 1);
     CK(cudaMemcpyAsync(am, c->d.scal + fb::S_CFLRAW, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (before) CK(cudaMemcpyAsync(status, c->d.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    if (before && (*before = *status)) return FB_OK;
+    if (before) {
+        std::memcpy(before, h + fb::kScalStatus, sizeof(int));
+        if (*before) return FB_OK;
+    }
+    coefs(c, ns, 1, c->al, c->ga, c->ro);
     double dt = c->dt;
     if (ns > 0) {
         dt = c->hc.deck.cflmax / *am;
@@ -1145,15 +1150,27 @@ int end_side(fb_ctx *c) {
     return FB_OK;
 }
 
-// Takes back the marker set-up on the side branch of a step that ends before its
-// forcing: the branch joins (nothing of the step still runs when the caller next
-// writes the markers), and the spreading table is empty for the next set-up.
-int undo_marker_setup(fb_ctx *c) {
-    if (!c->d.nlm) return FB_OK;
-    CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
-    fb::launch_table_clear(c->d, c->stream);
-    c->own_launches += 1;
-    CK(cudaGetLastError());
+// A step at variable dt may end behind its marker set-up (dt refused, or an error
+// of the step before).  Its scalars and status word are noted ahead of the fork:
+// behind it the set-up may already have raised an error of its own.
+int note_state(fb_ctx *c, double *h) {
+    CK(cudaMemcpyAsync(h, c->d.scal, (fb::kScalStatus + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    return FB_OK;
+}
+
+// Ends such a step as if it had not begun: the side branch joins (nothing of the
+// step still runs when the caller next writes the markers), the spreading table is
+// empty for the next set-up, and the status word is what it was.  scalars: the
+// CFL number and the mean w too (a refused dt leaves those that it was refused by).
+int undo_start(fb_ctx *c, const double *h, bool scalars) {
+    if (c->d.nlm) {
+        CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+        fb::launch_table_clear(c->d, c->stream);
+        c->own_launches += 1;
+        CK(cudaGetLastError());
+    }
+    CK(cudaMemcpyAsync(c->d.status, h + fb::kScalStatus, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    if (scalars) CK(cudaMemcpyAsync(c->d.scal, h, fb::S_COUNT * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return FB_OK;
 }
@@ -1164,14 +1181,21 @@ int undo_marker_setup(fb_ctx *c) {
 // step ends the step here.
 int enqueue_fluid_start(fb_ctx *c, int ns, int *before = nullptr) {
     int r;
+    double *h = c->coef_pin + c->coef_cap + 1;
+    if (c->vardt && (r = note_state(c, h))) return r;
     if (c->d.nlm) {
         if ((r = fork_side(c))) return r;
         enqueue_marker_setup(c, c->side);
         if ((r = end_side(c))) return r;
     }
-    if (c->vardt && ((r = vardt_update(c, ns, before)) || (before && *before))) {
-        const int u = undo_marker_setup(c);
-        return r ? r : u;
+    if (c->vardt) {
+        r = vardt_update(c, ns, h, before);
+        const bool stopped = !r && before && *before;
+        if (stopped || r == FB_ERR_CFL) {
+            const int u = undo_start(c, h, stopped);
+            return r ? r : u;
+        }
+        if (r) return r;
     }
     return enqueue_substeps(c, ns, false);
 }

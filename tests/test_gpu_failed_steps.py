@@ -1,0 +1,76 @@
+"""What a step that ends with an error leaves behind: the same, whether it is
+taken by fb_advance, by a batch, by the separate calls or stage by stage.
+
+* At variable dt the step that raises an error is counted, with its history
+  row, and the next one leaves no trace.
+"""
+import numpy as np
+import pytest
+
+import fribois2d_b200 as fb
+from fribois2d_b200 import case as cases
+
+pytestmark = pytest.mark.gpu
+
+STATE = ("q2", "q3", "pr", "ru2", "ru3", "lmcc", "lmvel", "lmnor", "rigid", "press", "tau", "qb2n", "qb3n", "dq3x2o")
+
+
+def _open(c, path):
+    s = fb.Solver(path)
+    q2 = s.get("q2")
+    q2[1:c.n3m + 1] += c.v_perturbation()
+    s.set("q2", q2)
+    return s
+
+
+def _fails(call, code):
+    with pytest.raises(fb.FBError) as e:
+        call()
+    assert e.value.code == code
+
+
+def _move(c, y, z):
+    """The body's centre at (y, z)."""
+    c.vert = c.vert + (np.array([y, z]) - c.params.cmposi)
+    c.params.cmposi = (y, z)
+
+
+@pytest.mark.parametrize("nsst", [3, 1])
+def test_variable_dt_counts_the_failing_step(nsst, tmp_path):
+    # the body drifts into the second cell at the upper wall, where the support
+    # does not fit: the marker set-up of the step that follows raises the error
+    c = cases.tiny_cylinder()
+    c.params.idtv = False
+    c.params.nsst = nsst
+    c.params.cflmax = 0.25
+    c.params.dtmax = 0.02
+    c.params.cbody = False
+    c.params.ipert = (1.0, 0.0, 0.0)
+    c.params.kk = (0.0, 0.0, 0.0)
+    rm = 0.5 * (c.ycoord[1:] + c.ycoord[:-1])
+    _move(c, 0.5 * (rm[-3] + rm[-2]) - 0.5 - 0.05, 3.0)
+    path = c.write(str(tmp_path / "deck"))
+    a, b = _open(c, path), _open(c, path)
+    rows, code = [], 0
+    for ns in range(20):
+        try:
+            a.fluid_tsch(ns)
+        except fb.FBError as e:
+            code = e.code
+        try:
+            a.rigid(ns)
+        except fb.FBError as e:
+            assert e.code == code
+        rows.append(a.last_history())
+        if code:
+            break
+    assert code and len(rows) > 2
+    _fails(lambda: b.advance(0, 20), code)
+    np.testing.assert_array_equal(b.last_history(), rows[-1])
+    for f in STATE:
+        np.testing.assert_array_equal(b.get(f), a.get(f), err_msg=f)
+    sa, sb = a.scalars(), b.scalars()
+    for f in ("time", "dt", "dt_o", "cflm", "q3avg", "nbcv", "nbcw", "pravg"):
+        assert sb[f] == sa[f], f
+    for s in (a, b):
+        s.close()
