@@ -1212,10 +1212,10 @@ int enqueue_report(fb_ctx *c) {
     return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
 
-// The end of a step behind its last updvp (loads, rigid update, report), the
+// The end of step ns behind its last updvp (loads, rigid update, report), the
 // next one's explicit terms (next) on the side branch behind the rigid update.
 // pend: the step's last pressure mean is still to be subtracted.
-int enqueue_step_end(fb_ctx *c, bool pend, bool next) {
+int enqueue_step_end(fb_ctx *c, int ns, bool pend, bool next) {
     const Dev &d = c->d;
     const bool close = c->hc.deck.cbody && fb::step_closes(d.nlm);
     int r;
@@ -1229,6 +1229,7 @@ int enqueue_step_end(fb_ctx *c, bool pend, bool next) {
     if (close) fb::launch_step_close(d, c->hist_cap, c->stream);
     else fb::launch_rigid(d, c->hist_cap, c->stream);
     c->own_launches += 1;
+    coefs(c, ns, 1, c->al, c->ga, c->ro);   // FB_SCALARS: as behind fb_rigid
     if (next) {
         if ((r = fork_side(c))) return r;
         enqueue_nl_rhs(c, 1, 1, true, c->side);
@@ -1247,7 +1248,7 @@ int enqueue_step(fb_ctx *c, int ns, int *before = nullptr) {
     fb::launch_submean_boucqt(c->d, c->stream, true);
     c->own_launches += 1;
     CK(cudaGetLastError());
-    return c->d.nlm ? enqueue_step_end(c, false, false) : FB_OK;
+    return c->d.nlm ? enqueue_step_end(c, ns, false, false) : FB_OK;
 }
 
 // The end of a step and the next one up to its last updvp.  nl_rhs of the next
@@ -1256,11 +1257,13 @@ int enqueue_step(fb_ctx *c, int ns, int *before = nullptr) {
 // blocks kept the probes waiting, 28.9 us instead of 10 at 1024 x 768, and the
 // rigid update's one block, sharing its SM with them, took 19.6 us instead of 8.)
 int enqueue_next_step(fb_ctx *c) {
-    const int r = enqueue_step_end(c, true, true);
+    const int r = enqueue_step_end(c, 1, true, true);
     if (r) return r;
     enqueue_marker_setup(c, c->stream);
     CK(cudaGetLastError());
-    return enqueue_substeps(c, 1, true);
+    const int e = enqueue_substeps(c, 1, true);
+    coefs(c, 1, 1, c->al, c->ga, c->ro);   // (as enqueue_step_end leaves them)
+    return e;
 }
 
 void drop_graph(fb_ctx *c) {
@@ -1319,7 +1322,7 @@ int capture_step(fb_ctx *c, int steps = 1) {
                  // (Adams-Bashforth: the two other means are zero and stay so)
                  fb::launch_submean_boucqt(c->d, c->stream, true);
                  c->own_launches += 1;
-                 return enqueue_step_end(c, false, false);
+                 return enqueue_step_end(c, 1, false, false);
              })))
             return r;
         c->step_kernels = c->own_launches;
