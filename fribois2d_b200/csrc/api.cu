@@ -973,7 +973,7 @@ int stage_impl(fb_ctx *c, int stage, int ns, int n) {
             fb::launch_mls_setup(d, st);
             fb::launch_spread_chains(d, st);
         }
-        fb::launch_mls_interp(d, st, n == 1);
+        fb::launch_mls_interp(d, st, n == 1, false);
         fb::launch_mls_spread(d, st);
         break;
     case FB_ST_HELSOLVE:
@@ -1107,7 +1107,7 @@ int enqueue_substeps(fb_ctx *c, int ns, bool follows) {
         if (d.nlm) {
             if (n == 1) CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
             // the weights are ready: interpolation and spreading only
-            fb::launch_mls_interp(d, c->stream, n == 1);
+            fb::launch_mls_interp(d, c->stream, n == 1, cfl);
             fb::launch_mls_spread(d, c->stream);
             c->own_launches += 2;
         }

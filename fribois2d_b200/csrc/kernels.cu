@@ -1099,12 +1099,14 @@ __global__ void k_mls_setup(Dev d) {
 // support loads are independent, and each lane forms the sum of the nine
 // products in node order from the group's shuffles (the sequential sum).
 // clear (substep 1): the spreading table, read for the last time by
-// k_spread_chains, is emptied for the next step.
+// k_spread_chains, is emptied for the next step.  cfl (substep 1 at fixed dt): a
+// CFL number beyond the limit, which nl_rhs has just formed, ends the step's
+// forcing here in every substep (divg makes it the step's number).
 constexpr int kInterpLanes = 16;
 // kWait: the body waits for the kernel before it (nl_rhs, which writes
 // rhs2/rhs3, or the spreading chains) with everything else loaded.
 template <bool kWait>
-__device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
+__device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear, bool cfl) {
     const int T = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = T / kInterpLanes, m = T % kInterpLanes, lane = threadIdx.x & 31;
     const bool have = t < 2 * d.nlm;
@@ -1131,7 +1133,9 @@ __device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
         }
     }
     if (kWait) FB_GRID_WAIT();
-    const bool stopped = (*d.status != 0);
+    const bool over = cfl && !(d.scal[S_CFLNEXT] * d.dt <= d.cfllim);
+    if (over && T == 0) raise_status(d, FB_ERR_CFL);
+    const bool stopped = over || *d.status != 0;
     if (clear && have && m == kInterpLanes - 1) clear_entry(d, tt);   // (a lane without a node)
     const double prod = rp ? phim * (qv + *rp) : phim * 0.0;
     double u = 0.0;
@@ -1147,7 +1151,7 @@ __device__ __forceinline__ void mls_interp_body(const Dev &d, bool clear) {
     c[m] = cl * phim * f;
 }
 
-__global__ void k_mls_interp(Dev d, int clear) { mls_interp_body<true>(d, clear != 0); }
+__global__ void k_mls_interp(Dev d, int clear, int cfl) { mls_interp_body<true>(d, clear != 0, cfl != 0); }
 
 // the spreading table emptied on its own: a step that ends between its marker
 // set-up and its interpolation (a refused dt)
@@ -2679,10 +2683,10 @@ __global__ void kg_spread_chains(const GroupCase *__restrict__ g) {
     spread_chains_body(d);
 }
 
-__global__ void kg_mls_interp(const GroupCase *__restrict__ g, int clear) {
+__global__ void kg_mls_interp(const GroupCase *__restrict__ g, int first) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    mls_interp_body<false>(d, clear != 0);
+    mls_interp_body<false>(d, first != 0, first != 0);   // (batches have a fixed dt)
 }
 
 __global__ void kg_mls_spread(const GroupCase *__restrict__ g) {
@@ -2818,8 +2822,9 @@ void launch_mls_setup(const Dev &d, cudaStream_t s, bool find) {
     if (d.nlm) pdl(find ? k_mls_setup<true> : k_mls_setup<false>, dim3(setup_blocks(d.nlm)), dim3(kSetupThreads),
                    0, s, d);
 }
-void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear) {
-    if (d.nlm) pdl(k_mls_interp, dim3((2 * d.nlm * kInterpLanes + 255) / 256), dim3(256), 0, s, d, clear ? 1 : 0);
+void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear, bool cfl) {
+    if (d.nlm)
+        pdl(k_mls_interp, dim3((2 * d.nlm * kInterpLanes + 255) / 256), dim3(256), 0, s, d, clear ? 1 : 0, cfl ? 1 : 0);
 }
 void launch_table_clear(const Dev &d, cudaStream_t s) {
     if (d.nlm) pdl(k_table_clear, dim3((2 * d.nlm + 127) / 128), dim3(128), 0, s, d);

@@ -33,8 +33,9 @@ void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s
 void launch_lgrdist(const Dev &d, cudaStream_t s);
 // find: the nearest nodes (lgrdistribution) in the same launch
 void launch_mls_setup(const Dev &d, cudaStream_t s, bool find = false);
-// clear: empty the spreading table behind k_spread_chains (substep 1)
-void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear);
+// clear: empty the spreading table behind k_spread_chains (substep 1); cfl: check
+// the CFL number of nl_rhs (kNlCfl) ahead of the forcing
+void launch_mls_interp(const Dev &d, cudaStream_t s, bool clear, bool cfl);
 // empty the spreading table behind a set-up that no interpolation follows
 void launch_table_clear(const Dev &d, cudaStream_t s);
 void launch_mls_spread(const Dev &d, cudaStream_t s);
@@ -42,7 +43,8 @@ void launch_spread_chains(const Dev &d, cudaStream_t s);
 void launch_helsolve(const Dev &d, const SubDev &sd, cudaStream_t s);
 // rmax (may be null): n2m row maxima of |dph| accumulated for the INT8 digit cut
 // extra: the fused step's work on the same launch (kDivBoucqt: boucqt;
-// kDivCfl: the CFL number of nl_rhs made the step's, and its check)
+// kDivCfl: the CFL number of nl_rhs made the step's, and its check, which the
+// forcing has made before where there are markers)
 constexpr int kDivBoucqt = 1, kDivCfl = 2;
 void launch_divg(const Dev &d, double usdtal, cudaStream_t s, double *rmax = nullptr, int extra = 0);
 // slot: a scalar slot that keeps the pressure mean beside S_PRAVG (-1: none)

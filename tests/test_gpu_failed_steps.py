@@ -1,6 +1,7 @@
 """What a step that ends with an error leaves behind: the same, whether it is
 taken by fb_advance, by a batch, by the separate calls or stage by stage.
 
+* A CFL number beyond the limit holds the forcing back in every substep.
 * At variable dt the step that raises an error is counted, with its history
   row, and the next one leaves no trace.
 """
@@ -33,6 +34,42 @@ def _move(c, y, z):
     """The body's centre at (y, z)."""
     c.vert = c.vert + (np.array([y, z]) - c.params.cmposi)
     c.params.cmposi = (y, z)
+
+
+@pytest.mark.parametrize("how", ["advance", "fluid_tsch", "batch"])
+@pytest.mark.parametrize("nsst", [3, 1])
+def test_cfl_error_holds_the_forcing_back(how, nsst, tmp_path):
+    if how == "batch" and nsst == 1:
+        pytest.skip("batches are RK3")
+    c = cases.tiny_cylinder()
+    c.params.nsst = nsst
+    c.params.cfllim = 1e-6
+    path = c.write(str(tmp_path / "deck"))
+    a, b = _open(c, path), _open(c, path)
+    a.set_substep(0, 1)
+    assert a.stage("cfl") == fb.FB_ERR_CFL
+    for n in range(1, nsst + 1):
+        a.set_substep(0, n)
+        for st in ("boucdq", "nl_rhs", "lgrdistribution", "forcing", "helsolve", "divg", "phcalc", "updvp",
+                   "pr_submean"):
+            if st != "lgrdistribution" or n == 1:
+                assert a.stage(st, n) == fb.FB_ERR_CFL
+    if how == "batch":
+        other = _open(c, path)
+        batch = fb.Batch([b, other])
+        assert batch.info()["groups"] == 1
+        _fails(lambda: batch.advance(1), fb.FB_ERR_CFL)
+        batch.close()
+        other.close()
+    else:
+        _fails(lambda: b.advance(0, 1) if how == "advance" else b.fluid_tsch(0), fb.FB_ERR_CFL)
+    # the stages' and the step's launches sum the same terms in other block
+    # shapes (boucdq's flux, the pressure mean): a few roundings of order one
+    # values, where a forced substep differs by the forcing itself, O(0.1)
+    for f in ("q2", "q3", "pr"):
+        np.testing.assert_allclose(b.get(f), a.get(f), rtol=0, atol=1e-11, err_msg=f)
+    for s in (a, b):
+        s.close()
 
 
 @pytest.mark.parametrize("nsst", [3, 1])
