@@ -216,8 +216,9 @@ __device__ __forceinline__ void boucdq_body(const Dev &d, double ga, double ro) 
 }
 
 // pr_submean (updvp.F90:336) of a step's three pressure means, in order, for
-// the entries of pr that updvp never rewrites and no stencil reads (j = n2,
-// k = 0, k = n3); one block
+// the entries of pr that updvp never rewrites and no stencil of the step reads
+// (j = n2, k = 0, k = n3); one block.  (The probes of the loads read row k = 0
+// ahead of it and subtract the three means themselves.)
 __device__ __forceinline__ void edge_means_body(const Dev &d) {
     const int t = threadIdx.x + blockDim.x * threadIdx.y, nt = blockDim.x * blockDim.y;
     const double m1 = d.scal[S_PRAVG1], m2 = d.scal[S_PRAVG2], m3 = d.scal[S_PRAVG];
@@ -1803,8 +1804,9 @@ constexpr int kLoadLanes = kNodeLanes;
 constexpr int kLoadMk = 2;   // markers per block: the three groups of a marker in one block
 constexpr int kLoadThreads = 3 * kLoadMk * kLoadLanes;
 
-// pend: the step's last pressure mean is still to be subtracted from pr; the
-// value is the one pr_submean would have stored.
+// pend: the step's last pressure mean is still to be subtracted from pr (in row
+// k = 0, which a probe beside the inflow reads, all three of them); the value is
+// the one pr_submean would have stored.
 // vals (may be null): the block's markers' values in shared memory, 24 each
 template <bool kWait>
 __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double *vals) {
@@ -1960,10 +1962,13 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
     double f0 = 0.0, fym = 0.0, fzm = 0.0, g2r = 1.0, g3r = 1.0;
     if (act) {
         const double *f = (idir == 1) ? d.q2 : (idir == 2 ? d.q3 : d.pr);
-        const double mean = (pend && idir == 3) ? d.scal[S_PRAVG] : 0.0;   // (x - 0.0 is x)
+        const bool late = pend && idir == 3;
+        const double mean = late ? d.scal[S_PRAVG] : 0.0;   // (x - 0.0 is x)
         f0 = Fv(f, ej, ek) - mean;
-        fym = Fv(f, ej - 1, ek) - mean;
-        fzm = Fv(f, ej, ek - 1) - mean;
+        fym = Fv(f, ej - 1, ek) - mean;   // (ej >= 2)
+        double fk = Fv(f, ej, ek - 1);
+        if (late && ek == 1) fk = (fk - d.scal[S_PRAVG1]) - d.scal[S_PRAVG2];   // row 0: no updvp has rewritten it
+        fzm = fk - mean;
         g2r = d.g2rc[ej];
         g3r = d.g3rc[ek];
     }
