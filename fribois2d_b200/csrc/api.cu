@@ -619,6 +619,7 @@ int create_impl(const char *dir, int device, fb_ctx *c) {
         if ((st = dnew(c, &d.hlen, nlm * 2 * fb::kSD))) return st;
     }
     if ((st = dnew(c, &d.probe, nlm * 24))) return st;
+    if ((st = dnew(c, &d.lfin, nlm * 3))) return st;
     if ((st = dnew(c, &d.press, nlm))) return st;
     if ((st = dnew(c, &d.tau, nlm * 2))) return st;
     if ((st = dnew(c, &d.bcerrv, nlm))) return st;

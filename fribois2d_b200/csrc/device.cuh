@@ -73,6 +73,7 @@ struct Dev {
     int *hlist;              // per head slot: the chain's next kHeadList slots in order (then chain[])
     int *hlen;               // per head slot: the chain's length after the head
     double *probe;           // [marker][24]: ucy(7), ucz(7), pc(7), tan(2), flag
+    double *lfin;            // [marker][3]: press, tau(2) as the finishing probes leave them
     double *press, *tau, *bcerrv, *bcerrw;
     // rigid body
     double *rigid;           // cmp_n, cmv_n, cma_n, cmp_np1, cmv_np1, cma_np1

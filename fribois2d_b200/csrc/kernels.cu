@@ -2040,7 +2040,8 @@ __device__ __forceinline__ void carried_tangent(const Dev &d, int n, double &tan
 // tangent (loads_transfer.F90:177-185) from its first two probes.  kFinish: a
 // marker with a tangent of its own is finished here (press, tau), one outside
 // the channel gets zeros, and only those whose tangent carries over from
-// another marker are left to the launch that sums the loads.
+// another marker are left to the launch that sums the loads.  The values go to
+// d.lfin: only that launch knows that no probe has failed.
 template <bool kFinish, bool kWait>
 __device__ __forceinline__ void loads_probe_tan_body(const Dev &d, bool pend) {
     if (!d.nlm) return;
@@ -2073,9 +2074,9 @@ __device__ __forceinline__ void loads_probe_tan_body(const Dev &d, bool pend) {
         }
     }
     if (kFinish && done) {
-        d.press[n] = press;
-        d.tau[2 * n] = tau[0];
-        d.tau[2 * n + 1] = tau[1];
+        d.lfin[3 * n] = press;
+        d.lfin[3 * n + 1] = tau[0];
+        d.lfin[3 * n + 2] = tau[1];
     }
 }
 
@@ -2501,11 +2502,13 @@ __device__ __forceinline__ void close_body(const Dev &d, int hist_rows) {
     else if (tid >= 64 && tid < 67) mcon[tid - 64] = d.rbmcon[tid - 64];
     const double time = d.scal[S_TIME], stepd = d.scal[S_STEP], cflm = d.scal[S_CFLM];
     const double c0 = d.rigid[0], c1 = d.rigid[1];
-    FB_GRID_WAIT();   // (the probes before it write press, tau, bcerrv, bcerrw, probe)
-    const bool good = *d.status == 0;
+    FB_GRID_WAIT();   // (the probes before it write lfin, bcerrv, bcerrw, probe and the status)
+    const bool good = *d.status == 0;   // else press and tau stay what they were
     double f[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // fyp, fzp, fyv, fzv, mom, the checkbcs sums
     for (int i = tid; i < nlm; i += nt) {
-        double p = d.press[i], tau[2] = {d.tau[2 * i], d.tau[2 * i + 1]};
+        const double p0 = d.press[i], t0 = d.tau[2 * i], t1 = d.tau[2 * i + 1];
+        const double pn = d.lfin[3 * i], tn0 = d.lfin[3 * i + 1], tn1 = d.lfin[3 * i + 2];
+        double p = good ? pn : p0, tau[2] = {good ? tn0 : t0, good ? tn1 : t1};
         const double A = d.lmA[i], ny = d.lmnor[2 * i], nz = d.lmnor[2 * i + 1];
         const double y = d.lmcc[2 * i], z = d.lmcc[2 * i + 1], ev = d.bcerrv[i], ew = d.bcerrw[i];
         const double *pb = d.probe + static_cast<size_t>(i) * 24;
@@ -2513,6 +2516,8 @@ __device__ __forceinline__ void close_body(const Dev &d, int hist_rows) {
             double tany = 0.0, tanz = 0.0;
             carried_tangent(d, i, tany, tanz);
             finish_marker(d, i, pb, tany, tanz, p, tau);
+        }
+        if (good) {
             d.press[i] = p;
             d.tau[2 * i] = tau[0];
             d.tau[2 * i + 1] = tau[1];

@@ -2,6 +2,7 @@
 taken by fb_advance, by a batch, by the separate calls or stage by stage.
 
 * A CFL number beyond the limit holds the forcing back in every substep.
+* Loads whose probes fail leave press and tau as they were.
 * At variable dt the step that raises an error is counted, with its history
   row, and the next one leaves no trace.
 """
@@ -28,6 +29,16 @@ def _fails(call, code):
     with pytest.raises(fb.FBError) as e:
         call()
     assert e.value.code == code
+
+
+def _uniform(nlm):
+    """A cylinder on a grid uniform along z; finer for more than 2048 markers."""
+    if nlm <= 500:
+        c = cases.tiny_cylinder(n3m=96, nlm=nlm)
+    else:
+        c = cases.viv_cylinder(n3m=576, n2m=256, ywin=(-2.0, 2.0), zdom=(-3.0, 9.0), ydom=(-3.0, 3.0), nlm=nlm)
+    c.zcoord = cases.uniform_axis(12.0, c.n3m)
+    return c, 12.0 / c.n3m
 
 
 def _move(c, y, z):
@@ -68,6 +79,30 @@ def test_cfl_error_holds_the_forcing_back(how, nsst, tmp_path):
     # values, where a forced substep differs by the forcing itself, O(0.1)
     for f in ("q2", "q3", "pr"):
         np.testing.assert_allclose(b.get(f), a.get(f), rtol=0, atol=1e-11, err_msg=f)
+    for s in (a, b):
+        s.close()
+
+
+@pytest.mark.parametrize("nlm", [40, 2048, 2049])
+def test_failed_probes_leave_the_loads(nlm, tmp_path):
+    # markers down to the fourth line from the inflow: supported, but a probe's
+    # search needs five lines on either side.  They come last in the order of the
+    # markers, so that with many of them others' probes have ended before
+    c, h = _uniform(nlm)
+    _move(c, 3.0, 0.5 + 3.6 * h)
+    v = np.roll(c.vert[:-1], int(0.45 * nlm), axis=0)
+    c.vert = np.concatenate([v, v[:1]])
+    path = c.write(str(tmp_path / "deck"))
+    a, b = _open(c, path), _open(c, path)
+    before = np.linspace(1.0, 2.0, nlm)
+    for s in (a, b):
+        s.set("press", before)
+    _fails(lambda: a.fluid_tsch(0), fb.FB_ERR_MARKER_OUT)
+    _fails(lambda: a.rigid(0), fb.FB_ERR_MARKER_OUT)
+    _fails(lambda: b.advance(0, 1), fb.FB_ERR_MARKER_OUT)
+    np.testing.assert_array_equal(a.get("press"), before)
+    for f in STATE:
+        np.testing.assert_array_equal(b.get(f), a.get(f), err_msg=f)
     for s in (a, b):
         s.close()
 
