@@ -24,6 +24,7 @@
 #include "device.cuh"
 #include "host.h"
 #include "kernels.h"
+#include "pdl.h"
 #include "tc_gemm.h"
 #include "tri.h"
 
@@ -2349,7 +2350,12 @@ int fb_time_stage(fb_ctx *c, int stage, int n, int reps, double *ms) {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    for (int i = 0; i < reps && !r; ++i) r = stage_impl(c, stage, c->cur_ns, n);
+    for (int i = 0; i < reps && !r; ++i) {
+        // a stage behind itself: its early loads are another launch's stores
+        fb::pdl_full_next = true;
+        r = stage_impl(c, stage, c->cur_ns, n);
+    }
+    fb::pdl_full_next = false;
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (r || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);

@@ -1824,17 +1824,10 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
     double *pb = d.probe + static_cast<size_t>(n) * 24;
     const double pos[2] = {d.lmcc[2 * n], d.lmcc[2 * n + 1]};
     const bool inside = (d.zz[1] < pos[1] && pos[1] < d.zz[d.n3]);
-    if (have && m == 0) {
-        if (idir == 1) {
-            pb[23] = inside ? 0.0 : -1.0;
-            if (vals) vals[24 * (threadIdx.x / (3 * kLoadLanes)) + 23] = inside ? 0.0 : -1.0;
-            d.bcerrv[n] = 0.0;
-        }
-        if (idir == 2) d.bcerrw[n] = 0.0;
-    }
-    const bool stopped = __shfl_sync(kAll, static_cast<int>(*d.status != 0), base) != 0;
-    const bool ok = have && !stopped && inside;
-
+    // (an early look at the status: without a set-up of this step there are no
+    // support nodes to read; the one behind the wait decides what is stored)
+    const bool early = __shfl_sync(kAll, static_cast<int>(*d.status != 0), base) != 0;
+    const bool live = have && inside && !early;
 
     const double hpr = d.ddmin * d.kprobe;
     const double probe[2] = {pos[0] + d.lmnor[2 * n] * hpr, pos[1] + d.lmnor[2 * n + 1] * hpr};
@@ -1851,7 +1844,7 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
     // probe within 5 lines of the marker's own; lane i holds lines js + i, ks + i
     constexpr int off = 5;
     const int js = mj - off, ks = mk - off;
-    const bool inrange = ok && js >= 1 && mj + off <= d.n2 && ks >= 1 && mk + off <= d.n3;
+    const bool inrange = live && js >= 1 && mj + off <= d.n2 && ks >= 1 && mk + off <= d.n3;
     const double *ya = (idir == 1) ? d.rc : d.rm;
     const double *za = (idir == 2) ? d.zz : d.zm;
     double vy = inf, vz = inf;
@@ -1878,9 +1871,7 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
     const bool bad = inrange && node && (ej < 1 || ej + 1 > dimy || ek < 1 || ek + 1 > dimz);
     const bool supported = group_none(bad, base) && inrange;
     const int ej0 = __shfl_sync(kAll, ej, base);
-    const bool good = supported && ej0 >= 2;
-    if (ok && !good && m == 0) raise_status(d, FB_ERR_MARKER_OUT);
-    const bool act = good && node;
+    const bool found = supported && ej0 >= 2, act = found && node;
 
     // MLS_SF_d (MLSint.F90:173-258) with compute_AB_d (:342-402)
     double sc0 = 0.0, sc1 = 0.0, w0 = 0.0, w1 = 0.0, w2 = 0.0;
@@ -1949,11 +1940,13 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
         p2 = p2 + gam[a][2] * B0 + gam[a][0] * B2;
     }
     // All of the above depends on the markers alone: kWait waits only here for
-    // the kernel before it (updvp or pr_submean, which write q2, q3 and pr)
+    // the kernel before it (updvp or pr_submean, which write q2, q3 and pr, or the
+    // launch that sums the loads of the probes before)
     if (kWait) FB_GRID_WAIT();
+    const int status = __ldcg(d.status);
     // checkbcs: the velocity at the marker from the substep-1 weights
     double prod = 0.0;
-    if (ok && idir <= 2 && node) {
+    if (live && idir <= 2 && node) {
         const int t2 = 2 * n + idir - 1;
         const int *eu = d.eulins + static_cast<size_t>(t2) * 2 * kSD;
         const double *q = (idir == 1) ? d.q2 : d.q3;
@@ -1971,6 +1964,17 @@ __device__ __forceinline__ void loads_probe_body(const Dev &d, bool pend, double
         fzm = fk - mean;
         g2r = d.g2rc[ej];
         g3r = d.g3rc[ek];
+    }
+    const bool stopped = __shfl_sync(kAll, static_cast<int>(status != 0), base) != 0;
+    const bool ok = live && !stopped, good = found && !stopped;
+    if (have && m == 0) {
+        if (idir == 1) {
+            pb[23] = inside ? 0.0 : -1.0;
+            if (vals) vals[24 * (threadIdx.x / (3 * kLoadLanes)) + 23] = inside ? 0.0 : -1.0;
+            d.bcerrv[n] = 0.0;
+        }
+        if (idir == 2) d.bcerrw[n] = 0.0;
+        if (ok && !good) raise_status(d, FB_ERR_MARKER_OUT);
     }
     // getpbup (loads_transfer.F90:285-357) for this quantity; the last two: the
     // partition of unity and checkbcs's velocity

@@ -1,11 +1,8 @@
 // Programmatic dependent launch: kernels of one stream launched with the
 // programmatic-stream-serialization attribute may be scheduled while the
-// kernel before them drains; each such kernel starts with FB_GRID_WAIT, which
-// returns once the preceding grid has completed and its writes are visible.
-// Every kernel that this header launches waits before its first access to
-// global memory that earlier kernels write (grouped kernels first stage their
-// case's view, which only the host writes), so ordering is the stream's as
-// without the attribute.
+// kernel before them drains.  Every block of such a kernel passes FB_GRID_WAIT,
+// which returns once the preceding grid has completed and its writes are
+// visible.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -21,13 +18,25 @@
 // this grid's blocks have started: a waiting grid never holds slots that this
 // one still needs.
 //
-// What a kernel may read before its wait: the kernel before it has triggered,
+// What a kernel may do before its wait: the kernel before it has triggered,
 // that is, every block of it has passed its own wait, so everything earlier is
 // complete and visible; only what the kernel directly before it writes is not.
-// The kernels of the time step use that: they load the operands that come from
-// further back, and do the work that depends on them alone, ahead of their wait
-// (marked there with what the kernel before them writes).  Nothing is stored
-// ahead of it that an earlier kernel still running could read.
+// So a kernel may load what that one does not write, and work on it, ahead of
+// its wait; it stores nothing and raises no status there.  These load early, each
+// marked with what the kernel before it writes, and may follow directly only
+// kernels that leave the rest alone:
+//   k_nl_rhs_tma        ru2, ru3: not behind nl_rhs itself
+//   k_mls_interp        q2, q3, markers, MLS weights: not behind updvp, helsolve,
+//                       the marker set-up, or a launch that moves the markers
+//   k_mls_spread        rhs2, rhs3 and the chains: not behind nl_rhs or the chains
+//   k_helsolve_win      q2, q3 and its coefficients: not behind updvp or itself
+//   k_updvp_prcalc_tma  q2, q3, pr: not behind helsolve or itself
+//   k_loads_probe       markers: not behind a launch that moves them
+//   k_step_close        markers, body state, scalars: behind the probes only
+//   k_ymodes, k_i8x8_gemm, the 3xTF32 products: constants and the base operand
+// Kernels that find their case in device memory (grouped launches) wait first.
+// A caller that cannot promise the order makes the next launch an ordinary one
+// (pdl_full_next): it then starts behind the complete kernel before it.
 #define FB_GRID_WAIT() asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory")
 
 namespace fb {
@@ -40,6 +49,9 @@ inline bool pdl_enabled() {
     return on;
 }
 
+// set by this thread for its next launch, which clears it
+inline thread_local bool pdl_full_next = false;
+
 template <typename... KArgs, typename... Args>
 inline void pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
     cudaLaunchConfig_t cfg{};
@@ -51,7 +63,7 @@ inline void pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cuda
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = (pdl_enabled() && !std::exchange(pdl_full_next, false)) ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
