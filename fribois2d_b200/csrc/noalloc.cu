@@ -17,7 +17,9 @@
 // take the kCounters counters in turn, and each also clears the one half a
 // turn away: two calls whose kernels overlap on the GPU (different streams, no
 // ordering between them) race on the partials, and a counter that such a race
-// left wrong is right again before its next use.
+// left wrong is right again before its next use.  A captured call cannot take
+// turns: it has a counter of its own, which its graph clears ahead of the kernel
+// in every replay.
 //
 // What bounds it: latency.  With one block per row, a single thread that
 // combined all rows in order and a memset node for the counter a call took
@@ -38,8 +40,9 @@ constexpr int kThreads = 256;
 constexpr unsigned kMaxBlocks = 2 * 148;   // two per SM
 constexpr unsigned kCounters = 64;
 
-// [0, 2*kMaxBlocks): per-block (max, sum) pairs; then the completion counters
-__device__ __align__(256) double g_cfl_scratch[2 * kMaxBlocks + kCounters / 2];
+// [0, 2*kMaxBlocks): per-block (max, sum) pairs; then the completion counters,
+// the captured calls' one last
+__device__ __align__(256) double g_cfl_scratch[2 * kMaxBlocks + kCounters / 2 + 1];
 
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
@@ -73,7 +76,7 @@ __device__ __forceinline__ void block_max_sum(double &mx, double &sm, double *sh
 // pass (their loads all issued before the first use); the last block combines
 // the blocks' partials; q fields are (j, k) at q[k*pitch + j-1]
 __global__ void __launch_bounds__(kThreads, 2)
-    k_cfl_rows(double *scratch, unsigned slot, const double *__restrict__ q2, const double *__restrict__ q3, int pitch,
+    k_cfl_rows(double *scratch, unsigned slot, unsigned other, const double *__restrict__ q2, const double *__restrict__ q3, int pitch,
                int n2m, int n3m, const double *__restrict__ rc, const double *__restrict__ zz,
                const double *__restrict__ udx2m, const double *__restrict__ udx3m, double dt, double rext2,
                double alx3, double *out) {
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         out[0] = mx * dt;
         out[1] = sm / (rext2 * alx3);
         counter[slot] = 0u;
-        counter[(slot + kCounters / 2) % kCounters] = 0u;
+        counter[other] = 0u;
     }
 }
 
@@ -166,7 +169,7 @@ extern "C" int fb_cfl_noalloc(const double *q2, const double *q3, int pitch, int
     const int n2m = n2 - 1, n3m = n3 - 1;
     if (n3m > FB_NOALLOC_MAX_ROWS) {
         std::fprintf(stderr,
-                     "fribois2d: fb_cfl_noalloc: %d z cells exceed the fixed scratch capacity of %d rows\n",
+                     "fribois2d: fb_cfl_noalloc: %d z cells exceed the limit of %d\n",
                      n3m, FB_NOALLOC_MAX_ROWS);
         return FB_ERR_UNSUPPORTED;
     }
@@ -176,7 +179,17 @@ extern "C" int fb_cfl_noalloc(const double *q2, const double *q3, int pitch, int
     if (!scratch) return FB_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     static std::atomic<unsigned> calls{0};
-    const unsigned slot = calls.fetch_add(1, std::memory_order_relaxed) % kCounters;
+    unsigned slot, other;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return FB_ERR_CUDA;
+    if (cap == cudaStreamCaptureStatusNone) {
+        slot = calls.fetch_add(1, std::memory_order_relaxed) % kCounters;
+        other = (slot + kCounters / 2) % kCounters;
+    } else {
+        slot = other = kCounters;
+        unsigned *counter = reinterpret_cast<unsigned *>(scratch + 2 * kMaxBlocks) + slot;
+        if (cudaMemsetAsync(counter, 0, sizeof(unsigned), st) != cudaSuccess) return FB_ERR_CUDA;
+    }
     // the launch's own status (cudaGetLastError would also return, and clear,
     // an earlier error of the caller's); the runtime may still report an
     // earlier asynchronous error here
@@ -184,7 +197,7 @@ extern "C" int fb_cfl_noalloc(const double *q2, const double *q3, int pitch, int
     cfg.gridDim = dim3(static_cast<unsigned>(n3m) < kMaxBlocks ? static_cast<unsigned>(n3m) : kMaxBlocks);
     cfg.blockDim = dim3(kThreads);
     cfg.stream = st;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_cfl_rows, scratch, slot, q2, q3, pitch, n2m, n3m, rc, zz, udx2m,
-                                             udx3m, dt, rext2, alx3, out);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_cfl_rows, scratch, slot, other, q2, q3, pitch, n2m, n3m, rc, zz,
+                                             udx2m, udx3m, dt, rext2, alx3, out);
     return e == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }

@@ -352,8 +352,8 @@ int fb_eigen_tridiag(int n, const double *am, const double *ac, const double *ap
  * out[1] = the area-weighted mean of w -- from the caller's own device arrays:
  * q2, q3 as (j, k) at q[k*pitch + j-1], k = 0..n3; rc (n2), zz (n3),
  * udx2m (n2-1), udx3m (n3-1) 0-based; out: 2 doubles of device memory.
- * The partial results go to a fixed array inside the library (room for
- * FB_NOALLOC_MAX_ROWS rows of z cells; larger grids return FB_ERR_UNSUPPORTED).
+ * The partial results go to a fixed array inside the library.  Grids of more
+ * than FB_NOALLOC_MAX_ROWS z cells return FB_ERR_UNSUPPORTED.
  * The first call on a device looks up that array's address (make it before
  * any stream capture); every call shares the array, so calls whose kernels
  * overlap on the GPU race.  Asynchronous on `stream` (a cudaStream_t, or NULL).
