@@ -367,8 +367,7 @@ int build_substeps(fb_ctx *c) {
     const size_t nd = c->coef_h.size(), ni = std::max<size_t>(c->coef_hi.size(), 1);
     if ((st = dnew(c, &c->coef_d, nd))) return st;
     if ((st = dnew(c, &c->coef_di, ni))) return st;
-    // + the CFL number of a step, the scalars and status ahead of it
-    CK(cudaMallocHost(&c->coef_pin, (nd + 1 + fb::kScalStatus + 1) * sizeof(double)));
+    CK(cudaMallocHost(&c->coef_pin, (nd + fb::kScalAll) * sizeof(double)));   // + a step's scalars (vardt_update)
     CK(cudaMallocHost(&c->coef_pini, ni * sizeof(int)));
     c->coef_cap = nd;
     c->coef_capi = ni;
@@ -628,7 +627,7 @@ int create_impl(const char *dir, int device, fb_ctx *c) {
     if ((st = dnew(c, &d.rigid, 18))) return st;
     if ((st = h2d(c, d.rigid, c->hc.rigid, 18 * sizeof(double)))) return st;
     if ((st = dnew(c, &d.forces, 8))) return st;
-    if ((st = dnew(c, &d.scal, fb::kScalStatus + 1))) return st;
+    if ((st = dnew(c, &d.scal, fb::kScalAll))) return st;
     d.status = reinterpret_cast<int *>(d.scal + fb::kScalStatus);
     c->hist_cap = 4096;
     if ((st = dnew(c, &d.hist, static_cast<size_t>(c->hist_cap) * FB_HIST_COLS))) return st;
@@ -1036,24 +1035,23 @@ int stage_impl(fb_ctx *c, int stage, int ns, int n) {
 }
 
 // variable dt (fluid_tsch.F90:34-48): the CFL number of the current field
-// sets dt = cflmax / cflm (at most dtmax) from the second step on.  Runs cfl and
-// waits for it; before is the status word ahead of this step (h: note_state's
-// copy), which ends it here when it is set.
-int vardt_update(fb_ctx *c, int ns, const double *h, int *before) {
+// sets dt = cflmax / cflm (at most dtmax) from the second step on.  Runs cfl, waits
+// for it and reads the scalars into h; before is the status word ahead of this step
+// (as k_note has kept it), which ends it here when it is set.
+int vardt_update(fb_ctx *c, int ns, double *h, int *before) {
     fb::launch_cfl(c->d, c->stream);
     c->own_launches += 1;
     CK(cudaGetLastError());
-    double *am = c->coef_pin + c->coef_cap;
-    CK(cudaMemcpyAsync(am, c->d.scal + fb::S_CFLRAW, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(h, c->d.scal, fb::kScalAll * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     if (before) {
-        std::memcpy(before, h + fb::kScalStatus, sizeof(int));
+        std::memcpy(before, h + fb::kScalNoted + fb::kScalStatus, sizeof(int));
         if (*before) return FB_OK;
     }
     coefs(c, ns, 1, c->al, c->ga, c->ro);
     double dt = c->dt;
     if (ns > 0) {
-        dt = c->hc.deck.cflmax / *am;
+        dt = c->hc.deck.cflmax / h[fb::S_CFLRAW];
         if (dt > c->hc.deck.dtmax) dt = c->hc.deck.dtmax;
     }
     if (!(dt >= 1.0e-8)) return FB_ERR_CFL;
@@ -1152,18 +1150,12 @@ int end_side(fb_ctx *c) {
     return FB_OK;
 }
 
-// A step at variable dt may end behind its marker set-up (dt refused, or an error
-// of the step before).  Its scalars and status word are noted ahead of the fork:
-// behind it the set-up may already have raised an error of its own.
-int note_state(fb_ctx *c, double *h) {
-    CK(cudaMemcpyAsync(h, c->d.scal, (fb::kScalStatus + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    return FB_OK;
-}
-
-// Ends such a step as if it had not begun: the side branch joins (nothing of the
+// Ends a step at variable dt behind its marker set-up (dt refused, or an error of
+// the step before) as if it had not begun: the side branch joins (nothing of the
 // step still runs when the caller next writes the markers), the spreading table is
-// empty for the next set-up, and the status word is what it was.  scalars: the
-// CFL number and the mean w too (a refused dt leaves those that it was refused by).
+// empty for the next set-up, and the status word is what it was ahead of the set-up,
+// which may have raised an error of its own.  scalars: the CFL number and the mean w
+// too (a refused dt leaves those that it was refused by).  h: vardt_update's.
 int undo_start(fb_ctx *c, const double *h, bool scalars) {
     if (c->d.nlm) {
         CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
@@ -1171,8 +1163,10 @@ int undo_start(fb_ctx *c, const double *h, bool scalars) {
         c->own_launches += 1;
         CK(cudaGetLastError());
     }
-    CK(cudaMemcpyAsync(c->d.status, h + fb::kScalStatus, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    if (scalars) CK(cudaMemcpyAsync(c->d.scal, h, fb::S_COUNT * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    const double *noted = h + fb::kScalNoted;
+    CK(cudaMemcpyAsync(c->d.status, noted + fb::kScalStatus, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    if (scalars)
+        CK(cudaMemcpyAsync(c->d.scal, noted, fb::S_COUNT * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return FB_OK;
 }
@@ -1183,8 +1177,11 @@ int undo_start(fb_ctx *c, const double *h, bool scalars) {
 // step ends the step here.
 int enqueue_fluid_start(fb_ctx *c, int ns, int *before = nullptr) {
     int r;
-    double *h = c->coef_pin + c->coef_cap + 1;
-    if (c->vardt && (r = note_state(c, h))) return r;
+    double *h = c->coef_pin + c->coef_cap;
+    if (c->vardt) {
+        fb::launch_note(c->d, c->stream);
+        c->own_launches += 1;
+    }
     if (c->d.nlm) {
         if ((r = fork_side(c))) return r;
         enqueue_marker_setup(c, c->side);

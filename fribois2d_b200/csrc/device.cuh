@@ -167,9 +167,9 @@ enum Scal {
     // (divg of that substep makes them S_CFLM, S_CFLRAW, S_Q3AVG)
     S_PRAVG1 = S_COUNT, S_PRAVG2, S_CFLNEXT, S_Q3NEXT, S_SLOTS
 };
-// the status word lies behind the scalars, on a line of its own: one copy reads
-// both (the variable-dt step)
-constexpr int kScalStatus = 16;
+// the status word lies behind the scalars, on a line of its own, and k_note's copy
+// of both behind it: one copy to the host reads all of them (the variable-dt step)
+constexpr int kScalStatus = 16, kScalNoted = 32, kScalAll = kScalNoted + kScalStatus + 1;
 static_assert(S_SLOTS <= kScalStatus, "scalar slots");
 
 __host__ __device__ inline size_t fidx(const Dev &d, int j, int k) {

@@ -12,6 +12,8 @@ constexpr int kRedSlot = 65536;  // block partials per reduction slot
 
 cudaError_t kernels_configure();   // shared-memory limits (once per device)
 void launch_cfl(const Dev &d, cudaStream_t s);
+// keep the scalars and the status word beside them (scal + kScalNoted)
+void launch_note(const Dev &d, cudaStream_t s);
 void launch_boucdq(const Dev &d, double ga, double ro, cudaStream_t s);
 // TMA descriptors of the fields that the stencil tiles stage (q2, q3, pr for
 // k_nl_rhs, dph for k_updvp_prcalc): 2-D arrays (j - 1 fastest, row k,
