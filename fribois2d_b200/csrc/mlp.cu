@@ -594,28 +594,31 @@ int ensure(fb_mlp *m, int B) {
 }
 
 // buffers of the one-launch epochs: n samples, nbt minibatches per epoch
+// (FB_ERR_CUDA: the device has no room; nothing is kept then)
 int ensure_train(fb_mlp *m, int n, int nbt) {
-    if (n > m->tcap_n) {
-        cudaFree(m->TX);
-        cudaFree(m->TT);
+    if (n <= m->tcap_n && nbt <= m->tcap_b) return FB_OK;
+    const size_t cn = static_cast<size_t>(std::max(n, m->tcap_n)), cb = static_cast<size_t>(std::max(nbt, m->tcap_b));
+    auto release = [m] {
+        for (float **p : {&m->TX, &m->TT, &m->TC, &m->TL}) {
+            cudaFree(*p);
+            *p = nullptr;
+        }
         cudaFree(m->TI);
-        m->TX = m->TT = nullptr;
         m->TI = nullptr;
-        m->tcap_n = 0;
-        MK(cudaMalloc(&m->TX, sizeof(float) * static_cast<size_t>(n) * m->sh.nin));
-        MK(cudaMalloc(&m->TT, sizeof(float) * static_cast<size_t>(n) * m->sh.nout));
-        MK(cudaMalloc(&m->TI, sizeof(int) * static_cast<size_t>(n)));
-        m->tcap_n = n;
+        m->tcap_n = m->tcap_b = 0;
+    };
+    release();
+    if (cudaMalloc(&m->TX, sizeof(float) * cn * m->sh.nin) != cudaSuccess ||
+        cudaMalloc(&m->TT, sizeof(float) * cn * m->sh.nout) != cudaSuccess ||
+        cudaMalloc(&m->TI, sizeof(int) * cn) != cudaSuccess ||
+        cudaMalloc(&m->TC, sizeof(float) * 2 * cb) != cudaSuccess ||
+        cudaMalloc(&m->TL, sizeof(float) * cb) != cudaSuccess) {
+        cudaGetLastError();
+        release();
+        return FB_ERR_CUDA;
     }
-    if (nbt > m->tcap_b) {
-        cudaFree(m->TC);
-        cudaFree(m->TL);
-        m->TC = m->TL = nullptr;
-        m->tcap_b = 0;
-        MK(cudaMalloc(&m->TC, sizeof(float) * 2 * static_cast<size_t>(nbt)));
-        MK(cudaMalloc(&m->TL, sizeof(float) * static_cast<size_t>(nbt)));
-        m->tcap_b = nbt;
-    }
+    m->tcap_n = static_cast<int>(cn);
+    m->tcap_b = static_cast<int>(cb);
     return FB_OK;
 }
 
@@ -627,13 +630,11 @@ void grad_on_device(fb_mlp *m, int B) {
     k_mlp_reduce<<<(m->sh.n + 255) / 256, 256>>>(m->sh.n, nb, m->Gb, m->G, m->Lb, m->loss, B);
 }
 
-// fb_mlp_train with one launch per epoch (k_mlp_epoch); the host shuffles the
+// fb_mlp_train with one launch per epoch (k_mlp_epoch) on ensure_train's buffers; the host shuffles the
 // next epoch's order while the device works on the current one
 int train_epochs(fb_mlp *m, const float *x, const float *t, int n, int epochs, int batch, float lr, uint64_t seed,
                  float *loss_out, int ctas, size_t smem) {
     const int nbt = n / batch, used = nbt * batch;
-    int st = ensure_train(m, n, nbt);
-    if (st) return st;
     MK(cudaFuncSetAttribute(k_mlp_epoch, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTrainSmemMax)));
     MK(cudaMemcpy(m->TX, x, sizeof(float) * static_cast<size_t>(n) * m->sh.nin, cudaMemcpyHostToDevice));
     MK(cudaMemcpy(m->TT, t, sizeof(float) * static_cast<size_t>(n) * m->sh.nout, cudaMemcpyHostToDevice));
@@ -789,9 +790,10 @@ int fb_mlp_train(fb_mlp *m, const float *x, const float *t, int n, int epochs, i
     batch = std::min(batch, n);
     const int groups = (batch + kS - 1) / kS, ctas = std::min(kTrainCtas, groups);
     const size_t smem = train_smem(m->sh, train_slots(batch, ctas), ctas);
-    if (smem <= kTrainSmemMax) return train_epochs(m, x, t, n, epochs, batch, lr, seed, loss_out, ctas, smem);
-    // batches whose gradient slots do not fit the cluster's shared memory: one
-    // minibatch at a time
+    if (smem <= kTrainSmemMax && ensure_train(m, n, n / batch) == FB_OK)
+        return train_epochs(m, x, t, n, epochs, batch, lr, seed, loss_out, ctas, smem);
+    // batches whose gradient slots do not fit the cluster's shared memory, or more
+    // samples than the device has room for: one minibatch at a time
     int st = ensure(m, batch);
     if (st) return st;
     const int ni = m->sh.nin, no = m->sh.nout;
