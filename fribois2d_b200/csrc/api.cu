@@ -1398,12 +1398,16 @@ OutChunks g_out;
 // chunks: the copy engine fills one while several host threads empty the other
 // into the caller's array, whose first-touch page faults they share.  (The
 // driver's own staging copied 4.3 GB/s: 18 of the 108 ms of 50 steps at 2048 x
-// 1536 with three fields read at the end.)
+// 1536 with three fields read at the end.)  Memory that the copy engine reaches by
+// itself (pinned, managed) takes one direct copy: 457 us for a field of that size,
+// 754 through the chunks.
 int copy_out(fb_ctx *c, double *host, const double *dev, size_t pitch, size_t width, size_t rows) {
     constexpr size_t kDirect = 512u << 10, kChunk = OutChunks::kBytes;
     std::unique_lock<std::mutex> busy(g_out.busy, std::defer_lock);
     char *buf = nullptr;
-    if (rows * width > kDirect && width <= kChunk) {
+    cudaPointerAttributes at{};
+    if (rows * width > kDirect && width <= kChunk && cudaPointerGetAttributes(&at, host) == cudaSuccess &&
+        at.type == cudaMemoryTypeUnregistered) {
         CK(cudaStreamSynchronize(c->stream));   // (the chunks are not held while the GPU works)
         if (busy.try_lock()) buf = g_out.get(c->out_user);
     }

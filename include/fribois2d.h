@@ -267,6 +267,10 @@ int fb_read_restart(fb_ctx *ctx, const char *dir);
 /* dims: n2, n3, nlm, nsst, field pitch, Poisson pitch, pivoting flags,
  * helsolve windows of substep 1 (y | z << 8; 0 = full line scans) */
 int fb_get_dims(fb_ctx *ctx, int32_t dims[8]);
+/* Both copies are ordered behind the context's work; the read has arrived on
+ * return.  A field of more than 512 KiB into pageable memory is staged through
+ * pinned chunks that up to eight host threads empty (one reading thread of the
+ * process at a time; others copy directly); pinned memory takes one direct copy. */
 int fb_get_array(fb_ctx *ctx, int id, double *host, int64_t n);
 int fb_set_array(fb_ctx *ctx, int id, const double *host, int64_t n);
 int fb_get_iarray(fb_ctx *ctx, int id, int32_t *host, int64_t n);
