@@ -966,7 +966,7 @@ int stage_impl(fb_ctx *c, int stage, int ns, int n) {
     switch (stage) {
     case FB_ST_CFL: fb::launch_cfl(d, st); break;
     case FB_ST_BOUCDQ: fb::launch_boucdq(d, ga, ro, st); break;
-    case FB_ST_NL_RHS: fb::launch_nl_rhs(d, al, ga, ro, st, false, &c->nlmaps); break;
+    case FB_ST_NL_RHS: fb::launch_nl_rhs(d, al, ga, ro, st, false, c->nlmaps); break;
     case FB_ST_LGRDIST: fb::launch_lgrdist(d, st); break;
     case FB_ST_FORCING:
         if (!d.nlm) break;
@@ -1008,7 +1008,7 @@ int stage_impl(fb_ctx *c, int stage, int ns, int n) {
         fb::launch_scan_poisson(d, st);
         if ((r = gemm_bwd(c))) return r;
         break;
-    case FB_ST_UPDVP: fb::launch_updvp_prcalc(d, al, al * c->beta, st, false, &c->nlmaps); break;
+    case FB_ST_UPDVP: fb::launch_updvp_prcalc(d, al, al * c->beta, st, false, c->nlmaps); break;
     case FB_ST_PRSUBMEAN: fb::launch_submean_boucqt(d, st); break;
     case FB_ST_CHECKBCS:
     case FB_ST_LOADS: fb::launch_loads(d, st); break;
@@ -1075,7 +1075,7 @@ void enqueue_nl_rhs(fb_ctx *c, int ns, int n, bool follows, cudaStream_t st) {
     double al, ga, ro;
     coefs(c, ns, n, al, ga, ro);
     const bool pend = (n == 1) ? follows : c->d.nsst == 3;
-    fb::launch_nl_rhs(c->d, al, ga, ro, st, pend, &c->nlmaps,
+    fb::launch_nl_rhs(c->d, al, ga, ro, st, pend, c->nlmaps,
                       fb::kNlBoucdq | (n == 1 && !c->vardt ? fb::kNlCfl : 0) | (follows ? fb::kNlMeans : 0));
     c->own_launches += 1;
 }
@@ -1120,7 +1120,7 @@ int enqueue_substeps(fb_ctx *c, int ns, bool follows) {
                         fb::kDivBoucqt | (cfl ? fb::kDivCfl : 0));
         c->own_launches += 1;
         if ((r = stage_impl(c, FB_ST_PHCALC, ns, n))) return r;
-        fb::launch_updvp_prcalc(d, al, al * c->beta, c->stream, pend, &c->nlmaps,
+        fb::launch_updvp_prcalc(d, al, al * c->beta, c->stream, pend, c->nlmaps,
                                 !defer || n == 3 ? -1 : n == 1 ? fb::S_PRAVG1 : fb::S_PRAVG2);
         c->own_launches += 1;
         CK(cudaGetLastError());

@@ -575,12 +575,6 @@ __device__ __forceinline__ void nl_rhs_body(const Dev &d, double al, double ga, 
     if (kCfl) cfl_finish(d, cmx, csm, nb);
 }
 
-__global__ void __launch_bounds__(256, kNlBlocksPerSM) k_nl_rhs(Dev d, double al, double ga, double ro, int pend) {
-    extern __shared__ __align__(16) unsigned char nl_smem[];
-    FB_GRID_WAIT();
-    nl_rhs_body<false>(d, al, ga, ro, reinterpret_cast<NlTile *>(nl_smem), pend != 0, gridDim.x);
-}
-
 // the three field boxes of a tile, issued by one thread on the buffer's
 // mbarrier.  The proxy fence orders the threads' earlier reads (and the pend
 // pass's writes) of this buffer before the copies overwrite it.  Boxes that
@@ -1755,12 +1749,6 @@ __device__ __forceinline__ void updvp_prcalc_body(const Dev &d, double al, doubl
     }
 }
 
-__global__ void __launch_bounds__(256, kUpBlocksPerSM) k_updvp_prcalc(Dev d, double al, double be, int pend, int slot) {
-    extern __shared__ __align__(16) unsigned char up_smem[];
-    FB_GRID_WAIT();
-    updvp_prcalc_body<false>(d, al, be, reinterpret_cast<UpTile *>(up_smem), pend != 0, slot);
-}
-
 __global__ void __launch_bounds__(256, kUpBlocksPerSM)
     k_updvp_prcalc_tma(const __grid_constant__ Dev d, const __grid_constant__ NlMaps m, double al, double be,
                        int pend, int slot) {
@@ -2740,11 +2728,10 @@ __global__ void kg_submean_boucqt(const GroupCase *__restrict__ g, int deferred)
     submean_boucqt_body(d, deferred != 0);
 }
 
-template <bool kFinish>
-__global__ void __launch_bounds__(kLoadThreads, 5) kg_loads_probe(const GroupCase *__restrict__ g, int pend) {
+__global__ void __launch_bounds__(kLoadThreads, 5) kg_loads_probe(const GroupCase *__restrict__ g) {
     __shared__ Dev d;
     if (!stage_case(g, &d)) return;
-    loads_probe_tan_body<kFinish, false>(d, pend != 0);
+    loads_probe_tan_body<false, false>(d, false);
 }
 
 __global__ void __launch_bounds__(kLoadFin) kg_loads_finish(const GroupCase *__restrict__ g) {
@@ -2792,7 +2779,7 @@ void launch_note(const Dev &d, cudaStream_t s) { pdl(k_note, dim3(1), dim3(32), 
 void launch_boucdq(const Dev &d, double ga, double ro, cudaStream_t s) { pdl(k_boucdq, dim3(1), dim3(1024), 0, s, d, ga, ro); }
 int nl_tiles(const Dev &d) { return ((d.n2m + kNlJ - 1) / kNlJ) * ((d.n3m + kNlK - 1) / kNlK); }
 
-void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend, const NlMaps *maps,
+void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend, const NlMaps &maps,
                    int extra) {
     const int more = nl_more(extra);
     // all resident at once; beside the marker set-up of the step (kNlMeans) a
@@ -2801,11 +2788,8 @@ void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s
     // 1562, 1572, 1592 us per step at 2048 x 1536)
     const int slots = 148 * kNlBlocksPerSM - more - ((extra & kNlMeans) ? 148 * kNlBlocksPerSM / 16 : 0);
     const int blocks = std::min(nl_tiles(d), slots) + more;
-    if (maps)
-        pdl((extra & kNlCfl) ? k_nl_rhs_tma<true> : k_nl_rhs_tma<false>, dim3(blocks), dim3(32, 8), kNlSmemT, s, d,
-            *maps, al, ga, ro, pend ? 1 : 0, extra);
-    else
-        pdl(k_nl_rhs, dim3(blocks), dim3(32, 8), kNlSmem, s, d, al, ga, ro, pend ? 1 : 0);
+    pdl((extra & kNlCfl) ? k_nl_rhs_tma<true> : k_nl_rhs_tma<false>, dim3(blocks), dim3(32, 8), kNlSmemT, s, d, maps,
+        al, ga, ro, pend ? 1 : 0, extra);
 }
 
 // q2, q3, pr, dph as 2-D FP64 tensors: x = j - 1 (j = 1 .. n2), y = k (0 .. n3),
@@ -2880,10 +2864,9 @@ void launch_divg(const Dev &d, double usdtal, cudaStream_t s, double *rmax, int 
     // (the row maxima's reduction assumes these blocks)
     pdl(k_divg, divg_grid(d, extra), dim3(32, 8), 0, s, d, usdtal, rmax, extra);
 }
-void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, bool pend, const NlMaps *maps, int slot) {
+void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, bool pend, const NlMaps &maps, int slot) {
     const int blocks = std::min(nl_tiles(d), 148 * kUpBlocksPerSM);
-    if (maps) pdl(k_updvp_prcalc_tma, dim3(blocks), dim3(32, 8), kUpSmemT, s, d, *maps, al, be, pend ? 1 : 0, slot);
-    else pdl(k_updvp_prcalc, dim3(blocks), dim3(32, 8), kUpSmem, s, d, al, be, pend ? 1 : 0, slot);
+    pdl(k_updvp_prcalc_tma, dim3(blocks), dim3(32, 8), kUpSmemT, s, d, maps, al, be, pend ? 1 : 0, slot);
 }
 void launch_submean_boucqt(const Dev &d, cudaStream_t s, bool deferred) {
     dim3 b(32, 8);
@@ -2945,12 +2928,10 @@ cudaError_t kernels_configure() {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     };
-    allow(k_nl_rhs, kNlSmem);
     allow(k_nl_rhs_tma<false>, kNlSmemT);
     allow(k_nl_rhs_tma<true>, kNlSmemT);
     allow(kg_nl_rhs<false>, kNlSmem);
     allow(kg_nl_rhs<true>, kNlSmem);
-    allow(k_updvp_prcalc, kUpSmem);
     allow(k_updvp_prcalc_tma, kUpSmemT);
     allow(kg_updvp_prcalc, kUpSmem);
     allow(k_step_close, close_smem(kCloseMax));
@@ -2981,11 +2962,10 @@ void glaunch_submean_boucqt(const Group &g, cudaStream_t s, bool deferred) {
     dim3 b(32, 8);
     pdl(kg_submean_boucqt, zgrid(grid2(g.rep.n2, g.rep.n3 + 1, b), g), dim3(b), 0, s, g.cases, deferred ? 1 : 0);
 }
-void glaunch_loads(const Group &g, cudaStream_t s, bool pend) {
+void glaunch_loads(const Group &g, cudaStream_t s) {
     const Dev &d = g.rep;
     if (!d.nlm) return;
-    pdl(kg_loads_probe<false>, zgrid(dim3((d.nlm + kLoadMk - 1) / kLoadMk), g), dim3(kLoadThreads), 0, s, g.cases,
-        pend ? 1 : 0);
+    pdl(kg_loads_probe, zgrid(dim3((d.nlm + kLoadMk - 1) / kLoadMk), g), dim3(kLoadThreads), 0, s, g.cases);
     pdl(kg_loads_finish, zgrid(dim3((d.nlm + kLoadFin - 1) / kLoadFin), g), dim3(kLoadFin), 0, s, g.cases);
 }
 void glaunch_rigid(const Group &g, cudaStream_t s, int mode) {

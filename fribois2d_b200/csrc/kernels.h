@@ -16,22 +16,21 @@ void launch_cfl(const Dev &d, cudaStream_t s);
 void launch_note(const Dev &d, cudaStream_t s);
 void launch_boucdq(const Dev &d, double ga, double ro, cudaStream_t s);
 // TMA descriptors of the fields that the stencil tiles stage (q2, q3, pr for
-// k_nl_rhs, dph for k_updvp_prcalc): 2-D arrays (j - 1 fastest, row k,
+// k_nl_rhs_tma, dph for k_updvp_prcalc_tma): 2-D arrays (j - 1 fastest, row k,
 // k = 0 .. n3), one box per tile and field
 struct alignas(64) NlMaps {
     CUtensorMap q2, q3, pr, dph;
 };
 int encode_nl_maps(NlMaps *m, const Dev &d);   // FB_OK, or an error (no maps)
 // pend / deferred: the fused step's deferred pr_submean of RK3 substeps 1 and 2.
-// maps: stage the tiles with TMA (the single-case step); null: cp.async.
 // extra: the fused step's work on the same launch (kNlBoucdq: boucdq of this
 // substep in a block of its own; kNlCfl: the CFL number and the mean w of the
 // field the tiles hold; kNlMeans: the step before left all its pressure means to
 // be subtracted, and a block of its own brings the entries of pr that updvp does
 // not rewrite up to date)
 constexpr int kNlBoucdq = 1, kNlCfl = 2, kNlMeans = 4;
-void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend = false,
-                   const NlMaps *maps = nullptr, int extra = 0);
+void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s, bool pend,
+                   const NlMaps &maps, int extra = 0);
 void launch_lgrdist(const Dev &d, cudaStream_t s);
 // find: the nearest nodes (lgrdistribution) in the same launch
 void launch_mls_setup(const Dev &d, cudaStream_t s, bool find = false);
@@ -50,8 +49,8 @@ void launch_helsolve(const Dev &d, const SubDev &sd, cudaStream_t s);
 constexpr int kDivBoucqt = 1, kDivCfl = 2;
 void launch_divg(const Dev &d, double usdtal, cudaStream_t s, double *rmax = nullptr, int extra = 0);
 // slot: a scalar slot that keeps the pressure mean beside S_PRAVG (-1: none)
-void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, bool pend = false,
-                         const NlMaps *maps = nullptr, int slot = -1);
+void launch_updvp_prcalc(const Dev &d, double al, double be, cudaStream_t s, bool pend, const NlMaps &maps,
+                         int slot = -1);
 // mbox[0] = *d.status, mbox[1..8] = d.forces[0..7] (when forces); mbox in
 // mapped host memory
 void launch_publish(const Dev &d, bool forces, double *mbox, cudaStream_t s);
@@ -80,7 +79,7 @@ void glaunch_forcing(const Group &g, int n, cudaStream_t s); // interpolation an
 void glaunch_divg(const Group &g, int n, cudaStream_t s, int extra);
 void glaunch_updvp_prcalc(const Group &g, int n, cudaStream_t s, bool pend, int slot);
 void glaunch_submean_boucqt(const Group &g, cudaStream_t s, bool deferred = false);
-void glaunch_loads(const Group &g, cudaStream_t s, bool pend = false);
+void glaunch_loads(const Group &g, cudaStream_t s);
 void glaunch_rigid(const Group &g, cudaStream_t s, int mode = RIGID_STEP);
 void glaunch_diag(const Group &g, cudaStream_t s);
 
