@@ -838,7 +838,6 @@ __global__ void __launch_bounds__(256) k_i8_rowmax(const double *__restrict__ sr
     }
 }
 
-// grouped (blockIdx.z = case; a cluster never spans two cases)
 // S: digit slices; BN: output tile width, 64, 48, 32 or 16 (a 128 x 48 tile
 // puts 132 CTAs on a 768 x 1024 product where 128 x 64 tiles leave a third of
 // the 148 SMs idle; 32 and 16 spread small products over more SMs)

@@ -1,5 +1,5 @@
 """Test infrastructure: a NumPy restatement of the INT8 digit-slice product
-of fribois2d_b200/csrc/tc_gemm.cu (k_i8_rowmax, k_i8_digits, k_i8x8_gemm),
+of fribois2d_b200/csrc/tc_gemm.cu (k_i8_rowmax, k_i8_cut_rows, k_i8x8_gemm),
 used to check the device result bit for bit and the method's error bound.
 
 The method is the Ozaki scheme (Ozaki, Ogita, Oishi and Rump, "Error-free
