@@ -887,10 +887,10 @@ __device__ void wkernel(int wfun, double difc, double sdds, double &wc, double &
 }
 
 // Groups of kNodeLanes lanes work on one (marker, direction) each, support
-// node m on lane m < kSD; a sum over the support is formed in node order from
-// the group's shuffles (the sequential loop's sum).  Every lane of a warp
-// reaches every shuffle: a group that stops (outside the channel, an error)
-// carries on with its loads and stores switched off.
+// node m on lane m < kSD; a sum over the support is formed in node order
+// (group_sums; the sequential loop's sum).  Every lane of a warp reaches every
+// exchange: a group that stops (outside the channel, an error) carries on with
+// its loads and stores switched off.
 constexpr int kNodeLanes = 16;
 
 // N sums over the group's nodes through shared memory (buf: 10 N doubles of the
@@ -1793,10 +1793,10 @@ __global__ void k_submean_boucqt(Dev d, int deferred) {
 // groups also form checkbcs (ckbcs.F90:29-60) with the substep-1 weights.
 // One (marker, quantity) per group of kLoadLanes lanes, support node m on
 // lane m < kSD: the nodes' weights, moment terms and field reads are
-// independent, and every sum over the nodes is formed in node order from the
-// group's shuffles, so each result is that of the sequential loops.  Every
-// lane of a warp reaches every shuffle: a group that stops (outside the
-// channel, an error) carries on with its loads and stores switched off.
+// independent, and every sum over the nodes is formed in node order
+// (group_sums), so each result is that of the sequential loops.  Every lane of
+// a warp reaches every exchange: a group that stops (outside the channel, an
+// error) carries on with its loads and stores switched off.
 constexpr int kLoadLanes = kNodeLanes;
 constexpr int kLoadMk = 2;   // markers per block: the three groups of a marker in one block
 constexpr int kLoadThreads = 3 * kLoadMk * kLoadLanes;
@@ -2785,7 +2785,8 @@ void launch_nl_rhs(const Dev &d, double al, double ga, double ro, cudaStream_t s
     // all resident at once; beside the marker set-up of the step (kNlMeans) a
     // sixteenth of the slots is left to its small blocks, which otherwise waited
     // for these persistent ones (none, 20, 37, 74 or 148 slots left: 1568, 1559,
-    // 1562, 1572, 1592 us per step at 2048 x 1536)
+    // 1562, 1572, 1592 us per step at 2048 x 1536; 20 and 37 do not differ by more
+    // than two runs of one of them do)
     const int slots = 148 * kNlBlocksPerSM - more - ((extra & kNlMeans) ? 148 * kNlBlocksPerSM / 16 : 0);
     const int blocks = std::min(nl_tiles(d), slots) + more;
     pdl((extra & kNlCfl) ? k_nl_rhs_tma<true> : k_nl_rhs_tma<false>, dim3(blocks), dim3(32, 8), kNlSmemT, s, d, maps,

@@ -62,8 +62,10 @@ struct ResidualTask {    // one Poisson residual: phi -> hi, lo (ldd), row facto
 // their slices per operand: 7 balanced 8-bit digits (28 digit pairs; the time
 // step) and 8 sign-magnitude 7-bit digits (36 pairs; the public product
 // fb_gemm_i8x8, whose digits and summation order are its documented result).
-constexpr int kI8Step = 7;       // digit slices per operand of the time step
-constexpr int kI8S = 8;    // ... of fb_gemm_i8x8
+// The step's operands hold 55 bits of their row maximum, 54 where its mantissa is
+// above 0.994, the public product's 56: tc_gemm.cu has what that does to the error.
+constexpr int kI8Step = 7;    // digit slices per operand of the time step
+constexpr int kI8S = 8;       // ... of fb_gemm_i8x8
 constexpr int kI8BK = 128;    // K bytes per k-block (one 128-byte swizzle row)
 constexpr int kI8BN = 64;     // widest output tile
 // Largest K of one product: the last weight class sums S digit pairs (7 of at

@@ -670,8 +670,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_zlines(Dev d, SubDev sd, int nb
 // phases (forward and backward recurrences apart, their values exchanged
 // through shared memory) a tile of 32 x 64 made 53 thousand 8-byte accesses and
 // three blocks of 72 KB fitted an SM; the fused segments make 28 thousand
-// (coefficients in pairs) and 51 KB.  20.4 -> 15.9 us at 1024 x 768, 88.7 -> 70.9 at
-// 2048 x 1536 (K = 15), 8.2 -> 5.8 at 384 x 256, 7.0 -> 5.4 at 48 x 32 (32 rows).
+// (coefficients in pairs) and 51 KB.  Repeated behind itself (fb_time_stage):
+// 20.6 -> 16.6 us at 1024 x 768, 88.4 -> 72.9 at 2048 x 1536 (K = 15), 8.7 -> 6.2 at
+// 384 x 256 and 7.8 -> 5.6 at 48 x 32 (the last two with 32 instead of 64 rows too).
 constexpr int kWTj = 32;        // tile columns (j): one lane each in the z phase
 constexpr int kWSeg = 16;       // unknowns per thread segment
 constexpr int kWThreads = 192;  // six warps: the y segments of a 32 x 64 tile with K <= 16

@@ -151,8 +151,12 @@ int fb_rigid(fb_ctx *ctx, int ns, double *forcecomp);
 /* nsteps iterations of the reference main loop body (main.F90:85-97:
  * fluid_tsch, rigid, time += dt) starting at step index ns0, replayed from a
  * captured CUDA graph; hist (nsteps x FB_HIST_COLS, may be NULL) receives the
- * per-step history rows.  Status errors found on the device stop the call and
- * are returned after the step that raised them. */
+ * per-step history rows.  A status error found on the device is returned: at
+ * variable dt behind the step that raised it, which counts as taken (a refused
+ * dt is returned ahead of its step, and the context can go on); at fixed dt
+ * behind the captured steps of the call, at most 4096, which run on.  From the
+ * step that raised it on, the forcing is held back (a CFL number beyond cfllim:
+ * in that step too) and press and tau stay as they were. */
 int fb_advance(fb_ctx *ctx, int ns0, int nsteps, double *hist);
 
 /* Marker-side coupling for a host rigid-body solver (the reference's own
