@@ -1334,21 +1334,33 @@ int capture_step(fb_ctx *c, int steps = 1) {
 // 8 us; inside one the next kernel's launch is hidden.  So longer calls take kRun
 // joints per launch (100 steps on 48 x 32 / 384 x 256 / 731 x 561 / 1024 x 768:
 // 11.8 / 15.6 / 28.8 / 40.3 ms, joint by joint 12.2 / 16.1 / 29.9 / 40.7; at
-// 2048 x 1536 equal).  The graph is made in the first call that is long enough
-// to gain its making back, behind kAhead joints already enqueued, during which
-// the GPU stays busy: that call, with the making, takes 12.6 ms on 48 x 32 and
-// 12.9 without.  Without the memory for it the joints are launched one by one.
-constexpr int kRun = 8, kAhead = 16;
+// 2048 x 1536 equal).
+// The graph of kRun joints is made in the first call of kRunCall or more, behind
+// half of its joints, already enqueued, during which the GPU stays busy: its making
+// takes the host 2 ms, and 10 to 20 ms with a hundred other contexts alive (behind
+// the first 16 joints only, the first 100 steps of 128 contexts of up to 768 x 512
+// cells took 31.0 ms each, 23.2 so, 17.9 from then on; of a single 48 x 32 context
+// 12.2, 12.4 and 12.1).  Without the memory for it the joints are launched one by one.
+constexpr int kRun = 8, kRunCall = 48;
+int make_run(fb_ctx *c) {
+    const int r = capture_exec(c, &c->run_exec, [&] {
+        int e = FB_OK;
+        for (int k = 0; k < kRun && !e; ++k) e = enqueue_next_step(c);
+        return e;
+    });
+    if (r) return r;
+    // on the side stream, which is idle: on the context's it would wait for the joints
+    CK(cudaGraphUpload(c->run_exec, c->side));
+    CK(cudaStreamSynchronize(c->side));
+    return FB_OK;
+}
+
 int launch_joints(fb_ctx *c, int n) {
     int i = 0;
-    if (!c->run_exec && n >= kAhead + 4 * kRun) {
-        for (; i < kAhead; ++i) CK(cudaGraphLaunch(c->next_exec, c->stream));
-        const int r = capture_exec(c, &c->run_exec, [&] {
-            int e = FB_OK;
-            for (int k = 0; k < kRun && !e; ++k) e = enqueue_next_step(c);
-            return e;
-        });
-        if (r) {
+    if (!c->run_exec && n >= kRunCall) {
+        for (; i < n / 2; ++i) CK(cudaGraphLaunch(c->next_exec, c->stream));
+        if (make_run(c)) {
+            if (c->run_exec) cudaGraphExecDestroy(c->run_exec);
             c->run_exec = nullptr;
             cudaGetLastError();
         }
